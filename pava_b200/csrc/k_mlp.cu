@@ -1,12 +1,11 @@
-// The learned form selector's network: an MLP 12 -> 64 -> 64 -> 6 (ReLU, FP32) that predicts
-// the log-time of each of the six engine variants from a matrix's structural features
+// The learned form selector's network: an MLP 12 -> 64 -> 64 -> 32 (ReLU, FP32) that predicts
+// the log-time of each of the 32 engine forms from a matrix's structural features
 // (k_features.cu), trained on the GPU by the kernels below (forward, backward, Adam).
 //
-// Parameters, one flat float array of 5,382 entries:
-//   W1[64][12] @0   b1[64] @768   W2[64][64] @832   b2[64] @4928   W3[6][64] @4992   b3[6] @5376
-// Loss: masked mean squared error over the six outputs (a variant that failed on a matrix
-// has mask 0).  Every reduction runs in a fixed order (one thread owns one sum), so a
-// training run gives the same bits every time.
+// Parameters, one flat float array of 7,072 entries:
+//   W1[64][12] @0   b1[64] @768   W2[64][64] @832   b2[64] @4928   W3[32][64] @4992   b3[32] @7040
+// Loss: masked mean squared error over the outputs (a form that failed on a matrix has mask
+// 0).  Every reduction runs in a fixed order, so a training run gives the same bits every time.
 
 #include <math.h>
 #include <string.h>
@@ -24,125 +23,292 @@ constexpr int OW1 = 0, OB1 = OW1 + HID * IN, OW2 = OB1 + HID, OB2 = OW2 + HID * 
               OW3 = OB2 + HID, OB3 = OW3 + OUT * HID, NP = OB3 + OUT;
 static_assert(NP == PAVA_MLP_NPARAM, "parameter count");
 
-// One block of HID threads per sample.  Stores pre-activations Z1, Z2 and outputs O.
-__global__ void __launch_bounds__(HID)
-forward_kernel(const float *__restrict__ P, const float *__restrict__ X, int B,
-               float *__restrict__ Z1, float *__restrict__ Z2, float *__restrict__ O) {
-    __shared__ float xs[IN], h1[HID], h2[HID];
-    const int b = blockIdx.x, j = threadIdx.x;
-    if (b >= B) return;
-    if (j < IN) xs[j] = X[(long long)b * IN + j];
-    __syncthreads();
-    float z = P[OB1 + j];
-    for (int i = 0; i < IN; ++i) z = fmaf(P[OW1 + j * IN + i], xs[i], z);
-    Z1[(long long)b * HID + j] = z;
-    h1[j] = z > 0.f ? z : 0.f;
-    __syncthreads();
-    z = P[OB2 + j];
-    for (int k = 0; k < HID; ++k) z = fmaf(P[OW2 + j * HID + k], h1[k], z);
-    Z2[(long long)b * HID + j] = z;
-    h2[j] = z > 0.f ? z : 0.f;
-    __syncthreads();
-    if (j < OUT) {
-        float o = P[OB3 + j];
-        for (int k = 0; k < HID; ++k) o = fmaf(P[OW3 + j * HID + k], h2[k], o);
-        O[(long long)b * OUT + j] = o;
-    }
-}
+// The network on tiles of TS samples, one 512-thread CTA per tile (grid-stride), the weights in
+// shared memory for the whole launch.  GRAD = false: outputs O only.  GRAD = true: forward,
+// backward and weight gradients of the CTA's tiles; the gradient sums stay in registers over
+// the tiles (a 4 x 2 tile of W2 and 1 x 4 of W3 per thread, 2 of W1 for 384 threads, a bias
+// each for 160) and go to part[blockIdx.x][NP], the CTA's loss sum to part_loss[blockIdx.x];
+// reduce_kernel adds the CTAs.
+//
+// What bounds it: the latency of eight dependent phases between barriers, each a short chain of
+// shared-memory reads and FMAs; an epoch moves well under 4 MB and 85 MFLOP at 2,000 samples.
+// One CTA per sample read W2 with a stride of 256 bytes between lanes and left the weight
+// gradients to 28 CTAs of 2,000-step serial sums: 183 us a training step at 2,000 samples (forward
+// 51, backward 7, gradient 153, loss 42, Adam 4 us, each alone); this kernel and reduce_kernel
+// take 17 us a step, 12.5 us at 500 samples.
+// 16 samples per tile put 2,000 samples on 125 CTAs, one per SM (32 per tile would leave half
+// of the SMs idle there), and 16 warps hide more of each phase than 8 (22 us a step).  Each thread
+// has all of its weight loads in flight at once.
+//
+// Both kernels are launched as programmatic dependents of the one before: their launch and, here,
+// the read of the inputs overlap its end.
+//
+// Rows of W2 and W3 are padded to 68 floats: a warp's 16-byte reads down the rows (forward) and
+// its 4-byte reads along them (backward) are both free of bank conflicts.
+constexpr int TS = 16, NT = 512, LDW = HID + 4;
+constexpr int SH = TS * HID / NT, SO = TS * OUT / NT;  // samples per thread: hidden, output
+static_assert(SH == 2 && SO == 1 && NP % 4 == 0, "thread mapping");
+struct MlpSmem {
+    float w1[HID * IN], b1[HID], w2[HID * LDW], b2[HID], w3[OUT * LDW], b3[OUT];
+    float x[TS * IN], h1[TS * HID], h2[TS * HID], go[TS * OUT], g1[TS * HID], g2[TS * HID];
+    float red[NT / 32];
+};
+static_assert(sizeof(MlpSmem) <= 48 * 1024, "default shared memory limit");
 
-// Per-sample backward: dO = 2 mask (O - T) / count, then dZ2 and dZ1 through the ReLUs.
-__global__ void __launch_bounds__(HID)
-backward_kernel(const float *__restrict__ P, int B, const float *__restrict__ Z1,
-                const float *__restrict__ Z2, const float *__restrict__ O,
-                const float *__restrict__ T, const float *__restrict__ Mk, float inv_count,
-                float *__restrict__ dO, float *__restrict__ dZ1, float *__restrict__ dZ2) {
-    __shared__ float go[OUT], g2[HID];
-    const int b = blockIdx.x, j = threadIdx.x;
-    if (b >= B) return;
-    if (j < OUT) {
-        const long long q = (long long)b * OUT + j;
-        const float g = 2.f * Mk[q] * (O[q] - T[q]) * inv_count;
-        go[j] = g;
-        dO[q] = g;
-    }
-    __syncthreads();
-    float s = 0.f;
-    for (int t = 0; t < OUT; ++t) s = fmaf(go[t], P[OW3 + t * HID + j], s);
-    const float d2 = Z2[(long long)b * HID + j] > 0.f ? s : 0.f;
-    g2[j] = d2;
-    dZ2[(long long)b * HID + j] = d2;
-    __syncthreads();
-    s = 0.f;
-    for (int k = 0; k < HID; ++k) s = fmaf(g2[k], P[OW2 + k * HID + j], s);
-    dZ1[(long long)b * HID + j] = Z1[(long long)b * HID + j] > 0.f ? s : 0.f;
-}
-
-// One thread per parameter: its gradient summed over the batch in sample order.
-__global__ void grad_kernel(const float *__restrict__ X, int B, const float *__restrict__ Z1,
-                            const float *__restrict__ Z2, const float *__restrict__ dO,
-                            const float *__restrict__ dZ1, const float *__restrict__ dZ2,
-                            float *__restrict__ G) {
-    const int p = blockIdx.x * blockDim.x + threadIdx.x;
-    if (p >= NP) return;
-    float s = 0.f;
-    if (p < OB1) {
-        const int j = (p - OW1) / IN, i = (p - OW1) % IN;
-        for (int b = 0; b < B; ++b) s = fmaf(dZ1[(long long)b * HID + j], X[(long long)b * IN + i], s);
-    } else if (p < OW2) {
-        const int j = p - OB1;
-        for (int b = 0; b < B; ++b) s += dZ1[(long long)b * HID + j];
-    } else if (p < OB2) {
-        const int j = (p - OW2) / HID, k = (p - OW2) % HID;
-        for (int b = 0; b < B; ++b) {
-            const float h = Z1[(long long)b * HID + k];
-            s = fmaf(dZ2[(long long)b * HID + j], h > 0.f ? h : 0.f, s);
+template <bool GRAD>
+__global__ void __launch_bounds__(NT)
+mlp_kernel(const float *P, const float *__restrict__ X, int B,
+           const float *__restrict__ T, const float *__restrict__ Mk, float inv_count,
+           float *O, float *part, float *part_loss) {
+    __shared__ __align__(16) MlpSmem S;
+    const int t = threadIdx.x;
+    const int tiles = (B + TS - 1) / TS;
+    auto load_x = [&](int tile) {
+        const int b0 = tile * TS, nb = min(TS, B - b0);
+        for (int q = t; q < TS * IN; q += NT) S.x[q] = q < nb * IN ? X[(long long)b0 * IN + q] : 0.f;
+    };
+    asm volatile("griddepcontrol.launch_dependents;");
+    load_x(blockIdx.x);  // the grid has at most one CTA per tile
+    // the step before has to be done: it wrote the weights, and read part
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    {
+        constexpr int NV = (NP / 4 + NT - 1) / NT;
+        float4 v[NV];
+#pragma unroll
+        for (int i = 0; i < NV; ++i) {
+            const int q = i * NT + t;
+            if (q < NP / 4) v[i] = reinterpret_cast<const float4 *>(P)[q];
         }
-    } else if (p < OW3) {
-        const int j = p - OB2;
-        for (int b = 0; b < B; ++b) s += dZ2[(long long)b * HID + j];
-    } else if (p < OB3) {
-        const int t = (p - OW3) / HID, k = (p - OW3) % HID;
-        for (int b = 0; b < B; ++b) {
-            const float h = Z2[(long long)b * HID + k];
-            s = fmaf(dO[(long long)b * OUT + t], h > 0.f ? h : 0.f, s);
+#pragma unroll
+        for (int i = 0; i < NV; ++i) {
+            const int q = 4 * (i * NT + t);  // the four entries lie in one row of one matrix
+            if (q >= NP) continue;
+            float *d = q < OB1   ? S.w1 + q
+                       : q < OW2 ? S.b1 + (q - OB1)
+                       : q < OB2 ? S.w2 + (q - OW2) / HID * LDW + (q - OW2) % HID
+                       : q < OW3 ? S.b2 + (q - OB2)
+                       : q < OB3 ? S.w3 + (q - OW3) / HID * LDW + (q - OW3) % HID
+                                 : S.b3 + (q - OB3);
+            *reinterpret_cast<float4 *>(d) = v[i];
         }
-    } else {
-        const int t = p - OB3;
-        for (int b = 0; b < B; ++b) s += dO[(long long)b * OUT + t];
     }
-    G[p] = s;
-}
 
-// Masked mean squared error, one block: strided partial sums, then a fixed tree.
-__global__ void __launch_bounds__(256)
-loss_kernel(const float *__restrict__ O, const float *__restrict__ T,
-            const float *__restrict__ Mk, long long n, float inv_count, float *__restrict__ out) {
-    __shared__ float part[256];
-    float s = 0.f;
-    for (long long q = threadIdx.x; q < n; q += 256) {
-        const float d = O[q] - T[q];
-        s = fmaf(Mk[q] * d, d, s);
-    }
-    part[threadIdx.x] = s;
-    __syncthreads();
-    for (int w = 128; w > 0; w >>= 1) {
-        if (threadIdx.x < w) part[threadIdx.x] += part[threadIdx.x + w];
+    const int j = t & (HID - 1), s0 = (t / HID) * SH;  // hidden unit and SH samples
+    const int o = t & (OUT - 1), s1 = (t / OUT) * SO;  // output and SO samples
+    const int tj = (t >> 5) * 4, tk = (t & 31) * 2;    // W2 tile: rows tj.., columns tk, tk + 1
+    const int to = t >> 4, tq = (t & 15) * 4;          // W3 tile: row to, columns tq..
+    const int ti = (t >> 6) * 2;                       // W1: unit j, inputs ti, ti + 1 (t < 384)
+    float a2[4][2] = {}, a3[4] = {}, a1[2] = {}, ab = 0.f, loss = 0.f;
+
+    for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
+        const int b0 = tile * TS, nb = min(TS, B - b0);
+        if (tile != blockIdx.x) {
+            __syncthreads();  // the previous tile's arrays are done with
+            load_x(tile);
+        }
         __syncthreads();
+        // layer 1 (samples past the batch: zero activations, so they add nothing below)
+        float z[SH];
+#pragma unroll
+        for (int u = 0; u < SH; ++u) z[u] = S.b1[j];
+#pragma unroll
+        for (int i = 0; i < IN; ++i) {
+            const float w = S.w1[j * IN + i];
+#pragma unroll
+            for (int u = 0; u < SH; ++u) z[u] = fmaf(w, S.x[(s0 + u) * IN + i], z[u]);
+        }
+#pragma unroll
+        for (int u = 0; u < SH; ++u) S.h1[(s0 + u) * HID + j] = s0 + u < nb && z[u] > 0.f ? z[u] : 0.f;
+        __syncthreads();
+        // layer 2
+#pragma unroll
+        for (int u = 0; u < SH; ++u) z[u] = S.b2[j];
+#pragma unroll 8
+        for (int k = 0; k < HID; k += 4) {
+            const float4 w = *reinterpret_cast<const float4 *>(&S.w2[j * LDW + k]);
+#pragma unroll
+            for (int u = 0; u < SH; ++u) {
+                const float4 h = *reinterpret_cast<const float4 *>(&S.h1[(s0 + u) * HID + k]);
+                z[u] = fmaf(w.x, h.x, z[u]);
+                z[u] = fmaf(w.y, h.y, z[u]);
+                z[u] = fmaf(w.z, h.z, z[u]);
+                z[u] = fmaf(w.w, h.w, z[u]);
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < SH; ++u) S.h2[(s0 + u) * HID + j] = s0 + u < nb && z[u] > 0.f ? z[u] : 0.f;
+        __syncthreads();
+        // output layer, its loss and gradient
+        float y[SO];
+#pragma unroll
+        for (int u = 0; u < SO; ++u) y[u] = S.b3[o];
+#pragma unroll 8
+        for (int k = 0; k < HID; k += 4) {
+            const float4 w = *reinterpret_cast<const float4 *>(&S.w3[o * LDW + k]);
+#pragma unroll
+            for (int u = 0; u < SO; ++u) {
+                const float4 h = *reinterpret_cast<const float4 *>(&S.h2[(s1 + u) * HID + k]);
+                y[u] = fmaf(w.x, h.x, y[u]);
+                y[u] = fmaf(w.y, h.y, y[u]);
+                y[u] = fmaf(w.z, h.z, y[u]);
+                y[u] = fmaf(w.w, h.w, y[u]);
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < SO; ++u) {
+            const bool in = s1 + u < nb;
+            const long long q = (long long)(b0 + s1 + u) * OUT + o;
+            if (!GRAD) {
+                if (in) O[q] = y[u];
+            } else {
+                const float d = in ? y[u] - T[q] : 0.f, mk = in ? Mk[q] : 0.f;
+                loss = fmaf(mk * d, d, loss);
+                S.go[(s1 + u) * OUT + o] = in ? 2.f * mk * d * inv_count : 0.f;
+            }
+        }
+        if (!GRAD) continue;
+        __syncthreads();
+        // dZ2 = (dO W3) through the ReLU
+#pragma unroll
+        for (int u = 0; u < SH; ++u) z[u] = 0.f;
+#pragma unroll
+        for (int k = 0; k < OUT; k += 4) {
+            float w[4];
+#pragma unroll
+            for (int e = 0; e < 4; ++e) w[e] = S.w3[(k + e) * LDW + j];
+#pragma unroll
+            for (int u = 0; u < SH; ++u) {
+                const float4 g = *reinterpret_cast<const float4 *>(&S.go[(s0 + u) * OUT + k]);
+                z[u] = fmaf(g.x, w[0], z[u]);
+                z[u] = fmaf(g.y, w[1], z[u]);
+                z[u] = fmaf(g.z, w[2], z[u]);
+                z[u] = fmaf(g.w, w[3], z[u]);
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < SH; ++u)
+            S.g2[(s0 + u) * HID + j] = S.h2[(s0 + u) * HID + j] > 0.f ? z[u] : 0.f;
+        __syncthreads();
+        // dZ1 = (dZ2 W2) through the ReLU
+#pragma unroll
+        for (int u = 0; u < SH; ++u) z[u] = 0.f;
+#pragma unroll 8
+        for (int k = 0; k < HID; k += 4) {
+            float w[4];
+#pragma unroll
+            for (int e = 0; e < 4; ++e) w[e] = S.w2[(k + e) * LDW + j];
+#pragma unroll
+            for (int u = 0; u < SH; ++u) {
+                const float4 g = *reinterpret_cast<const float4 *>(&S.g2[(s0 + u) * HID + k]);
+                z[u] = fmaf(g.x, w[0], z[u]);
+                z[u] = fmaf(g.y, w[1], z[u]);
+                z[u] = fmaf(g.z, w[2], z[u]);
+                z[u] = fmaf(g.w, w[3], z[u]);
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < SH; ++u)
+            S.g1[(s0 + u) * HID + j] = S.h1[(s0 + u) * HID + j] > 0.f ? z[u] : 0.f;
+        __syncthreads();
+        // weight gradients, summed over the samples in order
+#pragma unroll 8
+        for (int s = 0; s < TS; ++s) {
+            const float4 g = *reinterpret_cast<const float4 *>(&S.g2[s * HID + tj]);
+            const float2 h = *reinterpret_cast<const float2 *>(&S.h1[s * HID + tk]);
+            const float4 h2 = *reinterpret_cast<const float4 *>(&S.h2[s * HID + tq]);
+            const float go = S.go[s * OUT + to];
+            const float gv[4] = {g.x, g.y, g.z, g.w};
+#pragma unroll
+            for (int r = 0; r < 4; ++r) {
+                a2[r][0] = fmaf(gv[r], h.x, a2[r][0]);
+                a2[r][1] = fmaf(gv[r], h.y, a2[r][1]);
+            }
+            a3[0] = fmaf(go, h2.x, a3[0]);
+            a3[1] = fmaf(go, h2.y, a3[1]);
+            a3[2] = fmaf(go, h2.z, a3[2]);
+            a3[3] = fmaf(go, h2.w, a3[3]);
+            if (t < 6 * HID) {
+                const float g1 = S.g1[s * HID + j];
+                a1[0] = fmaf(g1, S.x[s * IN + ti], a1[0]);
+                a1[1] = fmaf(g1, S.x[s * IN + ti + 1], a1[1]);
+                if (t < HID) ab += g1;
+                else if (t < 2 * HID) ab += S.g2[s * HID + j];
+                else if (t < 2 * HID + OUT) ab += S.go[s * OUT + o];
+            }
+        }
     }
-    if (threadIdx.x == 0) *out = part[0] * inv_count;
+    if (!GRAD) return;
+    float *G = part + (long long)blockIdx.x * NP;
+#pragma unroll
+    for (int r = 0; r < 4; ++r)
+        *reinterpret_cast<float2 *>(&G[OW2 + (tj + r) * HID + tk]) = make_float2(a2[r][0], a2[r][1]);
+    *reinterpret_cast<float4 *>(&G[OW3 + to * HID + tq]) = make_float4(a3[0], a3[1], a3[2], a3[3]);
+    if (t < 6 * HID)
+        *reinterpret_cast<float2 *>(&G[OW1 + j * IN + ti]) = make_float2(a1[0], a1[1]);
+    if (t < HID) G[OB1 + t] = ab;
+    else if (t < 2 * HID) G[OB2 + j] = ab;
+    else if (t < 2 * HID + OUT) G[OB3 + o] = ab;
+    // the CTA's loss: fixed butterfly per warp, then the warps in order
+#pragma unroll
+    for (int d = 16; d > 0; d >>= 1) loss += __shfl_xor_sync(FULL, loss, d);
+    if ((t & 31) == 0) S.red[t >> 5] = loss;
+    __syncthreads();
+    if (t == 0) {
+        float l = 0.f;
+        for (int w = 0; w < NT / 32; ++w) l += S.red[w];
+        part_loss[blockIdx.x] = l;
+    }
 }
 
-__global__ void adam_kernel(float *__restrict__ P, const float *__restrict__ G,
-                            float *__restrict__ Mm, float *__restrict__ Vv, float lr, float b1,
-                            float b2, float eps, float c1, float c2) {
-    const int p = blockIdx.x * blockDim.x + threadIdx.x;
-    if (p >= NP) return;
-    const float g = G[p];
-    const float m = b1 * Mm[p] + (1.f - b1) * g;
-    const float v = b2 * Vv[p] + (1.f - b2) * g * g;
-    Mm[p] = m;
-    Vv[p] = v;
-    P[p] -= lr * (m * c1) / (sqrtf(v * c2) + eps);
+// Sums the CTAs' gradients in a fixed order (warp w of RW takes the parts w, w + RW, ..., then the
+// RW sums in order), 32 parameters per block, and either stores them (G) or applies an Adam
+// step at once.  Block 0 also sums the loss.  Bound by latency: one round of L2 reads (3.5 MB at
+// 125 parts, eight in flight per thread), the sum of the warps, the Adam step.
+constexpr int RW = 16;
+struct AdamStep {
+    float *P, *Mm, *Vv;  // P = nullptr: store the gradient in G instead
+    float lr, b1, b2, eps, c1, c2;
+};
+__global__ void __launch_bounds__(RW * 32)
+reduce_kernel(const float *part, const float *part_loss, int parts,
+              float inv_count, float *G, float *loss, AdamStep st) {
+    __shared__ float red[RW][32];
+    asm volatile("griddepcontrol.launch_dependents;");
+    asm volatile("griddepcontrol.wait;" ::: "memory");  // mlp_kernel's parts
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int p = blockIdx.x * 32 + lane;
+    static_assert(NP % 32 == 0 && NP % 4 == 0 && OW2 % 4 == 0 && OW3 % 4 == 0, "32 per block");
+    float m0 = 0.f, v0 = 0.f, p0 = 0.f;
+    if (w == 0 && st.P) {  // in flight beside the parts
+        m0 = st.Mm[p];
+        v0 = st.Vv[p];
+        p0 = st.P[p];
+    }
+    float s = 0.f;
+#pragma unroll 8
+    for (int c = w; c < parts; c += RW) s += part[(long long)c * NP + p];
+    red[w][lane] = s;
+    __syncthreads();
+    if (w == 0) {
+        float g = red[0][lane];
+#pragma unroll
+        for (int q = 1; q < RW; ++q) g += red[q][lane];
+        if (!st.P) {
+            G[p] = g;
+        } else {
+            const float m = st.b1 * m0 + (1.f - st.b1) * g;
+            const float v = st.b2 * v0 + (1.f - st.b2) * g * g;
+            st.Mm[p] = m;
+            st.Vv[p] = v;
+            st.P[p] = p0 - st.lr * (m * st.c1) / (sqrtf(v * st.c2) + st.eps);
+        }
+    } else if (w == 1 && blockIdx.x == 0) {
+        float l = 0.f;
+        for (int c = lane; c < parts; c += 32) l += part_loss[c];
+#pragma unroll
+        for (int d = 16; d > 0; d >>= 1) l += __shfl_xor_sync(FULL, l, d);
+        if (lane == 0) *loss = l * inv_count;
+    }
 }
 
 // (x - mean) / std per feature.
@@ -169,9 +335,12 @@ struct pava_mlp {
     float *P = nullptr, *G = nullptr, *Mm = nullptr, *Vv = nullptr;  // params, grad, Adam
     float *mu = nullptr, *sd = nullptr;                              // feature normalisation
     int B = 0, cap = 0;
-    float *X = nullptr, *T = nullptr, *Mk = nullptr;                 // current batch
-    float *Z1 = nullptr, *Z2 = nullptr, *O = nullptr, *dO = nullptr, *dZ1 = nullptr,
-          *dZ2 = nullptr, *loss = nullptr;
+    float *X = nullptr, *T = nullptr, *Mk = nullptr, *O = nullptr;   // current batch
+    float *part = nullptr, *part_loss = nullptr;                     // per-CTA gradients, losses
+    float *loss = nullptr;
+    float *hist = nullptr;                                           // losses of a training run
+    int hist_cap = 0;
+    int max_ctas = 1;                                                // two per SM
     float inv_count = 0.f;
     int step = 0;
 };
@@ -186,24 +355,42 @@ pava_status mfail(cudaError_t e, const char *where) {
 }
 
 void free_batch(pava_mlp *m) {
-    float **bufs[] = {&m->X, &m->T, &m->Mk, &m->Z1, &m->Z2, &m->O, &m->dO, &m->dZ1, &m->dZ2};
+    float **bufs[] = {&m->X, &m->T, &m->Mk, &m->O, &m->part, &m->part_loss};
     for (float **b : bufs) { cudaFree(*b); *b = nullptr; }
     m->cap = 0;
 }
 
+int mlp_ctas(const pava_mlp *m, int B) {
+    const int tiles = (B + TS - 1) / TS;
+    return tiles < m->max_ctas ? tiles : m->max_ctas;
+}
+
 cudaError_t run_forward(pava_mlp *m) {
-    forward_kernel<<<m->B, HID>>>(m->P, m->X, m->B, m->Z1, m->Z2, m->O);
+    mlp_kernel<false><<<mlp_ctas(m, m->B), NT>>>(m->P, m->X, m->B, nullptr, nullptr, 0.f, m->O,
+                                                 nullptr, nullptr);
     return cudaGetLastError();
 }
 
-cudaError_t run_gradient(pava_mlp *m) {
-    cudaError_t e = run_forward(m);
+// The gradient of the current batch: into m->G (st.P null), or straight into an Adam step.
+cudaError_t run_gradient(pava_mlp *m, float *loss, const AdamStep &st) {
+    const int ctas = mlp_ctas(m, m->B);
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)ctas);
+    cfg.blockDim = dim3(NT);
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    cudaError_t e = cudaLaunchKernelEx(
+        &cfg, mlp_kernel<true>, (const float *)m->P, (const float *)m->X, m->B,
+        (const float *)m->T, (const float *)m->Mk, m->inv_count, (float *)nullptr, m->part,
+        m->part_loss);
     if (e != cudaSuccess) return e;
-    backward_kernel<<<m->B, HID>>>(m->P, m->B, m->Z1, m->Z2, m->O, m->T, m->Mk, m->inv_count,
-                                   m->dO, m->dZ1, m->dZ2);
-    grad_kernel<<<(NP + 255) / 256, 256>>>(m->X, m->B, m->Z1, m->Z2, m->dO, m->dZ1, m->dZ2, m->G);
-    loss_kernel<<<1, 256>>>(m->O, m->T, m->Mk, (long long)m->B * OUT, m->inv_count, m->loss);
-    return cudaGetLastError();
+    cfg.gridDim = dim3(NP / 32);
+    cfg.blockDim = dim3(RW * 32);
+    return cudaLaunchKernelEx(&cfg, reduce_kernel, (const float *)m->part,
+                              (const float *)m->part_loss, ctas, m->inv_count, m->G, loss, st);
 }
 
 }  // namespace
@@ -215,7 +402,11 @@ pava_status pava_mlp_create(uint64_t seed, pava_mlp **out) {
     *out = nullptr;
     pava_mlp *m = new (std::nothrow) pava_mlp();
     if (!m) return PAVA_E_NOMEM;
-    cudaError_t e = cudaMalloc(&m->P, sizeof(float) * NP);
+    int dev = 0, sms = 1;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    m->max_ctas = 2 * sms;
+    if (e == cudaSuccess) e = cudaMalloc(&m->P, sizeof(float) * NP);
     if (e == cudaSuccess) e = cudaMalloc(&m->G, sizeof(float) * NP);
     if (e == cudaSuccess) e = cudaMalloc(&m->Mm, sizeof(float) * NP);
     if (e == cudaSuccess) e = cudaMalloc(&m->Vv, sizeof(float) * NP);
@@ -283,15 +474,13 @@ pava_status pava_mlp_set_batch(pava_mlp *m, int B, const float *X, const float *
     if (B > m->cap) {
         free_batch(m);
         const size_t b = (size_t)B;
+        const size_t ctas = (size_t)mlp_ctas(m, B);
         e = cudaMalloc(&m->X, sizeof(float) * b * IN);
         if (e == cudaSuccess) e = cudaMalloc(&m->T, sizeof(float) * b * OUT);
         if (e == cudaSuccess) e = cudaMalloc(&m->Mk, sizeof(float) * b * OUT);
-        if (e == cudaSuccess) e = cudaMalloc(&m->Z1, sizeof(float) * b * HID);
-        if (e == cudaSuccess) e = cudaMalloc(&m->Z2, sizeof(float) * b * HID);
         if (e == cudaSuccess) e = cudaMalloc(&m->O, sizeof(float) * b * OUT);
-        if (e == cudaSuccess) e = cudaMalloc(&m->dO, sizeof(float) * b * OUT);
-        if (e == cudaSuccess) e = cudaMalloc(&m->dZ1, sizeof(float) * b * HID);
-        if (e == cudaSuccess) e = cudaMalloc(&m->dZ2, sizeof(float) * b * HID);
+        if (e == cudaSuccess) e = cudaMalloc(&m->part, sizeof(float) * ctas * NP);
+        if (e == cudaSuccess) e = cudaMalloc(&m->part_loss, sizeof(float) * ctas);
         if (e != cudaSuccess) { free_batch(m); return mfail(e, "mlp batch"); }
         m->cap = B;
     }
@@ -326,7 +515,7 @@ pava_status pava_mlp_forward(pava_mlp *m, float *Y) {
 
 pava_status pava_mlp_gradient(pava_mlp *m, float *grad, float *loss) {
     if (!m || m->B < 1) { set_last_error("no batch set"); return PAVA_E_INVALID_ARG; }
-    cudaError_t e = run_gradient(m);
+    cudaError_t e = run_gradient(m, m->loss, AdamStep{});
     if (e == cudaSuccess && grad) e = cudaMemcpy(grad, m->G, sizeof(float) * NP, cudaMemcpyDeviceToHost);
     if (e == cudaSuccess && loss) e = cudaMemcpy(loss, m->loss, sizeof(float), cudaMemcpyDeviceToHost);
     return e == cudaSuccess ? PAVA_SUCCESS : mfail(e, "mlp gradient");
@@ -335,20 +524,24 @@ pava_status pava_mlp_gradient(pava_mlp *m, float *grad, float *loss) {
 pava_status pava_mlp_train(pava_mlp *m, int epochs, float lr, float *loss_hist) {
     if (!m || m->B < 1 || epochs < 0) { set_last_error("no batch set"); return PAVA_E_INVALID_ARG; }
     const float b1 = 0.9f, b2 = 0.999f, eps = 1e-8f;
-    std::vector<float> hist((size_t)epochs, 0.f);
     cudaError_t e = cudaSuccess;
+    if (epochs > m->hist_cap) {  // one loss per step, copied back once at the end
+        cudaFree(m->hist);
+        m->hist = nullptr;
+        m->hist_cap = 0;
+        e = cudaMalloc(&m->hist, sizeof(float) * (size_t)epochs);
+        if (e != cudaSuccess) return mfail(e, "mlp train");
+        m->hist_cap = epochs;
+    }
     for (int ep = 0; ep < epochs && e == cudaSuccess; ++ep) {
-        e = run_gradient(m);
         ++m->step;
         const float c1 = 1.f / (1.f - powf(b1, (float)m->step));
         const float c2 = 1.f / (1.f - powf(b2, (float)m->step));
-        adam_kernel<<<(NP + 255) / 256, 256>>>(m->P, m->G, m->Mm, m->Vv, lr, b1, b2, eps, c1, c2);
-        if (e == cudaSuccess) e = cudaGetLastError();
-        if (e == cudaSuccess && loss_hist)
-            e = cudaMemcpyAsync(&hist[ep], m->loss, sizeof(float), cudaMemcpyDeviceToHost, nullptr);
+        e = run_gradient(m, m->hist + ep, AdamStep{m->P, m->Mm, m->Vv, lr, b1, b2, eps, c1, c2});
     }
     if (e == cudaSuccess) e = cudaDeviceSynchronize();
-    if (e == cudaSuccess && loss_hist) memcpy(loss_hist, hist.data(), sizeof(float) * hist.size());
+    if (e == cudaSuccess && loss_hist && epochs > 0)
+        e = cudaMemcpy(loss_hist, m->hist, sizeof(float) * (size_t)epochs, cudaMemcpyDeviceToHost);
     return e == cudaSuccess ? PAVA_SUCCESS : mfail(e, "mlp train");
 }
 
@@ -356,7 +549,7 @@ pava_status pava_mlp_destroy(pava_mlp *m) {
     if (!m) return PAVA_SUCCESS;
     free_batch(m);
     cudaFree(m->P); cudaFree(m->G); cudaFree(m->Mm); cudaFree(m->Vv);
-    cudaFree(m->mu); cudaFree(m->sd); cudaFree(m->loss);
+    cudaFree(m->mu); cudaFree(m->sd); cudaFree(m->loss); cudaFree(m->hist);
     delete m;
     return PAVA_SUCCESS;
 }
