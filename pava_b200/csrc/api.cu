@@ -123,13 +123,19 @@ void free_handle_buffers(pava::Handle &h) {
     h.rp = nullptr; h.ci = nullptr; h.v = nullptr;
 }
 
+// Lanes per row of the plain CSR SpMV by the mean row length: the fastest of the measured widths.
+// Narrow groups cost rounds on long rows, wide ones idle lanes and shuffles on short rows (FP64,
+// us at 2 / 4 / 8 / 16 / 32 lanes): mean 5 (Laplacian) 53 / 72 / 122; mean 12 49 / 45 / 47 / 72;
+// power law, mean 16, 112 / 106 / 96 / 107; mean 24 (banded) 133 / 82 / 80 / 119 / 223; mean 27
+// (stencil) 342 / 190 / 158 / 240 / 426; mean 64 100 / 113 / 76 / 79 / 88; mean 100 100 / 76 /
+// 80 / 72 / 76; mean 300 221 / 121 / 72 / 82 / 65.
 int auto_lanes_per_row(int m, int nnz) {
     const double mean = m > 0 ? (double)nnz / m : 0.0;
     if (mean <= 2) return 1;
-    if (mean <= 4) return 2;
-    if (mean <= 8) return 4;
-    if (mean <= 16) return 8;
-    if (mean <= 32) return 16;
+    if (mean <= 6) return 2;
+    if (mean <= 12.5) return 4;
+    if (mean <= 80) return 8;
+    if (mean <= 160) return 16;
     return 32;
 }
 

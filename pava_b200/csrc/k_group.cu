@@ -4,8 +4,8 @@
 // A group of GL lanes (a power of two <= 32) owns one row at a time.  Inside the group, KC
 // lanes span the k right-hand sides (lane c holds columns c, c + KC, ..., KPL of them) and
 // ES = GL / KC element slices split the row's nonzeros (slice e takes elements e, e + ES, ...).
-// For k = 1 this is the vector-CSR kernel with GL lanes per row; for k = 32, GL = KC = 32 it is
-// one warp per row reading 256-byte rows of X.  A slice's partial sums are combined over the
+// For k = 32, GL = KC = 32 it is one warp per row reading 256-byte rows of X.  One right-hand
+// side has a kernel of its own (csr_spmv_kernel).  A slice's partial sums are combined over the
 // ES slices with a fixed xor butterfly, so every call gives the same bits.
 //
 // The launch is persistent: the grid is sized to the resident capacity of the GPU and warps
@@ -366,6 +366,141 @@ csr_window_kernel(const int *__restrict__ rp, const int *__restrict__ ci,
     }
 }
 
+// SpMV on plain CSR (one right-hand side): groups of GL lanes own a row at a time, lane gi taking
+// elements gi, gi + GL, ...; a fixed butterfly adds the lanes.  Rows of very uneven length are kept
+// off the critical path:
+//
+//  * a row longer than LONG = 4 U GL is summed by the whole warp, WU elements per lane at a time:
+//    in its group it would run len / (U GL) dependent rounds while the other groups wait;
+//  * a row longer than HUGE_ROW waits until the CTA's tiles are done and is summed by all of its
+//    warps.  Each warp keeps up to LIST such rows (and sums further ones alone), so which rows
+//    take which way depends on the matrix and the launch shape only, and results repeat bit
+//    for bit.  Nothing is kept in global memory: calls on one handle may overlap.
+//
+// What bounds it: on power-law rows the chain row pointer -> values and columns -> x of each round
+// and the gathers (one L1 wavefront each on random columns); on regular rows instruction issue.
+// Compile-time GL and 32-bit offsets keep a round short enough for six CTAs per SM.  FP64, L2
+// flushed, against one group per row whatever its length: power-law rows (700,001, mean 16,
+// longest about 7,000) 457 -> 96 us, 4,194,304 rows 806 -> 400 us; 27-point stencil 128^3 190 ->
+// 158 us, dense blocks 158 -> 132 us (8 lanes each).  Reading the row pointers of 32 rows at once,
+// and keeping the next round's loads in flight at four CTAs per SM, were slower (96-107 us and
+// 125 us on the 700,001 rows; 172 and 221 us on the stencil), as were HUGE_ROW = 2,048 (39
+// against 33 us on 100,003 power-law rows) and seven or eight CTAs (spills).
+constexpr int HUGE_ROW = 1024, LIST = 8;
+constexpr int SPMV_MINB = 6;
+
+template <int GL, typename VT>
+__global__ void __launch_bounds__(GROUP_THREADS, SPMV_MINB)
+csr_spmv_kernel(const int *__restrict__ rp, const int *__restrict__ ci, const VT *__restrict__ v,
+                const VT *__restrict__ x, long long ldx, double *__restrict__ y, long long ldy,
+                int m, int tile_rows, int n, unsigned long long *err) {
+    constexpr int U = 4, WU = 4, GPW = 32 / GL, WARPS = GROUP_THREADS / 32;
+    constexpr int LONG = GL < 32 ? 4 * U * GL : HUGE_ROW;
+    __shared__ int s_list[WARPS][LIST], s_cnt[WARPS];
+    __shared__ double s_sum[WARPS];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int grp = lane / GL, gi = lane % GL;
+    const uint64_t pf = policy_evict_first(), pl = policy_evict_last();
+    const long long ntiles = ((long long)m + tile_rows - 1) / tile_rows;
+    const long long nwarps = ((long long)gridDim.x * blockDim.x) >> 5;
+    const int rounds = tile_rows / GPW;
+
+    auto gather = [&](int col) -> VT {
+        if (!guard(err, col >= 0 && col < n, G_X, col)) return VT(0);
+        return ld_x(x + (long long)col * ldx, pl);
+    };
+    // elements [j0, j1) of a row, this thread taking j0 + first, then every `step`-th
+    auto strided = [&](int j0, int j1, unsigned first, unsigned step) -> double {
+        Acc<VT> acc;
+        const VT *vr = v + j0;
+        const int *cr = ci + j0;
+        const unsigned len = (unsigned)(j1 - j0);  // unsigned offsets: no overflow near 2^31
+        for (unsigned j = first; j < len; j += WU * step) {
+            VT val[WU], xv[WU];
+            int col[WU];
+#pragma unroll
+            for (int u = 0; u < WU; ++u) {
+                const bool in = j + u * step < len;
+                val[u] = in ? ld_val(vr + j + u * step, pf) : VT(0);
+                col[u] = in ? ld_col(cr + j + u * step, pf) : -1;
+            }
+#pragma unroll
+            for (int u = 0; u < WU; ++u) xv[u] = col[u] >= 0 ? gather(col[u]) : VT(0);
+#pragma unroll
+            for (int u = 0; u < WU; ++u)
+                if (col[u] >= 0) acc.add(val[u], xv[u]);
+        }
+        return acc.value();
+    };
+
+    int cnt = 0;
+    for (unsigned t = (blockIdx.x * GROUP_THREADS + threadIdx.x) >> 5; t < (unsigned)ntiles;
+         t += (unsigned)nwarps) {
+        // row of the tile's first round (< m + tile_rows <= 2^31 + 2^20: unsigned)
+        unsigned r = t * (unsigned)tile_rows + grp;
+        for (int i = 0; i < rounds; ++i, r += GPW) {
+            int a = 0, b = 0;
+            if (r < (unsigned)m) {
+                a = rp[r];
+                b = rp[r + 1];
+            }
+            const int len = b - a;
+            const bool is_long = len > LONG;
+            const VT *vr = v + a;
+            const int *cr = ci + a;
+            Acc<VT> acc;
+            for (int j = gi; j < (is_long ? 0 : len); j += U * GL) {
+                VT val[U];
+                int col[U];
+#pragma unroll
+                for (int u = 0; u < U; ++u) {
+                    const bool in = j + u * GL < len;
+                    val[u] = in ? ld_val(vr + (j + u * GL), pf) : VT(0);
+                    col[u] = in ? ld_col(cr + (j + u * GL), pf) : -1;
+                }
+#pragma unroll
+                for (int u = 0; u < U; ++u)
+                    if (col[u] >= 0) acc.add(val[u], gather(col[u]));
+            }
+            double s = acc.value();
+#pragma unroll
+            for (int o = 1; o < GL; o <<= 1) s += __shfl_xor_sync(FULL, s, o);
+            if (r < (unsigned)m && gi == 0 && !is_long) y[r * ldy] = s;
+            // long rows, one after the other, by the whole warp
+            unsigned todo = __ballot_sync(FULL, is_long && gi == 0);
+            while (todo) {
+                const int src = __ffs(todo) - 1;
+                todo &= todo - 1;
+                const int al = __shfl_sync(FULL, a, src), bl = __shfl_sync(FULL, b, src);
+                const int rl = __shfl_sync(FULL, (int)r, src);
+                if (bl - al > HUGE_ROW && cnt < LIST) {
+                    if (lane == 0) s_list[w][cnt] = rl;
+                    ++cnt;
+                    continue;
+                }
+                const double sl = warp_sum(strided(al, bl, lane, 32));
+                if (lane == 0) y[rl * ldy] = sl;
+            }
+        }
+    }
+    if (lane == 0) s_cnt[w] = cnt;
+    __syncthreads();
+    for (int q = 0; q < WARPS * LIST; ++q) {
+        if (q % LIST >= s_cnt[q / LIST]) continue;  // the same for every thread
+        const int rl = s_list[q / LIST][q % LIST];
+        const double t = warp_sum(strided(rp[rl], rp[rl + 1], threadIdx.x, GROUP_THREADS));
+        if (lane == 0) s_sum[w] = t;
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            double sum = s_sum[0];
+#pragma unroll
+            for (int k = 1; k < WARPS; ++k) sum += s_sum[k];
+            y[rl * ldy] = sum;
+        }
+        __syncthreads();  // s_sum is written again by the next row
+    }
+}
+
 int ilog2(int v) {
     int s = 0;
     while ((1 << s) < v) ++s;
@@ -409,6 +544,31 @@ cudaError_t launch_window(const Handle &h, const VT *x, long long ldx, double *y
     });
 }
 
+// One right-hand side, one column lane: the SpMV kernel for the group width.
+template <typename VT>
+cudaError_t launch_spmv(const Handle &h, const VT *x, long long ldx, double *y, long long ldy,
+                        cudaStream_t s) {
+    const int tr = h.rows_per_tile;
+    const long long ntiles = ((long long)h.m + tr - 1) / tr;
+    const long long want = (ntiles + (GROUP_THREADS / 32) - 1) / (GROUP_THREADS / 32);
+    const long long cap = (long long)h.sm_count * SPMV_MINB;
+    const unsigned grid = (unsigned)(want < cap ? (want > 0 ? want : 1) : cap);
+    auto go = [&](auto GLC) {
+        csr_spmv_kernel<decltype(GLC)::value, VT><<<grid, GROUP_THREADS, 0, s>>>(
+            h.rp, h.ci, (const VT *)h.v, x, ldx, y, ldy, h.m, tr, h.n, guard_word());
+        return cudaGetLastError();
+    };
+    switch (h.lanes_per_row) {
+        case 1: return go(std::integral_constant<int, 1>());
+        case 2: return go(std::integral_constant<int, 2>());
+        case 4: return go(std::integral_constant<int, 4>());
+        case 8: return go(std::integral_constant<int, 8>());
+        case 16: return go(std::integral_constant<int, 16>());
+        case 32: return go(std::integral_constant<int, 32>());
+        default: return cudaErrorInvalidValue;
+    }
+}
+
 template <int KPL, typename VT>
 cudaError_t launch_rows(const Handle &h, const VT *x, long long ldx, double *y, long long ldy,
                         int k, cudaStream_t s) {
@@ -426,7 +586,9 @@ cudaError_t launch_rows(const Handle &h, const VT *x, long long ldx, double *y, 
     return with_kc(kc, [&](auto KCC) {
         constexpr int KCT = decltype(KCC)::value;
         constexpr int VW2 = KPL >= 2 ? 2 : 1;
-        if (vec2)
+        if constexpr (KPL == 1 && KCT == 0)
+            return cudaErrorInvalidValue;  // one column in one lane: launch_spmv
+        else if (vec2)
             csr_group_kernel<KPL, VT, KCT, VW2><<<grid, GROUP_THREADS, 0, s>>>(
                 h.rp, h.ci, (const VT *)h.v, x, ldx, y, ldy, h.m, k, gs, ks, tr, h.n,
                 guard_word());
@@ -451,6 +613,8 @@ cudaError_t launch_group(const Handle &h, const void *X, long long ldx, void *Y,
             default: return cudaErrorInvalidValue;
         }
     }
+    if (k == 1 && h.col_lanes == 1 && h.cols_per_lane == 1)
+        return launch_spmv<VT>(h, x, ldx, y, ldy, s);
     switch (h.cols_per_lane) {
         case 1: return launch_rows<1, VT>(h, x, ldx, y, ldy, k, s);
         case 2: return launch_rows<2, VT>(h, x, ldx, y, ldy, k, s);
