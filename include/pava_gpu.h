@@ -201,7 +201,9 @@ pava_status pava_spmv_host_async(pava_handle *h, const void *x_host, void *y_hos
 pava_status pava_spmv_host_wait(pava_handle *h);
 pava_status pava_get_info(const pava_handle *h, pava_info *out);
 
-/* anonymouslibHandle::destroy / asCSR (csr5/anonymouslib_avx512.h:80-104,258-262). */
+/* anonymouslibHandle::destroy / asCSR (csr5/anonymouslib_avx512.h:80-104,258-262).  Waits for the
+ * handle's device.  The library keeps up to 1 GiB of freed device memory per device for later
+ * conversions. */
 pava_status pava_destroy(pava_handle *h);
 
 /* Message of the last failed call on this thread ("" if none). */

@@ -90,37 +90,37 @@ std::atomic<unsigned long long> g_mem_limit{0};
 
 // A handle's device allocation: counted in *acc and refused, as an allocation failure, when it
 // would take the handle past the memory limit.
-cudaError_t budget_malloc(void **p, size_t bytes, size_t *acc) {
+cudaError_t budget_malloc(void **p, size_t bytes, size_t *acc, cudaStream_t s) {
     *p = nullptr;
     if (bytes == 0) bytes = 1;
     const unsigned long long lim = g_mem_limit.load();
     if (lim && acc && (unsigned long long)*acc + bytes > lim) return cudaErrorMemoryAllocation;
-    cudaError_t e = cudaMalloc(p, bytes);
+    cudaError_t e = pava::pool_malloc(p, bytes, s);
     if (e == cudaSuccess && acc) *acc += bytes;
     return e;
 }
 
 template <typename T>
-cudaError_t dalloc(T **p, size_t count, size_t *acc) {
-    return budget_malloc((void **)p, sizeof(T) * (count ? count : 1), acc);
+cudaError_t dalloc(T **p, size_t count, size_t *acc, cudaStream_t s) {
+    return budget_malloc((void **)p, sizeof(T) * (count ? count : 1), acc, s);
 }
 
-void free_handle_buffers(pava::Handle &h) {
-    cudaFree(h.arp);
-    cudaFree(h.vals);
-    cudaFree(h.cols);
-    cudaFree(h.flags);
-    cudaFree(h.meta);
-    cudaFree(h.tile_ptr);
-    cudaFree(h.colbase);
-    cudaFree(h.carry_head);
-    cudaFree(h.carry_tail);
-    cudaFree(h.rp);
-    cudaFree(h.ci);
-    cudaFree(h.v);
+// The handle's device buffers, detached from it.
+constexpr int HANDLE_BUFFERS = 12;
+void take_handle_buffers(pava::Handle &h, void *(&ps)[HANDLE_BUFFERS]) {
+    void *all[HANDLE_BUFFERS] = {h.arp, h.vals, h.cols, h.flags, h.meta, h.tile_ptr, h.colbase,
+                                 h.carry_head, h.carry_tail, h.rp, h.ci, h.v};
+    memcpy(ps, all, sizeof(all));
     h.arp = nullptr; h.vals = nullptr; h.cols = nullptr; h.flags = nullptr; h.meta = nullptr;
     h.tile_ptr = nullptr; h.colbase = nullptr; h.carry_head = nullptr; h.carry_tail = nullptr;
     h.rp = nullptr; h.ci = nullptr; h.v = nullptr;
+}
+
+// Frees them while a handle is being made: they were used on s alone.
+void free_handle_buffers(pava::Handle &h, cudaStream_t s) {
+    void *ps[HANDLE_BUFFERS];
+    take_handle_buffers(h, ps);
+    for (void *p : ps) pava::pool_free(p, s);
 }
 
 // Lanes per row of the plain CSR SpMV by the mean row length: the fastest of the measured widths.
@@ -191,14 +191,14 @@ bool resolve_group_shape(const pava::Handle &h, int k, pava::Handle &out, std::s
 
 // Builds the augmented row pointer and sizes the chunked element space (CVR, CSR5).
 pava_status plan_chunks(pava::Handle &h, const int *rp, cudaStream_t s) {
-    PAVA_CUDA(dalloc(&h.arp, (size_t)h.m + 2, &h.device_bytes), "cudaMalloc(arp)");
+    PAVA_CUDA(dalloc(&h.arp, (size_t)h.m + 2, &h.device_bytes, s), "cudaMalloc(arp)");
     int *d_nempty = nullptr;
-    PAVA_CUDA(cudaMallocAsync(&d_nempty, sizeof(int), s), "cudaMallocAsync");
+    PAVA_CUDA(pava::pool_malloc(&d_nempty, 1, s), "cudaMallocAsync");
     cudaError_t e = pava::build_augmented_rowptr(rp, h.m, 0, h.arp, d_nempty, s);
     int nempty = 0;
     if (e == cudaSuccess) e = cudaMemcpyAsync(&nempty, d_nempty, sizeof(int), cudaMemcpyDeviceToHost, s);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-    cudaFreeAsync(d_nempty, s);
+    pava::pool_free(d_nempty, s);
     if (e != cudaSuccess) return fail_cuda(e, "augmented row pointer");
     h.n_empty = nempty;
     h.n_aug = (long long)h.nnz + nempty;
@@ -221,38 +221,38 @@ pava_status convert(pava::Handle &h, const int *rp, const int *ci, const double 
         pava_status st = plan_chunks(h, rp, s);
         if (st != PAVA_SUCCESS) return st;
         const size_t padded = (size_t)(h.nchunks * h.L);
-        PAVA_CUDA(budget_malloc(&h.vals, sv * (padded ? padded : 1), &h.device_bytes),
+        PAVA_CUDA(budget_malloc(&h.vals, sv * (padded ? padded : 1), &h.device_bytes, s),
                   "cudaMalloc(vals)");
-        PAVA_CUDA(budget_malloc(&h.cols, si * (padded ? padded : 1), &h.device_bytes),
+        PAVA_CUDA(budget_malloc(&h.cols, si * (padded ? padded : 1), &h.device_bytes, s),
                   "cudaMalloc(cols)");
-        PAVA_CUDA(dalloc(&h.carry_head, (size_t)h.nchunks, &h.device_bytes), "cudaMalloc(carry)");
-        PAVA_CUDA(dalloc(&h.carry_tail, (size_t)h.nchunks, &h.device_bytes), "cudaMalloc(carry)");
+        PAVA_CUDA(dalloc(&h.carry_head, (size_t)h.nchunks, &h.device_bytes, s), "cudaMalloc(carry)");
+        PAVA_CUDA(dalloc(&h.carry_tail, (size_t)h.nchunks, &h.device_bytes, s), "cudaMalloc(carry)");
         if (h.index_mode == PAVA_INDEX_DELTA16) {
-            PAVA_CUDA(dalloc(&h.colbase, (size_t)h.nchunks, &h.device_bytes), "cudaMalloc(colbase)");
+            PAVA_CUDA(dalloc(&h.colbase, (size_t)h.nchunks, &h.device_bytes, s), "cudaMalloc(colbase)");
             PAVA_CUDA(pava::chunk_colbase(h, rp, ci, s), "chunk column bases");
         }
         int *d_ovf = nullptr;
-        PAVA_CUDA(cudaMallocAsync(&d_ovf, sizeof(int), s), "cudaMallocAsync");
+        PAVA_CUDA(pava::pool_malloc(&d_ovf, 1, s), "cudaMallocAsync");
         cudaError_t e = cudaMemsetAsync(d_ovf, 0, sizeof(int), s);
         if (h.format == PAVA_FORMAT_CVR) {
-            if (e == cudaSuccess) e = dalloc(&h.flags, (size_t)h.nchunks * h.S, &h.device_bytes);
+            if (e == cudaSuccess) e = dalloc(&h.flags, (size_t)h.nchunks * h.S, &h.device_bytes, s);
             h.meta_stride = sizeof(pava::CvrMeta);
             if (e == cudaSuccess)
-                e = dalloc((pava::CvrMeta **)&h.meta, (size_t)h.nchunks, &h.device_bytes);
+                e = dalloc((pava::CvrMeta **)&h.meta, (size_t)h.nchunks, &h.device_bytes, s);
             if (e == cudaSuccess) e = pava::cvr_convert(h, rp, ci, v, d_ovf, s);
         } else {
             h.ntiles = h.nchunks * h.G;
-            if (e == cudaSuccess) e = dalloc(&h.flags, (size_t)h.ntiles * 32, &h.device_bytes);
-            if (e == cudaSuccess) e = dalloc(&h.tile_ptr, (size_t)h.ntiles, &h.device_bytes);
+            if (e == cudaSuccess) e = dalloc(&h.flags, (size_t)h.ntiles * 32, &h.device_bytes, s);
+            if (e == cudaSuccess) e = dalloc(&h.tile_ptr, (size_t)h.ntiles, &h.device_bytes, s);
             h.meta_stride = sizeof(pava::ChunkHdr);
             if (e == cudaSuccess)
-                e = dalloc((pava::ChunkHdr **)&h.meta, (size_t)h.nchunks, &h.device_bytes);
+                e = dalloc((pava::ChunkHdr **)&h.meta, (size_t)h.nchunks, &h.device_bytes, s);
             if (e == cudaSuccess) e = pava::csr5_convert(h, rp, ci, v, d_ovf, s);
         }
         int ovf = 0;
         if (e == cudaSuccess) e = cudaMemcpyAsync(&ovf, d_ovf, sizeof(int), cudaMemcpyDeviceToHost, s);
         if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-        cudaFreeAsync(d_ovf, s);
+        pava::pool_free(d_ovf, s);
         if (e != cudaSuccess) return fail_cuda(e, "conversion");
         h.d16_overflow = ovf ? 1 : 0;
         if (ovf)
@@ -262,13 +262,13 @@ pava_status convert(pava::Handle &h, const int *rp, const int *ci, const double 
         h.nchunks = ((long long)h.m + 31) / 32;
         h.L = 32;
         h.meta_stride = sizeof(pava::SellSlice);
-        PAVA_CUDA(dalloc((pava::SellSlice **)&h.meta, (size_t)h.nchunks, &h.device_bytes),
+        PAVA_CUDA(dalloc((pava::SellSlice **)&h.meta, (size_t)h.nchunks, &h.device_bytes, s),
                   "cudaMalloc(slices)");
         int *d_off = nullptr, *d_tot = nullptr, *d_ovf = nullptr;
         int total_blk = 0, ovf = 0;
-        cudaError_t e = cudaMallocAsync(&d_off, sizeof(int) * (size_t)(h.nchunks + 1), s);
-        if (e == cudaSuccess) e = cudaMallocAsync(&d_tot, sizeof(int), s);
-        if (e == cudaSuccess) e = cudaMallocAsync(&d_ovf, sizeof(int), s);
+        cudaError_t e = pava::pool_malloc(&d_off, (size_t)(h.nchunks + 1), s);
+        if (e == cudaSuccess) e = pava::pool_malloc(&d_tot, 1, s);
+        if (e == cudaSuccess) e = pava::pool_malloc(&d_ovf, 1, s);
         if (e == cudaSuccess) e = cudaMemsetAsync(d_ovf, 0, sizeof(int), s);
         if (e == cudaSuccess && h.nchunks > 0) e = pava::sell_plan(h, rp, ci, d_off, d_tot, s);
         if (e == cudaSuccess && h.nchunks > 0)
@@ -286,27 +286,27 @@ pava_status convert(pava::Handle &h, const int *rp, const int *ci, const double 
             st = fail(PAVA_E_TOO_LARGE, "SELL: padded elements exceed the int32 element space");
         } else {
             h.n_aug = padded;
-            e = budget_malloc(&h.vals, sv * (size_t)(padded ? padded : 1), &h.device_bytes);
+            e = budget_malloc(&h.vals, sv * (size_t)(padded ? padded : 1), &h.device_bytes, s);
             if (e == cudaSuccess)
-                e = budget_malloc(&h.cols, si * (size_t)(padded ? padded : 1), &h.device_bytes);
+                e = budget_malloc(&h.cols, si * (size_t)(padded ? padded : 1), &h.device_bytes, s);
             if (e == cudaSuccess && h.nchunks > 0) e = pava::sell_fill(h, rp, ci, v, d_off, d_ovf, s);
             if (e == cudaSuccess) e = cudaMemcpyAsync(&ovf, d_ovf, sizeof(int), cudaMemcpyDeviceToHost, s);
             if (e == cudaSuccess) e = cudaStreamSynchronize(s);
             if (e != cudaSuccess) st = fail_cuda(e, "SELL conversion");
         }
-        cudaFreeAsync(d_off, s);
-        cudaFreeAsync(d_tot, s);
-        cudaFreeAsync(d_ovf, s);
+        pava::pool_free(d_off, s);
+        pava::pool_free(d_tot, s);
+        pava::pool_free(d_ovf, s);
         if (st != PAVA_SUCCESS) return st;
         h.d16_overflow = ovf ? 1 : 0;
         if (ovf)
             return fail(PAVA_E_UNSUPPORTED_PARAMS,
                         "16-bit column offsets: a slice's columns span more than 65534");
     } else {  // plain CSR: private copies (values narrowed to float for FP32C)
-        PAVA_CUDA(dalloc(&h.rp, (size_t)h.m + 1, &h.device_bytes), "cudaMalloc(rp)");
-        PAVA_CUDA(dalloc(&h.ci, (size_t)h.nnz, &h.device_bytes), "cudaMalloc(ci)");
+        PAVA_CUDA(dalloc(&h.rp, (size_t)h.m + 1, &h.device_bytes, s), "cudaMalloc(rp)");
+        PAVA_CUDA(dalloc(&h.ci, (size_t)h.nnz, &h.device_bytes, s), "cudaMalloc(ci)");
         const size_t nv = (size_t)(h.nnz ? h.nnz : 1);
-        PAVA_CUDA(budget_malloc(&h.v, sv * nv, &h.device_bytes), "cudaMalloc(v)");
+        PAVA_CUDA(budget_malloc(&h.v, sv * nv, &h.device_bytes, s), "cudaMalloc(v)");
         PAVA_CUDA(cudaMemcpyAsync(h.rp, rp, sizeof(int) * ((size_t)h.m + 1),
                                   cudaMemcpyDeviceToDevice, s), "copy rp");
         if (h.nnz > 0) {
@@ -555,6 +555,21 @@ pava_status pava_create(const pava_csr *A, int format, const pava_opts *opts, vo
         }
     }
 
+    // conversion allocates and waits: not on a stream that is being captured
+    cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
+    ce = cudaStreamIsCapturing(s, &capturing);
+    if (ce == cudaSuccess && capturing != cudaStreamCaptureStatusNone)
+        ce = cudaErrorStreamCaptureUnsupported;
+    if (ce != cudaSuccess) { delete H; return fail_cuda(ce, "conversion"); }
+    const size_t held = pava::pool_reserved();
+    // a failed conversion leaves the pool as it found it
+    auto give_back = [&]() {
+        free_handle_buffers(h, s);
+        cudaStreamSynchronize(s);
+        pava::pool_trim(held);
+        delete H;
+    };
+
     // inputs on the device
     const int *rp = A->row_ptr, *ci = A->col_idx;
     const double *v = A->vals;
@@ -562,34 +577,34 @@ pava_status pava_create(const pava_csr *A, int format, const pava_opts *opts, vo
     double *t_v = nullptr;
     pava_status st = PAVA_SUCCESS;
     auto cleanup_tmp = [&]() {
-        cudaFree(t_rp); cudaFree(t_ci); cudaFree(t_v);
+        pava::pool_free(t_rp, s); pava::pool_free(t_ci, s); pava::pool_free(t_v, s);
     };
     if (!A->on_device) {
-        ce = cudaMalloc(&t_rp, sizeof(int) * ((size_t)h.m + 1));
-        if (ce == cudaSuccess) ce = cudaMalloc(&t_ci, sizeof(int) * (size_t)(h.nnz ? h.nnz : 1));
-        if (ce == cudaSuccess) ce = cudaMalloc(&t_v, sizeof(double) * (size_t)(h.nnz ? h.nnz : 1));
+        ce = pava::pool_malloc(&t_rp, (size_t)h.m + 1, s);
+        if (ce == cudaSuccess) ce = pava::pool_malloc(&t_ci, (size_t)h.nnz, s);
+        if (ce == cudaSuccess) ce = pava::pool_malloc(&t_v, (size_t)h.nnz, s);
         if (ce == cudaSuccess)
             ce = cudaMemcpyAsync(t_rp, rp, sizeof(int) * ((size_t)h.m + 1), cudaMemcpyHostToDevice, s);
         if (ce == cudaSuccess && h.nnz)
             ce = cudaMemcpyAsync(t_ci, ci, sizeof(int) * (size_t)h.nnz, cudaMemcpyHostToDevice, s);
         if (ce == cudaSuccess && h.nnz)
             ce = cudaMemcpyAsync(t_v, v, sizeof(double) * (size_t)h.nnz, cudaMemcpyHostToDevice, s);
-        if (ce != cudaSuccess) { cleanup_tmp(); delete H; return fail_cuda(ce, "copying the CSR to the device"); }
+        if (ce != cudaSuccess) { cleanup_tmp(); give_back(); return fail_cuda(ce, "copying the CSR to the device"); }
         rp = t_rp; ci = t_ci; v = t_v;
     }
     // validation
     {
         int *d_err = nullptr;
         int herr = 0;
-        ce = cudaMallocAsync(&d_err, sizeof(int), s);
+        ce = pava::pool_malloc(&d_err, 1, s);
         if (ce == cudaSuccess) ce = pava::launch_validate(rp, ci, h.m, h.n, h.nnz, d_err, s);
         if (ce == cudaSuccess) ce = cudaMemcpyAsync(&herr, d_err, sizeof(int), cudaMemcpyDeviceToHost, s);
         if (ce == cudaSuccess) ce = cudaStreamSynchronize(s);
-        cudaFreeAsync(d_err, s);
-        if (ce != cudaSuccess) { cleanup_tmp(); delete H; return fail_cuda(ce, "CSR validation"); }
+        pava::pool_free(d_err, s);
+        if (ce != cudaSuccess) { cleanup_tmp(); give_back(); return fail_cuda(ce, "CSR validation"); }
         if (herr) {
             cleanup_tmp();
-            delete H;
+            give_back();
             return fail(PAVA_E_INVALID_CSR, "row_ptr not monotone, row_ptr[0]/row_ptr[m] wrong, or column out of range (" +
                                                 std::to_string(herr) + " violations)");
         }
@@ -601,7 +616,7 @@ pava_status pava_create(const pava_csr *A, int format, const pava_opts *opts, vo
     st = convert(h, rp, ci, v, s);
     if (st == PAVA_E_UNSUPPORTED_PARAMS && auto_index && h.d16_overflow) {
         // a column does not fit 16 bits: convert again with 32-bit columns
-        free_handle_buffers(h);
+        free_handle_buffers(h, s);
         h.device_bytes = 0;
         h.index_mode = PAVA_INDEX_I32;
         st = convert(h, rp, ci, v, s);
@@ -618,8 +633,7 @@ pava_status pava_create(const pava_csr *A, int format, const pava_opts *opts, vo
     cudaEventDestroy(e1);
     cleanup_tmp();
     if (st != PAVA_SUCCESS) {
-        free_handle_buffers(h);
-        delete H;
+        give_back();
         return st;
     }
     *out = H;
@@ -776,7 +790,9 @@ pava_status pava_get_info(const pava_handle *H, pava_info *out) {
 pava_status pava_destroy(pava_handle *H) {
     if (!H) return PAVA_SUCCESS;
     free_pipe(H->pipe);
-    free_handle_buffers(H->h);
+    void *ps[HANDLE_BUFFERS];
+    take_handle_buffers(H->h, ps);
+    pava::pool_free_synced(ps, HANDLE_BUFFERS);
     cudaFree(H->x_dev);
     cudaFree(H->y_dev);
     delete H;

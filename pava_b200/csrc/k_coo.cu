@@ -99,20 +99,28 @@ extern "C" pava_status pava_coo_to_csr_device(int m, int n, long long nnz, const
     unsigned long long *keys = nullptr, *keys2 = nullptr;
     double *v = nullptr, *v2 = nullptr;
     void *tmp = nullptr;
+    cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
+    cudaError_t e = cudaStreamIsCapturing(s, &capturing);
+    if (e == cudaSuccess && capturing != cudaStreamCaptureStatusNone)
+        e = cudaErrorStreamCaptureUnsupported;
+    const size_t held = pool_reserved();
     auto cleanup = [&]() {
-        cudaFree(flag); cudaFree(mpos); cudaFree(d_bad); cudaFree(keys); cudaFree(keys2);
-        cudaFree(v); cudaFree(tmp);
+        pool_free(flag, s); pool_free(mpos, s); pool_free(d_bad, s); pool_free(keys, s);
+        pool_free(keys2, s); pool_free(v, s); pool_free(tmp, s);
     };
     auto fail_e = [&](cudaError_t e) {
         cleanup();
-        cudaFree(rp); cudaFree(ci); cudaFree(v2);
+        pool_free(rp, s); pool_free(ci, s); pool_free(v2, s);
+        cudaStreamSynchronize(s);
+        pool_trim(held);
         set_last_error(std::string("COO -> CSR: ") + cudaGetErrorString(e));
         return e == cudaErrorMemoryAllocation ? PAVA_E_NOMEM : PAVA_E_CUDA;
     };
     const size_t nz = (size_t)(nnz ? nnz : 1);
-    cudaError_t e = cudaMalloc(&flag, sizeof(int) * nz);
-    if (e == cudaSuccess) e = cudaMalloc(&mpos, sizeof(int) * nz);
-    if (e == cudaSuccess) e = cudaMalloc(&d_bad, sizeof(int) * 2);
+    if (e != cudaSuccess) return fail_e(e);  // it allocates and waits
+    e = pool_malloc(&flag, nz, s);
+    if (e == cudaSuccess) e = pool_malloc(&mpos, nz, s);
+    if (e == cudaSuccess) e = pool_malloc(&d_bad, 2, s);
     if (e == cudaSuccess) e = cudaMemsetAsync(d_bad, 0, sizeof(int) * 2, s);
     if (e == cudaSuccess && nnz > 0) {
         coo_flags_kernel<<<grid_of(nnz), 256, 0, s>>>(rows, cols, nnz, index_base, m, n,
@@ -121,13 +129,13 @@ extern "C" pava_status pava_coo_to_csr_device(int m, int n, long long nnz, const
     }
     size_t tb = 0;
     if (e == cudaSuccess && nnz > 0) e = cub::DeviceScan::ExclusiveSum(nullptr, tb, flag, mpos, (int)nnz, s);
-    if (e == cudaSuccess && nnz > 0) e = cudaMalloc(&tmp, tb ? tb : 1);
+    if (e == cudaSuccess && nnz > 0) e = pool_malloc(&tmp, tb, s);
     if (e == cudaSuccess && nnz > 0) e = cub::DeviceScan::ExclusiveSum(tmp, tb, flag, mpos, (int)nnz, s);
     if (e == cudaSuccess && nnz > 0)  // mirrored count = mpos[last] + flag[last]
         e = cub::DeviceReduce::Sum(nullptr, tb, flag, d_bad + 1, (int)nnz, s);
-    cudaFree(tmp);
+    pool_free(tmp, s);
     tmp = nullptr;
-    if (e == cudaSuccess && nnz > 0) e = cudaMalloc(&tmp, tb ? tb : 1);
+    if (e == cudaSuccess && nnz > 0) e = pool_malloc(&tmp, tb, s);
     if (e == cudaSuccess && nnz > 0) e = cub::DeviceReduce::Sum(tmp, tb, flag, d_bad + 1, (int)nnz, s);
     int h[2] = {0, 0};
     if (e == cudaSuccess) e = cudaMemcpyAsync(h, d_bad, sizeof(h), cudaMemcpyDeviceToHost, s);
@@ -145,23 +153,23 @@ extern "C" pava_status pava_coo_to_csr_device(int m, int n, long long nnz, const
         return PAVA_E_TOO_LARGE;
     }
     const size_t tz = (size_t)(total ? total : 1);
-    e = cudaMalloc(&keys, sizeof(unsigned long long) * tz);
-    if (e == cudaSuccess) e = cudaMalloc(&keys2, sizeof(unsigned long long) * tz);
-    if (e == cudaSuccess) e = cudaMalloc(&v, sizeof(double) * tz);
-    if (e == cudaSuccess) e = cudaMalloc(&v2, sizeof(double) * tz);
-    if (e == cudaSuccess) e = cudaMalloc(&rp, sizeof(int) * ((size_t)m + 1));
-    if (e == cudaSuccess) e = cudaMalloc(&ci, sizeof(int) * tz);
+    e = pool_malloc(&keys, tz, s);
+    if (e == cudaSuccess) e = pool_malloc(&keys2, tz, s);
+    if (e == cudaSuccess) e = pool_malloc(&v, tz, s);
+    if (e == cudaSuccess) e = pool_malloc(&v2, tz, s);
+    if (e == cudaSuccess) e = pool_malloc(&rp, (size_t)m + 1, s);
+    if (e == cudaSuccess) e = pool_malloc(&ci, tz, s);
     if (e == cudaSuccess && nnz > 0) {
         coo_keys_kernel<<<grid_of(nnz), 256, 0, s>>>(rows, cols, vals, nnz, index_base, mpos,
                                                      symmetric, keys, v);
         e = cudaGetLastError();
     }
-    cudaFree(tmp);
+    pool_free(tmp, s);
     tmp = nullptr;
     if (e == cudaSuccess && total > 0)
         e = cub::DeviceRadixSort::SortPairs(nullptr, tb, keys, keys2, v, v2, (int)total, 0,
                                             key_bits(m), s);
-    if (e == cudaSuccess && total > 0) e = cudaMalloc(&tmp, tb ? tb : 1);
+    if (e == cudaSuccess && total > 0) e = pool_malloc(&tmp, tb, s);
     if (e == cudaSuccess && total > 0)
         e = cub::DeviceRadixSort::SortPairs(tmp, tb, keys, keys2, v, v2, (int)total, 0,
                                             key_bits(m), s);

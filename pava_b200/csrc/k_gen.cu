@@ -347,9 +347,9 @@ extern "C" pava_status pava_gen_device(const pava_gen_params *q, uint64_t seed, 
 extern "C" pava_status pava_free_device_csr(pava_csr *A) {
     if (!A) return PAVA_SUCCESS;
     if (A->on_device) {
-        cudaFree((void *)A->row_ptr);
-        cudaFree((void *)A->col_idx);
-        cudaFree((void *)A->vals);
+        // as cudaFree does, after whatever still uses them
+        void *ps[3] = {(void *)A->row_ptr, (void *)A->col_idx, (void *)A->vals};
+        pava::pool_free_synced(ps, 3);
     }
     memset(A, 0, sizeof(*A));
     return PAVA_SUCCESS;

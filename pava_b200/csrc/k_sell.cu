@@ -327,7 +327,7 @@ cudaError_t sell_plan(Handle &h, const int *rp, const int *ci, int *d_blk_off, i
     const long long ns = h.nchunks;
     const long long threads = ns * 32;
     int *nblk = nullptr;
-    cudaError_t e = cudaMallocAsync(&nblk, sizeof(int) * (size_t)(ns + 1), s);
+    cudaError_t e = pool_malloc(&nblk, (size_t)(ns + 1), s);
     if (e != cudaSuccess) return e;
     sell_plan_kernel<<<(unsigned)((threads + 255) / 256), 256, 0, s>>>(
         rp, ci, h.m, ns, h.index_mode == PAVA_INDEX_DELTA16 ? 1 : 0, (SellSlice *)h.meta, nblk);
@@ -338,13 +338,13 @@ cudaError_t sell_plan(Handle &h, const int *rp, const int *ci, int *d_blk_off, i
     if (e == cudaSuccess)
         e = cub::DeviceScan::ExclusiveSum(nullptr, tmp_bytes, nblk, d_blk_off, (int)(ns + 1), s);
     void *tmp = nullptr;
-    if (e == cudaSuccess) e = cudaMallocAsync(&tmp, tmp_bytes ? tmp_bytes : 1, s);
+    if (e == cudaSuccess) e = pool_malloc(&tmp, tmp_bytes, s);
     if (e == cudaSuccess)
         e = cub::DeviceScan::ExclusiveSum(tmp, tmp_bytes, nblk, d_blk_off, (int)(ns + 1), s);
     if (e == cudaSuccess)
         e = cudaMemcpyAsync(d_total_blk, d_blk_off + ns, sizeof(int), cudaMemcpyDeviceToDevice, s);
-    if (tmp) cudaFreeAsync(tmp, s);
-    cudaFreeAsync(nblk, s);
+    pool_free(tmp, s);
+    pool_free(nblk, s);
     return e;
 }
 

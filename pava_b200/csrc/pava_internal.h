@@ -74,6 +74,25 @@ struct Handle {
     int d16_overflow = 0;    // the last conversion found a column outside the 16-bit range
 };
 
+// Device memory of handles, conversions and their temporaries: a memory pool per device (and
+// context) that keeps at most POOL_KEEP bytes of what was freed, so that converting a new matrix
+// does not pay the driver for its buffers each time.  All calls are thread-safe; memory is
+// ordered on the stream it is allocated and freed on.
+constexpr size_t POOL_KEEP = (size_t)1 << 30;
+cudaError_t pool_malloc(void **p, size_t bytes, cudaStream_t s);
+template <typename T> cudaError_t pool_malloc(T **p, size_t count, cudaStream_t s) {
+    return pool_malloc((void **)p, sizeof(T) * (count ? count : 1), s);
+}
+// Frees memory whose last use is ordered before this point of s (NULL pointers are skipped).
+void pool_free(void *p, cudaStream_t s);
+// Frees memory that work on any stream may still use: waits for the device first, as cudaFree
+// does.  Where the wait is not possible (a stream is capturing) the memory is kept until a later
+// call can wait.
+void pool_free_synced(void *const *ps, int count);
+// Bytes the pool holds, and giving back what is unused above `keep`.
+size_t pool_reserved();
+void pool_trim(size_t keep);
+
 // Sets the message pava_last_error() returns on this thread.
 void set_last_error(const std::string &msg);
 
