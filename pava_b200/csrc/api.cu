@@ -189,72 +189,86 @@ bool resolve_group_shape(const pava::Handle &h, int k, pava::Handle &out, std::s
     return true;
 }
 
-// Builds the augmented row pointer and sizes the chunked element space (CVR, CSR5).
-pava_status plan_chunks(pava::Handle &h, const int *rp, cudaStream_t s) {
-    PAVA_CUDA(dalloc(&h.arp, (size_t)h.m + 2, &h.device_bytes, s), "cudaMalloc(arp)");
-    int *d_nempty = nullptr;
-    PAVA_CUDA(pava::pool_malloc(&d_nempty, 1, s), "cudaMallocAsync");
-    cudaError_t e = pava::build_augmented_rowptr(rp, h.m, 0, h.arp, d_nempty, s);
-    int nempty = 0;
-    if (e == cudaSuccess) e = cudaMemcpyAsync(&nempty, d_nempty, sizeof(int), cudaMemcpyDeviceToHost, s);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-    pava::pool_free(d_nempty, s);
-    if (e != cudaSuccess) return fail_cuda(e, "augmented row pointer");
+// Sizes the chunked element space (CVR, CSR5) once the number of empty rows is known and
+// completes the augmented row pointer.
+pava_status plan_chunks(pava::Handle &h, int nempty, cudaStream_t s) {
     h.n_empty = nempty;
     h.n_aug = (long long)h.nnz + nempty;
     h.nchunks = (h.n_aug + h.L - 1) / h.L;
     const long long padded = h.nchunks * h.L;
     if (padded >= (long long)INT_MAX - 64)
         return fail(PAVA_E_TOO_LARGE, "matrix exceeds the int32 element space after padding");
-    const int pt = (int)padded;
-    PAVA_CUDA(cudaMemcpyAsync(h.arp + h.m + 1, &pt, sizeof(int), cudaMemcpyHostToDevice, s),
-              "cudaMemcpyAsync(arp)");
-    PAVA_CUDA(cudaStreamSynchronize(s), "cudaStreamSynchronize");
+    PAVA_CUDA(pava::set_int(h.arp + h.m + 1, (int)padded, s), "augmented row pointer");
     return PAVA_SUCCESS;
 }
 
-pava_status convert(pava::Handle &h, const int *rp, const int *ci, const double *v,
-                    cudaStream_t s) {
+// Converts the validated CSR (device arrays) into the handle's form.  nempty: empty rows, for the
+// chunked forms, whose h.arp[0..m] is complete.  auto_index: fall back to 32-bit columns when
+// 16-bit offsets do not reach.
+pava_status convert(pava::Handle &h, const int *rp, const int *ci, const double *v, int nempty,
+                    bool auto_index, cudaStream_t s) {
     const size_t sv = value_bytes(h.precision);
-    const size_t si = h.index_mode == PAVA_INDEX_DELTA16 ? 2 : 4;
     if (h.format == PAVA_FORMAT_CVR || h.format == PAVA_FORMAT_CSR5) {
-        pava_status st = plan_chunks(h, rp, s);
+        pava_status st = plan_chunks(h, nempty, s);
         if (st != PAVA_SUCCESS) return st;
+        const bool cvr = h.format == PAVA_FORMAT_CVR;
         const size_t padded = (size_t)(h.nchunks * h.L);
         PAVA_CUDA(budget_malloc(&h.vals, sv * (padded ? padded : 1), &h.device_bytes, s),
                   "cudaMalloc(vals)");
-        PAVA_CUDA(budget_malloc(&h.cols, si * (padded ? padded : 1), &h.device_bytes, s),
-                  "cudaMalloc(cols)");
         PAVA_CUDA(dalloc(&h.carry_head, (size_t)h.nchunks, &h.device_bytes, s), "cudaMalloc(carry)");
         PAVA_CUDA(dalloc(&h.carry_tail, (size_t)h.nchunks, &h.device_bytes, s), "cudaMalloc(carry)");
-        if (h.index_mode == PAVA_INDEX_DELTA16) {
-            PAVA_CUDA(dalloc(&h.colbase, (size_t)h.nchunks, &h.device_bytes, s), "cudaMalloc(colbase)");
-            PAVA_CUDA(pava::chunk_colbase(h, rp, ci, s), "chunk column bases");
-        }
-        int *d_ovf = nullptr;
-        PAVA_CUDA(pava::pool_malloc(&d_ovf, 1, s), "cudaMallocAsync");
-        cudaError_t e = cudaMemsetAsync(d_ovf, 0, sizeof(int), s);
-        if (h.format == PAVA_FORMAT_CVR) {
-            if (e == cudaSuccess) e = dalloc(&h.flags, (size_t)h.nchunks * h.S, &h.device_bytes, s);
+        if (cvr) {
+            PAVA_CUDA(dalloc(&h.flags, (size_t)h.nchunks * h.S, &h.device_bytes, s), "cudaMalloc(flags)");
             h.meta_stride = sizeof(pava::CvrMeta);
-            if (e == cudaSuccess)
-                e = dalloc((pava::CvrMeta **)&h.meta, (size_t)h.nchunks, &h.device_bytes, s);
-            if (e == cudaSuccess) e = pava::cvr_convert(h, rp, ci, v, d_ovf, s);
+            PAVA_CUDA(dalloc((pava::CvrMeta **)&h.meta, (size_t)h.nchunks, &h.device_bytes, s),
+                      "cudaMalloc(meta)");
         } else {
             h.ntiles = h.nchunks * h.G;
-            if (e == cudaSuccess) e = dalloc(&h.flags, (size_t)h.ntiles * 32, &h.device_bytes, s);
-            if (e == cudaSuccess) e = dalloc(&h.tile_ptr, (size_t)h.ntiles, &h.device_bytes, s);
+            PAVA_CUDA(dalloc(&h.flags, (size_t)h.ntiles * 32, &h.device_bytes, s), "cudaMalloc(flags)");
+            PAVA_CUDA(dalloc(&h.tile_ptr, (size_t)h.ntiles, &h.device_bytes, s), "cudaMalloc(tile_ptr)");
             h.meta_stride = sizeof(pava::ChunkHdr);
-            if (e == cudaSuccess)
-                e = dalloc((pava::ChunkHdr **)&h.meta, (size_t)h.nchunks, &h.device_bytes, s);
-            if (e == cudaSuccess) e = pava::csr5_convert(h, rp, ci, v, d_ovf, s);
+            PAVA_CUDA(dalloc((pava::ChunkHdr **)&h.meta, (size_t)h.nchunks, &h.device_bytes, s),
+                      "cudaMalloc(meta)");
         }
+        // rows of the chunks' (CVR) or tiles' (CSR5) first elements
+        int *first = h.tile_ptr, *d_ovf = nullptr;
+        if (cvr) PAVA_CUDA(pava::pool_malloc(&first, (size_t)h.nchunks, s), "cudaMalloc(chunk rows)");
+        cudaError_t e = cvr ? pava::chunk_rows(h.arp, h.m, h.L, h.nchunks, first, s)
+                            : pava::chunk_rows(h.arp, h.m, 32LL * h.sigma, h.ntiles, first, s);
         int ovf = 0;
-        if (e == cudaSuccess) e = cudaMemcpyAsync(&ovf, d_ovf, sizeof(int), cudaMemcpyDeviceToHost, s);
-        if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+        if (h.index_mode == PAVA_INDEX_DELTA16) {
+            if (e == cudaSuccess) e = dalloc(&h.colbase, (size_t)h.nchunks, &h.device_bytes, s);
+            if (e == cudaSuccess) e = pava::pool_malloc(&d_ovf, 1, s);
+            if (e == cudaSuccess) e = cudaMemsetAsync(d_ovf, 0, sizeof(int), s);
+            if (e == cudaSuccess)
+                e = pava::chunk_colbase(h, rp, ci, first, cvr ? 1 : h.G, d_ovf, s);
+        }
+        auto run = [&]() {
+            const size_t si = h.index_mode == PAVA_INDEX_DELTA16 ? 2 : 4;
+            if (e == cudaSuccess)
+                e = budget_malloc(&h.cols, si * (padded ? padded : 1), &h.device_bytes, s);
+            if (e == cudaSuccess)
+                e = cvr ? pava::cvr_convert(h, rp, ci, v, first, d_ovf, s)
+                        : pava::csr5_convert(h, rp, ci, v, d_ovf, s);
+            if (e == cudaSuccess && d_ovf)
+                e = cudaMemcpyAsync(&ovf, d_ovf, sizeof(int), cudaMemcpyDeviceToHost, s);
+            if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+        };
+        run();
         pava::pool_free(d_ovf, s);
+        d_ovf = nullptr;
+        if (e == cudaSuccess && ovf && auto_index) {  // a column out of reach: 32-bit columns
+            pava::pool_free(h.cols, s);
+            pava::pool_free(h.colbase, s);
+            h.cols = nullptr;
+            h.colbase = nullptr;
+            h.device_bytes -= 2 * (padded ? padded : 1) + sizeof(int) * (size_t)(h.nchunks ? h.nchunks : 1);
+            h.index_mode = PAVA_INDEX_I32;
+            ovf = 0;
+            run();
+        }
+        if (cvr) pava::pool_free(first, s);
         if (e != cudaSuccess) return fail_cuda(e, "conversion");
-        h.d16_overflow = ovf ? 1 : 0;
         if (ovf)
             return fail(PAVA_E_UNSUPPORTED_PARAMS,
                         "16-bit column offsets: a chunk's columns span more than 65534");
@@ -264,17 +278,16 @@ pava_status convert(pava::Handle &h, const int *rp, const int *ci, const double 
         h.meta_stride = sizeof(pava::SellSlice);
         PAVA_CUDA(dalloc((pava::SellSlice **)&h.meta, (size_t)h.nchunks, &h.device_bytes, s),
                   "cudaMalloc(slices)");
-        int *d_off = nullptr, *d_tot = nullptr, *d_ovf = nullptr;
-        int total_blk = 0, ovf = 0;
+        int *d_off = nullptr, *d_res = nullptr;
+        int res[2] = {0, 0};  // blocks, columns out of 16-bit reach
         cudaError_t e = pava::pool_malloc(&d_off, (size_t)(h.nchunks + 1), s);
-        if (e == cudaSuccess) e = pava::pool_malloc(&d_tot, 1, s);
-        if (e == cudaSuccess) e = pava::pool_malloc(&d_ovf, 1, s);
-        if (e == cudaSuccess) e = cudaMemsetAsync(d_ovf, 0, sizeof(int), s);
-        if (e == cudaSuccess && h.nchunks > 0) e = pava::sell_plan(h, rp, ci, d_off, d_tot, s);
+        if (e == cudaSuccess) e = pava::pool_malloc(&d_res, 2, s);
         if (e == cudaSuccess && h.nchunks > 0)
-            e = cudaMemcpyAsync(&total_blk, d_tot, sizeof(int), cudaMemcpyDeviceToHost, s);
+            e = pava::sell_plan(h, rp, ci, h.index_mode == PAVA_INDEX_DELTA16, d_off, d_res, s);
+        if (e == cudaSuccess && h.nchunks > 0)
+            e = cudaMemcpyAsync(res, d_res, sizeof(res), cudaMemcpyDeviceToHost, s);
         if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-        const long long padded = (long long)total_blk * 128;
+        const long long padded = (long long)res[0] * 128;
         pava_status st = PAVA_SUCCESS;
         if (e != cudaSuccess) {
             st = fail_cuda(e, "SELL plan");
@@ -284,24 +297,23 @@ pava_status convert(pava::Handle &h, const int *rp, const int *ci, const double 
                           std::to_string(padded) + " for " + std::to_string(h.nnz) + " nonzeros)");
         } else if (padded >= (long long)INT_MAX - 64) {
             st = fail(PAVA_E_TOO_LARGE, "SELL: padded elements exceed the int32 element space");
+        } else if (res[1] && !auto_index) {
+            st = fail(PAVA_E_UNSUPPORTED_PARAMS,
+                      "16-bit column offsets: a slice's columns span more than 65534");
         } else {
+            if (res[1]) h.index_mode = PAVA_INDEX_I32;
+            const size_t si = h.index_mode == PAVA_INDEX_DELTA16 ? 2 : 4;
             h.n_aug = padded;
             e = budget_malloc(&h.vals, sv * (size_t)(padded ? padded : 1), &h.device_bytes, s);
             if (e == cudaSuccess)
                 e = budget_malloc(&h.cols, si * (size_t)(padded ? padded : 1), &h.device_bytes, s);
-            if (e == cudaSuccess && h.nchunks > 0) e = pava::sell_fill(h, rp, ci, v, d_off, d_ovf, s);
-            if (e == cudaSuccess) e = cudaMemcpyAsync(&ovf, d_ovf, sizeof(int), cudaMemcpyDeviceToHost, s);
+            if (e == cudaSuccess && h.nchunks > 0) e = pava::sell_fill(h, rp, ci, v, d_off, s);
             if (e == cudaSuccess) e = cudaStreamSynchronize(s);
             if (e != cudaSuccess) st = fail_cuda(e, "SELL conversion");
         }
         pava::pool_free(d_off, s);
-        pava::pool_free(d_tot, s);
-        pava::pool_free(d_ovf, s);
+        pava::pool_free(d_res, s);
         if (st != PAVA_SUCCESS) return st;
-        h.d16_overflow = ovf ? 1 : 0;
-        if (ovf)
-            return fail(PAVA_E_UNSUPPORTED_PARAMS,
-                        "16-bit column offsets: a slice's columns span more than 65534");
     } else {  // plain CSR: private copies (values narrowed to float for FP32C)
         PAVA_CUDA(dalloc(&h.rp, (size_t)h.m + 1, &h.device_bytes, s), "cudaMalloc(rp)");
         PAVA_CUDA(dalloc(&h.ci, (size_t)h.nnz, &h.device_bytes, s), "cudaMalloc(ci)");
@@ -592,35 +604,43 @@ pava_status pava_create(const pava_csr *A, int format, const pava_opts *opts, vo
         if (ce != cudaSuccess) { cleanup_tmp(); give_back(); return fail_cuda(ce, "copying the CSR to the device"); }
         rp = t_rp; ci = t_ci; v = t_v;
     }
-    // validation
-    {
-        int *d_err = nullptr;
-        int herr = 0;
-        ce = pava::pool_malloc(&d_err, 1, s);
-        if (ce == cudaSuccess) ce = pava::launch_validate(rp, ci, h.m, h.n, h.nnz, d_err, s);
-        if (ce == cudaSuccess) ce = cudaMemcpyAsync(&herr, d_err, sizeof(int), cudaMemcpyDeviceToHost, s);
-        if (ce == cudaSuccess) ce = cudaStreamSynchronize(s);
-        pava::pool_free(d_err, s);
-        if (ce != cudaSuccess) { cleanup_tmp(); give_back(); return fail_cuda(ce, "CSR validation"); }
-        if (herr) {
-            cleanup_tmp();
-            give_back();
-            return fail(PAVA_E_INVALID_CSR, "row_ptr not monotone, row_ptr[0]/row_ptr[m] wrong, or column out of range (" +
-                                                std::to_string(herr) + " violations)");
-        }
-    }
+    // validation and, for the chunked forms, the augmented row pointer (it reads row_ptr alone and
+    // is only used once that is known to be sound): one wait for both
     cudaEvent_t e0 = nullptr, e1 = nullptr;
     cudaEventCreate(&e0);
     cudaEventCreate(&e1);
-    cudaEventRecord(e0, s);
-    st = convert(h, rp, ci, v, s);
-    if (st == PAVA_E_UNSUPPORTED_PARAMS && auto_index && h.d16_overflow) {
-        // a column does not fit 16 bits: convert again with 32-bit columns
-        free_handle_buffers(h, s);
-        h.device_bytes = 0;
-        h.index_mode = PAVA_INDEX_I32;
-        st = convert(h, rp, ci, v, s);
+    auto drop_events = [&]() {
+        cudaEventDestroy(e0);
+        cudaEventDestroy(e1);
+    };
+    int *d_chk = nullptr, chk[2] = {0, 0};  // violations, empty rows
+    {
+        ce = pava::pool_malloc(&d_chk, 2, s);
+        if (ce == cudaSuccess) ce = pava::launch_validate(rp, ci, h.m, h.n, h.nnz, d_chk, s);
+        cudaEventRecord(e0, s);
+        const bool chunked = format == PAVA_FORMAT_CVR || format == PAVA_FORMAT_CSR5;
+        if (ce == cudaSuccess && chunked) ce = dalloc(&h.arp, (size_t)h.m + 2, &h.device_bytes, s);
+        if (ce == cudaSuccess && chunked)
+            ce = pava::build_augmented_rowptr(rp, h.m, h.arp, d_chk + 1, s);
+        if (ce == cudaSuccess)
+            ce = cudaMemcpyAsync(chk, d_chk, sizeof(int) * (chunked ? 2 : 1), cudaMemcpyDeviceToHost, s);
+        if (ce == cudaSuccess) ce = cudaStreamSynchronize(s);
+        pava::pool_free(d_chk, s);
+        if (ce != cudaSuccess) {
+            drop_events();
+            cleanup_tmp();
+            give_back();
+            return fail_cuda(ce, "CSR validation");
+        }
+        if (chk[0]) {
+            drop_events();
+            cleanup_tmp();
+            give_back();
+            return fail(PAVA_E_INVALID_CSR, "row_ptr not monotone, row_ptr[0]/row_ptr[m] wrong, or column out of range (" +
+                                                std::to_string(chk[0]) + " violations)");
+        }
     }
+    st = convert(h, rp, ci, v, chk[1], auto_index, s);
     if (st == PAVA_SUCCESS) {
         cudaEventRecord(e1, s);
         ce = cudaEventSynchronize(e1);
@@ -629,8 +649,7 @@ pava_status pava_create(const pava_csr *A, int format, const pava_opts *opts, vo
         if (ce != cudaSuccess) st = fail_cuda(ce, "conversion");
         h.convert_ms = ms;
     }
-    cudaEventDestroy(e0);
-    cudaEventDestroy(e1);
+    drop_events();
     cleanup_tmp();
     if (st != PAVA_SUCCESS) {
         give_back();

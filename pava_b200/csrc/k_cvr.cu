@@ -49,52 +49,56 @@ __device__ __forceinline__ RowSrc row_src(const int *rp, const int *arp, int m, 
     return r;
 }
 
-template <typename IT> __device__ __forceinline__ IT encode_col(int col, int base, int *ovf);
-template <> __device__ __forceinline__ int encode_col<int>(int col, int, int *) { return col; }
-template <> __device__ __forceinline__ short encode_col<short>(int col, int base, int *ovf) {
-    if (col < 0) return DELTA_NONE;
-    const int d = col - base;
-    if (d < -32767 || d > 32767) { atomicOr(ovf, 1); return DELTA_NONE; }
-    return (short)d;
-}
-
 template <typename VT, typename IT>
 __device__ __forceinline__ void put_elem(VT *vals, IT *cols, long long cbase, int i, int lane,
                                          const int *ci, const double *v, int e, RowSrc src,
-                                         int col_base, int *ovf) {
+                                         int col_base) {
     double val = 0.0;
-    int col = -1;
+    IT col = sizeof(IT) == 2 ? (IT)DELTA_NONE : (IT)-1;
     if (!src.dummy) {
         val = v[e + src.base];
-        col = ci[e + src.base];
+        col = (IT)(ci[e + src.base] - (sizeof(IT) == 2 ? col_base : 0));
     }
     vals[cbase + vals_offset<VT>(i, lane)] = (VT)val;
-    cols[cbase + cols_offset(i, lane)] = encode_col<IT>(col, col_base, ovf);
+    cols[cbase + cols_offset(i, lane)] = col;
 }
 
+// A warp per chunk, its lanes walking the CSR along their own rows.  Bound by the latency of the S
+// dependent steps of a walk and its scattered reads (64 L1 wavefronts per step), which many
+// resident warps hide: staging the chunk's CSR range in shared memory first left 8-16 warps per
+// SM and was slower (908 against 722 us for 66 M power-law nonzeros, S = 64, 32-bit columns).
 constexpr int CONV_WARPS = 4;
 
 template <typename VT, typename IT>
 __global__ void __launch_bounds__(CONV_WARPS * 32)
 cvr_convert_kernel(const int *__restrict__ rp, const int *__restrict__ ci,
                    const double *__restrict__ v, const int *__restrict__ arp, int m,
-                   long long nchunks, int S, VT *__restrict__ vals, IT *__restrict__ cols,
-                   unsigned *__restrict__ flags, CvrMeta *__restrict__ meta,
-                   const int *__restrict__ colbase, int *ovf) {
+                   long long nchunks, int S, const int *__restrict__ first,
+                   VT *__restrict__ vals, IT *__restrict__ cols, unsigned *__restrict__ flags,
+                   CvrMeta *__restrict__ meta, const int *__restrict__ colbase,
+                   const int *__restrict__ ovf) {
     __shared__ int s_len[CONV_WARPS][64];
     __shared__ int s_src[CONV_WARPS][64];
     __shared__ int s_row[CONV_WARPS][64];
     __shared__ int s_off[CONV_WARPS][65];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const long long c = (long long)blockIdx.x * CONV_WARPS + w;
-    if (c >= nchunks) return;  // warp-uniform
+    if (c >= nchunks) return;  // warp-uniform: no block-wide barrier below
+    if (sizeof(IT) == 2 && *ovf) return;
     const long long L = 32LL * S;
     const long long s = c * L, e = s + L;
-    const int nr = m + 2;  // arp entries (rows 0..m, m = padding row)
-    const int r_first = upper_bound_m1(arp, nr, s);
-    const int r_last = upper_bound_m1(arp, nr, e - 1);
-    const int nrows = r_last - r_first + 1;
+    const int r_first = first[c];
     const int col_base = sizeof(IT) == 2 ? colbase[c] : 0;  // of the 16-bit offsets
+    // the row that holds element e - 1: the one before the next chunk's first row, unless that
+    // row runs across the boundary; the last chunk ends in its padding (row m), if it has any
+    int r_last;
+    if (c + 1 < nchunks) {
+        r_last = first[c + 1];
+        if ((long long)arp[r_last] == e) --r_last;
+    } else {
+        r_last = (long long)arp[m] == e ? m - 1 : m;
+    }
+    const int nrows = r_last - r_first + 1;
     const unsigned lt = lanemask_lt();
 
     int g = lane, row = -1, cur = 0, rem = 0;
@@ -123,7 +127,7 @@ cvr_convert_kernel(const int *__restrict__ rp, const int *__restrict__ ci,
             }
             next_g += __popc(b);
         }
-        put_elem<VT, IT>(vals, cols, s, i, lane, ci, v, cur, src, col_base, ovf);
+        put_elem<VT, IT>(vals, cols, s, i, lane, ci, v, cur, src, col_base);
         ++cur;
         --rem;
         if (rem == 0) fword |= 1u << (i & 31);
@@ -180,7 +184,7 @@ cvr_convert_kernel(const int *__restrict__ rp, const int *__restrict__ ci,
         int slen = s_len[w][j], sa = s_src[w][j];
         src = row_src(rp, arp, m, s_row[w][j]);
         for (int t = 0; t < T; ++t, ++i) {
-            put_elem<VT, IT>(vals, cols, s, i, lane, ci, v, sa + off, src, col_base, ovf);
+            put_elem<VT, IT>(vals, cols, s, i, lane, ci, v, sa + off, src, col_base);
             ++off;
             const bool slot_end = (off == slen);
             if (slot_end || t == T - 1) fword |= 1u << (i & 31);
@@ -367,11 +371,11 @@ cvr_spmv_kernel(const CvrMeta *__restrict__ meta, const unsigned *__restrict__ f
 }
 
 template <typename VT, typename IT>
-cudaError_t convert_t(Handle &h, const int *rp, const int *ci, const double *v, int *ovf,
-                      cudaStream_t s) {
+cudaError_t convert_t(Handle &h, const int *rp, const int *ci, const double *v, const int *first,
+                      const int *ovf, cudaStream_t s) {
     const long long blocks = (h.nchunks + CONV_WARPS - 1) / CONV_WARPS;
     cvr_convert_kernel<VT, IT><<<(unsigned)blocks, CONV_WARPS * 32, 0, s>>>(
-        rp, ci, v, h.arp, h.m, h.nchunks, h.S, (VT *)h.vals, (IT *)h.cols, h.flags,
+        rp, ci, v, h.arp, h.m, h.nchunks, h.S, first, (VT *)h.vals, (IT *)h.cols, h.flags,
         (CvrMeta *)h.meta, h.colbase, ovf);
     return cudaGetLastError();
 }
@@ -408,14 +412,14 @@ cudaError_t spmv_t(const Handle &h, const void *x, void *y, cudaStream_t s) {
 
 }  // namespace
 
-cudaError_t cvr_convert(Handle &h, const int *rp, const int *ci, const double *v, int *ovf,
-                        cudaStream_t s) {
+cudaError_t cvr_convert(Handle &h, const int *rp, const int *ci, const double *v, const int *first,
+                        const int *ovf, cudaStream_t s) {
     if (h.nchunks <= 0) return cudaSuccess;
     const bool f32 = h.precision == PAVA_PREC_FP32C, d16 = h.index_mode == PAVA_INDEX_DELTA16;
-    if (!f32 && !d16) return convert_t<double, int>(h, rp, ci, v, ovf, s);
-    if (!f32 && d16) return convert_t<double, short>(h, rp, ci, v, ovf, s);
-    if (f32 && !d16) return convert_t<float, int>(h, rp, ci, v, ovf, s);
-    return convert_t<float, short>(h, rp, ci, v, ovf, s);
+    if (!f32 && !d16) return convert_t<double, int>(h, rp, ci, v, first, ovf, s);
+    if (!f32 && d16) return convert_t<double, short>(h, rp, ci, v, first, ovf, s);
+    if (f32 && !d16) return convert_t<float, int>(h, rp, ci, v, first, ovf, s);
+    return convert_t<float, short>(h, rp, ci, v, first, ovf, s);
 }
 
 cudaError_t cvr_spmv(const Handle &h, const void *x, void *y, cudaStream_t s) {

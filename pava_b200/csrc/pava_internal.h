@@ -71,7 +71,6 @@ struct Handle {
 
     double convert_ms = 0.0;
     size_t device_bytes = 0;
-    int d16_overflow = 0;    // the last conversion found a column outside the 16-bit range
 };
 
 // Device memory of handles, conversions and their temporaries: a memory pool per device (and
@@ -126,19 +125,26 @@ inline int csr5_wave_tiles(long long tiles, long long warps) {
 // Kernel launchers (stream-ordered; return cudaGetLastError()).
 cudaError_t launch_validate(const int *rp, const int *ci, int m, int n, int nnz, int *d_err,
                             cudaStream_t s);
-cudaError_t build_augmented_rowptr(const int *rp, int m, long long padded_total, int *arp,
-                                   int *d_nempty, cudaStream_t s);
+// arp[0..m]; arp[m + 1], the padded total, is the caller's (set_int).
+cudaError_t build_augmented_rowptr(const int *rp, int m, int *arp, int *d_nempty, cudaStream_t s);
+cudaError_t set_int(int *p, int v, cudaStream_t s);
+// rows[t] = row of augmented element t*T, t in [0, count) (arp complete).
+cudaError_t chunk_rows(const int *arp, int m, long long T, long long count, int *rows,
+                       cudaStream_t s);
 
 // DELTA16 base column of every warp chunk (h.colbase): the midpoint of the chunk's smallest
-// and largest column.
-cudaError_t chunk_colbase(const Handle &h, const int *rp, const int *ci, cudaStream_t s);
+// and largest column; *ovf is set to 1 when a chunk's columns span too much for 16-bit offsets.
+// first[c * stride]: row of chunk c's first element.
+cudaError_t chunk_colbase(const Handle &h, const int *rp, const int *ci, const int *first,
+                          int stride, int *ovf, cudaStream_t s);
 
-// Conversions set *ovf (device) to 1 when a 16-bit column offset does not fit.
-cudaError_t cvr_convert(Handle &h, const int *rp, const int *ci, const double *v, int *ovf,
-                        cudaStream_t s);
+// Conversions.  With 16-bit offsets they do nothing when *ovf (device) is set.  first: CVR, the
+// row of each chunk's first element; CSR5, h.tile_ptr is complete.
+cudaError_t cvr_convert(Handle &h, const int *rp, const int *ci, const double *v, const int *first,
+                        const int *ovf, cudaStream_t s);
 cudaError_t cvr_spmv(const Handle &h, const void *x, void *y, cudaStream_t s);
 
-cudaError_t csr5_convert(Handle &h, const int *rp, const int *ci, const double *v, int *ovf,
+cudaError_t csr5_convert(Handle &h, const int *rp, const int *ci, const double *v, const int *ovf,
                          cudaStream_t s);
 cudaError_t csr5_spmv(const Handle &h, const void *x, void *y, cudaStream_t s);
 
@@ -146,11 +152,12 @@ cudaError_t carry_fixup(const Handle &h, void *y, cudaStream_t s);
 
 // SELL: sell_plan fills the slice descriptors (h.meta, h.nchunks slices) except their offsets
 // and writes the exclusive scan of the slices' block counts to d_blk_off[0..nslices], the total
-// to *d_total_blk; sell_fill writes the padded streams and the offsets.
-cudaError_t sell_plan(Handle &h, const int *rp, const int *ci, int *d_blk_off, int *d_total_blk,
-                      cudaStream_t s);
+// to d_res[0], and 1 to d_res[1] when want_base and a slice's columns span too much for 16-bit
+// offsets (0 otherwise); sell_fill writes the padded streams and the offsets.
+cudaError_t sell_plan(Handle &h, const int *rp, const int *ci, bool want_base, int *d_blk_off,
+                      int *d_res, cudaStream_t s);
 cudaError_t sell_fill(Handle &h, const int *rp, const int *ci, const double *v,
-                      const int *d_blk_off, int *ovf, cudaStream_t s);
+                      const int *d_blk_off, cudaStream_t s);
 cudaError_t sell_spmv(const Handle &h, const void *x, void *y, cudaStream_t s);
 // SELL SpMM, Y = A X with X row-major n x k; leading dimensions ldx, ldy in elements.  Lanes per
 // row (h.lanes_per_row): 4 (k <= 32), 8 (k <= 64) or 16 (k <= 64); 0 = 4 for k <= 16, else 8.
