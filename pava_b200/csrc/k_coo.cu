@@ -2,12 +2,17 @@
 // symmetric expansion and 1-based shift, utils/basicMatrix.cpp:63-253, and convertCOO2CSR,
 // :350-415, which calls MKL's mkl_dcsrcoo there).
 //
-// Entries are keyed (row << 32 | column) and sorted by a stable LSD radix sort (cub), so rows
-// and the columns inside a row come out ascending and duplicates stay as separate entries in
+// Rows and the columns inside a row come out ascending and duplicates stay as separate entries in
 // input order -- the same result as the host conversion, pava_coo_to_csr.  With `symmetric`,
-// every off-diagonal entry (r, c) also yields (c, r), as a symmetric Matrix Market file
-// stores one triangle.  The row pointer is then read off the sorted keys: element j writes
-// rp[r] = j for every row r in (row[j-1], row[j]].
+// every off-diagonal entry (r, c) also yields (c, r), as a symmetric Matrix Market file stores
+// one triangle; among equal (row, column) the entries come before the mirrored ones.
+//
+// The entries are bucketed by row (count, scan, scatter) and each row is sorted by (column,
+// mirrored, input position), which are all different, so the result does not depend on the order
+// in which the scatter's atomics ran.  Against one stable radix sort of (row << 32 | column) with
+// its values -- 7 passes of 32 bytes per entry -- an entry is written and read once as a 16-byte
+// record: 80^3 stencil from its triangle (6.9 M entries, 13.6 M nonzeros) 1.50 -> 0.30 ms of
+// kernels.
 
 #include <string.h>
 
@@ -19,62 +24,198 @@ namespace pava {
 
 namespace {
 
-unsigned grid_of(long long work) {
+unsigned grid_of(long long work, long long cap) {
     long long b = (work + 255) / 256;
     if (b < 1) b = 1;
-    if (b > 16384) b = 16384;
+    if (b > cap) b = cap;
     return (unsigned)b;
 }
 
-// flag[k] = 1 for an off-diagonal entry when mirroring; counts indices out of range.
-__global__ void coo_flags_kernel(const int *__restrict__ rows, const int *__restrict__ cols,
-                                 long long nnz, int base, int m, int n, int symmetric,
-                                 int *__restrict__ flag, int *__restrict__ bad) {
-    const long long stride = (long long)gridDim.x * blockDim.x;
-    int nb = 0;
-    for (long long k = (long long)blockIdx.x * blockDim.x + threadIdx.x; k < nnz; k += stride) {
-        const int r = rows[k] - base, c = cols[k] - base;
-        const bool ok = r >= 0 && r < m && c >= 0 && c < n && (!symmetric || (c < m && r < n));
-        nb += !ok;
-        flag[k] = (ok && symmetric && r != c) ? 1 : 0;
+struct CooStat {
+    unsigned long long mirrored;    // entries the symmetric expansion adds
+    unsigned long long long_total;  // nonzeros in rows longer than RANK_MAX
+    int bad, nlong;                 // entries outside the matrix, rows longer than RANK_MAX
+};
+
+// A record of the scatter: key = column << 32 | mirrored << 31 | input position, and the value.
+struct CooRec {
+    unsigned long long key;
+    double val;
+};
+
+// Adds `on` lanes' counts to their rows' counters, one atomic per run of equal rows in
+// neighbouring lanes (sorted inputs have long ones), and returns the lane's slot.  All 32 lanes.
+__device__ __forceinline__ int run_add(int *cnt, int row, bool on, int lane) {
+    const int left = __shfl_up_sync(FULL, row, 1);
+    const unsigned act = __ballot_sync(FULL, on);
+    const bool lead = on && (lane == 0 || !((act >> (lane - 1)) & 1u) || left != row);
+    const unsigned leads = __ballot_sync(FULL, lead);
+    // a run ends before the next leader or the next inactive lane
+    int base = 0, src = lane;
+    if (on) src = 31 - __clz(leads & (0xffffffffu >> (31 - lane)));
+    if (lead) {
+        const unsigned stop = (leads | ~act) & ~(0xffffffffu >> (31 - lane));
+        const int end = stop ? __ffs(stop) - 1 : 32;
+        base = atomicAdd(&cnt[row], end - lane);
     }
-    if (nb) atomicAdd(bad, nb);
+    base = __shfl_sync(FULL, base, src);
+    return base + (lane - src);
 }
 
-__global__ void coo_keys_kernel(const int *__restrict__ rows, const int *__restrict__ cols,
-                                const double *__restrict__ vals, long long nnz, int base,
-                                const int *__restrict__ mirror_pos, int symmetric,
-                                unsigned long long *__restrict__ keys, double *__restrict__ v) {
+// Entries per row (mirrored ones included); counts indices out of range.
+__global__ void __launch_bounds__(256)
+coo_count_kernel(const int *__restrict__ rows, const int *__restrict__ cols, long long nnz,
+                 int base, int m, int n, int symmetric, int *__restrict__ cnt,
+                 CooStat *__restrict__ st) {
+    const int lane = threadIdx.x & 31;
     const long long stride = (long long)gridDim.x * blockDim.x;
-    for (long long k = (long long)blockIdx.x * blockDim.x + threadIdx.x; k < nnz; k += stride) {
-        const unsigned long long r = (unsigned)(rows[k] - base), c = (unsigned)(cols[k] - base);
-        keys[k] = (r << 32) | c;
-        v[k] = vals[k];
-        if (symmetric && r != c) {
-            const long long q = nnz + mirror_pos[k];
-            keys[q] = (c << 32) | r;
-            v[q] = vals[k];
+    int nb = 0, nm = 0;
+    for (long long k0 = (long long)blockIdx.x * blockDim.x + (threadIdx.x & ~31); k0 < nnz;
+         k0 += stride) {
+        const long long k = k0 + lane;
+        const bool in = k < nnz;
+        const long long r = in ? (long long)rows[k] - base : -1, c = in ? (long long)cols[k] - base : -1;
+        const bool ok = r >= 0 && r < m && c >= 0 && c < n && (!symmetric || (c < m && r < n));
+        nb += in && !ok;
+        run_add(cnt, (int)r, ok, lane);
+        if (symmetric) {
+            const bool mir = ok && r != c;
+            nm += mir;
+            run_add(cnt, (int)c, mir, lane);
+        }
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        nb += __shfl_xor_sync(FULL, nb, o);
+        nm += __shfl_xor_sync(FULL, nm, o);
+    }
+    // one atomic per block: all of them go to the same address
+    __shared__ int s_bad, s_mir;
+    if (threadIdx.x == 0) s_bad = s_mir = 0;
+    __syncthreads();
+    if (lane == 0 && nb) atomicAdd(&s_bad, nb);
+    if (lane == 0 && nm) atomicAdd(&s_mir, nm);
+    __syncthreads();
+    if (threadIdx.x == 0 && s_bad) atomicAdd(&st->bad, s_bad);
+    if (threadIdx.x == 0 && s_mir) atomicAdd(&st->mirrored, (unsigned long long)s_mir);
+}
+
+// Rows are sorted by counting, for each entry, the smaller keys of its row: up to RANK_MAX
+// entries.  Longer rows (listed here) are sorted by cub's segmented sort.
+constexpr int RANK_MAX = 256;
+__global__ void coo_long_kernel(const int *__restrict__ cnt, int m, CooStat *__restrict__ st,
+                                const int *__restrict__ rp, int *__restrict__ row,
+                                int *__restrict__ begin, int *__restrict__ end) {
+    const long long r = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (r >= m) return;
+    const int len = cnt ? cnt[r] : rp[r + 1] - rp[r];
+    if (len <= RANK_MAX) return;
+    const int q = atomicAdd(&st->nlong, 1);
+    const unsigned long long off = atomicAdd(&st->long_total, (unsigned long long)len);
+    if (row) {
+        row[q] = (int)r;
+        begin[q] = (int)off;
+        end[q] = (int)off + len;
+    }
+}
+
+// Entry k into the next free slot of its row (cur: the rows' cursors, starting at rp).
+__global__ void __launch_bounds__(256)
+coo_scatter_kernel(const int *__restrict__ rows, const int *__restrict__ cols,
+                   const double *__restrict__ vals, long long nnz, int base, int symmetric,
+                   int *__restrict__ cur, CooRec *__restrict__ rec) {
+    const int lane = threadIdx.x & 31;
+    const long long stride = (long long)gridDim.x * blockDim.x;
+    for (long long k0 = (long long)blockIdx.x * blockDim.x + (threadIdx.x & ~31); k0 < nnz;
+         k0 += stride) {
+        const long long k = k0 + lane;
+        const bool in = k < nnz;
+        const int r = in ? rows[k] - base : -1, c = in ? cols[k] - base : -1;
+        const double v = in ? vals[k] : 0.0;
+        auto put = [&](int at, int col, unsigned tie) {
+            const unsigned long long key = ((unsigned long long)(unsigned)col << 32) | tie;
+            *reinterpret_cast<ulonglong2 *>(rec + at) =
+                make_ulonglong2(key, (unsigned long long)__double_as_longlong(v));
+        };
+        const int at = run_add(cur, r, in, lane);
+        if (in) put(at, c, (unsigned)k);
+        if (symmetric) {
+            const bool mir = in && r != c;
+            const int at2 = run_add(cur, c, mir, lane);
+            if (mir) put(at2, r, (unsigned)k | 0x80000000u);
         }
     }
 }
 
-// Row pointer and columns from the sorted keys; j = total stands for a virtual element of
-// row m, which closes every remaining row.
-__global__ void coo_rowptr_kernel(const unsigned long long *__restrict__ keys, long long total,
-                                  int m, int *__restrict__ rp, int *__restrict__ ci) {
-    const long long stride = (long long)gridDim.x * blockDim.x;
-    for (long long j = (long long)blockIdx.x * blockDim.x + threadIdx.x; j <= total; j += stride) {
-        const long long row = j < total ? (long long)(keys[j] >> 32) : m;
-        const long long prev = j > 0 ? (long long)(keys[j - 1] >> 32) : -1;
-        for (long long r = prev + 1; r <= row; ++r) rp[r] = (int)j;
-        if (j < total) ci[j] = (int)(keys[j] & 0xffffffffull);
+// A warp per 32 rows, in batches of whole rows of at most CAP entries: keys in shared memory, an
+// entry's place in its row is the number of smaller keys there.  Bound by the shared-memory reads
+// (row length per entry) and the bytes (16 read, 12 written).
+constexpr int SORT_WARPS = 4, CAP = 512;
+static_assert(RANK_MAX <= CAP, "a row fits a batch");
+__global__ void __launch_bounds__(SORT_WARPS * 32)
+coo_sort_kernel(const int *__restrict__ rp, int m, const CooRec *__restrict__ rec,
+                int *__restrict__ ci, double *__restrict__ v) {
+    __shared__ unsigned long long s_key[SORT_WARPS][CAP];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const long long r = ((long long)blockIdx.x * SORT_WARPS + w) * 32 + lane;
+    if (r - lane >= m) return;  // warp-uniform: no block-wide barrier below
+    const int s = rp[r < m ? r : m], e = rp[r < m ? r + 1 : m];
+    const bool is_long = e - s > RANK_MAX;
+    unsigned long long *key = s_key[w];
+    int i = 0;
+    while (i < 32) {  // rows [i, j) of the 32
+        const int base = __shfl_sync(FULL, s, i);
+        const unsigned stop = __ballot_sync(FULL, lane >= i && (is_long || e - base > CAP));
+        const int j = stop ? __ffs(stop) - 1 : 32;
+        if (j == i) {  // a long row
+            ++i;
+            continue;
+        }
+        const int n = __shfl_sync(FULL, e, j - 1) - base;
+        for (int q = lane; q < n; q += 32) key[q] = rec[base + q].key;
+        __syncwarp();
+        for (int q0 = 0; q0 < n; q0 += 32) {
+            const int q = q0 + lane < n ? q0 + lane : n - 1;
+            int row = i;  // the last row of the batch that starts at or before q
+#pragma unroll
+            for (int d = 16; d > 0; d >>= 1) {
+                const int t = row + d;
+                const int st = __shfl_sync(FULL, s, t & 31) - base;
+                if (t < j && st <= q) row = t;
+            }
+            const int a = __shfl_sync(FULL, s, row) - base, b = __shfl_sync(FULL, e, row) - base;
+            const unsigned long long mine = key[q];
+            int rank = 0;
+#pragma unroll 4
+            for (int t = a; t < b; ++t) rank += key[t] < mine;
+            if (q0 + lane < n) {
+                ci[base + a + rank] = (int)(mine >> 32);
+                v[base + a + rank] = rec[base + q].val;
+            }
+        }
+        __syncwarp();  // the next batch overwrites the keys
+        i = j;
     }
 }
 
-int key_bits(int m) {
-    int b = 0;
-    while ((1ll << b) < (long long)m + 1) ++b;
-    return 32 + b;
+// Long rows: keys out to a packed array, and the sorted keys back as columns and values.
+__global__ void coo_long_pack_kernel(const int *__restrict__ rp, const int *__restrict__ row,
+                                     const int *__restrict__ begin, const CooRec *__restrict__ rec,
+                                     unsigned long long *__restrict__ keys) {
+    const int r = row[blockIdx.x], a = rp[r], len = rp[r + 1] - a, o = begin[blockIdx.x];
+    for (int t = threadIdx.x; t < len; t += blockDim.x) keys[o + t] = rec[a + t].key;
+}
+__global__ void coo_long_unpack_kernel(const int *__restrict__ rp, const int *__restrict__ row,
+                                       const int *__restrict__ begin,
+                                       const unsigned long long *__restrict__ keys,
+                                       const double *__restrict__ vals, int *__restrict__ ci,
+                                       double *__restrict__ v) {
+    const int r = row[blockIdx.x], a = rp[r], len = rp[r + 1] - a, o = begin[blockIdx.x];
+    for (int t = threadIdx.x; t < len; t += blockDim.x) {
+        const unsigned long long key = keys[o + t];
+        ci[a + t] = (int)(key >> 32);
+        v[a + t] = vals[key & 0x7fffffffull];
+    }
 }
 
 }  // namespace
@@ -95,9 +236,11 @@ extern "C" pava_status pava_coo_to_csr_device(int m, int n, long long nnz, const
     }
     if (nnz > 2147483000LL) { set_last_error("more than 2^31 entries"); return PAVA_E_TOO_LARGE; }
     cudaStream_t s = (cudaStream_t)stream;
-    int *flag = nullptr, *mpos = nullptr, *d_bad = nullptr, *rp = nullptr, *ci = nullptr;
-    unsigned long long *keys = nullptr, *keys2 = nullptr;
-    double *v = nullptr, *v2 = nullptr;
+    int *cnt = nullptr, *cur = nullptr, *rp = nullptr, *ci = nullptr, *seg = nullptr;
+    CooStat *d_st = nullptr;
+    CooRec *rec = nullptr;
+    unsigned long long *keys = nullptr;
+    double *v = nullptr;
     void *tmp = nullptr;
     cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
     cudaError_t e = cudaStreamIsCapturing(s, &capturing);
@@ -105,77 +248,101 @@ extern "C" pava_status pava_coo_to_csr_device(int m, int n, long long nnz, const
         e = cudaErrorStreamCaptureUnsupported;
     const size_t held = pool_reserved();
     auto cleanup = [&]() {
-        pool_free(flag, s); pool_free(mpos, s); pool_free(d_bad, s); pool_free(keys, s);
-        pool_free(keys2, s); pool_free(v, s); pool_free(tmp, s);
+        pool_free(cnt, s); pool_free(cur, s); pool_free(seg, s); pool_free(d_st, s);
+        pool_free(rec, s); pool_free(keys, s); pool_free(tmp, s);
     };
-    auto fail_e = [&](cudaError_t e) {
+    auto give_back = [&]() {
         cleanup();
-        pool_free(rp, s); pool_free(ci, s); pool_free(v2, s);
+        pool_free(rp, s); pool_free(ci, s); pool_free(v, s);
         cudaStreamSynchronize(s);
         pool_trim(held);
-        set_last_error(std::string("COO -> CSR: ") + cudaGetErrorString(e));
-        return e == cudaErrorMemoryAllocation ? PAVA_E_NOMEM : PAVA_E_CUDA;
     };
-    const size_t nz = (size_t)(nnz ? nnz : 1);
+    auto fail_e = [&](cudaError_t err) {
+        give_back();
+        set_last_error(std::string("COO -> CSR: ") + cudaGetErrorString(err));
+        return err == cudaErrorMemoryAllocation ? PAVA_E_NOMEM : PAVA_E_CUDA;
+    };
     if (e != cudaSuccess) return fail_e(e);  // it allocates and waits
-    e = pool_malloc(&flag, nz, s);
-    if (e == cudaSuccess) e = pool_malloc(&mpos, nz, s);
-    if (e == cudaSuccess) e = pool_malloc(&d_bad, 2, s);
-    if (e == cudaSuccess) e = cudaMemsetAsync(d_bad, 0, sizeof(int) * 2, s);
+    // entries per row -> row pointer
+    e = pool_malloc(&cnt, (size_t)m + 1, s);
+    if (e == cudaSuccess) e = pool_malloc(&rp, (size_t)m + 1, s);
+    if (e == cudaSuccess) e = pool_malloc(&d_st, 1, s);
+    if (e == cudaSuccess) e = cudaMemsetAsync(cnt, 0, sizeof(int) * ((size_t)m + 1), s);
+    if (e == cudaSuccess) e = cudaMemsetAsync(d_st, 0, sizeof(CooStat), s);
     if (e == cudaSuccess && nnz > 0) {
-        coo_flags_kernel<<<grid_of(nnz), 256, 0, s>>>(rows, cols, nnz, index_base, m, n,
-                                                      symmetric, flag, d_bad);
+        coo_count_kernel<<<grid_of(nnz, 148 * 16), 256, 0, s>>>(rows, cols, nnz, index_base, m, n, symmetric,
+                                                      cnt, d_st);
+        e = cudaGetLastError();
+    }
+    const unsigned row_blocks = (unsigned)(((long long)m + 255) / 256);
+    if (e == cudaSuccess && m > 0) {
+        coo_long_kernel<<<row_blocks, 256, 0, s>>>(cnt, m, d_st, nullptr, nullptr, nullptr, nullptr);
         e = cudaGetLastError();
     }
     size_t tb = 0;
-    if (e == cudaSuccess && nnz > 0) e = cub::DeviceScan::ExclusiveSum(nullptr, tb, flag, mpos, (int)nnz, s);
-    if (e == cudaSuccess && nnz > 0) e = pool_malloc(&tmp, tb, s);
-    if (e == cudaSuccess && nnz > 0) e = cub::DeviceScan::ExclusiveSum(tmp, tb, flag, mpos, (int)nnz, s);
-    if (e == cudaSuccess && nnz > 0)  // mirrored count = mpos[last] + flag[last]
-        e = cub::DeviceReduce::Sum(nullptr, tb, flag, d_bad + 1, (int)nnz, s);
-    pool_free(tmp, s);
-    tmp = nullptr;
-    if (e == cudaSuccess && nnz > 0) e = pool_malloc(&tmp, tb, s);
-    if (e == cudaSuccess && nnz > 0) e = cub::DeviceReduce::Sum(tmp, tb, flag, d_bad + 1, (int)nnz, s);
-    int h[2] = {0, 0};
-    if (e == cudaSuccess) e = cudaMemcpyAsync(h, d_bad, sizeof(h), cudaMemcpyDeviceToHost, s);
+    if (e == cudaSuccess)
+        e = cub::DeviceScan::ExclusiveSum(nullptr, tb, cnt, rp, (long long)m + 1, s);
+    if (e == cudaSuccess) e = pool_malloc(&tmp, tb, s);
+    if (e == cudaSuccess)
+        e = cub::DeviceScan::ExclusiveSum(tmp, tb, cnt, rp, (long long)m + 1, s);
+    CooStat h = {};
+    if (e == cudaSuccess) e = cudaMemcpyAsync(&h, d_st, sizeof(h), cudaMemcpyDeviceToHost, s);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
     if (e != cudaSuccess) return fail_e(e);
-    if (h[0]) {
-        cleanup();
-        set_last_error("COO -> CSR: " + std::to_string(h[0]) + " entries outside the matrix");
+    if (h.bad) {
+        give_back();
+        set_last_error("COO -> CSR: " + std::to_string(h.bad) + " entries outside the matrix");
         return PAVA_E_INVALID_CSR;
     }
-    const long long total = nnz + h[1];
+    const long long total = nnz + (long long)h.mirrored;
     if (total > 2147483000LL) {
-        cleanup();
+        give_back();
         set_last_error("more than 2^31 entries after the symmetric expansion");
         return PAVA_E_TOO_LARGE;
     }
     const size_t tz = (size_t)(total ? total : 1);
-    e = pool_malloc(&keys, tz, s);
-    if (e == cudaSuccess) e = pool_malloc(&keys2, tz, s);
-    if (e == cudaSuccess) e = pool_malloc(&v, tz, s);
-    if (e == cudaSuccess) e = pool_malloc(&v2, tz, s);
-    if (e == cudaSuccess) e = pool_malloc(&rp, (size_t)m + 1, s);
     if (e == cudaSuccess) e = pool_malloc(&ci, tz, s);
-    if (e == cudaSuccess && nnz > 0) {
-        coo_keys_kernel<<<grid_of(nnz), 256, 0, s>>>(rows, cols, vals, nnz, index_base, mpos,
-                                                     symmetric, keys, v);
-        e = cudaGetLastError();
+    if (e == cudaSuccess) e = pool_malloc(&v, tz, s);
+    if (total > 0) {
+        if (e == cudaSuccess) e = pool_malloc(&rec, tz, s);
+        cur = cnt;  // the counts are in rp: their array becomes the rows' cursors
+        cnt = nullptr;
+        if (e == cudaSuccess)
+            e = cudaMemcpyAsync(cur, rp, sizeof(int) * (size_t)m, cudaMemcpyDeviceToDevice, s);
+        if (e == cudaSuccess) {
+            coo_scatter_kernel<<<grid_of(nnz, 16384), 256, 0, s>>>(rows, cols, vals, nnz, index_base,
+                                                            symmetric, cur, rec);
+            const long long warps = ((long long)m + 31) / 32;
+            coo_sort_kernel<<<(unsigned)((warps + SORT_WARPS - 1) / SORT_WARPS), SORT_WARPS * 32, 0,
+                              s>>>(rp, m, rec, ci, v);
+            e = cudaGetLastError();
+        }
     }
-    pool_free(tmp, s);
-    tmp = nullptr;
-    if (e == cudaSuccess && total > 0)
-        e = cub::DeviceRadixSort::SortPairs(nullptr, tb, keys, keys2, v, v2, (int)total, 0,
-                                            key_bits(m), s);
-    if (e == cudaSuccess && total > 0) e = pool_malloc(&tmp, tb, s);
-    if (e == cudaSuccess && total > 0)
-        e = cub::DeviceRadixSort::SortPairs(tmp, tb, keys, keys2, v, v2, (int)total, 0,
-                                            key_bits(m), s);
-    if (e == cudaSuccess) {
-        coo_rowptr_kernel<<<grid_of(total + 1), 256, 0, s>>>(keys2, total, m, rp, ci);
-        e = cudaGetLastError();
+    if (e == cudaSuccess && h.nlong > 0) {
+        const size_t nl = (size_t)h.nlong, lt = (size_t)h.long_total;
+        e = pool_malloc(&seg, 3 * nl, s);
+        if (e == cudaSuccess) e = pool_malloc(&keys, 2 * lt, s);
+        if (e == cudaSuccess) e = cudaMemsetAsync(d_st, 0, sizeof(CooStat), s);
+        if (e == cudaSuccess) {
+            coo_long_kernel<<<row_blocks, 256, 0, s>>>(nullptr, m, d_st, rp, seg, seg + nl,
+                                                       seg + 2 * nl);
+            coo_long_pack_kernel<<<(unsigned)nl, 256, 0, s>>>(rp, seg, seg + nl, rec, keys);
+            e = cudaGetLastError();
+        }
+        pool_free(tmp, s);
+        tmp = nullptr;
+        if (e == cudaSuccess)
+            e = cub::DeviceSegmentedSort::SortKeys(nullptr, tb, keys, keys + lt, (int)lt, (int)nl,
+                                                   seg + nl, seg + 2 * nl, s);
+        if (e == cudaSuccess) e = pool_malloc(&tmp, tb, s);
+        if (e == cudaSuccess)
+            e = cub::DeviceSegmentedSort::SortKeys(tmp, tb, keys, keys + lt, (int)lt, (int)nl,
+                                                   seg + nl, seg + 2 * nl, s);
+        if (e == cudaSuccess) {
+            coo_long_unpack_kernel<<<(unsigned)nl, 256, 0, s>>>(rp, seg, seg + nl, keys + lt, vals,
+                                                               ci, v);
+            e = cudaGetLastError();
+        }
     }
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
     if (e != cudaSuccess) return fail_e(e);
@@ -185,7 +352,7 @@ extern "C" pava_status pava_coo_to_csr_device(int m, int n, long long nnz, const
     out->nnz = (int)total;
     out->row_ptr = rp;
     out->col_idx = ci;
-    out->vals = v2;
+    out->vals = v;
     out->on_device = 1;
     return PAVA_SUCCESS;
 }
