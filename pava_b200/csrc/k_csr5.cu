@@ -232,8 +232,7 @@ csr5_spmv_kernel(const ChunkHdr *__restrict__ hdr, const int *__restrict__ tile_
                  double *__restrict__ carry_tail, long long nchunks, int G, int m, int n,
                  unsigned long long *err) {
     constexpr int NBT = SIGMA / 4;  // blocks per tile
-    // the carry fixup that follows may launch now; it waits for this grid to finish
-    asm volatile("griddepcontrol.launch_dependents;");
+    pdl_trigger();
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const uint64_t pf = policy_evict_first(), pl = policy_evict_last();
     const long long nwarps = (long long)gridDim.x * SPMV_WARPS;
@@ -263,6 +262,7 @@ csr5_spmv_kernel(const ChunkHdr *__restrict__ hdr, const int *__restrict__ tile_
         VT x0[4];
         {
             const CBlk<IT> c0 = CBlk<IT>::load(cb, 0, lane, pf);
+            pdl_wait();  // x, and y and the carries, which the product before may still use
 #pragma unroll
             for (int q = 0; q < 4; ++q) x0[q] = c0.gather(q, xb, pl, xlo, xhi, err);
         }
@@ -394,8 +394,7 @@ csr5_spmv_f32_kernel(const ChunkHdr *__restrict__ hdr, const int *__restrict__ t
                      unsigned long long *err) {
     using VT = float;
     constexpr int NBT = SIGMA / 4;  // blocks per tile
-    // the carry fixup that follows may launch now; it waits for this grid to finish
-    asm volatile("griddepcontrol.launch_dependents;");
+    pdl_trigger();
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const uint64_t pf = policy_evict_first(), pl = policy_evict_last();
     const long long nwarps = (long long)gridDim.x * SPMV_WARPS;
@@ -428,6 +427,7 @@ csr5_spmv_f32_kernel(const ChunkHdr *__restrict__ hdr, const int *__restrict__ t
         VT x0[4];
         {
             const CBlk<IT> c0 = CBlk<IT>::load(cb, 0, lane, pf);
+            pdl_wait();  // x, and y and the carries, which the product before may still use
 #pragma unroll
             for (int q = 0; q < 4; ++q) x0[q] = c0.gather(q, xb, pl, xlo, xhi, err);
         }
@@ -554,17 +554,15 @@ cudaError_t convert_t(Handle &h, const int *rp, const int *ci, const double *v, 
 }
 
 template <int SG, typename VT, typename IT>
-void launch_sg(const Handle &h, unsigned grid, const void *x, void *y, cudaStream_t s) {
-    if constexpr (sizeof(VT) == 4)
-        csr5_spmv_f32_kernel<SG, IT><<<grid, SPMV_WARPS * 32, 0, s>>>(
-            (const ChunkHdr *)h.meta, h.tile_ptr, h.flags, (const float *)h.vals,
-            (const IT *)h.cols, (const float *)x, (double *)y, h.carry_head,
-            h.carry_tail, h.nchunks, h.G, h.m, h.n, guard_word());
-    else
-        csr5_spmv_kernel<SG, VT, IT><<<grid, SPMV_WARPS * 32, 0, s>>>(
-            (const ChunkHdr *)h.meta, h.tile_ptr, h.flags, (const VT *)h.vals,
-            (const IT *)h.cols, (const VT *)x, (double *)y, h.carry_head,
-            h.carry_tail, h.nchunks, h.G, h.m, h.n, guard_word());
+cudaError_t launch_sg(const Handle &h, unsigned grid, const void *x, void *y, cudaStream_t s) {
+    auto go = [&](auto kernel) {
+        return launch_product(kernel, grid, SPMV_WARPS * 32, 0, s, (const ChunkHdr *)h.meta,
+                              h.tile_ptr, h.flags, (const VT *)h.vals, (const IT *)h.cols,
+                              (const VT *)x, (double *)y, h.carry_head, h.carry_tail, h.nchunks,
+                              h.G, h.m, h.n, guard_word());
+    };
+    if constexpr (sizeof(VT) == 4) return go(csr5_spmv_f32_kernel<SG, IT>);
+    else return go(csr5_spmv_kernel<SG, VT, IT>);
 }
 
 template <typename VT, typename IT>
@@ -573,14 +571,13 @@ cudaError_t spmv_t(const Handle &h, const void *x, void *y, cudaStream_t s) {
     const long long cap = (long long)h.sm_count * (sizeof(VT) == 8 ? PAVA_CSR5_MINB : PAVA_CSR5_MINB32);
     const unsigned grid = (unsigned)(want < cap ? want : cap);
     switch (h.sigma) {
-        case 8: launch_sg<8, VT, IT>(h, grid, x, y, s); break;
-        case 12: launch_sg<12, VT, IT>(h, grid, x, y, s); break;
-        case 16: launch_sg<16, VT, IT>(h, grid, x, y, s); break;
-        case 24: launch_sg<24, VT, IT>(h, grid, x, y, s); break;
-        case 32: launch_sg<32, VT, IT>(h, grid, x, y, s); break;
+        case 8: return launch_sg<8, VT, IT>(h, grid, x, y, s);
+        case 12: return launch_sg<12, VT, IT>(h, grid, x, y, s);
+        case 16: return launch_sg<16, VT, IT>(h, grid, x, y, s);
+        case 24: return launch_sg<24, VT, IT>(h, grid, x, y, s);
+        case 32: return launch_sg<32, VT, IT>(h, grid, x, y, s);
         default: return cudaErrorInvalidValue;
     }
-    return cudaGetLastError();
 }
 
 }  // namespace

@@ -245,8 +245,7 @@ cvr_spmv_kernel(const CvrMeta *__restrict__ meta, const unsigned *__restrict__ f
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const uint64_t pf = policy_evict_first(), pl = policy_evict_last();
     const unsigned lt = lanemask_lt();
-    // the carry fixup that follows may launch now; it waits for this grid to finish
-    asm volatile("griddepcontrol.launch_dependents;");
+    pdl_trigger();
     const long long nwarps = (long long)gridDim.x * SPMV_WARPS;
 
     for (long long c = (long long)blockIdx.x * SPMV_WARPS + w; c < nchunks; c += nwarps) {
@@ -276,6 +275,7 @@ cvr_spmv_kernel(const CvrMeta *__restrict__ meta, const unsigned *__restrict__ f
         VT x0[4];
         {
             const CBlk<IT> c0 = CBlk<IT>::load(cb, 0, lane, pf);
+            pdl_wait();  // x, and y and the carries, which the product before may still use
 #pragma unroll
             for (int q = 0; q < 4; ++q) x0[q] = c0.gather(q, xb, pl, xlo, xhi, err);
         }
@@ -385,29 +385,18 @@ cudaError_t spmv_t(const Handle &h, const void *x, void *y, cudaStream_t s) {
     const long long want = (h.nchunks + SPMV_WARPS - 1) / SPMV_WARPS;
     const long long cap = (long long)h.sm_count * (sizeof(VT) == 8 ? PAVA_CVR_MINB : PAVA_CVR_MINB32);
     const unsigned grid = (unsigned)(want < cap ? want : cap);
-    const CvrMeta *meta = (const CvrMeta *)h.meta;
-    const VT *xv = (const VT *)x;
-    double *yv = (double *)y;
+    auto go = [&](auto kernel) {
+        return launch_product(kernel, grid, SPMV_WARPS * 32, 0, s, (const CvrMeta *)h.meta,
+                              h.flags, (const VT *)h.vals, (const IT *)h.cols, (const VT *)x,
+                              h.colbase, (double *)y, h.carry_head, h.carry_tail, h.nchunks, h.m,
+                              h.n, guard_word());
+    };
     switch (h.S) {
-        case 32:
-            cvr_spmv_kernel<32, VT, IT><<<grid, SPMV_WARPS * 32, 0, s>>>(
-                meta, h.flags, (const VT *)h.vals, (const IT *)h.cols, xv, h.colbase, yv,
-                h.carry_head, h.carry_tail, h.nchunks, h.m, h.n, guard_word());
-            break;
-        case 64:
-            cvr_spmv_kernel<64, VT, IT><<<grid, SPMV_WARPS * 32, 0, s>>>(
-                meta, h.flags, (const VT *)h.vals, (const IT *)h.cols, xv, h.colbase, yv,
-                h.carry_head, h.carry_tail, h.nchunks, h.m, h.n, guard_word());
-            break;
-        case 128:
-            cvr_spmv_kernel<128, VT, IT><<<grid, SPMV_WARPS * 32, 0, s>>>(
-                meta, h.flags, (const VT *)h.vals, (const IT *)h.cols, xv, h.colbase, yv,
-                h.carry_head, h.carry_tail, h.nchunks, h.m, h.n, guard_word());
-            break;
-        default:
-            return cudaErrorInvalidValue;
+        case 32: return go(cvr_spmv_kernel<32, VT, IT>);
+        case 64: return go(cvr_spmv_kernel<64, VT, IT>);
+        case 128: return go(cvr_spmv_kernel<128, VT, IT>);
+        default: return cudaErrorInvalidValue;
     }
-    return cudaGetLastError();
 }
 
 }  // namespace

@@ -128,6 +128,8 @@ csr_group_kernel(const int *__restrict__ rp, const int *__restrict__ ci,
                  double *__restrict__ Y, long long ldy, int m, int k, int gl_shift,
                  int kc_shift, int tile_rows, int n, unsigned long long *err) {
     constexpr int U = group_unroll<KPL>();
+    pdl_trigger();
+    pdl_wait();
     const int lane = threadIdx.x & 31;
     const int gl = 1 << gl_shift, kc = 1 << kc_shift;
     const int grp = lane >> gl_shift;          // group within the warp
@@ -220,6 +222,8 @@ csr_window_kernel(const int *__restrict__ rp, const int *__restrict__ ci,
     VT *xs = reinterpret_cast<VT *>(smem_raw);
     constexpr int WARPS = GROUP_THREADS / 32;
     __shared__ int s_min[WARPS], s_max[WARPS];
+    pdl_trigger();
+    pdl_wait();
     const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
     const int gl = 1 << gl_shift, kc = 1 << kc_shift;
     const int grp = lane >> gl_shift;
@@ -398,6 +402,8 @@ csr_spmv_kernel(const int *__restrict__ rp, const int *__restrict__ ci, const VT
     constexpr int LONG = GL < 32 ? 4 * U * GL : HUGE_ROW;
     __shared__ int s_list[WARPS][LIST], s_cnt[WARPS];
     __shared__ double s_sum[WARPS];
+    pdl_trigger();
+    pdl_wait();
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const int grp = lane / GL, gi = lane % GL;
     const uint64_t pf = policy_evict_first(), pl = policy_evict_last();
@@ -537,10 +543,10 @@ cudaError_t launch_window(const Handle &h, const VT *x, long long ldx, double *y
             csr_window_kernel<KPL, VT, KCT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
             WINDOW_SMEM);
         if (attr != cudaSuccess) return attr;
-        csr_window_kernel<KPL, VT, KCT><<<grid, GROUP_THREADS, smem, s>>>(
-            h.rp, h.ci, (const VT *)h.v, x, ldx, y, ldy, h.m, k, ilog2(h.lanes_per_row),
-            ilog2(h.col_lanes), tr, max_w, h.n, guard_word());
-        return cudaGetLastError();
+        return launch_product(csr_window_kernel<KPL, VT, KCT>, grid, GROUP_THREADS, smem, s, h.rp,
+                              h.ci, (const VT *)h.v, x, ldx, y, ldy, h.m, k,
+                              ilog2(h.lanes_per_row), ilog2(h.col_lanes), tr, max_w, h.n,
+                              guard_word());
     });
 }
 
@@ -554,9 +560,9 @@ cudaError_t launch_spmv(const Handle &h, const VT *x, long long ldx, double *y, 
     const long long cap = (long long)h.sm_count * SPMV_MINB;
     const unsigned grid = (unsigned)(want < cap ? (want > 0 ? want : 1) : cap);
     auto go = [&](auto GLC) {
-        csr_spmv_kernel<decltype(GLC)::value, VT><<<grid, GROUP_THREADS, 0, s>>>(
-            h.rp, h.ci, (const VT *)h.v, x, ldx, y, ldy, h.m, tr, h.n, guard_word());
-        return cudaGetLastError();
+        return launch_product(csr_spmv_kernel<decltype(GLC)::value, VT>, grid, GROUP_THREADS, 0, s,
+                              h.rp, h.ci, (const VT *)h.v, x, ldx, y, ldy, h.m, tr, h.n,
+                              guard_word());
     };
     switch (h.lanes_per_row) {
         case 1: return go(std::integral_constant<int, 1>());
@@ -586,17 +592,17 @@ cudaError_t launch_rows(const Handle &h, const VT *x, long long ldx, double *y, 
     return with_kc(kc, [&](auto KCC) {
         constexpr int KCT = decltype(KCC)::value;
         constexpr int VW2 = KPL >= 2 ? 2 : 1;
-        if constexpr (KPL == 1 && KCT == 0)
+        if constexpr (KPL == 1 && KCT == 0) {
             return cudaErrorInvalidValue;  // one column in one lane: launch_spmv
-        else if (vec2)
-            csr_group_kernel<KPL, VT, KCT, VW2><<<grid, GROUP_THREADS, 0, s>>>(
-                h.rp, h.ci, (const VT *)h.v, x, ldx, y, ldy, h.m, k, gs, ks, tr, h.n,
-                guard_word());
-        else
-            csr_group_kernel<KPL, VT, KCT, 1><<<grid, GROUP_THREADS, 0, s>>>(
-                h.rp, h.ci, (const VT *)h.v, x, ldx, y, ldy, h.m, k, gs, ks, tr, h.n,
-                guard_word());
-        return cudaGetLastError();
+        } else {
+            auto go = [&](auto kernel) {
+                return launch_product(kernel, grid, GROUP_THREADS, 0, s, h.rp, h.ci,
+                                      (const VT *)h.v, x, ldx, y, ldy, h.m, k, gs, ks, tr, h.n,
+                                      guard_word());
+            };
+            return vec2 ? go(csr_group_kernel<KPL, VT, KCT, VW2>)
+                        : go(csr_group_kernel<KPL, VT, KCT, 1>);
+        }
     });
 }
 

@@ -215,6 +215,7 @@ sell_spmv_kernel(const SellSlice *__restrict__ meta, const VT *__restrict__ vals
     using ST = Stage<VT, IT>;
     constexpr int KB = ST::KB;
     extern __shared__ __align__(128) unsigned char smem[];
+    pdl_trigger();
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     unsigned char *wbase = smem + w * ST::WARP_BYTES;  // [barriers | value stages | column stages]
     const unsigned bar0 = (unsigned)__cvta_generic_to_shared(wbase);
@@ -263,6 +264,8 @@ sell_spmv_kernel(const SellSlice *__restrict__ meta, const VT *__restrict__ vals
 #pragma unroll
     for (int k = 0; k < STAGES; ++k)
         if (ps < nslices) { issue(k); ++pending; }
+
+    pdl_wait();  // x, and y, which the product before may still use: only copies of the format above
 
     // consumer cursor: slice cs, next block cb; it writes the rows of empty slices
     long long cs = first;
@@ -366,10 +369,10 @@ cudaError_t spmv_t(const Handle &h, const void *x, void *y, cudaStream_t s) {
     const long long want = (h.nchunks + SELL_WARPS - 1) / SELL_WARPS;
     const long long cap = (long long)h.sm_count * CTAS_PER_SM;
     const unsigned grid = (unsigned)(want < cap ? want : cap);
-    sell_spmv_kernel<VT, IT><<<grid, SELL_WARPS * 32, ST::CTA_BYTES, s>>>(
-        (const SellSlice *)h.meta, (const VT *)h.vals, (const IT *)h.cols, (const VT *)x,
-        (double *)y, h.nchunks, h.m, h.n, guard_word(), wait_word());
-    return cudaGetLastError();
+    return launch_product(sell_spmv_kernel<VT, IT>, grid, SELL_WARPS * 32, ST::CTA_BYTES, s,
+                          (const SellSlice *)h.meta, (const VT *)h.vals, (const IT *)h.cols,
+                          (const VT *)x, (double *)y, h.nchunks, h.m, h.n, guard_word(),
+                          wait_word());
 }
 
 }  // namespace

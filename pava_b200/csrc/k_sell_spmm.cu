@@ -86,6 +86,7 @@ sell_spmm_kernel(const SellSlice *__restrict__ meta, const VT *__restrict__ vals
     using ST = SpmmStage<VT, IT, G>;
     constexpr int KB = SpmmShape<G>::KB;
     extern __shared__ __align__(128) unsigned char smem[];
+    pdl_trigger();
     const int tid = threadIdx.x;
     const int r = tid / G;   // the thread's row within the slice
     const int lg = tid % G;  // its column slot
@@ -143,6 +144,8 @@ sell_spmm_kernel(const SellSlice *__restrict__ meta, const VT *__restrict__ vals
             issue(kk);
             ++pending;
         }
+
+    pdl_wait();  // X, and Y, which the product before may still use: only copies of the format above
 
     // consumer cursor; the rows of empty slices are written as zeros
     long long cs = s_first;
@@ -262,10 +265,10 @@ cudaError_t spmm_launch(const Handle &h, const VT *X, long long ldx, double *Y, 
     }
     const long long cap = (long long)h.sm_count * SpmmShape<G>::CTAS_PER_SM;
     const unsigned grid = (unsigned)(h.nchunks < cap ? h.nchunks : cap);
-    sell_spmm_kernel<VT, IT, G, KPL, VW><<<grid, SpmmShape<G>::THREADS, ST::BYTES, s>>>(
-        (const SellSlice *)h.meta, (const VT *)h.vals, (const IT *)h.cols, X, ldx, Y, ldy,
-        h.nchunks, h.m, h.n, k, guard_word(), wait_word());
-    return cudaGetLastError();
+    return launch_product(sell_spmm_kernel<VT, IT, G, KPL, VW>, grid, SpmmShape<G>::THREADS,
+                          ST::BYTES, s, (const SellSlice *)h.meta, (const VT *)h.vals,
+                          (const IT *)h.cols, X, ldx, Y, ldy, h.nchunks, h.m, h.n, k,
+                          guard_word(), wait_word());
 }
 
 // KPL = the columns per lane that cover k with G lanes; pairs per read where they can be

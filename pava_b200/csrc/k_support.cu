@@ -217,6 +217,7 @@ __global__ void __launch_bounds__(128)
 carry_fixup_kernel(const char *__restrict__ meta, size_t stride, const int *__restrict__ arp,
                    long long L, const double *carry_head, const double *carry_tail, double *y,
                    long long nchunks, int m, unsigned long long *err) {
+    pdl_trigger();
     const int lane = threadIdx.x & 31;
     const long long c1 = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     // the headers belong to the matrix: read before the wait
@@ -230,9 +231,7 @@ carry_fixup_kernel(const char *__restrict__ meta, size_t stride, const int *__re
         if ((sh & 1u) && !((sh & 2u) && H->nrows == 1)) R = H->r_first;
         two = P->nrows > 1 || !(psh & 1u);
     }
-    // launched as a programmatic dependent of the SpMV kernel: wait until that grid has
-    // finished and its carries are visible (returns at once for an ordinary launch)
-    asm volatile("griddepcontrol.wait;" ::: "memory");
+    pdl_wait();  // the SpMV kernel's carries
     if (R >= m || !guard(err, R >= -1, G_Y, R)) R = -1;
     if (R >= 0 && two) y[R] = carry_tail[c1 - 1] + carry_head[c1];
     unsigned todo = __ballot_sync(FULL, R >= 0 && !two);
@@ -377,22 +376,9 @@ cudaError_t set_int(int *p, int v, cudaStream_t s) {
 cudaError_t carry_fixup(const Handle &h, void *y, cudaStream_t s) {
     if (h.nchunks <= 0) return cudaSuccess;
     const long long blocks = (h.nchunks + 127) / 128;
-    // programmatic dependent launch: the fixup grid is launched while the SpMV grid runs (its
-    // launch latency hidden) and waits for it in griddepcontrol.wait
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)blocks);
-    cfg.blockDim = dim3(128);
-    cfg.dynamicSmemBytes = 0;
-    cfg.stream = s;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, carry_fixup_kernel, (const char *)h.meta, h.meta_stride,
-                              (const int *)h.arp, h.L, (const double *)h.carry_head,
-                              (const double *)h.carry_tail, (double *)y, h.nchunks, h.m,
-                              guard_word());
+    return launch_product(carry_fixup_kernel, (unsigned)blocks, 128, 0, s, (const char *)h.meta,
+                          h.meta_stride, h.arp, h.L, h.carry_head, h.carry_tail, (double *)y,
+                          h.nchunks, h.m, guard_word());
 }
 
 }  // namespace pava

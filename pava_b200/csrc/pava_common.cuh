@@ -7,6 +7,14 @@ namespace pava {
 
 constexpr unsigned FULL = 0xffffffffu;
 
+// Programmatic dependent launch (launch_product): lets the next kernel's grid launch, and waits
+// until the grids before this one are done and their writes visible (returns at once after an
+// ordinary launch).
+__device__ __forceinline__ void pdl_trigger() {
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 __device__ __forceinline__ unsigned lanemask_lt() {
     unsigned r;
     asm("mov.u32 %0, %%lanemask_lt;" : "=r"(r));

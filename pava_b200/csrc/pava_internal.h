@@ -92,6 +92,28 @@ void pool_free_synced(void *const *ps, int count);
 size_t pool_reserved();
 void pool_trim(size_t keep);
 
+// Launches a product kernel as a programmatic dependent of the kernel before it in the stream.
+// All product kernels let their dependents launch at once (pdl_trigger) and call pdl_wait before
+// they read x or write anything, so consecutive products overlap one's launch and first reads of
+// the format, which only conversion writes, with the end of the other; behind any other kernel
+// the launch waits as an ordinary one does.  512 x 512 Laplacian, CVR (SpMV and fixup): 12.3 ->
+// 10.3 us a product in a loop; 128^3 stencil, SELL FP32C: 74.5 -> 71.6 us.
+template <typename... KArgs, typename... Args>
+cudaError_t launch_product(void (*kernel)(KArgs...), unsigned grid, unsigned threads,
+                           size_t smem, cudaStream_t s, Args... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
+}
+
 // Sets the message pava_last_error() returns on this thread.
 void set_last_error(const std::string &msg);
 
