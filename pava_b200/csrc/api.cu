@@ -706,9 +706,24 @@ pava_status pava_spmm(pava_handle *H, int k, const void *X, long long ldx, void 
         if (e != cudaSuccess) return fail_cuda(e, "spmm launch");
         return PAVA_SUCCESS;
     }
-    pava::Handle g;
+    // Handles without a shape of their own: rows staged per warp for k >= 3, two columns per lane
+    // in groups of four lanes for k = 2 (FP64, banded / stencil / blocks: staged 123 / 137 / 98 us,
+    // groups 105 / 123 / 96; k = 3: 127 / 143 / 97 against 154 / 176 / 129).
+    const bool own_shape = h.lanes_per_row || h.col_lanes || h.cols_per_lane || h.rows_per_tile ||
+                           h.x_window;
+    if (!own_shape && k > 2) {
+        const cudaError_t e = pava::csr_spmm_staged(h, X, ldx, Y, ldy, k, 0, 0, (cudaStream_t)stream);
+        if (e != cudaSuccess) return fail_cuda(e, "spmm launch");
+        return PAVA_SUCCESS;
+    }
+    pava::Handle g, asked = h;
+    if (!own_shape && k == 2) {
+        asked.lanes_per_row = 4;
+        asked.col_lanes = 1;
+        asked.cols_per_lane = 2;
+    }
     std::string why;
-    if (!resolve_group_shape(h, k, g, why)) return fail(PAVA_E_UNSUPPORTED_PARAMS, why);
+    if (!resolve_group_shape(asked, k, g, why)) return fail(PAVA_E_UNSUPPORTED_PARAMS, why);
     cudaError_t e = pava::csr_spmm(g, X, ldx, Y, ldy, k, (cudaStream_t)stream);
     if (e != cudaSuccess) return fail_cuda(e, "spmm launch");
     return PAVA_SUCCESS;

@@ -1,5 +1,6 @@
 // CSR row-group kernel: SpMV and multi-RHS SpMM (Y = A X, X row-major n x k) on plain CSR,
-// FP64 or FP32-compensated, for short-row and batched matrices.
+// FP64 or FP32 storage (one right-hand side: compensated FP32 sums), for short-row and batched
+// matrices.  SpMM without a shape of its own runs k_csr_spmm.cu instead.
 //
 // A group of GL lanes (a power of two <= 32) owns one row at a time.  Inside the group, KC
 // lanes span the k right-hand sides (lane c holds columns c, c + KC, ..., KPL of them) and
@@ -24,24 +25,14 @@ namespace pava {
 
 namespace {
 
-__device__ __forceinline__ double ld_val(const double *p, uint64_t pol) {
-    double r;
-    asm volatile("ld.global.nc.L1::no_allocate.L2::cache_hint.f64 %0, [%1], %2;"
-                 : "=d"(r) : "l"(p), "l"(pol));
-    return r;
-}
-__device__ __forceinline__ float ld_val(const float *p, uint64_t pol) {
-    float r;
-    asm volatile("ld.global.nc.L1::no_allocate.L2::cache_hint.f32 %0, [%1], %2;"
-                 : "=f"(r) : "l"(p), "l"(pol));
-    return r;
-}
-__device__ __forceinline__ int ld_col(const int *p, uint64_t pol) {
-    int r;
-    asm volatile("ld.global.nc.L1::no_allocate.L2::cache_hint.s32 %0, [%1], %2;"
-                 : "=r"(r) : "l"(p), "l"(pol));
-    return r;
-}
+// A row's sum for one right-hand side.  FP32 values and x: a product of two FP32 numbers is exact in
+// FP64, so the exact products are summed there -- one conversion and one FMA per right-hand side,
+// where a compensated FP32 sum takes ten operations, and more accurate.
+struct ColAcc {
+    double s = 0.0;
+    __device__ __forceinline__ void add(double v, double x) { s = fma(v, x, s); }
+    __device__ __forceinline__ double value() const { return s; }
+};
 
 // Rows shared by several column lanes (KCT = KC > 1, a compile-time count so that the KC
 // elements of a round unroll): the group loads its row's nonzeros
@@ -49,12 +40,14 @@ __device__ __forceinline__ int ld_col(const int *p, uint64_t pol) {
 // stream), with the next round's loads in flight while the current round is consumed; each
 // element reaches the lanes that need it by shuffle.  Slice e takes elements e, e + ES, ... in
 // ascending order, as the per-lane loop does, so the sums have the same bits.  The round count
-// is the maximum over the warp's groups so that every shuffle has all 32 lanes.
-template <int KPL, int KCT, int VW, typename VT, typename XREAD>
-__device__ __forceinline__ void coop_row(int a, int b, int gi, int gl, int es, int e, int kc,
-                                         int lane, const int *__restrict__ ci,
-                                         const VT *__restrict__ v, const bool (&colok)[KPL],
-                                         XREAD xread, Acc<VT> (&acc)[KPL], uint64_t pf) {
+// is the maximum over the warp's groups so that every shuffle has all 32 lanes.  The X reads of
+// UB elements are in flight together: an element past the row's end has column -1, for which
+// xload gives zeros.
+template <int KPL, int KCT, typename VT, typename XLOAD>
+__device__ __forceinline__ void coop_row(int a, int b, int gi, int gl, int es, int e, int lane,
+                                         const int *__restrict__ ci, const VT *__restrict__ v,
+                                         XLOAD xload, ColAcc (&acc)[KPL], uint64_t pf) {
+    constexpr int UB = KPL >= 4 ? 1 : (KCT < 4 / KPL ? KCT : 4 / KPL);
     int rounds = (b - a + gl - 1) / gl;
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
@@ -63,7 +56,7 @@ __device__ __forceinline__ void coop_row(int a, int b, int gi, int gl, int es, i
     }
     const int gbase = lane & ~(gl - 1);
     VT pv = VT(0);
-    int pc = 0;
+    int pc = -1;
     if (a + gi < b) {
         pv = ld_val(v + a + gi, pf);
         pc = ld_col(ci + a + gi, pf);
@@ -72,36 +65,27 @@ __device__ __forceinline__ void coop_row(int a, int b, int gi, int gl, int es, i
         const VT cv = pv;
         const int cc = pc;
         const int base = a + rd * gl;
+        pv = VT(0);
+        pc = -1;
         if (base + gl + gi < b) {  // next round in flight
             pv = ld_val(v + base + gl + gi, pf);
             pc = ld_col(ci + base + gl + gi, pf);
         }
 #pragma unroll
-        for (int u = 0; u < KCT; ++u) {
-            const int o = e + u * es;
-            const VT val = __shfl_sync(FULL, cv, gbase + o);
-            const int col = __shfl_sync(FULL, cc, gbase + o);
-            if (base + o < b) {
+        for (int u0 = 0; u0 < KCT; u0 += UB) {
+            VT val[UB], xv[UB][KPL];
 #pragma unroll
-                for (int q = 0; q < KPL / VW; ++q)
-                    if (colok[q * VW]) xread(col, q, val, acc);
+            for (int u = 0; u < UB; ++u) {
+                const int o = gbase + e + (u0 + u) * es;
+                val[u] = __shfl_sync(FULL, cv, o);
+                xload(__shfl_sync(FULL, cc, o), xv[u]);
             }
+#pragma unroll
+            for (int u = 0; u < UB; ++u)
+#pragma unroll
+                for (int p = 0; p < KPL; ++p) acc[p].add((double)val[u], (double)xv[u][p]);
         }
     }
-}
-
-// Two adjacent right-hand sides of X in one 16-byte (8-byte for FP32) read.
-__device__ __forceinline__ double2 ld_x2(const double *p, uint64_t pol) {
-    double2 r;
-    asm volatile("ld.global.nc.L2::cache_hint.v2.f64 {%0, %1}, [%2], %3;"
-                 : "=d"(r.x), "=d"(r.y) : "l"(p), "l"(pol));
-    return r;
-}
-__device__ __forceinline__ float2 ld_x2(const float *p, uint64_t pol) {
-    float2 r;
-    asm volatile("ld.global.nc.L2::cache_hint.v2.f32 {%0, %1}, [%2], %3;"
-                 : "=f"(r.x), "=f"(r.y) : "l"(p), "l"(pol));
-    return r;
 }
 
 // Column of accumulator p of a lane whose first column slot is cl: VW = 1 interleaves single
@@ -143,19 +127,29 @@ csr_group_kernel(const int *__restrict__ rp, const int *__restrict__ ci,
     const long long nwarps = ((long long)gridDim.x * blockDim.x) >> 5;
     const int rounds = tile_rows / gpw;        // rows per group per tile
 
-    bool colok[KPL];
+    // column offsets of the lane's reads; a slot past k reads nothing
+    int xoff[KPL];
 #pragma unroll
-    for (int p = 0; p < KPL; ++p) colok[p] = col_of<VW>(cl, p, kc) < k;
-    // reads the VW columns of slot q of X row `col` and accumulates them
-    auto xread = [&](int col, int q, VT val, Acc<VT>(&acc)[KPL]) {
-        if (!guard(err, col >= 0 && col < n, G_X, col)) return;
-        const VT *xr = X + (long long)col * ldx + col_of<VW>(cl, q * VW, kc);
-        if (VW == 2) {
-            const auto x2 = ld_x2(xr, pl);
-            acc[2 * q].add(val, x2.x);
-            acc[2 * q + 1].add(val, x2.y);
-        } else {
-            acc[q].add(val, ld_x(xr, pl));
+    for (int p = 0; p < KPL; ++p) {
+        const int c = col_of<VW>(cl, p, kc);
+        xoff[p] = c < k ? c : -1;
+    }
+    // the lane's KPL columns of X row `col` (zeros for column -1)
+    auto xload = [&](int col, VT(&xv)[KPL]) {
+        const bool in = col >= 0 && guard(err, col < n, G_X, col);
+        const VT *xr = X + (long long)col * ldx;
+#pragma unroll
+        for (int p = 0; p < KPL; p += VW) {
+            xv[p] = VT(0);
+            if constexpr (VW == 2) xv[p + 1] = VT(0);
+            if (!in || xoff[p] < 0) continue;
+            if constexpr (VW == 2) {
+                const auto x2 = ld_x2(xr + xoff[p], pl);
+                xv[p] = x2.x;
+                xv[p + 1] = x2.y;
+            } else {
+                xv[p] = ld_x(xr + xoff[p], pl);
+            }
         }
     };
 
@@ -169,36 +163,36 @@ csr_group_kernel(const int *__restrict__ rp, const int *__restrict__ ci,
                 a = rp[r];
                 b = rp[r + 1];
             }
-            Acc<VT> acc[KPL];
-            int j = a + e;
-            if (KCT) {
-                coop_row<KPL, KCT, VW>(a, b, gi, gl, es, e, kc, lane, ci, v, colok, xread, acc,
-                                       pf);
-                j = b;
-            }
-            // U elements at a time (the last batch predicated): all value and column loads
-            // first, then all gathers, so up to U memory round trips overlap even on short rows
-            for (; j < b; j += U * es) {
-                VT val[U];
-                int col[U];
-                bool in[U];
+            ColAcc acc[KPL];
+            if constexpr (KCT != 0) {
+                coop_row<KPL, KCT>(a, b, gi, gl, es, e, lane, ci, v, xload, acc, pf);
+            } else {
+                // U elements at a time: all value and column loads first, then all gathers, so up to U
+                // memory round trips overlap even on short rows
+                const unsigned len = (unsigned)(b - a);
+                for (unsigned j = e; j < len; j += U * es) {
+                    VT val[U], xv[U][KPL];
+                    int col[U];
 #pragma unroll
-                for (int u = 0; u < U; ++u) {
-                    in[u] = j + u * es < b;
-                    val[u] = in[u] ? ld_val(v + j + u * es, pf) : VT(0);
-                    col[u] = in[u] ? ld_col(ci + j + u * es, pf) : 0;
+                    for (int u = 0; u < U; ++u) {
+                        const bool in = j + u * es < len;
+                        val[u] = in ? ld_val(v + a + (j + u * es), pf) : VT(0);
+                        col[u] = in ? ld_col(ci + a + (j + u * es), pf) : -1;
+                    }
+#pragma unroll
+                    for (int u = 0; u < U; ++u) xload(col[u], xv[u]);
+#pragma unroll
+                    for (int u = 0; u < U; ++u)
+#pragma unroll
+                        for (int p = 0; p < KPL; ++p) acc[p].add((double)val[u], (double)xv[u][p]);
                 }
-#pragma unroll
-                for (int u = 0; u < U; ++u)
-#pragma unroll
-                    for (int q = 0; q < KPL / VW; ++q)
-                        if (in[u] && colok[q * VW]) xread(col[u], q, val[u], acc);
             }
 #pragma unroll
             for (int p = 0; p < KPL; ++p) {
                 double s = acc[p].value();
                 for (int o = kc; o < gl; o <<= 1) s += __shfl_xor_sync(FULL, s, o);
-                if (valid && e == 0 && colok[p]) Y[r * ldy + col_of<VW>(cl, p, kc)] = s;
+                if (valid && e == 0 && col_of<VW>(cl, p, kc) < k)
+                    Y[r * ldy + col_of<VW>(cl, p, kc)] = s;
             }
         }
     }
@@ -306,22 +300,29 @@ csr_window_kernel(const int *__restrict__ rp, const int *__restrict__ ci,
                 a = rp[r];
                 b = rp[r + 1];
             }
-            Acc<VT> acc[KPL];
+            ColAcc acc[KPL];
             int j = a + e;
-            if (KCT) {
+            if constexpr (KCT != 0) {
                 if (staged)
-                    coop_row<KPL, KCT, 1>(
-                        a, b, gi, gl, es, e, kc, lane, ci, v, colok,
-                        [&](int col, int p, VT val, Acc<VT>(&ac)[KPL]) {
-                            ac[p].add(val, xs[(col - cmin) * k + cl + p * kc]);
+                    coop_row<KPL, KCT>(
+                        a, b, gi, gl, es, e, lane, ci, v,
+                        [&](int col, VT(&xv)[KPL]) {
+#pragma unroll
+                            for (int p = 0; p < KPL; ++p)
+                                xv[p] = col >= 0 && colok[p] ? xs[(col - cmin) * k + cl + p * kc]
+                                                             : VT(0);
                         },
                         acc, pf);
                 else
-                    coop_row<KPL, KCT, 1>(
-                        a, b, gi, gl, es, e, kc, lane, ci, v, colok,
-                        [&](int col, int p, VT val, Acc<VT>(&ac)[KPL]) {
-                            if (guard(err, col >= 0 && col < n, G_X, col))
-                                ac[p].add(val, ld_x(X + (long long)col * ldx + cl + p * kc, pl));
+                    coop_row<KPL, KCT>(
+                        a, b, gi, gl, es, e, lane, ci, v,
+                        [&](int col, VT(&xv)[KPL]) {
+                            const bool in = col >= 0 && guard(err, col < n, G_X, col);
+#pragma unroll
+                            for (int p = 0; p < KPL; ++p)
+                                xv[p] = in && colok[p]
+                                            ? ld_x(X + (long long)col * ldx + cl + p * kc, pl)
+                                            : VT(0);
                         },
                         acc, pf);
                 j = b;
@@ -641,6 +642,8 @@ __global__ void narrow_kernel(const double *__restrict__ src, float *__restrict_
 cudaError_t csr_spmm(const Handle &h, const void *X, long long ldx, void *Y, long long ldy,
                      int k, cudaStream_t s) {
     if (h.m <= 0 || k <= 0) return cudaSuccess;
+    if (csr_staged_shape(h, k))
+        return csr_spmm_staged(h, X, ldx, Y, ldy, k, h.lanes_per_row, h.cols_per_lane, s);
     if (h.precision == PAVA_PREC_FP32C) return launch_group<float>(h, X, ldx, Y, ldy, k, s);
     return launch_group<double>(h, X, ldx, Y, ldy, k, s);
 }

@@ -207,4 +207,38 @@ __device__ __forceinline__ unsigned ld_flag(const unsigned *p) {
     return r;
 }
 
+// One element of a plain CSR's streams.
+__device__ __forceinline__ double ld_val(const double *p, uint64_t pol) {
+    double r;
+    asm volatile("ld.global.nc.L1::no_allocate.L2::cache_hint.f64 %0, [%1], %2;"
+                 : "=d"(r) : "l"(p), "l"(pol));
+    return r;
+}
+__device__ __forceinline__ float ld_val(const float *p, uint64_t pol) {
+    float r;
+    asm volatile("ld.global.nc.L1::no_allocate.L2::cache_hint.f32 %0, [%1], %2;"
+                 : "=f"(r) : "l"(p), "l"(pol));
+    return r;
+}
+__device__ __forceinline__ int ld_col(const int *p, uint64_t pol) {
+    int r;
+    asm volatile("ld.global.nc.L1::no_allocate.L2::cache_hint.s32 %0, [%1], %2;"
+                 : "=r"(r) : "l"(p), "l"(pol));
+    return r;
+}
+
+// Two adjacent right-hand sides of X in one 16-byte (8-byte for FP32) read.
+__device__ __forceinline__ double2 ld_x2(const double *p, uint64_t pol) {
+    double2 r;
+    asm volatile("ld.global.nc.L2::cache_hint.v2.f64 {%0, %1}, [%2], %3;"
+                 : "=d"(r.x), "=d"(r.y) : "l"(p), "l"(pol));
+    return r;
+}
+__device__ __forceinline__ float2 ld_x2(const float *p, uint64_t pol) {
+    float2 r;
+    asm volatile("ld.global.nc.L2::cache_hint.v2.f32 {%0, %1}, [%2], %3;"
+                 : "=f"(r.x), "=f"(r.y) : "l"(p), "l"(pol));
+    return r;
+}
+
 }  // namespace pava

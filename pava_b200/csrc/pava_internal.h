@@ -200,6 +200,11 @@ cudaError_t sell_spmm(const Handle &h, const void *X, long long ldx, void *Y, lo
 cudaError_t csr_spmv(const Handle &h, const void *x, void *y, cudaStream_t s);
 cudaError_t csr_spmm(const Handle &h, const void *X, long long ldx, void *Y, long long ldy,
                      int k, cudaStream_t s);
+// SpMM with the rows staged per warp (k_csr_spmm.cu), k in 1 .. 128, in the engine's own shape for
+// k; csr_spmm runs it too for the shapes csr_staged_shape accepts.
+cudaError_t csr_spmm_staged(const Handle &h, const void *X, long long ldx, void *Y, long long ldy,
+                            int k, int lanes, int cols, cudaStream_t s);
+bool csr_staged_shape(const Handle &shape, int k);
 cudaError_t narrow_to_float(const double *src, float *dst, long long n, cudaStream_t s);
 
 }  // namespace pava
