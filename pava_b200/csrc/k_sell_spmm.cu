@@ -1,19 +1,33 @@
 // SELL SpMM: Y = A X for k right-hand sides (X row-major n x k, Y row-major m x k) on a SELL
 // handle.
 //
-// A CTA of 32 G threads takes one 32-row slice at a time (slices in turn over the grid): G
-// lanes per row (4, 8 or 16), 32 / G rows per warp.  Thread t owns row t / G of the slice and,
-// of that row's k outputs, the KPL columns of slot g = t % G (VW = 2: the pairs g, g + G, ... of
-// adjacent columns, each read as one vector) -- so the G lanes of a row read a whole row of X
-// per nonzero, and each thread keeps its KPL sums in registers for the whole slice.
+// A CTA of 32 G threads takes one 32-row slice at a time: G lanes per row (4, 8 or 16), 32 / G rows
+// per warp.  Thread t owns row t / G of the slice and, of that row's k outputs, the KPL columns of
+// slot g = t % G (VW = 2: the pairs g, g + G, ... of adjacent columns, each read as one vector)
+// -- so the G lanes of a row read a whole row of X per nonzero, and each thread keeps its KPL sums
+// in registers for the whole slice.  CTAs take runs of one or two neighbouring slices in
+// turn.
 //
 // The slice's value and column streams come into shared memory by bulk asynchronous copies
-// (k_bulk.cuh), G blocks per piece, two pieces in flight per CTA: thread 0 issues the
-// copies of the piece after next while the CTA sums the current one.  A row's four elements of
-// a block are one 16-byte shared-memory read per stream (the G lanes of the row read the same
-// address: a broadcast), where the row-group kernel (k_group.cu) passes every element to the
-// lanes of its row by shuffles.  Padding elements (value 0, no column) read X row 0 and add
-// nothing.
+// (k_bulk.cuh), KB blocks per piece, two pieces in flight per CTA: thread 0 issues the copies of
+// the piece after next while the CTA sums the current one.  A row's four elements of a block are
+// one 16-byte shared-memory read per stream (the G lanes of the row read the same address: a
+// broadcast), where the row-group kernel (k_group.cu) passes every element to the lanes of its
+// row by shuffles.  Padding (value 0, no column) reads a row of zeros instead of X; the blocks before
+// the slice's shortest row ends carry no test for it.  The CTA meets once per piece: each thread
+// waits for the copies on the mbarrier, and the barrier that hands the piece back also carries
+// whether a wait gave up.
+//
+// What bounds it: the X reads, 8 k bytes per nonzero into registers (128 bytes per SM and clock:
+// 179 us for 25 M banded nonzeros at k = 32) and their latency, so the reads of all four elements
+// of a block are in flight before the first is used, without predicates, and the cursor of the
+// copies lives in shared memory to leave the registers to them.  FP64, 32-bit / 16-bit columns,
+// L2 flushed, against reads used one by one, a select per column for padding and two barriers per
+// piece: banded (1,048,576 rows, 24 each) k = 8 195 / 202 -> 115 / 107 us, k = 32 336 / 357 -> 328 /
+// 320; stencil 100^3 k = 8 181 / 189 -> 119 / 109, k = 32 335 / 390 -> 330 / 324; dense blocks
+// (400,000 rows) k = 8 181 / 186 -> 82 / 78, k = 32 274 / 297 -> 261 / 258.  One 1,024-thread CTA per
+// SM whose groups share runs of 8-32 slices raised the L1 hit rate from 75 to 90 % on the
+// banded matrix and ran it like this form (k = 32: 317 us), but the blocks in 290.
 //
 // No counterpart in the reference (its SpMV takes one vector; main.cpp:554-587 runs one matrix
 // and one vector at a time).
@@ -21,6 +35,7 @@
 #include <atomic>
 #include <climits>
 #include <cstdint>
+#include <type_traits>
 
 #include "k_bulk.cuh"
 #include "k_stream.cuh"
@@ -30,14 +45,17 @@ namespace pava {
 
 namespace {
 
-// The shape of G lanes per row: 32 G threads per CTA (32 rows), 32 / G CTAs per SM (32 warps),
-// pieces of G blocks (about 100 KB of stages per SM for FP64 values and 32-bit columns, which
-// leaves L1 room for the X rows neighbouring slices share; pieces of 2 G blocks were 5-10 %
-// slower, of G / 2 blocks 4-7 % slower).
+// The shape of G lanes per row: 32 G threads per CTA (32 rows), 32 / G CTAs per SM (32 warps), pieces
+// of KB blocks (100 KB of stages per SM for FP64 values and 32-bit columns with 8 or 16 lanes, which
+// leaves L1 room for the X rows neighbouring slices share).
 constexpr int SPMM_UNROLL = 2;  // blocks of a piece unrolled together
+// Neighbouring slices a CTA takes in a row: they share X rows, but long runs keep distant regions
+// of X alive at once (stencil, k = 16: 249, 251, 254 and 304 us at 1, 2, 4 and 16; FP32C 214, 202,
+// 200, 208).  One at a time where the matrix has fewer than four runs per resident CTA.
+constexpr int RUN = 2;  // a power of two
 template <int G> struct SpmmShape {
     static_assert(G == 4 || G == 8 || G == 16, "lanes per row");
-    static constexpr int THREADS = 32 * G, CTAS_PER_SM = 32 / G, KB = G;
+    static constexpr int THREADS = 32 * G, CTAS_PER_SM = 32 / G, KB = G == 4 ? 8 : G;
 };
 template <typename VT, typename IT, int G> struct SpmmStage {
     static constexpr int VBYTES = SpmmShape<G>::KB * 128 * (int)sizeof(VT);
@@ -45,19 +63,8 @@ template <typename VT, typename IT, int G> struct SpmmStage {
     static constexpr int BYTES = 2 * (VBYTES + CBYTES) + 128;  // two pieces + barriers
 };
 
-// Two adjacent columns of an X row in one read (16 bytes FP64, 8 bytes FP32), kept in L2.
-__device__ __forceinline__ double2 ld_xpair(const double *p, uint64_t pol) {
-    double2 r;
-    asm volatile("ld.global.nc.L2::cache_hint.v2.f64 {%0, %1}, [%2], %3;"
-                 : "=d"(r.x), "=d"(r.y) : "l"(p), "l"(pol));
-    return r;
-}
-__device__ __forceinline__ float2 ld_xpair(const float *p, uint64_t pol) {
-    float2 r;
-    asm volatile("ld.global.nc.L2::cache_hint.v2.f32 {%0, %1}, [%2], %3;"
-                 : "=f"(r.x), "=f"(r.y) : "l"(p), "l"(pol));
-    return r;
-}
+// What padding reads in place of a row of X: it adds 0 * 0, whatever X holds.
+__device__ double g_zero_row[SELL_SPMM_MAX_K];
 
 // Column of sum p of a lane whose column slot is lg (0 .. G-1).
 template <int G, int VW>
@@ -77,12 +84,13 @@ __device__ __forceinline__ void row_cols(const short *pc, int i, int r, int (&c)
     c[2] = (int)(a.y << 16) >> 16; c[3] = (int)a.y >> 16;
 }
 
-template <typename VT, typename IT, int G, int KPL, int VW>
+// LD: the type of X's leading dimension; int (VW = 2) makes a row address one multiply-add.
+template <typename VT, typename IT, int G, int KPL, int VW, typename LD>
 __global__ void __launch_bounds__(SpmmShape<G>::THREADS, SpmmShape<G>::CTAS_PER_SM)
 sell_spmm_kernel(const SellSlice *__restrict__ meta, const VT *__restrict__ vals,
-                 const IT *__restrict__ cols, const VT *__restrict__ X, long long ldx,
-                 double *__restrict__ Y, long long ldy, long long nslices, int m, int n, int k,
-                 unsigned long long *err, unsigned long long *wait_err) {
+                 const IT *__restrict__ cols, const VT *__restrict__ X, LD ldx,
+                 double *__restrict__ Y, long long ldy, int ns, int run, int m, int n, int k,
+                  unsigned long long *err, unsigned long long *wait_err) {
     using ST = SpmmStage<VT, IT, G>;
     constexpr int KB = SpmmShape<G>::KB;
     extern __shared__ __align__(128) unsigned char smem[];
@@ -101,64 +109,60 @@ sell_spmm_kernel(const SellSlice *__restrict__ meta, const VT *__restrict__ vals
     }
     __syncthreads();
     const uint64_t pl = policy_evict_last();
-    bool colok[KPL];
-#pragma unroll
-    for (int p = 0; p < KPL; ++p) colok[p] = spmm_col<G, VW>(lg, p) < k;
-    // the CTA's slices, in turn over the grid (a contiguous run of slices per CTA, whose
-    // neighbours share X rows, was measured slower on the stencil)
-    const long long step = gridDim.x, s_first = blockIdx.x, s_end = nslices;
 
-    // producer cursor (the CTA's slices with blocks; thread 0 issues the copies)
-    long long ps = s_first;
-    int pb = 0;
-    SellSlice pm{0, 0, 0, 0u};
-    auto p_find = [&]() {
-        for (; ps < s_end; ps += step) {
+    // the CTA's slices: runs of `run` (a power of two), in turn over the grid
+    const int first = (int)blockIdx.x * run, hop = ((int)gridDim.x - 1) * run + 1;
+    auto next = [&](int s) { return s + (((s + 1) & (run - 1)) ? 1 : hop); };
+
+    // Producer: thread 0 issues the copies of the slices' pieces.  Its cursor lives in shared memory,
+    // so that it costs no registers: slice, next block, the slice's offset and blocks, and the
+    // copies issued that the consumer has not waited for.
+    int *cur = reinterpret_cast<int *>(smem + 16);
+    auto p_find = [&](int ps) {
+        SellSlice pm{0, 0, 0, 0u};
+        for (; ps < ns; ps = next(ps)) {
             pm = meta[ps];
             if (pm.nblk > 0) break;
         }
+        cur[0] = ps;
+        cur[1] = 0;
+        cur[2] = pm.off;
+        cur[3] = pm.nblk;
     };
-    p_find();
-    auto issue = [&](int kk) {
-        const int len = min(KB, pm.nblk - pb);
-        const long long e0 = (long long)pm.off + (long long)pb * 128;
-        if (tid == 0) {
-            const unsigned vb = (unsigned)(len * 128 * (int)sizeof(VT));
-            const unsigned cb = (unsigned)(len * 128 * (int)sizeof(IT));
-            proxy_fence();  // the stage's last reads come before the copy's writes
-            mbar_expect_tx(bar0 + 8 * kk, vb + cb);
-            bulk_g2s(sv0 + kk * ST::VBYTES, vals + e0, vb, bar0 + 8 * kk);
-            bulk_g2s(sc0 + kk * ST::CBYTES, cols + e0, cb, bar0 + 8 * kk);
-        }
-        pb += KB;
-        if (pb >= pm.nblk) {
-            pb = 0;
-            ps += step;
-            p_find();
-        }
+    auto issue = [&](int kk) {  // thread 0 alone
+        const int ps = cur[0], pb = cur[1], off = cur[2], nblk = cur[3];
+        if (ps >= ns) return;
+        const int len = min(KB, nblk - pb);
+        const long long e0 = (long long)off + (long long)pb * 128;
+        const unsigned vb = (unsigned)(len * 128 * (int)sizeof(VT));
+        const unsigned cb = (unsigned)(len * 128 * (int)sizeof(IT));
+        proxy_fence();  // the stage's last reads come before the copy's writes
+        mbar_expect_tx(bar0 + 8 * kk, vb + cb);
+        bulk_g2s(sv0 + kk * ST::VBYTES, vals + e0, vb, bar0 + 8 * kk);
+        bulk_g2s(sc0 + kk * ST::CBYTES, cols + e0, cb, bar0 + 8 * kk);
+        cur[4] += 1;
+        if (pb + KB < nblk) cur[1] = pb + KB;
+        else p_find(next(ps));
     };
-    int pending = 0;
-#pragma unroll
-    for (int kk = 0; kk < 2; ++kk)
-        if (ps < s_end) {
-            issue(kk);
-            ++pending;
-        }
-
+    if (tid == 0) {
+        cur[4] = 0;
+        p_find(first);
+        issue(0);
+        issue(1);
+    }
     pdl_wait();  // X, and Y, which the product before may still use: only copies of the format above
 
     // consumer cursor; the rows of empty slices are written as zeros
-    long long cs = s_first;
-    int cb = 0;
-    SellSlice cm{0, 0, 0, 0u};
-    auto store_row = [&](long long slice, const double (&acc)[KPL]) {
-        const long long row = slice * 32 + r;
+    int cs = first, cb = 0;
+    int nblk = 0, base = 0, pads = 0;  // of slice cs: blocks, base column, first block with padding
+    auto store_row = [&](int slice, const double (&acc)[KPL]) {
+        const long long row = (long long)slice * 32 + r;
         if (row >= m) return;
         double *yr = Y + row * ldy;
 #pragma unroll
         for (int p = 0; p < KPL; p += VW) {
-            if (!colok[p]) continue;
             const int c = spmm_col<G, VW>(lg, p);
+            if (c >= k) continue;
             if constexpr (VW == 2)
                 *reinterpret_cast<double2 *>(yr + c) = make_double2(acc[p], acc[p + 1]);
             else
@@ -169,9 +173,12 @@ sell_spmm_kernel(const SellSlice *__restrict__ meta, const VT *__restrict__ vals
         double zero[KPL];
 #pragma unroll
         for (int p = 0; p < KPL; ++p) zero[p] = 0.0;
-        for (; cs < s_end; cs += step) {
-            cm = meta[cs];
-            if (cm.nblk > 0) break;
+        for (; cs < ns; cs = next(cs)) {
+            const SellSlice cm = meta[cs];
+            nblk = cm.nblk;
+            base = sizeof(IT) == 2 ? cm.colbase : 0;
+            pads = (cm.flags & 1u) ? (int)(cm.flags >> 1) : nblk;
+            if (nblk > 0) break;
             store_row(cs, zero);
         }
     };
@@ -181,69 +188,85 @@ sell_spmm_kernel(const SellSlice *__restrict__ meta, const VT *__restrict__ vals
     double acc[KPL];
 #pragma unroll
     for (int p = 0; p < KPL; ++p) acc[p] = 0.0;
-    while (cs < s_end) {
-        // every thread waits (bounded); the CTA gives up together if any thread did
-        const bool ok = mbar_wait(bar0 + 8 * kk, (phases >> kk) & 1u);
-        if (__syncthreads_or(!ok)) {
-            if (tid == 0) {
-                atomicAdd(&wait_err[0], 1ull);
-                atomicCAS(&wait_err[1], 0ull, (unsigned long long)cs + 1);
-            }
-            break;
-        }
-        phases ^= 1u << kk;
-        --pending;
-        const int len = min(KB, cm.nblk - cb);
-        const VT *pv = sv + kk * (ST::VBYTES / (int)sizeof(VT));
-        const IT *pc = sc + kk * (ST::CBYTES / (int)sizeof(IT));
-        const int xbase = sizeof(IT) == 2 ? cm.colbase : 0;  // base of the 16-bit offsets
-#pragma unroll SPMM_UNROLL
-        for (int i = 0; i < len; ++i) {
-            int c[4];
-            row_cols(pc, i, r, c);
-            const VBlk<VT> vv = VBlk<VT>::load_smem(pv, i, r);
+    // column offsets of the lane's reads; a slot past k reads column 0 and is never stored
+    int xoff[KPL / VW];
 #pragma unroll
-            for (int q = 0; q < 4; ++q) {
-                const bool real = sizeof(IT) == 2 ? c[q] != DELTA_NONE : c[q] >= 0;
-                const int col = c[q] + xbase;
-                const bool use = real && guard(err, col >= 0 && col < n, G_X, col);
-                const VT *xr = X + (long long)(use ? col : 0) * ldx;  // row 0: a safe read
-                const double v = (double)vv.get(q);
+    for (int p = 0; p < KPL; p += VW) {
+        const int c = spmm_col<G, VW>(lg, p);
+        xoff[p / VW] = c < k ? c : 0;
+    }
+    auto sum_block = [&](const VT *pv, const IT *pc, int i, auto pads_tag) {
+        constexpr bool PADS = decltype(pads_tag)::value;
+        // elements whose X reads are in flight together: a block's four, where registers allow
+        constexpr int QB = KPL >= 8 || PADS ? 2 : 4;
+        int c[4];
+        row_cols(pc, i, r, c);
+        const VBlk<VT> vv = VBlk<VT>::load_smem(pv, i, r);
+#pragma unroll
+        for (int q0 = 0; q0 < 4; q0 += QB) {
+            VT xv[QB][KPL];
+#pragma unroll
+            for (int q = 0; q < QB; ++q) {
+                const int cq = c[q0 + q];
+                const bool real = !PADS || (sizeof(IT) == 2 ? cq != DELTA_NONE : cq >= 0);
+                const bool use = real && guard(err, cq + base >= 0 && cq + base < n, G_X, cq + base);
+                const VT *xr = use ? X + (long long)(cq + base) * ldx
+                                   : reinterpret_cast<const VT *>(g_zero_row);
 #pragma unroll
                 for (int p = 0; p < KPL; p += VW) {
-                    if (!colok[p]) continue;
-                    const int cc = spmm_col<G, VW>(lg, p);
                     if constexpr (VW == 2) {
-                        const auto x2 = ld_xpair(xr + cc, pl);
-                        acc[p] = fma(v, use ? (double)x2.x : 0.0, acc[p]);
-                        acc[p + 1] = fma(v, use ? (double)x2.y : 0.0, acc[p + 1]);
+                        const auto x2 = ld_x2(xr + xoff[p / 2], pl);
+                        xv[q][p] = x2.x;
+                        xv[q][p + 1] = x2.y;
                     } else {
-                        const VT xv = ld_x(xr + cc, pl);
-                        acc[p] = fma(v, use ? (double)xv : 0.0, acc[p]);
+                        xv[q][p] = ld_x(xr + xoff[p], pl);
                     }
                 }
             }
+#pragma unroll
+            for (int q = 0; q < QB; ++q) {
+                const double v = (double)vv.get(q0 + q);
+#pragma unroll
+                for (int p = 0; p < KPL; ++p) acc[p] = fma(v, (double)xv[q][p], acc[p]);
+            }
         }
+    };
+    while (cs < ns) {
+        const bool ok = mbar_wait(bar0 + 8 * kk, (phases >> kk) & 1u);
+        phases ^= 1u << kk;
+        const int len = ok ? min(KB, nblk - cb) : 0;
+        const VT *pv = sv + kk * (ST::VBYTES / (int)sizeof(VT));
+        const IT *pc = sc + kk * (ST::CBYTES / (int)sizeof(IT));
+        const int clean = max(0, min(len, pads - cb));  // blocks before the padding
+#pragma unroll SPMM_UNROLL
+        for (int i = 0; i < clean; ++i) sum_block(pv, pc, i, std::false_type());
+#pragma unroll SPMM_UNROLL
+        for (int i = clean; i < len; ++i) sum_block(pv, pc, i, std::true_type());
+        const int done = cs;
         cb += KB;
-        if (cb >= cm.nblk) {  // the slice's last piece
+        if (cb >= nblk) {  // the slice's last piece
             store_row(cs, acc);
 #pragma unroll
             for (int p = 0; p < KPL; ++p) acc[p] = 0.0;
             cb = 0;
-            cs += step;
+            cs = next(cs);
             c_find();
         }
-        __syncthreads();  // every thread is done with stage kk
-        if (ps < s_end) {
-            issue(kk);
-            ++pending;
+        // every thread is done with stage kk; the CTA gives up together if any wait did
+        if (__syncthreads_or(!ok)) {
+            if (tid == 0) {
+                atomicAdd(&wait_err[0], 1ull);
+                atomicCAS(&wait_err[1], 0ull, (unsigned long long)done + 1);
+                // the copies still in flight land before the CTA exits: this piece's, the next's
+                mbar_wait(bar0 + 8 * kk, ((phases >> kk) & 1u) ^ 1u);
+                if (cur[4] > 1) mbar_wait(bar0 + 8 * (kk ^ 1), (phases >> (kk ^ 1)) & 1u);
+            }
+            break;
         }
-        kk ^= 1;
-    }
-    // only after a wait gave up: let the copies still in flight land before the CTA exits
-    for (; pending > 0; --pending) {
-        mbar_wait(bar0 + 8 * kk, (phases >> kk) & 1u);
-        phases ^= 1u << kk;
+        if (tid == 0) {
+            cur[4] -= 1;
+            issue(kk);
+        }
         kk ^= 1;
     }
 }
@@ -252,30 +275,32 @@ template <typename VT, typename IT, int G, int KPL, int VW>
 cudaError_t spmm_launch(const Handle &h, const VT *X, long long ldx, double *Y, long long ldy,
                         int k, cudaStream_t s) {
     using ST = SpmmStage<VT, IT, G>;
+    using LD = std::conditional_t<VW == 2, int, long long>;
+    constexpr auto kernel = sell_spmm_kernel<VT, IT, G, KPL, VW, LD>;
     // more than the default 48 KB of dynamic shared memory: opted into once per device
     static std::atomic<unsigned long long> opted{0};
     if (h.device < 0 || h.device >= 64) return cudaErrorInvalidDevice;
     const unsigned long long bit = 1ull << h.device;
     if (!(opted.load() & bit)) {
-        const cudaError_t e = cudaFuncSetAttribute(sell_spmm_kernel<VT, IT, G, KPL, VW>,
-                                                   cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                   ST::BYTES);
+        const cudaError_t e = cudaFuncSetAttribute(
+            kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, ST::BYTES);
         if (e != cudaSuccess) return e;
         opted.fetch_or(bit);
     }
     const long long cap = (long long)h.sm_count * SpmmShape<G>::CTAS_PER_SM;
-    const unsigned grid = (unsigned)(h.nchunks < cap ? h.nchunks : cap);
-    return launch_product(sell_spmm_kernel<VT, IT, G, KPL, VW>, grid, SpmmShape<G>::THREADS,
-                          ST::BYTES, s, (const SellSlice *)h.meta, (const VT *)h.vals,
-                          (const IT *)h.cols, X, ldx, Y, ldy, h.nchunks, h.m, h.n, k,
-                          guard_word(), wait_word());
+    const int run = h.nchunks >= 4 * RUN * cap ? RUN : 1;
+    const long long runs = (h.nchunks + run - 1) / run;
+    const unsigned grid = (unsigned)(runs < cap ? runs : cap);
+    return launch_product(kernel, grid, SpmmShape<G>::THREADS, ST::BYTES, s,
+                          (const SellSlice *)h.meta, (const VT *)h.vals, (const IT *)h.cols, X,
+                          (LD)ldx, Y, ldy, (int)h.nchunks, run, h.m, h.n, k, guard_word(), wait_word());
 }
 
 // KPL = the columns per lane that cover k with G lanes; pairs per read where they can be
 template <typename VT, typename IT, int G, int KPL>
 cudaError_t spmm_vw(const Handle &h, const VT *X, long long ldx, double *Y, long long ldy,
                     int k, cudaStream_t s) {
-    const bool vec2 = KPL >= 2 && k % 2 == 0 && ldx % 2 == 0 && ldy % 2 == 0 &&
+    const bool vec2 = KPL >= 2 && k % 2 == 0 && ldx % 2 == 0 && ldy % 2 == 0 && ldx <= INT_MAX &&
                       reinterpret_cast<uintptr_t>(X) % (2 * sizeof(VT)) == 0 &&
                       reinterpret_cast<uintptr_t>(Y) % 16 == 0;
     if constexpr (KPL >= 2)
