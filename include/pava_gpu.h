@@ -81,7 +81,8 @@ typedef struct pava_opts {
                              matrix gives fewer than 24 chunks of 64 steps per SM) */
     int sigma;            /* CSR5: elements per lane per tile, 8, 12, 16, 24 or 32 (default 16) */
     int tiles_per_chunk;  /* CSR5: tiles per warp chunk, 1 .. 64 (default 4; 2 or 1 when a
-                             matrix gives fewer than 4 x 24 tiles per SM), or PAVA_TILES_WAVE
+                             matrix gives fewer than 4 x 24 tiles per SM; FP64 with columns
+                             scattered over x: 1 .. 8, balanced), or PAVA_TILES_WAVE
                              (-1): the count in 1 .. 8 that fills the last wave of resident
                              warps best for this matrix */
     int precision;        /* pava_precision */

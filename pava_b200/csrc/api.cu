@@ -613,17 +613,20 @@ pava_status pava_create(const pava_csr *A, int format, const pava_opts *opts, vo
         cudaEventDestroy(e0);
         cudaEventDestroy(e1);
     };
-    int *d_chk = nullptr, chk[2] = {0, 0};  // violations, empty rows
+    int *d_chk = nullptr, chk[3] = {0, 0, 0};  // violations, empty rows, sampled lines of x
     {
-        ce = pava::pool_malloc(&d_chk, 2, s);
+        ce = pava::pool_malloc(&d_chk, 3, s);
         if (ce == cudaSuccess) ce = pava::launch_validate(rp, ci, h.m, h.n, h.nnz, d_chk, s);
         cudaEventRecord(e0, s);
         const bool chunked = format == PAVA_FORMAT_CVR || format == PAVA_FORMAT_CSR5;
         if (ce == cudaSuccess && chunked) ce = dalloc(&h.arp, (size_t)h.m + 2, &h.device_bytes, s);
         if (ce == cudaSuccess && chunked)
             ce = pava::build_augmented_rowptr(rp, h.m, h.arp, d_chk + 1, s);
+        const bool sample = format == PAVA_FORMAT_CSR5;
+        if (ce == cudaSuccess && sample) ce = pava::sample_lines(ci, h.nnz, d_chk + 2, s);
         if (ce == cudaSuccess)
-            ce = cudaMemcpyAsync(chk, d_chk, sizeof(int) * (chunked ? 2 : 1), cudaMemcpyDeviceToHost, s);
+            ce = cudaMemcpyAsync(chk, d_chk, sizeof(int) * (sample ? 3 : chunked ? 2 : 1),
+                                 cudaMemcpyDeviceToHost, s);
         if (ce == cudaSuccess) ce = cudaStreamSynchronize(s);
         pava::pool_free(d_chk, s);
         if (ce != cudaSuccess) {
@@ -639,6 +642,14 @@ pava_status pava_create(const pava_csr *A, int format, const pava_opts *opts, vo
             return fail(PAVA_E_INVALID_CSR, "row_ptr not monotone, row_ptr[0]/row_ptr[m] wrong, or column out of range (" +
                                                 std::to_string(chk[0]) + " violations)");
         }
+    }
+    // scattered: more than half of the sampled nonzeros on a line of their own (over 0.9 on
+    // power-law matrices of 100,000 rows and more, under 0.05 on stencils, bands and dense blocks)
+    h.scattered = chk[2] > pava::LINE_WINDOW * pava::LINE_WINDOWS / 2 ? 1 : 0;
+    if (format == PAVA_FORMAT_CSR5 && h.scattered && !o.tiles_per_chunk &&
+        o.precision == PAVA_PREC_FP64) {
+        h.G = pava::csr5_scattered_tiles((long long)h.nnz / (32LL * h.sigma), 20LL * h.sm_count);
+        h.L = 32LL * h.sigma * h.G;
     }
     st = convert(h, rp, ci, v, chk[1], auto_index, s);
     if (st == PAVA_SUCCESS) {

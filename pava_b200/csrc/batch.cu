@@ -254,13 +254,9 @@ pava_status pava_autotune(const pava_csr *A, int k, int precision, int reps,
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
         return bfail(PAVA_E_CUDA, "no usable CUDA device");
     const std::vector<std::pair<int, pava_opts>> cand = candidates(k, precision);
-    // CSR5 forms whose wave-balanced tile count equals the default count are the same form:
-    // timed once, the twin copies the result
-    auto csr5_tiles = [&](const pava_opts &o) {
-        const long long tiles = (long long)A->nnz / (32LL * o.sigma), warps = 24LL * sms;
-        if (o.tiles_per_chunk == PAVA_TILES_WAVE) return pava::csr5_wave_tiles(tiles, warps);
-        return o.tiles_per_chunk ? o.tiles_per_chunk : pava::csr5_default_tiles(tiles, warps);
-    };
+    // CSR5 forms whose wave-balanced tile count equals the one the default form got are the same
+    // form: timed once, the twin copies the result
+    std::vector<long long> elems(cand.size(), 0);  // elements per chunk of the forms that ran
     const size_t sx = precision == PAVA_PREC_FP32C ? 4 : 8;
     void *X = nullptr, *Y = nullptr;
     cudaError_t e = cudaMalloc(&X, sx * (size_t)(A->n ? A->n : 1) * k);
@@ -286,7 +282,9 @@ pava_status pava_autotune(const pava_csr *A, int k, int precision, int reps,
             const pava_tune_entry &tw = entries[n - 3];
             if (tw.format == PAVA_FORMAT_CSR5 && tw.opts.tiles_per_chunk == 0 &&
                 tw.opts.sigma == t.opts.sigma && tw.opts.index_mode == t.opts.index_mode &&
-                csr5_tiles(tw.opts) == csr5_tiles(t.opts)) {
+                elems[n - 3] == 32LL * t.opts.sigma *
+                                    pava::csr5_wave_tiles((long long)A->nnz / (32LL * t.opts.sigma),
+                                                          24LL * sms)) {
                 t.ms = tw.ms;
                 t.status = tw.status;
                 continue;
@@ -295,6 +293,8 @@ pava_status pava_autotune(const pava_csr *A, int k, int precision, int reps,
         pava_handle *H = nullptr;
         t.status = pava_create(A, t.format, &t.opts, nullptr, &H);
         if (t.status != PAVA_SUCCESS) continue;
+        pava_info info;
+        if (pava_get_info(H, &info) == PAVA_SUCCESS) elems[n - 1] = info.elems_per_chunk;
         auto run = [&]() {
             return k == 1 ? pava_spmv(H, X, Y, nullptr) : pava_spmm(H, k, X, k, Y, k, nullptr);
         };

@@ -205,13 +205,16 @@ __device__ __forceinline__ void tile_combine(double head, double tail, bool seen
     }
 }
 
-#ifndef PAVA_CSR5_MINB32
-#define PAVA_CSR5_MINB32 3
-#endif
-#ifndef PAVA_CSR5_MINB
-#define PAVA_CSR5_MINB 3
-#endif
-constexpr int SPMV_WARPS = 8;
+// Warps per CTA and CTAs per SM: 24 warps per SM as three CTAs where the columns are local (FP64: 80
+// registers); where they are scattered (Handle::scattered) the gathers' latency counts, and 20
+// warps with the registers to keep more of a chunk in flight, or FP32 chunks over smaller CTAs, are
+// faster.  FP64, sigma 16, 32-bit columns: power law, 66 M nonzeros 338 -> 313 us a product in a
+// loop, 20 M 118 -> 107 with L2 flushed (110 -> 109 in a loop); local columns lose by it (stencil
+// 128^3 150 -> 155, dense blocks 114 -> 122).  16 warps with 128 registers: 302 us where 20 take
+// 300.  FP32C, sigma 32, L2 flushed: 66 M 308 -> 290, 20 M 112 -> 101.
+template <typename VT, bool SCAT> struct Csr5Shape {
+    static constexpr int WARPS = SCAT ? 4 : 8, CTAS = !SCAT ? 3 : sizeof(VT) == 8 ? 5 : 6;
+};
 
 // CSR5 SpMV (FP64 values; the FP32 form is csr5_spmv_f32_kernel below): one warp per chunk of
 // G tiles, walked as one pipelined run of 4-step blocks
@@ -223,8 +226,8 @@ constexpr int SPMV_WARPS = 8;
 // so the step has no branch; at the tile end piece 0 (the end of the row the lane started
 // with) joins the cross-lane combine and pieces 1 .. k-1, rows that start and end in the
 // lane, go to y.  Other tiles write each finished row as it ends.
-template <int SIGMA, typename VT, typename IT>
-__global__ void __launch_bounds__(SPMV_WARPS * 32, sizeof(VT) == 8 ? PAVA_CSR5_MINB : PAVA_CSR5_MINB32)
+template <int SIGMA, typename VT, typename IT, bool SCAT>
+__global__ void __launch_bounds__(Csr5Shape<VT, SCAT>::WARPS * 32, Csr5Shape<VT, SCAT>::CTAS)
 csr5_spmv_kernel(const ChunkHdr *__restrict__ hdr, const int *__restrict__ tile_ptr,
                  const unsigned *__restrict__ desc, const VT *__restrict__ vals,
                  const IT *__restrict__ cols, const VT *__restrict__ x,
@@ -232,6 +235,7 @@ csr5_spmv_kernel(const ChunkHdr *__restrict__ hdr, const int *__restrict__ tile_
                  double *__restrict__ carry_tail, long long nchunks, int G, int m, int n,
                  unsigned long long *err) {
     constexpr int NBT = SIGMA / 4;  // blocks per tile
+    constexpr int SPMV_WARPS = Csr5Shape<VT, SCAT>::WARPS;
     pdl_trigger();
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const uint64_t pf = policy_evict_first(), pl = policy_evict_last();
@@ -384,8 +388,8 @@ template <bool B> struct Flag { static constexpr bool value = B; };
 // choice and the tile-boundary checks are made once per tile instead of once per block.  The
 // compensated add makes this form instruction-issue bound, where the saved instructions are
 // time; the FP64 form is bandwidth bound, and unrolled it spills, so it keeps the block loop.
-template <int SIGMA, typename IT>
-__global__ void __launch_bounds__(SPMV_WARPS * 32, PAVA_CSR5_MINB32)
+template <int SIGMA, typename IT, bool SCAT>
+__global__ void __launch_bounds__(Csr5Shape<float, SCAT>::WARPS * 32, Csr5Shape<float, SCAT>::CTAS)
 csr5_spmv_f32_kernel(const ChunkHdr *__restrict__ hdr, const int *__restrict__ tile_ptr,
                      const unsigned *__restrict__ desc, const float *__restrict__ vals,
                      const IT *__restrict__ cols, const float *__restrict__ x,
@@ -394,6 +398,7 @@ csr5_spmv_f32_kernel(const ChunkHdr *__restrict__ hdr, const int *__restrict__ t
                      unsigned long long *err) {
     using VT = float;
     constexpr int NBT = SIGMA / 4;  // blocks per tile
+    constexpr int SPMV_WARPS = Csr5Shape<VT, SCAT>::WARPS;
     pdl_trigger();
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const uint64_t pf = policy_evict_first(), pl = policy_evict_last();
@@ -553,29 +558,30 @@ cudaError_t convert_t(Handle &h, const int *rp, const int *ci, const double *v, 
     }
 }
 
-template <int SG, typename VT, typename IT>
-cudaError_t launch_sg(const Handle &h, unsigned grid, const void *x, void *y, cudaStream_t s) {
+template <int SG, typename VT, typename IT, bool SCAT>
+cudaError_t launch_sg(const Handle &h, const void *x, void *y, cudaStream_t s) {
+    using SH = Csr5Shape<VT, SCAT>;
+    const long long want = (h.nchunks + SH::WARPS - 1) / SH::WARPS;
+    const long long cap = (long long)h.sm_count * SH::CTAS;
+    const unsigned grid = (unsigned)(want < cap ? want : cap);
     auto go = [&](auto kernel) {
-        return launch_product(kernel, grid, SPMV_WARPS * 32, 0, s, (const ChunkHdr *)h.meta,
+        return launch_product(kernel, grid, SH::WARPS * 32, 0, s, (const ChunkHdr *)h.meta,
                               h.tile_ptr, h.flags, (const VT *)h.vals, (const IT *)h.cols,
                               (const VT *)x, (double *)y, h.carry_head, h.carry_tail, h.nchunks,
                               h.G, h.m, h.n, guard_word());
     };
-    if constexpr (sizeof(VT) == 4) return go(csr5_spmv_f32_kernel<SG, IT>);
-    else return go(csr5_spmv_kernel<SG, VT, IT>);
+    if constexpr (sizeof(VT) == 4) return go(csr5_spmv_f32_kernel<SG, IT, SCAT>);
+    else return go(csr5_spmv_kernel<SG, VT, IT, SCAT>);
 }
 
-template <typename VT, typename IT>
+template <typename VT, typename IT, bool SCAT>
 cudaError_t spmv_t(const Handle &h, const void *x, void *y, cudaStream_t s) {
-    const long long want = (h.nchunks + SPMV_WARPS - 1) / SPMV_WARPS;
-    const long long cap = (long long)h.sm_count * (sizeof(VT) == 8 ? PAVA_CSR5_MINB : PAVA_CSR5_MINB32);
-    const unsigned grid = (unsigned)(want < cap ? want : cap);
     switch (h.sigma) {
-        case 8: return launch_sg<8, VT, IT>(h, grid, x, y, s);
-        case 12: return launch_sg<12, VT, IT>(h, grid, x, y, s);
-        case 16: return launch_sg<16, VT, IT>(h, grid, x, y, s);
-        case 24: return launch_sg<24, VT, IT>(h, grid, x, y, s);
-        case 32: return launch_sg<32, VT, IT>(h, grid, x, y, s);
+        case 8: return launch_sg<8, VT, IT, SCAT>(h, x, y, s);
+        case 12: return launch_sg<12, VT, IT, SCAT>(h, x, y, s);
+        case 16: return launch_sg<16, VT, IT, SCAT>(h, x, y, s);
+        case 24: return launch_sg<24, VT, IT, SCAT>(h, x, y, s);
+        case 32: return launch_sg<32, VT, IT, SCAT>(h, x, y, s);
         default: return cudaErrorInvalidValue;
     }
 }
@@ -595,10 +601,11 @@ cudaError_t csr5_convert(Handle &h, const int *rp, const int *ci, const double *
 cudaError_t csr5_spmv(const Handle &h, const void *x, void *y, cudaStream_t s) {
     if (h.nchunks <= 0) return cudaSuccess;
     const bool f32 = h.precision == PAVA_PREC_FP32C, d16 = h.index_mode == PAVA_INDEX_DELTA16;
-    if (!f32 && !d16) return spmv_t<double, int>(h, x, y, s);
-    if (!f32 && d16) return spmv_t<double, short>(h, x, y, s);
-    if (f32 && !d16) return spmv_t<float, int>(h, x, y, s);
-    return spmv_t<float, short>(h, x, y, s);
+    if (d16)  // columns within 65,534 of one another in every chunk
+        return f32 ? spmv_t<float, short, false>(h, x, y, s) : spmv_t<double, short, false>(h, x, y, s);
+    if (h.scattered)
+        return f32 ? spmv_t<float, int, true>(h, x, y, s) : spmv_t<double, int, true>(h, x, y, s);
+    return f32 ? spmv_t<float, int, false>(h, x, y, s) : spmv_t<double, int, false>(h, x, y, s);
 }
 
 }  // namespace pava

@@ -316,7 +316,35 @@ __global__ void chunk_colbase_kernel(const int *__restrict__ rp, const int *__re
     }
 }
 
+// Block b: the distinct lines (16 columns) of LINE_WINDOW consecutive nonzeros from its part of the
+// matrix, counted in a bitmap of hashed line numbers.
+__global__ void __launch_bounds__(256)
+sample_lines_kernel(const int *__restrict__ ci, int nnz, int *__restrict__ lines) {
+    constexpr int WORDS = 1024;  // 32 K bits for at most 1,024 lines
+    __shared__ unsigned bits[WORDS];
+    for (int i = threadIdx.x; i < WORDS; i += 256) bits[i] = 0;
+    __syncthreads();
+    const long long p0 = (long long)(nnz - LINE_WINDOW) * blockIdx.x / LINE_WINDOWS;
+    for (int i = threadIdx.x; i < LINE_WINDOW; i += 256) {
+        const unsigned h = ((unsigned)ci[p0 + i] >> 4) * 2654435761u >> 17;
+        atomicOr(&bits[h >> 5], 1u << (h & 31));
+    }
+    __syncthreads();
+    int n = 0;
+    for (int i = threadIdx.x; i < WORDS; i += 256) n += __popc(bits[i]);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) n += __shfl_xor_sync(FULL, n, o);
+    if ((threadIdx.x & 31) == 0) atomicAdd(lines, n);
+}
+
 }  // namespace
+
+cudaError_t sample_lines(const int *ci, int nnz, int *lines, cudaStream_t s) {
+    const cudaError_t e = cudaMemsetAsync(lines, 0, sizeof(int), s);
+    if (e != cudaSuccess || nnz < LINE_WINDOW) return e;  // too small to matter: not scattered
+    sample_lines_kernel<<<LINE_WINDOWS, 256, 0, s>>>(ci, nnz, lines);
+    return cudaGetLastError();
+}
 
 cudaError_t launch_validate(const int *rp, const int *ci, int m, int n, int nnz, int *d_err,
                             cudaStream_t s) {

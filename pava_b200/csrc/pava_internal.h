@@ -48,6 +48,7 @@ struct Handle {
     int S = 0;               // CVR: steps per chunk
     int sigma = 0, G = 0;    // CSR5: elements per lane per tile, tiles per chunk
     long long ntiles = 0;
+    int scattered = 0;       // CSR5: neighbouring nonzeros rarely share lines of x
     int lanes_per_row = 0;   // plain CSR: lanes per row group (GL)
     int col_lanes = 1;       //   lanes across the right-hand sides (KC)
     int cols_per_lane = 1;   //   right-hand sides per lane (KPL)
@@ -144,6 +145,20 @@ inline int csr5_wave_tiles(long long tiles, long long warps) {
     return best;
 }
 
+// Scattered columns, FP64: the G in 1..8 with the smallest cost of a warp's chunks, a chunk costing its
+// tiles and a fifth of a tile for its header, carries and start.  Sigma 16, us a product in a
+// loop at 1 / 2 / 3 / 4 / 6 / 8 tiles per chunk: 20 M nonzeros (13.5 tiles per resident warp)
+// 103 / 100 / 105 / 110 / 115 / 111; 66 M (43.5) 310 / 302 / 304 / 297 / 312 / 321.
+inline int csr5_scattered_tiles(long long tiles, long long warps) {
+    int best = 1;
+    long long best_t = -1;
+    for (int g = 1; g <= 8; ++g) {
+        const long long t = (tiles + g * warps - 1) / (g * warps) * (5 * g + 1);
+        if (best_t < 0 || t <= best_t) { best_t = t; best = g; }
+    }
+    return best;
+}
+
 // Kernel launchers (stream-ordered; return cudaGetLastError()).
 cudaError_t launch_validate(const int *rp, const int *ci, int m, int n, int nnz, int *d_err,
                             cudaStream_t s);
@@ -159,6 +174,11 @@ cudaError_t chunk_rows(const int *arp, int m, long long T, long long count, int 
 // first[c * stride]: row of chunk c's first element.
 cudaError_t chunk_colbase(const Handle &h, const int *rp, const int *ci, const int *first,
                           int stride, int *ovf, cudaStream_t s);
+
+// Lines of x (128 bytes of FP64) that LINE_WINDOWS samples of LINE_WINDOW consecutive nonzeros touch,
+// summed into *lines (device, zeroed here): a matrix whose samples reuse few lines is scattered.
+constexpr int LINE_WINDOW = 1024, LINE_WINDOWS = 32;
+cudaError_t sample_lines(const int *ci, int nnz, int *lines, cudaStream_t s);
 
 // Conversions.  With 16-bit offsets they do nothing when *ovf (device) is set.  first: CVR, the
 // row of each chunk's first element; CSR5, h.tile_ptr is complete.

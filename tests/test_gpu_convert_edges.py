@@ -99,3 +99,20 @@ def test_bad_column_found_at_any_alignment(cuda, shift, where):
         with pytest.raises(_abi.PavaError) as e:
             SpMatrix(A, "csr5", device_arrays=dev)
         assert e.value.status == _abi.E_INVALID_CSR
+
+
+@pytest.mark.parametrize("prec", [_abi.PREC_FP64, _abi.PREC_FP32C])
+@pytest.mark.parametrize("sigma", [8, 12, 16, 24, 32])
+@pytest.mark.parametrize("rows", [60, 61, 4000])  # below and above one sample of 1,024 nonzeros
+def test_scattered_columns(cuda, rows, sigma, prec):
+    torch = cuda
+    rng = np.random.default_rng(rows)
+    A = _csr([np.sort(rng.choice(200_000, 17, replace=False)) for _ in range(rows)], 200_000, 10)
+    x = M.uniform(A.n, seed=11, fp32=True)
+    yr, ab = O.csr_ref(A.rp, A.ci, A.v, x)
+    xd = torch.from_numpy(x).cuda()
+    xd = xd.float() if prec == _abi.PREC_FP32C else xd
+    mat = SpMatrix(A, "csr5", sigma=sigma, precision=prec)
+    y = mat.spmv(xd)
+    assert O.rel_error(y.cpu().numpy(), yr, ab, 1e-9 if prec else 1e-12)[0] == 0
+    assert torch.equal(y, mat.spmv(xd))
