@@ -222,16 +222,20 @@ cvr_convert_kernel(const int *__restrict__ rp, const int *__restrict__ ci,
 // software pipeline: value and flag streams are requested two blocks ahead, column streams
 // three blocks ahead, and the x gathers one block ahead of the block being summed, so each
 // lane keeps several 16-byte stream loads and four gathers in flight.
-#ifndef PAVA_CVR_MINB32
-#define PAVA_CVR_MINB32 3
-#endif
-#ifndef PAVA_CVR_MINB
-#define PAVA_CVR_MINB 2
-#endif
-constexpr int SPMV_WARPS = 8;
+// Warps per CTA and CTAs per SM.  FP64: 20 warps per SM with 96 registers for 16-bit columns, whose
+// gathers land near one another so that instruction issue counts, from the chunk count on that 16
+// warps per SM no longer hold at once; else DEEP, 16 warps with 128 registers, which keep more
+// gathers in flight.  A product in a loop, us, 16 / 20 warps: 16-bit columns, stencil 128^3
+// 164 / 144, 60^3 24.5 / 19.3, dense blocks 17 M nonzeros 57 / 48, Laplacian 512^2 (1,278 chunks)
+// 10.3 / 11.6; 32-bit columns, stencil 128^3 174 / 191, power law 66 M 310 / 349, 20 M 108 / 126.
+// 24 warps with 80 registers spill (stencil 196).  FP32: 24 warps.
+template <typename VT, bool DEEP> struct CvrShape {
+    static constexpr int WARPS = sizeof(VT) == 8 && !DEEP ? 4 : 8;
+    static constexpr int CTAS = sizeof(VT) == 4 ? 3 : DEEP ? 2 : 5;
+};
 
-template <int S, typename VT, typename IT>
-__global__ void __launch_bounds__(SPMV_WARPS * 32, sizeof(VT) == 8 ? PAVA_CVR_MINB : PAVA_CVR_MINB32)
+template <int S, typename VT, typename IT, bool DEEP>
+__global__ void __launch_bounds__(CvrShape<VT, DEEP>::WARPS * 32, CvrShape<VT, DEEP>::CTAS)
 cvr_spmv_kernel(const CvrMeta *__restrict__ meta, const unsigned *__restrict__ flags,
                 const VT *__restrict__ vals, const IT *__restrict__ cols,
                 const VT *__restrict__ x, const int *__restrict__ colbase,
@@ -239,13 +243,14 @@ cvr_spmv_kernel(const CvrMeta *__restrict__ meta, const unsigned *__restrict__ f
                 double *__restrict__ carry_tail, long long nchunks, int m, int n,
                 unsigned long long *err) {
     constexpr int L = 32 * S;
-    constexpr int NB = S / 4;
+    constexpr int NB = S / 4, SPMV_WARPS = CvrShape<VT, DEEP>::WARPS;
     __shared__ double s_tail[SPMV_WARPS][64];
     __shared__ int s_row[SPMV_WARPS][64];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const uint64_t pf = policy_evict_first(), pl = policy_evict_last();
     const unsigned lt = lanemask_lt();
     pdl_trigger();
+
     const long long nwarps = (long long)gridDim.x * SPMV_WARPS;
 
     for (long long c = (long long)blockIdx.x * SPMV_WARPS + w; c < nchunks; c += nwarps) {
@@ -380,21 +385,22 @@ cudaError_t convert_t(Handle &h, const int *rp, const int *ci, const double *v, 
     return cudaGetLastError();
 }
 
-template <typename VT, typename IT>
+template <typename VT, typename IT, bool DEEP>
 cudaError_t spmv_t(const Handle &h, const void *x, void *y, cudaStream_t s) {
-    const long long want = (h.nchunks + SPMV_WARPS - 1) / SPMV_WARPS;
-    const long long cap = (long long)h.sm_count * (sizeof(VT) == 8 ? PAVA_CVR_MINB : PAVA_CVR_MINB32);
+    using SH = CvrShape<VT, DEEP>;
+    const long long want = (h.nchunks + SH::WARPS - 1) / SH::WARPS;
+    const long long cap = (long long)h.sm_count * SH::CTAS;
     const unsigned grid = (unsigned)(want < cap ? want : cap);
     auto go = [&](auto kernel) {
-        return launch_product(kernel, grid, SPMV_WARPS * 32, 0, s, (const CvrMeta *)h.meta,
+        return launch_product(kernel, grid, SH::WARPS * 32, 0, s, (const CvrMeta *)h.meta,
                               h.flags, (const VT *)h.vals, (const IT *)h.cols, (const VT *)x,
                               h.colbase, (double *)y, h.carry_head, h.carry_tail, h.nchunks, h.m,
                               h.n, guard_word());
     };
     switch (h.S) {
-        case 32: return go(cvr_spmv_kernel<32, VT, IT>);
-        case 64: return go(cvr_spmv_kernel<64, VT, IT>);
-        case 128: return go(cvr_spmv_kernel<128, VT, IT>);
+        case 32: return go(cvr_spmv_kernel<32, VT, IT, DEEP>);
+        case 64: return go(cvr_spmv_kernel<64, VT, IT, DEEP>);
+        case 128: return go(cvr_spmv_kernel<128, VT, IT, DEEP>);
         default: return cudaErrorInvalidValue;
     }
 }
@@ -414,10 +420,10 @@ cudaError_t cvr_convert(Handle &h, const int *rp, const int *ci, const double *v
 cudaError_t cvr_spmv(const Handle &h, const void *x, void *y, cudaStream_t s) {
     if (h.nchunks <= 0) return cudaSuccess;
     const bool f32 = h.precision == PAVA_PREC_FP32C, d16 = h.index_mode == PAVA_INDEX_DELTA16;
-    if (!f32 && !d16) return spmv_t<double, int>(h, x, y, s);
-    if (!f32 && d16) return spmv_t<double, short>(h, x, y, s);
-    if (f32 && !d16) return spmv_t<float, int>(h, x, y, s);
-    return spmv_t<float, short>(h, x, y, s);
+    if (f32) return d16 ? spmv_t<float, short, true>(h, x, y, s) : spmv_t<float, int, true>(h, x, y, s);
+    if (!d16) return spmv_t<double, int, true>(h, x, y, s);
+    return h.nchunks <= 16LL * h.sm_count ? spmv_t<double, short, true>(h, x, y, s)
+                                          : spmv_t<double, short, false>(h, x, y, s);
 }
 
 }  // namespace pava

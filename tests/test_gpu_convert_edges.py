@@ -116,3 +116,26 @@ def test_scattered_columns(cuda, rows, sigma, prec):
     y = mat.spmv(xd)
     assert O.rel_error(y.cpu().numpy(), yr, ab, 1e-9 if prec else 1e-12)[0] == 0
     assert torch.equal(y, mat.spmv(xd))
+
+
+@pytest.mark.parametrize("extra", [-1, 0, 1, 3, 900])
+def test_cvr_chunks_around_a_full_gpu(cuda, extra):
+    """16 warps per SM hold one chunk each; 16-bit columns take another launch shape beyond that."""
+    torch = cuda
+    chunks = 16 * torch.cuda.get_device_properties(0).multi_processor_count + extra
+    m = chunks * 32                       # rows of 31 or 33 nonzeros: 1,024 elements to a chunk
+    lens = np.where(np.arange(m) % 2, 33, 31)
+    lens[-1] -= 1                         # not a whole number of elements
+    rp = np.concatenate([[0], np.cumsum(lens)])
+    k = np.arange(rp[-1]) - np.repeat(rp[:-1], lens)
+    ci = (np.repeat(np.arange(m), lens) // 32 * 5 + k * 7) % 20011
+    A = M.from_arrays(m, 20011, rp, ci.astype(np.int32), M.uniform(int(rp[-1]), seed=12, fp32=True))
+    x = M.uniform(A.n, seed=13, fp32=True)
+    yr, ab = O.csr_ref(A.rp, A.ci, A.v, x)
+    for prec, bound in ((_abi.PREC_FP64, 1e-12), (_abi.PREC_FP32C, 1e-9)):
+        for mode in (_abi.INDEX_DELTA16, _abi.INDEX_I32):
+            mat = SpMatrix(A, "cvr", precision=prec, index_mode=mode, steps=32)
+            xd = torch.from_numpy(x).cuda()
+            y = mat.spmv(xd.float() if prec == _abi.PREC_FP32C else xd).cpu().numpy()
+            assert O.rel_error(y, yr, ab, bound)[0] == 0, (prec, mode)
+            mat.close()
