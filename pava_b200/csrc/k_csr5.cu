@@ -205,15 +205,17 @@ __device__ __forceinline__ void tile_combine(double head, double tail, bool seen
     }
 }
 
-// Warps per CTA and CTAs per SM: 24 warps per SM as three CTAs where the columns are local (FP64: 80
-// registers); where they are scattered (Handle::scattered) the gathers' latency counts, and 20
-// warps with the registers to keep more of a chunk in flight, or FP32 chunks over smaller CTAs, are
-// faster.  FP64, sigma 16, 32-bit columns: power law, 66 M nonzeros 338 -> 313 us a product in a
-// loop, 20 M 118 -> 107 with L2 flushed (110 -> 109 in a loop); local columns lose by it (stencil
-// 128^3 150 -> 155, dense blocks 114 -> 122).  16 warps with 128 registers: 302 us where 20 take
-// 300.  FP32C, sigma 32, L2 flushed: 66 M 308 -> 290, 20 M 112 -> 101.
+// Warps of the one CTA per SM: 24, except for FP64 on scattered columns (Handle::scattered), where the
+// gathers' latency counts and 20 warps with 96 registers, which keep more of a chunk in flight, are
+// faster than 24 with 80: sigma 16, 32-bit columns, power law, 66 M nonzeros 338 -> 313 us a product in
+// a loop, 20 M 118 -> 107 with L2 flushed; local columns lose by it (stencil 128^3 150 -> 155, dense
+// blocks 114 -> 122).  16 warps with 128 registers: 302 us where 20 take 300.
+// One CTA puts that many neighbouring chunks on the SM, which share lines of x: 256 stacked small
+// matrices FP32 67 -> 51 us, FP64 105 -> 85, stencil 128^3 FP64 137 -> 134, power law of 102,000 rows
+// FP64 16.0 -> 12.0, against CTAs of 8 or 4 warps; CTAs of 12 or 10 lie between.
 template <typename VT, bool SCAT> struct Csr5Shape {
-    static constexpr int WARPS = SCAT ? 4 : 8, CTAS = !SCAT ? 3 : sizeof(VT) == 8 ? 5 : 6;
+    static_assert(!SCAT || sizeof(VT) == 8, "FP32 has one shape");
+    static constexpr int WARPS = SCAT ? 20 : 24, CTAS = 1;
 };
 
 // CSR5 SpMV (FP64 values; the FP32 form is csr5_spmv_f32_kernel below): one warp per chunk of
@@ -232,27 +234,26 @@ csr5_spmv_kernel(const ChunkHdr *__restrict__ hdr, const int *__restrict__ tile_
                  const unsigned *__restrict__ desc, const VT *__restrict__ vals,
                  const IT *__restrict__ cols, const VT *__restrict__ x,
                  double *__restrict__ y, double *__restrict__ carry_head,
-                 double *__restrict__ carry_tail, long long nchunks, int G, int m, int n,
+                 double *__restrict__ carry_tail, ChunkWalk<Csr5Shape<VT, SCAT>::WARPS> walk,
+                 int G, int m, int n,
                  unsigned long long *err) {
     constexpr int NBT = SIGMA / 4;  // blocks per tile
     constexpr int SPMV_WARPS = Csr5Shape<VT, SCAT>::WARPS;
     pdl_trigger();
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const uint64_t pf = policy_evict_first(), pl = policy_evict_last();
-    const long long nwarps = (long long)gridDim.x * SPMV_WARPS;
-    (void)w;
     constexpr int KSTK = 4;
     constexpr unsigned SLOT = SPMV_WARPS * 32 * 8;  // bytes between a thread's slots
     __shared__ __align__(16) double s_piece[KSTK * SPMV_WARPS * 32];
     const unsigned sbase = (unsigned)__cvta_generic_to_shared(&s_piece[threadIdx.x]);
 
-    for (long long c = (long long)blockIdx.x * SPMV_WARPS + w; c < nchunks; c += nwarps) {
+    for (unsigned c = walk.first(); walk.ok(c); c = walk.next(c)) {
         const ChunkHdr H = hdr[c];
         const int r_first = H.r_first, r_last = H.r_first + H.nrows - 1;
         const unsigned shared = H.shared;
         int carry_row = (shared & 1u) ? r_first : -1;
         double carry_val = 0.0;
-        const long long t0 = c * G;
+        const long long t0 = (long long)c * G;
         const VT *vb = vals + t0 * 32 * SIGMA;
         const IT *cb = cols + t0 * 32 * SIGMA;
         const int xbase = sizeof(IT) == 2 ? (int)((unsigned)H.aux >> 1) : 0;  // offsets' base
@@ -388,27 +389,27 @@ template <bool B> struct Flag { static constexpr bool value = B; };
 // choice and the tile-boundary checks are made once per tile instead of once per block.  The
 // compensated add makes this form instruction-issue bound, where the saved instructions are
 // time; the FP64 form is bandwidth bound, and unrolled it spills, so it keeps the block loop.
-template <int SIGMA, typename IT, bool SCAT>
-__global__ void __launch_bounds__(Csr5Shape<float, SCAT>::WARPS * 32, Csr5Shape<float, SCAT>::CTAS)
+template <int SIGMA, typename IT>
+__global__ void __launch_bounds__(Csr5Shape<float, false>::WARPS * 32, Csr5Shape<float, false>::CTAS)
 csr5_spmv_f32_kernel(const ChunkHdr *__restrict__ hdr, const int *__restrict__ tile_ptr,
                      const unsigned *__restrict__ desc, const float *__restrict__ vals,
                      const IT *__restrict__ cols, const float *__restrict__ x,
                      double *__restrict__ y, double *__restrict__ carry_head,
-                     double *__restrict__ carry_tail, long long nchunks, int G, int m, int n,
+                     double *__restrict__ carry_tail,
+                     ChunkWalk<Csr5Shape<float, false>::WARPS> walk, int G, int m, int n,
                      unsigned long long *err) {
     using VT = float;
     constexpr int NBT = SIGMA / 4;  // blocks per tile
-    constexpr int SPMV_WARPS = Csr5Shape<VT, SCAT>::WARPS;
+    constexpr int SPMV_WARPS = Csr5Shape<VT, false>::WARPS;
     pdl_trigger();
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const uint64_t pf = policy_evict_first(), pl = policy_evict_last();
-    const long long nwarps = (long long)gridDim.x * SPMV_WARPS;
     constexpr int KSTK = 4;
     constexpr unsigned SLOT = SPMV_WARPS * 32 * 8;  // bytes between a thread's slots
     __shared__ __align__(16) double s_piece[KSTK * SPMV_WARPS * 32];
     const unsigned sbase = (unsigned)__cvta_generic_to_shared(&s_piece[threadIdx.x]);
 
-    for (long long c = (long long)blockIdx.x * SPMV_WARPS + w; c < nchunks; c += nwarps) {
+    for (unsigned c = walk.first(); walk.ok(c); c = walk.next(c)) {
         const ChunkHdr H = hdr[c];
         const int r_first = H.r_first, r_last = H.r_first + H.nrows - 1;
         const unsigned shared = H.shared;
@@ -418,7 +419,7 @@ csr5_spmv_f32_kernel(const ChunkHdr *__restrict__ hdr, const int *__restrict__ t
         const bool chk = !SKIP || (H.aux & 1);
         int carry_row = (shared & 1u) ? r_first : -1;
         double carry_val = 0.0;
-        const long long t0 = c * G;
+        const long long t0 = (long long)c * G;
         const VT *vb = vals + t0 * 32 * SIGMA;
         const IT *cb = cols + t0 * 32 * SIGMA;
         const int xbase = sizeof(IT) == 2 ? (int)((unsigned)H.aux >> 1) : 0;  // offsets' base
@@ -561,16 +562,16 @@ cudaError_t convert_t(Handle &h, const int *rp, const int *ci, const double *v, 
 template <int SG, typename VT, typename IT, bool SCAT>
 cudaError_t launch_sg(const Handle &h, const void *x, void *y, cudaStream_t s) {
     using SH = Csr5Shape<VT, SCAT>;
-    const long long want = (h.nchunks + SH::WARPS - 1) / SH::WARPS;
     const long long cap = (long long)h.sm_count * SH::CTAS;
-    const unsigned grid = (unsigned)(want < cap ? want : cap);
+    const unsigned grid = (unsigned)(h.nchunks < cap ? h.nchunks : cap);
     auto go = [&](auto kernel) {
         return launch_product(kernel, grid, SH::WARPS * 32, 0, s, (const ChunkHdr *)h.meta,
                               h.tile_ptr, h.flags, (const VT *)h.vals, (const IT *)h.cols,
-                              (const VT *)x, (double *)y, h.carry_head, h.carry_tail, h.nchunks,
-                              h.G, h.m, h.n, guard_word());
+                              (const VT *)x, (double *)y, h.carry_head, h.carry_tail,
+                              ChunkWalk<SH::WARPS>::over(h.nchunks, grid), h.G, h.m, h.n,
+                              guard_word());
     };
-    if constexpr (sizeof(VT) == 4) return go(csr5_spmv_f32_kernel<SG, IT, SCAT>);
+    if constexpr (sizeof(VT) == 4) return go(csr5_spmv_f32_kernel<SG, IT>);
     else return go(csr5_spmv_kernel<SG, VT, IT, SCAT>);
 }
 
@@ -603,9 +604,8 @@ cudaError_t csr5_spmv(const Handle &h, const void *x, void *y, cudaStream_t s) {
     const bool f32 = h.precision == PAVA_PREC_FP32C, d16 = h.index_mode == PAVA_INDEX_DELTA16;
     if (d16)  // columns within 65,534 of one another in every chunk
         return f32 ? spmv_t<float, short, false>(h, x, y, s) : spmv_t<double, short, false>(h, x, y, s);
-    if (h.scattered)
-        return f32 ? spmv_t<float, int, true>(h, x, y, s) : spmv_t<double, int, true>(h, x, y, s);
-    return f32 ? spmv_t<float, int, false>(h, x, y, s) : spmv_t<double, int, false>(h, x, y, s);
+    if (f32) return spmv_t<float, int, false>(h, x, y, s);
+    return h.scattered ? spmv_t<double, int, true>(h, x, y, s) : spmv_t<double, int, false>(h, x, y, s);
 }
 
 }  // namespace pava

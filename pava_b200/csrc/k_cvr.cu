@@ -229,9 +229,13 @@ cvr_convert_kernel(const int *__restrict__ rp, const int *__restrict__ ci,
 // 164 / 144, 60^3 24.5 / 19.3, dense blocks 17 M nonzeros 57 / 48, Laplacian 512^2 (1,278 chunks)
 // 10.3 / 11.6; 32-bit columns, stencil 128^3 174 / 191, power law 66 M 310 / 349, 20 M 108 / 126.
 // 24 warps with 80 registers spill (stencil 196).  FP32: 24 warps.
+// Fewer, larger CTAs put more neighbouring chunks on one SM, where they share lines of x; the next
+// product's CTAs come in sooner with more, smaller ones.  FP32, one CTA of 24 against three of 8:
+// 256 stacked small matrices 87 -> 74 us, power law of 150,000 rows 17.3 -> 14.6 us.  FP64, two of 10
+// against five of 4: stacked matrices 98.5 -> 92 us, stencil 60^3 19.4 -> 19.2; one of 20: 79 and 22.8.
 template <typename VT, bool DEEP> struct CvrShape {
-    static constexpr int WARPS = sizeof(VT) == 8 && !DEEP ? 4 : 8;
-    static constexpr int CTAS = sizeof(VT) == 4 ? 3 : DEEP ? 2 : 5;
+    static constexpr int WARPS = sizeof(VT) == 4 ? 24 : DEEP ? 8 : 10;
+    static constexpr int CTAS = sizeof(VT) == 4 ? 1 : 2;
 };
 
 template <int S, typename VT, typename IT, bool DEEP>
@@ -240,7 +244,7 @@ cvr_spmv_kernel(const CvrMeta *__restrict__ meta, const unsigned *__restrict__ f
                 const VT *__restrict__ vals, const IT *__restrict__ cols,
                 const VT *__restrict__ x, const int *__restrict__ colbase,
                 double *__restrict__ y, double *__restrict__ carry_head,
-                double *__restrict__ carry_tail, long long nchunks, int m, int n,
+                double *__restrict__ carry_tail, ChunkWalk<CvrShape<VT, DEEP>::WARPS> walk, int m, int n,
                 unsigned long long *err) {
     constexpr int L = 32 * S;
     constexpr int NB = S / 4, SPMV_WARPS = CvrShape<VT, DEEP>::WARPS;
@@ -251,20 +255,18 @@ cvr_spmv_kernel(const CvrMeta *__restrict__ meta, const unsigned *__restrict__ f
     const unsigned lt = lanemask_lt();
     pdl_trigger();
 
-    const long long nwarps = (long long)gridDim.x * SPMV_WARPS;
-
-    for (long long c = (long long)blockIdx.x * SPMV_WARPS + w; c < nchunks; c += nwarps) {
+    for (unsigned c = walk.first(); walk.ok(c); c = walk.next(c)) {
         const CvrMeta *M = meta + c;
         const int r_first = M->h.r_first;
         const int r_last = r_first + M->h.nrows - 1;
         const unsigned shared = M->h.shared;
         const int i_t = M->i_t;
-        const VT *vb = vals + c * L;
-        const IT *cb = cols + c * L;
+        const VT *vb = vals + (long long)c * L;
+        const IT *cb = cols + (long long)c * L;
         const int xbase = sizeof(IT) == 2 ? colbase[c] : 0;  // base of the column offsets
         const VT *xb = x + xbase;
         const int xlo = -xbase, xhi = n - xbase;  // the offsets that stay inside x
-        const unsigned *fb = flags + c * S;
+        const unsigned *fb = flags + (long long)c * S;
         auto LF = [&](int b) { return ld_flag(fb + ((4 * b) >> 5) * 32 + lane); };
 
         Acc<VT> acc;
@@ -388,14 +390,14 @@ cudaError_t convert_t(Handle &h, const int *rp, const int *ci, const double *v, 
 template <typename VT, typename IT, bool DEEP>
 cudaError_t spmv_t(const Handle &h, const void *x, void *y, cudaStream_t s) {
     using SH = CvrShape<VT, DEEP>;
-    const long long want = (h.nchunks + SH::WARPS - 1) / SH::WARPS;
     const long long cap = (long long)h.sm_count * SH::CTAS;
-    const unsigned grid = (unsigned)(want < cap ? want : cap);
+    const unsigned grid = (unsigned)(h.nchunks < cap ? h.nchunks : cap);
     auto go = [&](auto kernel) {
         return launch_product(kernel, grid, SH::WARPS * 32, 0, s, (const CvrMeta *)h.meta,
                               h.flags, (const VT *)h.vals, (const IT *)h.cols, (const VT *)x,
-                              h.colbase, (double *)y, h.carry_head, h.carry_tail, h.nchunks, h.m,
-                              h.n, guard_word());
+                              h.colbase, (double *)y, h.carry_head, h.carry_tail,
+                              ChunkWalk<SH::WARPS>::over(h.nchunks, grid), h.m, h.n,
+                              guard_word());
     };
     switch (h.S) {
         case 32: return go(cvr_spmv_kernel<32, VT, IT, DEEP>);

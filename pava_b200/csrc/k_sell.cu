@@ -210,7 +210,7 @@ template <typename VT, typename IT>
 __global__ void __launch_bounds__(SELL_WARPS * 32, CTAS_PER_SM)
 sell_spmv_kernel(const SellSlice *__restrict__ meta, const VT *__restrict__ vals,
                  const IT *__restrict__ cols, const VT *__restrict__ x,
-                 double *__restrict__ y, long long nslices, int m, int n,
+                 double *__restrict__ y, ChunkWalk<SELL_WARPS> walk, int m, int n,
                  unsigned long long *err, unsigned long long *wait_err) {
     using ST = Stage<VT, IT>;
     constexpr int KB = ST::KB;
@@ -228,17 +228,16 @@ sell_spmv_kernel(const SellSlice *__restrict__ meta, const VT *__restrict__ vals
     }
     __syncwarp();
     const uint64_t pl = policy_evict_last();
-    const long long nwarps = (long long)gridDim.x * SELL_WARPS;
-    const long long first = (long long)blockIdx.x * SELL_WARPS + w;
+    const unsigned first = walk.first();
 
     // producer cursor: slice ps (with blocks), next block pb
-    long long ps = first;
+    unsigned ps = first;
     int pb = 0;
     SellSlice pm{0, 0, 0, 0u};
-    if (ps < nslices) pm = meta[ps];
-    while (ps < nslices && pm.nblk == 0) {
-        ps += nwarps;
-        if (ps < nslices) pm = meta[ps];
+    if (walk.ok(ps)) pm = meta[ps];
+    while (walk.ok(ps) && pm.nblk == 0) {
+        ps = walk.next(ps);
+        if (walk.ok(ps)) pm = meta[ps];
     }
     auto issue = [&](int k) {
         const int len = min(KB, pm.nblk - pb);
@@ -255,36 +254,36 @@ sell_spmv_kernel(const SellSlice *__restrict__ meta, const VT *__restrict__ vals
         if (pb >= pm.nblk) {
             pb = 0;
             do {
-                ps += nwarps;
-                if (ps < nslices) pm = meta[ps];
-            } while (ps < nslices && pm.nblk == 0);
+                ps = walk.next(ps);
+                if (walk.ok(ps)) pm = meta[ps];
+            } while (walk.ok(ps) && pm.nblk == 0);
         }
     };
     int pending = 0;
 #pragma unroll
     for (int k = 0; k < STAGES; ++k)
-        if (ps < nslices) { issue(k); ++pending; }
+        if (walk.ok(ps)) { issue(k); ++pending; }
 
     pdl_wait();  // x, and y, which the product before may still use: only copies of the format above
 
     // consumer cursor: slice cs, next block cb; it writes the rows of empty slices
-    long long cs = first;
+    unsigned cs = first;
     int cb = 0;
     SellSlice cm{0, 0, 0, 0u};
     auto skip_empty = [&]() {
-        while (cs < nslices) {
+        while (walk.ok(cs)) {
             cm = meta[cs];
             if (cm.nblk > 0) break;
-            const long long r = cs * 32 + lane;
+            const long long r = cs * 32ll + lane;
             if (r < m) y[r] = 0.0;
-            cs += nwarps;
+            cs = walk.next(cs);
         }
     };
     skip_empty();
     unsigned phases = 0;  // bit k: parity the consumer waits for on stage k
     int k = 0;
     RowAcc<VT> acc;
-    while (cs < nslices) {
+    while (walk.ok(cs)) {
         if (!mbar_wait(bar0 + 8 * k, (phases >> k) & 1u)) {
             if (lane == 0) {
                 atomicAdd(&wait_err[0], 1ull);
@@ -325,15 +324,15 @@ sell_spmv_kernel(const SellSlice *__restrict__ meta, const VT *__restrict__ vals
         }
         cb += KB;
         if (cb >= cm.nblk) {  // the slice's last piece
-            const long long r = cs * 32 + lane;
+            const long long r = cs * 32ll + lane;
             if (r < m) y[r] = acc.value();
             acc.reset();
             cb = 0;
-            cs += nwarps;
+            cs = walk.next(cs);
             skip_empty();
         }
         __syncwarp();  // every lane is done with stage k
-        if (ps < nslices) { issue(k); ++pending; }
+        if (walk.ok(ps)) { issue(k); ++pending; }
         k = k + 1 == STAGES ? 0 : k + 1;
     }
     // only after a wait gave up: let the copies still in flight land before the CTA exits
@@ -366,13 +365,12 @@ cudaError_t spmv_t(const Handle &h, const void *x, void *y, cudaStream_t s) {
         if (e != cudaSuccess) return e;
         opted.fetch_or(bit);
     }
-    const long long want = (h.nchunks + SELL_WARPS - 1) / SELL_WARPS;
     const long long cap = (long long)h.sm_count * CTAS_PER_SM;
-    const unsigned grid = (unsigned)(want < cap ? want : cap);
+    const unsigned grid = (unsigned)(h.nchunks < cap ? h.nchunks : cap);
     return launch_product(sell_spmv_kernel<VT, IT>, grid, SELL_WARPS * 32, ST::CTA_BYTES, s,
                           (const SellSlice *)h.meta, (const VT *)h.vals, (const IT *)h.cols,
-                          (const VT *)x, (double *)y, h.nchunks, h.m, h.n, guard_word(),
-                          wait_word());
+                          (const VT *)x, (double *)y, ChunkWalk<SELL_WARPS>::over(h.nchunks, grid),
+                          h.m, h.n, guard_word(), wait_word());
 }
 
 }  // namespace

@@ -139,3 +139,43 @@ def test_cvr_chunks_around_a_full_gpu(cuda, extra):
             y = mat.spmv(xd.float() if prec == _abi.PREC_FP32C else xd).cpu().numpy()
             assert O.rel_error(y, yr, ab, bound)[0] == 0, (prec, mode)
             mat.close()
+
+
+@pytest.mark.parametrize("units", [1, 2, 147, 149, 443, 445, 591, 593, 739, 741, 2367, 2369, 3553, 4737])
+def test_every_chunk_is_taken_once(cuda, units):
+    """Chunk and slice counts around the CTAs and the warps that 148 SMs hold in each kernel."""
+    torch = cuda
+    rng = np.random.default_rng(units)
+    m = 32 * units - 5                    # rows of 8: CSR5 chunks of 256 elements, slices of 32 rows
+    ci = np.sort((np.arange(m)[:, None] * 3 + np.arange(8) * 11 + rng.integers(0, 11, (m, 8))) % 4999, 1)
+    A = M.from_arrays(m, 4999, np.arange(0, 8 * m + 1, 8), ci.ravel().astype(np.int32),
+                      M.uniform(8 * m, seed=14, fp32=True))
+    x = M.uniform(A.n, seed=15, fp32=True)
+    yr, ab = O.csr_ref(A.rp, A.ci, A.v, x)
+    for fmt, kw in (("cvr", dict(steps=32)), ("csr5", dict(sigma=8, tiles_per_chunk=1)), ("sell", {})):
+        for prec, bound in ((_abi.PREC_FP64, 1e-12), (_abi.PREC_FP32C, 1e-9)):
+            for mode in (_abi.INDEX_DELTA16, _abi.INDEX_I32):
+                mat = SpMatrix(A, fmt, precision=prec, index_mode=mode, **kw)
+                xd = torch.from_numpy(x).cuda()
+                y = torch.full((m,), float("nan"), dtype=torch.float64, device="cuda")
+                mat.spmv(xd.float() if prec == _abi.PREC_FP32C else xd, y)
+                assert O.rel_error(y.cpu().numpy(), yr, ab, bound)[0] == 0, (fmt, prec, mode)
+                mat.close()
+
+
+@pytest.mark.parametrize("fmt,kw", [("cvr", dict(steps=32)), ("csr5", dict(sigma=8, tiles_per_chunk=4))])
+def test_rows_over_a_few_chunks(cuda, fmt, kw):
+    """Rows over 1 to 40 chunks of 1,024 elements, neighbours ending in the same 32 chunks."""
+    torch = cuda
+    rng = np.random.default_rng(16)
+    spans = [s for s in range(1, 12) for _ in range(5)] + [40, 33, 32, 31, 2, 2, 9, 8, 7]
+    lens = [int(s * 1024 + rng.integers(-500, 500)) for s in rng.permutation(spans)]
+    A = _csr([np.sort(rng.choice(50_000, k, replace=False)) for k in lens], 50_000, 17)
+    x = M.uniform(A.n, seed=18, fp32=True)
+    yr, ab = O.csr_ref(A.rp, A.ci, A.v, x)
+    for prec, bound in ((_abi.PREC_FP64, 1e-12), (_abi.PREC_FP32C, 1e-9)):
+        mat = SpMatrix(A, fmt, precision=prec, **kw)
+        xd = torch.from_numpy(x).cuda()
+        y = mat.spmv(xd.float() if prec == _abi.PREC_FP32C else xd)
+        assert O.rel_error(y.cpu().numpy(), yr, ab, bound)[0] == 0, prec
+        mat.close()
