@@ -208,11 +208,13 @@ __global__ void set_int_kernel(int *p, int v) { *p = v; }
 // One thread per chunk c1.  A row R that spans chunks c0 < c1 (it starts in c0 and ends in c1)
 // gets y[R] = carry_tail[c0] + sum(carry_head[c0+1 .. c1]); chunks in between lie entirely
 // inside R and hold their whole contribution in carry_head.  Nearly always c0 = c1 - 1, which the
-// header of c1 - 1 tells, so one round of independent reads is enough; longer rows are summed by
-// the warp, one after the other, in a fixed order (lane-strided partial sums, then a fixed
-// butterfly), so y is the same on every call.
+// header of c1 - 1 tells, so one round of independent reads is enough.  Rows over up to nine
+// chunks are summed by their thread, longer ones by the warp, one after the other, both in the same
+// fixed order (lane-strided partial sums, then a fixed butterfly), so y is the same on every call.
 // Bound by latency: a warp per chunk with the dependent reads header -> arp -> carries took 11.5 us
-// for 32,245 chunks and 4.7 us for 640 after the SpMV kernel, this form 6.2 and 3.5 us.
+// for 32,245 chunks and 4.7 us for 640 after the SpMV kernel, this form 6.2 and 3.5 us.  Power-law
+// matrices have many rows over three to nine chunks: summed by the warp too, they cost a product
+// of 100,000 to 700,000 rows about 1 us.
 __global__ void __launch_bounds__(128)
 carry_fixup_kernel(const char *__restrict__ meta, size_t stride, const int *__restrict__ arp,
                    long long L, const double *carry_head, const double *carry_tail, double *y,
@@ -223,6 +225,7 @@ carry_fixup_kernel(const char *__restrict__ meta, size_t stride, const int *__re
     // the headers belong to the matrix: read before the wait
     int R = -1;
     bool two = false;  // R starts in c1 - 1 and ends in c1
+    long long c0 = c1;
     if (c1 > 0 && c1 < nchunks) {
         const ChunkHdr *H = reinterpret_cast<const ChunkHdr *>(meta + c1 * stride);
         const ChunkHdr *P = reinterpret_cast<const ChunkHdr *>(meta + (c1 - 1) * stride);
@@ -230,22 +233,30 @@ carry_fixup_kernel(const char *__restrict__ meta, size_t stride, const int *__re
         // R ends in c1, unless it runs through c1 and beyond
         if ((sh & 1u) && !((sh & 2u) && H->nrows == 1)) R = H->r_first;
         two = P->nrows > 1 || !(psh & 1u);
+        if (R >= m || !guard(err, R >= -1, G_Y, R)) R = -1;
+        if (R >= 0) c0 = two ? c1 - 1 : (long long)arp[R] / L;
+        if (!guard(err, c0 >= 0 && c0 <= c1, G_CARRY, c0)) R = -1;
     }
     pdl_wait();  // the SpMV kernel's carries
-    if (R >= m || !guard(err, R >= -1, G_Y, R)) R = -1;
     if (R >= 0 && two) y[R] = carry_tail[c1 - 1] + carry_head[c1];
-    unsigned todo = __ballot_sync(FULL, R >= 0 && !two);
+    const bool few = c1 - c0 <= 8;
+    if (R >= 0 && !two && few) {
+        double h[8];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) h[j] = c0 + 1 + j <= c1 ? carry_head[c0 + 1 + j] : 0.0;
+        // the order of warp_sum, so a row's sum does not depend on the branch
+        y[R] = carry_tail[c0] + (((h[0] + h[4]) + (h[2] + h[6])) + ((h[1] + h[5]) + (h[3] + h[7])));
+    }
+    unsigned todo = __ballot_sync(FULL, R >= 0 && !few);
     while (todo) {
         const int src = __ffs(todo) - 1;
         todo &= todo - 1;
         const int row = __shfl_sync(FULL, R, src);
-        const long long c = __shfl_sync(FULL, c1, src);
-        const long long c0 = (long long)arp[row] / L;
-        if (!guard(err, c0 >= 0 && c0 <= c, G_CARRY, c0)) continue;
+        const long long c = __shfl_sync(FULL, c1, src), b = __shfl_sync(FULL, c0, src);
         double p = 0.0;
-        for (long long j = c0 + 1 + lane; j <= c; j += 32) p += carry_head[j];
+        for (long long j = b + 1 + lane; j <= c; j += 32) p += carry_head[j];
         p = warp_sum(p);
-        if (lane == 0) y[row] = carry_tail[c0] + p;
+        if (lane == 0) y[row] = carry_tail[b] + p;
     }
 }
 
