@@ -51,7 +51,8 @@ namespace {
 constexpr int SPMM_UNROLL = 2;  // blocks of a piece unrolled together
 // Neighbouring slices a CTA takes in a row: they share X rows, but long runs keep distant regions
 // of X alive at once (stencil, k = 16: 249, 251, 254 and 304 us at 1, 2, 4 and 16; FP32C 214, 202,
-// 200, 208).  One at a time where the matrix has fewer than four runs per resident CTA.
+// 200, 208).  One at a time where the matrix has few runs per resident CTA: fewer than 4 for FP32
+// (stencil 80^3, k = 32: 202 us one at a time, 196 in runs), 16 for FP64 (169 and 175).
 constexpr int RUN = 2;  // a power of two
 template <int G> struct SpmmShape {
     static_assert(G == 4 || G == 8 || G == 16, "lanes per row");
@@ -84,7 +85,7 @@ __device__ __forceinline__ void row_cols(const short *pc, int i, int r, int (&c)
     c[2] = (int)(a.y << 16) >> 16; c[3] = (int)a.y >> 16;
 }
 
-// LD: the type of X's leading dimension; int (VW = 2) makes a row address one multiply-add.
+// LD: the type of X's leading dimension; int makes a row address one multiply-add.
 template <typename VT, typename IT, int G, int KPL, int VW, typename LD>
 __global__ void __launch_bounds__(SpmmShape<G>::THREADS, SpmmShape<G>::CTAS_PER_SM)
 sell_spmm_kernel(const SellSlice *__restrict__ meta, const VT *__restrict__ vals,
@@ -188,17 +189,19 @@ sell_spmm_kernel(const SellSlice *__restrict__ meta, const VT *__restrict__ vals
     double acc[KPL];
 #pragma unroll
     for (int p = 0; p < KPL; ++p) acc[p] = 0.0;
-    // column offsets of the lane's reads; a slot past k reads column 0 and is never stored
+    // Column offsets of the lane's reads.  Only the last slot can lie past k: a pair of it reads the
+    // last columns, whose line other lanes read anyway; a single column of it is not read.
     int xoff[KPL / VW];
 #pragma unroll
     for (int p = 0; p < KPL; p += VW) {
         const int c = spmm_col<G, VW>(lg, p);
-        xoff[p / VW] = c < k ? c : 0;
+        xoff[p / VW] = c < k ? c : k - VW;
     }
+    const bool last = VW == 2 || spmm_col<G, VW>(lg, KPL - VW) < k;
     auto sum_block = [&](const VT *pv, const IT *pc, int i, auto pads_tag) {
         constexpr bool PADS = decltype(pads_tag)::value;
         // elements whose X reads are in flight together: a block's four, where registers allow
-        constexpr int QB = KPL >= 8 || PADS ? 2 : 4;
+        constexpr int QB = VW == 1 && KPL >= 3 ? 1 : KPL > 4 || PADS ? 2 : 4;
         int c[4];
         row_cols(pc, i, r, c);
         const VBlk<VT> vv = VBlk<VT>::load_smem(pv, i, r);
@@ -219,7 +222,7 @@ sell_spmm_kernel(const SellSlice *__restrict__ meta, const VT *__restrict__ vals
                         xv[q][p] = x2.x;
                         xv[q][p + 1] = x2.y;
                     } else {
-                        xv[q][p] = ld_x(xr + xoff[p], pl);
+                        xv[q][p] = p < KPL - 1 || last ? ld_x(xr + xoff[p], pl) : VT(0);
                     }
                 }
             }
@@ -271,11 +274,10 @@ sell_spmm_kernel(const SellSlice *__restrict__ meta, const VT *__restrict__ vals
     }
 }
 
-template <typename VT, typename IT, int G, int KPL, int VW>
+template <typename VT, typename IT, int G, int KPL, int VW, typename LD = int>
 cudaError_t spmm_launch(const Handle &h, const VT *X, long long ldx, double *Y, long long ldy,
                         int k, cudaStream_t s) {
     using ST = SpmmStage<VT, IT, G>;
-    using LD = std::conditional_t<VW == 2, int, long long>;
     constexpr auto kernel = sell_spmm_kernel<VT, IT, G, KPL, VW, LD>;
     // more than the default 48 KB of dynamic shared memory: opted into once per device
     static std::atomic<unsigned long long> opted{0};
@@ -288,7 +290,7 @@ cudaError_t spmm_launch(const Handle &h, const VT *X, long long ldx, double *Y, 
         opted.fetch_or(bit);
     }
     const long long cap = (long long)h.sm_count * SpmmShape<G>::CTAS_PER_SM;
-    const int run = h.nchunks >= 4 * RUN * cap ? RUN : 1;
+    const int run = h.nchunks >= (sizeof(VT) == 8 ? 16 : 4) * RUN * cap ? RUN : 1;
     const long long runs = (h.nchunks + run - 1) / run;
     const unsigned grid = (unsigned)(runs < cap ? runs : cap);
     return launch_product(kernel, grid, SpmmShape<G>::THREADS, ST::BYTES, s,
@@ -296,38 +298,53 @@ cudaError_t spmm_launch(const Handle &h, const VT *X, long long ldx, double *Y, 
                           (LD)ldx, Y, ldy, (int)h.nchunks, run, h.m, h.n, k, guard_word(), wait_word());
 }
 
-// KPL = the columns per lane that cover k with G lanes; pairs per read where they can be
+// KPL = ceil(k / G), so that a lane reads no slot that no lane needs (k = 21 on eight lanes: three,
+// not four); pairs per read where they can be, with KPL rounded up to even.  Single columns are read
+// element by element (QB = 1): two or four elements at once spill.  In a loop, us, KPL a power of two
+// with four elements in flight / this: k = 21, stencil 60^3 107 / 81 (FP32 91 / 71), dense blocks
+// 200,000 rows 185 / 126 (176 / 123); k = 13 dense blocks 106 / 83.
 template <typename VT, typename IT, int G, int KPL>
 cudaError_t spmm_vw(const Handle &h, const VT *X, long long ldx, double *Y, long long ldy,
                     int k, cudaStream_t s) {
-    const bool vec2 = KPL >= 2 && k % 2 == 0 && ldx % 2 == 0 && ldy % 2 == 0 && ldx <= INT_MAX &&
+    if (ldx > INT_MAX)  // 64-bit row offsets: one kernel for every k
+        return spmm_launch<VT, IT, 8, 8, 1, long long>(h, X, ldx, Y, ldy, k, s);
+    const bool vec2 = KPL >= 2 && k % 2 == 0 && ldx % 2 == 0 && ldy % 2 == 0 &&
                       reinterpret_cast<uintptr_t>(X) % (2 * sizeof(VT)) == 0 &&
                       reinterpret_cast<uintptr_t>(Y) % 16 == 0;
     if constexpr (KPL >= 2)
-        if (vec2) return spmm_launch<VT, IT, G, KPL, 2>(h, X, ldx, Y, ldy, k, s);
+        if (vec2) return spmm_launch<VT, IT, G, KPL + KPL % 2, 2>(h, X, ldx, Y, ldy, k, s);
     return spmm_launch<VT, IT, G, KPL, 1>(h, X, ldx, Y, ldy, k, s);
+}
+
+template <typename VT, typename IT, int G>
+cudaError_t spmm_g(const Handle &h, const VT *X, long long ldx, double *Y, long long ldy, int k,
+                   cudaStream_t s) {
+    switch ((k + G - 1) / G) {
+        case 1: return spmm_vw<VT, IT, G, 1>(h, X, ldx, Y, ldy, k, s);
+        case 2: return spmm_vw<VT, IT, G, 2>(h, X, ldx, Y, ldy, k, s);
+        case 3: return spmm_vw<VT, IT, G, 3>(h, X, ldx, Y, ldy, k, s);
+        case 4: return spmm_vw<VT, IT, G, 4>(h, X, ldx, Y, ldy, k, s);
+    }
+    if constexpr (G <= 8) {
+        switch ((k + G - 1) / G) {
+            case 5: return spmm_vw<VT, IT, G, 5>(h, X, ldx, Y, ldy, k, s);
+            case 6: return spmm_vw<VT, IT, G, 6>(h, X, ldx, Y, ldy, k, s);
+            case 7: return spmm_vw<VT, IT, G, 7>(h, X, ldx, Y, ldy, k, s);
+            case 8: return spmm_vw<VT, IT, G, 8>(h, X, ldx, Y, ldy, k, s);
+        }
+    }
+    return cudaErrorInvalidValue;
 }
 
 template <typename VT, typename IT>
 cudaError_t spmm_k(const Handle &h, const VT *X, long long ldx, double *Y, long long ldy, int k,
                    cudaStream_t s) {
-    const int g = sell_spmm_lanes(h.lanes_per_row, k);
-    if (g == 4) {
-        if (k <= 4) return spmm_vw<VT, IT, 4, 1>(h, X, ldx, Y, ldy, k, s);
-        if (k <= 8) return spmm_vw<VT, IT, 4, 2>(h, X, ldx, Y, ldy, k, s);
-        if (k <= 16) return spmm_vw<VT, IT, 4, 4>(h, X, ldx, Y, ldy, k, s);
-        if (k <= 32) return spmm_vw<VT, IT, 4, 8>(h, X, ldx, Y, ldy, k, s);
-    } else if (g == 8) {
-        if (k <= 8) return spmm_vw<VT, IT, 8, 1>(h, X, ldx, Y, ldy, k, s);
-        if (k <= 16) return spmm_vw<VT, IT, 8, 2>(h, X, ldx, Y, ldy, k, s);
-        if (k <= 32) return spmm_vw<VT, IT, 8, 4>(h, X, ldx, Y, ldy, k, s);
-        if (k <= 64) return spmm_vw<VT, IT, 8, 8>(h, X, ldx, Y, ldy, k, s);
-    } else if (g == 16) {
-        if (k <= 16) return spmm_vw<VT, IT, 16, 1>(h, X, ldx, Y, ldy, k, s);
-        if (k <= 32) return spmm_vw<VT, IT, 16, 2>(h, X, ldx, Y, ldy, k, s);
-        if (k <= 64) return spmm_vw<VT, IT, 16, 4>(h, X, ldx, Y, ldy, k, s);
+    switch (sell_spmm_lanes(h.lanes_per_row, k, sizeof(VT) == 4, (long long)h.nnz >= 16LL * h.m)) {
+        case 4: return spmm_g<VT, IT, 4>(h, X, ldx, Y, ldy, k, s);
+        case 8: return spmm_g<VT, IT, 8>(h, X, ldx, Y, ldy, k, s);
+        case 16: return spmm_g<VT, IT, 16>(h, X, ldx, Y, ldy, k, s);
+        default: return cudaErrorInvalidValue;
     }
-    return cudaErrorInvalidValue;
 }
 
 }  // namespace

@@ -202,12 +202,18 @@ cudaError_t sell_fill(Handle &h, const int *rp, const int *ci, const double *v,
                       const int *d_blk_off, cudaStream_t s);
 cudaError_t sell_spmv(const Handle &h, const void *x, void *y, cudaStream_t s);
 // SELL SpMM, Y = A X with X row-major n x k; leading dimensions ldx, ldy in elements.  Lanes per
-// row (h.lanes_per_row): 4 (k <= 32), 8 (k <= 64) or 16 (k <= 64); 0 = 4 for k <= 16, else 8.
+// row (h.lanes_per_row): 4 (k <= 32), 8 (k <= 64) or 16 (k <= 64); 0 = the engine's choice.
 // sell_spmm_lanes gives the lanes it uses for k, 0 when the handle's choice cannot serve k
 // (sell_spmm then returns cudaErrorInvalidValue).
 constexpr int SELL_SPMM_MAX_K = 64;
-inline int sell_spmm_lanes(int lanes_per_row, int k) {
-    const int g = lanes_per_row ? lanes_per_row : (k <= 16 ? 4 : 8);
+// The engine's choice (lanes_per_row 0): four lanes, whose warp reads eight rows' X at once, while the
+// sums fit its registers: FP32 up to k = 24, odd k up to 28; FP64 up to k = 12, or 16 where rows are
+// short (under 16 elements).  FP64 in a loop, us, 4 / 8 lanes: stencil 60^3 k = 13 70 / 63, k = 16
+// 58 / 46, banded 500,000 rows k = 15 167 / 119, dense blocks k = 12 75 / 77, Laplacian 900^2 k = 13
+// 75 / 93; FP32 banded k = 20 116 / 160, k = 27 157 / 186, stencil k = 32 101 / 78.
+inline int sell_spmm_lanes(int lanes_per_row, int k, bool f32 = false, bool long_rows = false) {
+    const int four = f32 ? (k % 2 ? 28 : 24) : long_rows ? 12 : 16;
+    const int g = lanes_per_row ? lanes_per_row : (k <= four ? 4 : 8);
     if (g == 4) return k <= 32 ? 4 : 0;
     if (g == 8 || g == 16) return k <= SELL_SPMM_MAX_K ? g : 0;
     return 0;

@@ -48,3 +48,41 @@ def test_pieces(cuda, name, A, index, prec):
                 yr, ab = O.csr_ref(A.rp, A.ci, A.v, X[:, j].copy())
                 assert O.rel_error(Yh[:, j].copy(), yr, ab, 1e-12)[0] == 0, (lanes, k, j)
         mat.close()
+
+
+@pytest.mark.parametrize("prec", [_abi.PREC_FP64, _abi.PREC_FP32C])
+@pytest.mark.parametrize("lanes", [0, 4, 8, 16])
+@pytest.mark.parametrize("per_row", [5, 20])
+def test_every_column_count(cuda, per_row, lanes, prec):
+    """Each number of columns per lane, whole and partly filled, aligned and not, short and long rows."""
+    torch = cuda
+    fp32 = prec == _abi.PREC_FP32C
+    A = _csr(np.full(300, per_row), 150, 8)
+    mat = SpMatrix(A, "sell", precision=prec, lanes_per_row=lanes)
+    top = 32 if lanes == 4 else 64
+    X = np.stack([M.uniform(A.n, seed=10 + j, fp32=True) for j in range(top)], 1)
+    refs = [O.csr_ref(A.rp, A.ci, A.v, X[:, j].copy()) for j in range(top)]
+    Xd = torch.from_numpy(X).cuda()
+    Xd = Xd.float() if fp32 else Xd
+    for k in range(1, top + 1):
+        for ld in {k, k + 1, k + 2}:
+            Xk = torch.full((A.n, ld), float("nan"), dtype=Xd.dtype, device="cuda")[:, :k]
+            Xk.copy_(Xd[:, :k])
+            Y = mat.spmm(Xk).cpu().numpy()
+            for j in {0, k // 2, k - 1}:
+                yr, ab = refs[j]
+                assert O.rel_error(Y[:, j].copy(), yr, ab, 1e-12)[0] == 0, (k, ld, j)
+
+
+@pytest.mark.parametrize("lanes,k", [(0, 3), (4, 32), (16, 64)])
+def test_leading_dimension_past_int(cuda, lanes, k):
+    torch = cuda
+    A = _csr([1, 0, 1] * 20, 2, 9)
+    ld = 2**31 + 5
+    X = torch.empty(ld + k, dtype=torch.float32, device="cuda").as_strided((2, k), (ld, 1))
+    X.copy_(torch.arange(2.0 * k, device="cuda").reshape(2, k))
+    mat = SpMatrix(A, "sell", precision=_abi.PREC_FP32C, lanes_per_row=lanes)
+    Y = mat.spmm(X).cpu().numpy()
+    for j in range(k):
+        yr, ab = O.csr_ref(A.rp, A.ci, A.v, X[:, j].double().cpu().numpy().copy())
+        assert O.rel_error(Y[:, j].copy(), yr, ab, 1e-12)[0] == 0, j
