@@ -205,17 +205,20 @@ __device__ __forceinline__ void tile_combine(double head, double tail, bool seen
     }
 }
 
-// Warps of the one CTA per SM: 24, except for FP64 on scattered columns (Handle::scattered), where the
-// gathers' latency counts and 20 warps with 96 registers, which keep more of a chunk in flight, are
-// faster than 24 with 80: sigma 16, 32-bit columns, power law, 66 M nonzeros 338 -> 313 us a product in
-// a loop, 20 M 118 -> 107 with L2 flushed; local columns lose by it (stencil 128^3 150 -> 155, dense
-// blocks 114 -> 122).  16 warps with 128 registers: 302 us where 20 take 300.
+// Warps per CTA and CTAs per SM.
+// FP64: 24 warps with 80 registers for 16-bit columns, 20 with 96 for 32-bit ones, which spill at 80 and
+// keep more of a chunk in flight at 96.  A product in a loop, us, 24 / 20 warps: 32-bit columns, stencil
+// 72^3 37.3 / 30.1, 128^3 158 / 150, dense blocks 17 M nonzeros 56 / 45, power law 66 M 338 / 294;
+// 16-bit columns, stencil 100^3 66.6 / 70.4, 128^3 135 / 143, Laplacian 2000^2 62 / 67 (dense blocks
+// 8.6 M 31.4 / 28.2).  16 warps with 128 registers: power law 302 where 20 took 300.
 // One CTA puts that many neighbouring chunks on the SM, which share lines of x: 256 stacked small
-// matrices FP32 67 -> 51 us, FP64 105 -> 85, stencil 128^3 FP64 137 -> 134, power law of 102,000 rows
+// matrices FP32 67 -> 51 us, FP64 105 -> 85, stencil 128^3 FP64 138 -> 135, power law of 102,000 rows
 // FP64 16.0 -> 12.0, against CTAs of 8 or 4 warps; CTAs of 12 or 10 lie between.
-template <typename VT, bool SCAT> struct Csr5Shape {
-    static_assert(!SCAT || sizeof(VT) == 8, "FP32 has one shape");
-    static constexpr int WARPS = SCAT ? 20 : 24, CTAS = 1;
+// FP32: one CTA of 24, but three of 8 for 32-bit columns that are not scattered (Handle::scattered):
+// stencil 128^3 115 -> 108, dense blocks 17 M 41.6 -> 38.6; power law 20 M 88 -> 90.
+template <typename VT, typename IT, bool SCAT> struct Csr5Shape {
+    static constexpr bool F64 = sizeof(VT) == 8, ONE = F64 || sizeof(IT) == 2 || SCAT;
+    static constexpr int WARPS = !ONE ? 8 : F64 && sizeof(IT) == 4 ? 20 : 24, CTAS = ONE ? 1 : 3;
 };
 
 // CSR5 SpMV (FP64 values; the FP32 form is csr5_spmv_f32_kernel below): one warp per chunk of
@@ -229,16 +232,16 @@ template <typename VT, bool SCAT> struct Csr5Shape {
 // with) joins the cross-lane combine and pieces 1 .. k-1, rows that start and end in the
 // lane, go to y.  Other tiles write each finished row as it ends.
 template <int SIGMA, typename VT, typename IT, bool SCAT>
-__global__ void __launch_bounds__(Csr5Shape<VT, SCAT>::WARPS * 32, Csr5Shape<VT, SCAT>::CTAS)
+__global__ void __launch_bounds__(Csr5Shape<VT, IT, SCAT>::WARPS * 32, Csr5Shape<VT, IT, SCAT>::CTAS)
 csr5_spmv_kernel(const ChunkHdr *__restrict__ hdr, const int *__restrict__ tile_ptr,
                  const unsigned *__restrict__ desc, const VT *__restrict__ vals,
                  const IT *__restrict__ cols, const VT *__restrict__ x,
                  double *__restrict__ y, double *__restrict__ carry_head,
-                 double *__restrict__ carry_tail, ChunkWalk<Csr5Shape<VT, SCAT>::WARPS> walk,
+                 double *__restrict__ carry_tail, ChunkWalk<Csr5Shape<VT, IT, SCAT>::WARPS> walk,
                  int G, int m, int n,
                  unsigned long long *err) {
     constexpr int NBT = SIGMA / 4;  // blocks per tile
-    constexpr int SPMV_WARPS = Csr5Shape<VT, SCAT>::WARPS;
+    constexpr int SPMV_WARPS = Csr5Shape<VT, IT, SCAT>::WARPS;
     pdl_trigger();
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const uint64_t pf = policy_evict_first(), pl = policy_evict_last();
@@ -389,18 +392,18 @@ template <bool B> struct Flag { static constexpr bool value = B; };
 // choice and the tile-boundary checks are made once per tile instead of once per block.  The
 // compensated add makes this form instruction-issue bound, where the saved instructions are
 // time; the FP64 form is bandwidth bound, and unrolled it spills, so it keeps the block loop.
-template <int SIGMA, typename IT>
-__global__ void __launch_bounds__(Csr5Shape<float, false>::WARPS * 32, Csr5Shape<float, false>::CTAS)
+template <int SIGMA, typename IT, bool SCAT>
+__global__ void __launch_bounds__(Csr5Shape<float, IT, SCAT>::WARPS * 32, Csr5Shape<float, IT, SCAT>::CTAS)
 csr5_spmv_f32_kernel(const ChunkHdr *__restrict__ hdr, const int *__restrict__ tile_ptr,
                      const unsigned *__restrict__ desc, const float *__restrict__ vals,
                      const IT *__restrict__ cols, const float *__restrict__ x,
                      double *__restrict__ y, double *__restrict__ carry_head,
                      double *__restrict__ carry_tail,
-                     ChunkWalk<Csr5Shape<float, false>::WARPS> walk, int G, int m, int n,
+                     ChunkWalk<Csr5Shape<float, IT, SCAT>::WARPS> walk, int G, int m, int n,
                      unsigned long long *err) {
     using VT = float;
     constexpr int NBT = SIGMA / 4;  // blocks per tile
-    constexpr int SPMV_WARPS = Csr5Shape<VT, false>::WARPS;
+    constexpr int SPMV_WARPS = Csr5Shape<VT, IT, SCAT>::WARPS;
     pdl_trigger();
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const uint64_t pf = policy_evict_first(), pl = policy_evict_last();
@@ -561,7 +564,7 @@ cudaError_t convert_t(Handle &h, const int *rp, const int *ci, const double *v, 
 
 template <int SG, typename VT, typename IT, bool SCAT>
 cudaError_t launch_sg(const Handle &h, const void *x, void *y, cudaStream_t s) {
-    using SH = Csr5Shape<VT, SCAT>;
+    using SH = Csr5Shape<VT, IT, SCAT>;
     const long long cap = (long long)h.sm_count * SH::CTAS;
     const unsigned grid = (unsigned)(h.nchunks < cap ? h.nchunks : cap);
     auto go = [&](auto kernel) {
@@ -571,7 +574,7 @@ cudaError_t launch_sg(const Handle &h, const void *x, void *y, cudaStream_t s) {
                               ChunkWalk<SH::WARPS>::over(h.nchunks, grid), h.G, h.m, h.n,
                               guard_word());
     };
-    if constexpr (sizeof(VT) == 4) return go(csr5_spmv_f32_kernel<SG, IT>);
+    if constexpr (sizeof(VT) == 4) return go(csr5_spmv_f32_kernel<SG, IT, SCAT>);
     else return go(csr5_spmv_kernel<SG, VT, IT, SCAT>);
 }
 
@@ -604,8 +607,8 @@ cudaError_t csr5_spmv(const Handle &h, const void *x, void *y, cudaStream_t s) {
     const bool f32 = h.precision == PAVA_PREC_FP32C, d16 = h.index_mode == PAVA_INDEX_DELTA16;
     if (d16)  // columns within 65,534 of one another in every chunk
         return f32 ? spmv_t<float, short, false>(h, x, y, s) : spmv_t<double, short, false>(h, x, y, s);
-    if (f32) return spmv_t<float, int, false>(h, x, y, s);
-    return h.scattered ? spmv_t<double, int, true>(h, x, y, s) : spmv_t<double, int, false>(h, x, y, s);
+    if (!f32) return spmv_t<double, int, false>(h, x, y, s);
+    return h.scattered ? spmv_t<float, int, true>(h, x, y, s) : spmv_t<float, int, false>(h, x, y, s);
 }
 
 }  // namespace pava
