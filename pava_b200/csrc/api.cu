@@ -622,11 +622,9 @@ pava_status pava_create(const pava_csr *A, int format, const pava_opts *opts, vo
         if (ce == cudaSuccess && chunked) ce = dalloc(&h.arp, (size_t)h.m + 2, &h.device_bytes, s);
         if (ce == cudaSuccess && chunked)
             ce = pava::build_augmented_rowptr(rp, h.m, h.arp, d_chk + 1, s);
-        const bool sample = format == PAVA_FORMAT_CSR5;
-        if (ce == cudaSuccess && sample) ce = pava::sample_lines(ci, h.nnz, d_chk + 2, s);
+        if (ce == cudaSuccess && chunked) ce = pava::sample_lines(ci, h.nnz, d_chk + 2, s);
         if (ce == cudaSuccess)
-            ce = cudaMemcpyAsync(chk, d_chk, sizeof(int) * (sample ? 3 : chunked ? 2 : 1),
-                                 cudaMemcpyDeviceToHost, s);
+            ce = cudaMemcpyAsync(chk, d_chk, sizeof(int) * (chunked ? 3 : 1), cudaMemcpyDeviceToHost, s);
         if (ce == cudaSuccess) ce = cudaStreamSynchronize(s);
         pava::pool_free(d_chk, s);
         if (ce != cudaSuccess) {

@@ -232,22 +232,24 @@ cvr_convert_kernel(const int *__restrict__ rp, const int *__restrict__ ci,
 // Fewer, larger CTAs put more neighbouring chunks on one SM, where they share lines of x; the next
 // product's CTAs come in sooner with more, smaller ones.  FP32, one CTA of 24 against three of 8:
 // 256 stacked small matrices 87 -> 74 us, power law of 150,000 rows 17.3 -> 14.6 us.  FP64, two of 10
-// against five of 4: stacked matrices 98.5 -> 92 us, stencil 60^3 19.4 -> 19.2; one of 20: 79 and 22.8.
-template <typename VT, bool DEEP> struct CvrShape {
-    static constexpr int WARPS = sizeof(VT) == 4 ? 24 : DEEP ? 8 : 10;
-    static constexpr int CTAS = sizeof(VT) == 4 ? 1 : 2;
+// against five of 4: stacked matrices 98.5 -> 92 us, stencil 60^3 19.4 -> 19.2; one of 20: 79 and 22.8,
+// so scattered columns (Handle::scattered) take that one.
+enum CvrMode { DEEP, LOCAL, SCATTERED };
+template <typename VT, CvrMode MODE> struct CvrShape {
+    static constexpr int WARPS = sizeof(VT) == 4 ? 24 : MODE == DEEP ? 8 : MODE == LOCAL ? 10 : 20;
+    static constexpr int CTAS = WARPS >= 20 ? 1 : 2;
 };
 
-template <int S, typename VT, typename IT, bool DEEP>
-__global__ void __launch_bounds__(CvrShape<VT, DEEP>::WARPS * 32, CvrShape<VT, DEEP>::CTAS)
+template <int S, typename VT, typename IT, CvrMode MODE>
+__global__ void __launch_bounds__(CvrShape<VT, MODE>::WARPS * 32, CvrShape<VT, MODE>::CTAS)
 cvr_spmv_kernel(const CvrMeta *__restrict__ meta, const unsigned *__restrict__ flags,
                 const VT *__restrict__ vals, const IT *__restrict__ cols,
                 const VT *__restrict__ x, const int *__restrict__ colbase,
                 double *__restrict__ y, double *__restrict__ carry_head,
-                double *__restrict__ carry_tail, ChunkWalk<CvrShape<VT, DEEP>::WARPS> walk, int m, int n,
+                double *__restrict__ carry_tail, ChunkWalk<CvrShape<VT, MODE>::WARPS> walk, int m, int n,
                 unsigned long long *err) {
     constexpr int L = 32 * S;
-    constexpr int NB = S / 4, SPMV_WARPS = CvrShape<VT, DEEP>::WARPS;
+    constexpr int NB = S / 4, SPMV_WARPS = CvrShape<VT, MODE>::WARPS;
     __shared__ double s_tail[SPMV_WARPS][64];
     __shared__ int s_row[SPMV_WARPS][64];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
@@ -387,9 +389,9 @@ cudaError_t convert_t(Handle &h, const int *rp, const int *ci, const double *v, 
     return cudaGetLastError();
 }
 
-template <typename VT, typename IT, bool DEEP>
+template <typename VT, typename IT, CvrMode MODE>
 cudaError_t spmv_t(const Handle &h, const void *x, void *y, cudaStream_t s) {
-    using SH = CvrShape<VT, DEEP>;
+    using SH = CvrShape<VT, MODE>;
     const long long cap = (long long)h.sm_count * SH::CTAS;
     const unsigned grid = (unsigned)(h.nchunks < cap ? h.nchunks : cap);
     auto go = [&](auto kernel) {
@@ -400,9 +402,9 @@ cudaError_t spmv_t(const Handle &h, const void *x, void *y, cudaStream_t s) {
                               guard_word());
     };
     switch (h.S) {
-        case 32: return go(cvr_spmv_kernel<32, VT, IT, DEEP>);
-        case 64: return go(cvr_spmv_kernel<64, VT, IT, DEEP>);
-        case 128: return go(cvr_spmv_kernel<128, VT, IT, DEEP>);
+        case 32: return go(cvr_spmv_kernel<32, VT, IT, MODE>);
+        case 64: return go(cvr_spmv_kernel<64, VT, IT, MODE>);
+        case 128: return go(cvr_spmv_kernel<128, VT, IT, MODE>);
         default: return cudaErrorInvalidValue;
     }
 }
@@ -422,10 +424,11 @@ cudaError_t cvr_convert(Handle &h, const int *rp, const int *ci, const double *v
 cudaError_t cvr_spmv(const Handle &h, const void *x, void *y, cudaStream_t s) {
     if (h.nchunks <= 0) return cudaSuccess;
     const bool f32 = h.precision == PAVA_PREC_FP32C, d16 = h.index_mode == PAVA_INDEX_DELTA16;
-    if (f32) return d16 ? spmv_t<float, short, true>(h, x, y, s) : spmv_t<float, int, true>(h, x, y, s);
-    if (!d16) return spmv_t<double, int, true>(h, x, y, s);
-    return h.nchunks <= 16LL * h.sm_count ? spmv_t<double, short, true>(h, x, y, s)
-                                          : spmv_t<double, short, false>(h, x, y, s);
+    if (f32) return d16 ? spmv_t<float, short, DEEP>(h, x, y, s) : spmv_t<float, int, DEEP>(h, x, y, s);
+    if (!d16) return spmv_t<double, int, DEEP>(h, x, y, s);
+    if (h.nchunks <= 16LL * h.sm_count) return spmv_t<double, short, DEEP>(h, x, y, s);
+    return h.scattered ? spmv_t<double, short, SCATTERED>(h, x, y, s)
+                       : spmv_t<double, short, LOCAL>(h, x, y, s);
 }
 
 }  // namespace pava

@@ -48,7 +48,7 @@ struct Handle {
     int S = 0;               // CVR: steps per chunk
     int sigma = 0, G = 0;    // CSR5: elements per lane per tile, tiles per chunk
     long long ntiles = 0;
-    int scattered = 0;       // CSR5: neighbouring nonzeros rarely share lines of x
+    int scattered = 0;       // CVR, CSR5: neighbouring nonzeros rarely share lines of x
     int lanes_per_row = 0;   // plain CSR: lanes per row group (GL)
     int col_lanes = 1;       //   lanes across the right-hand sides (KC)
     int cols_per_lane = 1;   //   right-hand sides per lane (KPL)

@@ -179,3 +179,20 @@ def test_rows_over_a_few_chunks(cuda, fmt, kw):
         y = mat.spmv(xd.float() if prec == _abi.PREC_FP32C else xd)
         assert O.rel_error(y.cpu().numpy(), yr, ab, bound)[0] == 0, prec
         mat.close()
+
+
+@pytest.mark.parametrize("units", [2369, 2960, 4001])
+def test_cvr_scattered_16_bit_columns(cuda, units):
+    """Random columns within 30,000: more chunks than 16 warps per SM hold, in one CTA per SM."""
+    torch = cuda
+    rng = np.random.default_rng(units)
+    m = 64 * units                        # 16 nonzeros per row, 1,024 elements to a chunk
+    ci = rng.integers(0, 30_000, 16 * m, dtype=np.int32)
+    A = M.from_arrays(m, 30_000, np.arange(0, 16 * m + 1, 16), ci, M.uniform(16 * m, seed=20, fp32=True))
+    x = M.uniform(A.n, seed=21, fp32=True)
+    yr, ab = O.csr_ref(A.rp, A.ci, A.v, x)
+    mat = SpMatrix(A, "cvr", index_mode=_abi.INDEX_DELTA16, steps=32)
+    xd = torch.from_numpy(x).cuda()
+    y = mat.spmv(xd)
+    assert O.rel_error(y.cpu().numpy(), yr, ab, 1e-12)[0] == 0
+    assert torch.equal(y, mat.spmv(xd))
