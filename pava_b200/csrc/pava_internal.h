@@ -126,9 +126,10 @@ unsigned long long *guard_word();
 // one's site + 1) on the current device; in every build.  nullptr when it cannot be resolved.
 unsigned long long *wait_word();
 
-// CSR5 tiles per chunk.  The persistent grid keeps `warps` warps resident (24 per SM); each
-// takes chunks in turn, so a chunk count just above a multiple of `warps` leaves a last wave
-// that few warps run.
+// CSR5 tiles per chunk.  The persistent grid keeps `warps` warps resident (24 per SM; FP64 on 32-bit
+// columns runs 20, and these rules count 24 for it too unless its columns are scattered); each
+// takes chunks in turn, so a chunk count just above a multiple of `warps` leaves a last wave that
+// few warps run.
 // Default: 4 tiles per chunk, fewer when that leaves fewer chunks than warps.
 inline int csr5_default_tiles(long long tiles, long long warps) {
     return tiles >= 4 * warps ? 4 : (tiles >= 2 * warps ? 2 : 1);
