@@ -215,6 +215,9 @@ __global__ void set_int_kernel(int *p, int v) { *p = v; }
 // for 32,245 chunks and 4.7 us for 640 after the SpMV kernel, this form 6.2 and 3.5 us.  Power-law
 // matrices have many rows over three to nine chunks: summed by the warp too, they cost a product
 // of 100,000 to 700,000 rows about 1 us.
+// FRESH: the kernel before wrote the headers too (the allocation-free product), so they are read
+// after the wait.
+template <bool FRESH>
 __global__ void __launch_bounds__(128)
 carry_fixup_kernel(const char *__restrict__ meta, size_t stride, const int *__restrict__ arp,
                    long long L, const double *carry_head, const double *carry_tail, double *y,
@@ -222,7 +225,8 @@ carry_fixup_kernel(const char *__restrict__ meta, size_t stride, const int *__re
     pdl_trigger();
     const int lane = threadIdx.x & 31;
     const long long c1 = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    // the headers belong to the matrix: read before the wait
+    if (FRESH) pdl_wait();
+    // otherwise the headers belong to the matrix: read before the wait
     int R = -1;
     bool two = false;  // R starts in c1 - 1 and ends in c1
     long long c0 = c1;
@@ -412,10 +416,10 @@ cudaError_t set_int(int *p, int v, cudaStream_t s) {
     return cudaGetLastError();
 }
 
-cudaError_t carry_fixup(const Handle &h, void *y, cudaStream_t s) {
+cudaError_t carry_fixup(const Handle &h, void *y, cudaStream_t s, bool fresh) {
     if (h.nchunks <= 0) return cudaSuccess;
     const long long blocks = (h.nchunks + 127) / 128;
-    return launch_product(carry_fixup_kernel, (unsigned)blocks, 128, 0, s, (const char *)h.meta,
+    return launch_product(fresh ? carry_fixup_kernel<true> : carry_fixup_kernel<false>, (unsigned)blocks, 128, 0, s, (const char *)h.meta,
                           h.meta_stride, h.arp, h.L, h.carry_head, h.carry_tail, (double *)y,
                           h.nchunks, h.m, guard_word());
 }

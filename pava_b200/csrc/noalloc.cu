@@ -193,7 +193,7 @@ extern "C" pava_status pava_spmv_csr_noalloc(int m, int n, int nnz, const int *r
         h.arp = const_cast<int *>(row_ptr);
         h.carry_head = head;
         h.carry_tail = tail;
-        e = carry_fixup(h, y, s);
+        e = carry_fixup(h, y, s, true);
         h.arp = nullptr;  // the Handle owns nothing here
         h.meta = nullptr;
         h.carry_head = nullptr;

@@ -191,7 +191,8 @@ cudaError_t csr5_convert(Handle &h, const int *rp, const int *ci, const double *
                          cudaStream_t s);
 cudaError_t csr5_spmv(const Handle &h, const void *x, void *y, cudaStream_t s);
 
-cudaError_t carry_fixup(const Handle &h, void *y, cudaStream_t s);
+// fresh: the kernel before it in the stream wrote the headers as well as the carries.
+cudaError_t carry_fixup(const Handle &h, void *y, cudaStream_t s, bool fresh = false);
 
 // SELL: sell_plan fills the slice descriptors (h.meta, h.nchunks slices) except their offsets
 // and writes the exclusive scan of the slices' block counts to d_blk_off[0..nslices], the total
