@@ -38,8 +38,9 @@ constexpr int WARPS = 8, PS = 16, MAX_K = 128;
 constexpr int LDC = PS + 4;                                            // ints per row of the stage
 template <typename VT> constexpr int LDV = sizeof(VT) == 8 ? PS + 2 : PS + 4;  // values per row
 
-// What elements past a row's end read in place of a row of X: they add 0 * 0.
-__device__ double g_zeros[MAX_K];
+// What elements past a row's end read in place of a row of X: they add 0 * 0.  Aligned for the pair
+// reads (ld_x2), which fault on an address that is no multiple of 16.
+__device__ __align__(16) double g_zeros[MAX_K];
 
 template <int G, int VW>
 __device__ __forceinline__ int slot_col(int lg, int p) {

@@ -64,8 +64,9 @@ template <typename VT, typename IT, int G> struct SpmmStage {
     static constexpr int BYTES = 2 * (VBYTES + CBYTES) + 128;  // two pieces + barriers
 };
 
-// What padding reads in place of a row of X: it adds 0 * 0, whatever X holds.
-__device__ double g_zero_row[SELL_SPMM_MAX_K];
+// What padding reads in place of a row of X: it adds 0 * 0, whatever X holds.  Aligned for the pair
+// reads (ld_x2).
+__device__ __align__(16) double g_zero_row[SELL_SPMM_MAX_K];
 
 // Column of sum p of a lane whose column slot is lg (0 .. G-1).
 template <int G, int VW>
