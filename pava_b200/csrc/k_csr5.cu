@@ -235,7 +235,7 @@ template <int SIGMA, typename VT, typename IT, bool SCAT>
 __global__ void __launch_bounds__(Csr5Shape<VT, IT, SCAT>::WARPS * 32, Csr5Shape<VT, IT, SCAT>::CTAS)
 csr5_spmv_kernel(const ChunkHdr *__restrict__ hdr, const int *__restrict__ tile_ptr,
                  const unsigned *__restrict__ desc, const VT *__restrict__ vals,
-                 const IT *__restrict__ cols, const VT *__restrict__ x,
+                 const IT *__restrict__ cols, const VT *x,
                  double *__restrict__ y, double *__restrict__ carry_head,
                  double *__restrict__ carry_tail, ChunkWalk<Csr5Shape<VT, IT, SCAT>::WARPS> walk,
                  int G, int m, int n,
@@ -396,7 +396,7 @@ template <int SIGMA, typename IT, bool SCAT>
 __global__ void __launch_bounds__(Csr5Shape<float, IT, SCAT>::WARPS * 32, Csr5Shape<float, IT, SCAT>::CTAS)
 csr5_spmv_f32_kernel(const ChunkHdr *__restrict__ hdr, const int *__restrict__ tile_ptr,
                      const unsigned *__restrict__ desc, const float *__restrict__ vals,
-                     const IT *__restrict__ cols, const float *__restrict__ x,
+                     const IT *__restrict__ cols, const float *x,
                      double *__restrict__ y, double *__restrict__ carry_head,
                      double *__restrict__ carry_tail,
                      ChunkWalk<Csr5Shape<float, IT, SCAT>::WARPS> walk, int G, int m, int n,

@@ -61,7 +61,7 @@ template <> __device__ __forceinline__ void row_vals(const float *p, float (&v)[
 template <typename VT, int G, int KPL, int VW, typename LD>
 __global__ void __launch_bounds__(WARPS * 32, 4)
 csr_spmm_kernel(const int *__restrict__ rp, const int *__restrict__ ci, const VT *__restrict__ v,
-                const VT *__restrict__ X, LD ldx, double *__restrict__ Y, long long ldy, int m,
+                const VT *X, LD ldx, double *__restrict__ Y, long long ldy, int m,
                 int n, int k, unsigned long long *err) {
     constexpr int R = 32 / G;               // rows at a time
     constexpr int NU = R * PS / 32;         // elements a lane stages per piece

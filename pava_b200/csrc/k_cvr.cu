@@ -244,7 +244,7 @@ template <int S, typename VT, typename IT, CvrMode MODE>
 __global__ void __launch_bounds__(CvrShape<VT, MODE>::WARPS * 32, CvrShape<VT, MODE>::CTAS)
 cvr_spmv_kernel(const CvrMeta *__restrict__ meta, const unsigned *__restrict__ flags,
                 const VT *__restrict__ vals, const IT *__restrict__ cols,
-                const VT *__restrict__ x, const int *__restrict__ colbase,
+                const VT *x, const int *__restrict__ colbase,
                 double *__restrict__ y, double *__restrict__ carry_head,
                 double *__restrict__ carry_tail, ChunkWalk<CvrShape<VT, MODE>::WARPS> walk, int m, int n,
                 unsigned long long *err) {

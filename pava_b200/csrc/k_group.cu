@@ -108,7 +108,7 @@ template <int KPL> constexpr int group_unroll() { return KPL == 1 ? 4 : (KPL == 
 template <int KPL, typename VT, int KCT, int VW>
 __global__ void __launch_bounds__(GROUP_THREADS, KCT ? COOP_MINB : group_minb<KPL>())
 csr_group_kernel(const int *__restrict__ rp, const int *__restrict__ ci,
-                 const VT *__restrict__ v, const VT *__restrict__ X, long long ldx,
+                 const VT *__restrict__ v, const VT *X, long long ldx,
                  double *__restrict__ Y, long long ldy, int m, int k, int gl_shift,
                  int kc_shift, int tile_rows, int n, unsigned long long *err) {
     constexpr int U = group_unroll<KPL>();
@@ -209,7 +209,7 @@ constexpr int WINDOW_SMEM = 100 * 1024;  // bytes of X per CTA (two CTAs per SM)
 template <int KPL, typename VT, int KCT>
 __global__ void __launch_bounds__(GROUP_THREADS, WINDOW_MINB)
 csr_window_kernel(const int *__restrict__ rp, const int *__restrict__ ci,
-                  const VT *__restrict__ v, const VT *__restrict__ X, long long ldx,
+                  const VT *__restrict__ v, const VT *X, long long ldx,
                   double *__restrict__ Y, long long ldy, int m, int k, int gl_shift,
                   int kc_shift, int tile_rows, int max_w, int n, unsigned long long *err) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -397,7 +397,7 @@ constexpr int SPMV_MINB = 6;
 template <int GL, typename VT>
 __global__ void __launch_bounds__(GROUP_THREADS, SPMV_MINB)
 csr_spmv_kernel(const int *__restrict__ rp, const int *__restrict__ ci, const VT *__restrict__ v,
-                const VT *__restrict__ x, long long ldx, double *__restrict__ y, long long ldy,
+                const VT *x, long long ldx, double *__restrict__ y, long long ldy,
                 int m, int tile_rows, unsigned by_cta, unsigned by_warp, int n,
                 unsigned long long *err) {
     constexpr int U = 4, WU = 4, GPW = 32 / GL, WARPS = GROUP_THREADS / 32;

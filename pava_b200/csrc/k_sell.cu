@@ -209,7 +209,7 @@ template <typename VT, typename IT> struct Stage {
 template <typename VT, typename IT>
 __global__ void __launch_bounds__(SELL_WARPS * 32, CTAS_PER_SM)
 sell_spmv_kernel(const SellSlice *__restrict__ meta, const VT *__restrict__ vals,
-                 const IT *__restrict__ cols, const VT *__restrict__ x,
+                 const IT *__restrict__ cols, const VT *x,
                  double *__restrict__ y, ChunkWalk<SELL_WARPS> walk, int m, int n,
                  unsigned long long *err, unsigned long long *wait_err) {
     using ST = Stage<VT, IT>;

@@ -90,7 +90,7 @@ __device__ __forceinline__ void row_cols(const short *pc, int i, int r, int (&c)
 template <typename VT, typename IT, int G, int KPL, int VW, typename LD>
 __global__ void __launch_bounds__(SpmmShape<G>::THREADS, SpmmShape<G>::CTAS_PER_SM)
 sell_spmm_kernel(const SellSlice *__restrict__ meta, const VT *__restrict__ vals,
-                 const IT *__restrict__ cols, const VT *__restrict__ X, LD ldx,
+                 const IT *__restrict__ cols, const VT *X, LD ldx,
                  double *__restrict__ Y, long long ldy, int ns, int run, int m, int n, int k,
                   unsigned long long *err, unsigned long long *wait_err) {
     using ST = SpmmStage<VT, IT, G>;

@@ -227,16 +227,16 @@ __device__ __forceinline__ int ld_col(const int *p, uint64_t pol) {
     return r;
 }
 
-// Two adjacent right-hand sides of X in one 16-byte (8-byte for FP32) read.
+// Two adjacent right-hand sides of X in one 16-byte (8-byte for FP32) read; not .nc, as ld_x.
 __device__ __forceinline__ double2 ld_x2(const double *p, uint64_t pol) {
     double2 r;
-    asm volatile("ld.global.nc.L2::cache_hint.v2.f64 {%0, %1}, [%2], %3;"
+    asm volatile("ld.global.L2::cache_hint.v2.f64 {%0, %1}, [%2], %3;"
                  : "=d"(r.x), "=d"(r.y) : "l"(p), "l"(pol));
     return r;
 }
 __device__ __forceinline__ float2 ld_x2(const float *p, uint64_t pol) {
     float2 r;
-    asm volatile("ld.global.nc.L2::cache_hint.v2.f32 {%0, %1}, [%2], %3;"
+    asm volatile("ld.global.L2::cache_hint.v2.f32 {%0, %1}, [%2], %3;"
                  : "=f"(r.x), "=f"(r.y) : "l"(p), "l"(pol));
     return r;
 }

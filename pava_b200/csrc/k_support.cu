@@ -216,11 +216,12 @@ __global__ void set_int_kernel(int *p, int v) { *p = v; }
 // matrices have many rows over three to nine chunks: summed by the warp too, they cost a product
 // of 100,000 to 700,000 rows about 1 us.
 // FRESH: the kernel before wrote the headers too (the allocation-free product), so they are read
-// after the wait.
+// after the wait, and without __restrict__: as the carries they are written while this kernel
+// waits, which rules out the read-only load path.
 template <bool FRESH>
 __global__ void __launch_bounds__(128)
-carry_fixup_kernel(const char *__restrict__ meta, size_t stride, const int *__restrict__ arp,
-                   long long L, const double *carry_head, const double *carry_tail, double *y,
+carry_fixup_kernel(const char *meta, size_t stride, const int *arp, long long L,
+                   const double *carry_head, const double *carry_tail, double *y,
                    long long nchunks, int m, unsigned long long *err) {
     pdl_trigger();
     const int lane = threadIdx.x & 31;

@@ -65,15 +65,17 @@ __device__ __forceinline__ unsigned ld_stream(const unsigned *p, uint64_t pol) {
     return r;
 }
 
-// x gather: read-only path through L1 (stencil rows reuse neighbours' x), kept in L2.
+// x gather through L1 (stencil rows reuse neighbours' x), kept in L2.  Not ld.global.nc, which is for
+// data that nothing writes while the kernel runs: a product starts while the one before, which may
+// write this x, still runs.
 __device__ __forceinline__ double ld_x(const double *p, uint64_t pol) {
     double r;
-    asm volatile("ld.global.nc.L2::cache_hint.f64 %0, [%1], %2;" : "=d"(r) : "l"(p), "l"(pol));
+    asm volatile("ld.global.L2::cache_hint.f64 %0, [%1], %2;" : "=d"(r) : "l"(p), "l"(pol));
     return r;
 }
 __device__ __forceinline__ float ld_x(const float *p, uint64_t pol) {
     float r;
-    asm volatile("ld.global.nc.L2::cache_hint.f32 %0, [%1], %2;" : "=f"(r) : "l"(p), "l"(pol));
+    asm volatile("ld.global.L2::cache_hint.f32 %0, [%1], %2;" : "=f"(r) : "l"(p), "l"(pol));
     return r;
 }
 
