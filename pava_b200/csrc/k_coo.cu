@@ -242,10 +242,16 @@ extern "C" pava_status pava_coo_to_csr_device(int m, int n, long long nnz, const
     unsigned long long *keys = nullptr;
     double *v = nullptr;
     void *tmp = nullptr;
+    // it allocates and waits: not on a stream that is being captured.  Nothing is held yet, and a
+    // wait or a trim here would end the caller's capture.
     cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
     cudaError_t e = cudaStreamIsCapturing(s, &capturing);
     if (e == cudaSuccess && capturing != cudaStreamCaptureStatusNone)
         e = cudaErrorStreamCaptureUnsupported;
+    if (e != cudaSuccess) {
+        set_last_error(std::string("COO -> CSR: ") + cudaGetErrorString(e));
+        return PAVA_E_CUDA;
+    }
     const size_t held = pool_reserved();
     auto cleanup = [&]() {
         pool_free(cnt, s); pool_free(cur, s); pool_free(seg, s); pool_free(d_st, s);
@@ -262,7 +268,6 @@ extern "C" pava_status pava_coo_to_csr_device(int m, int n, long long nnz, const
         set_last_error(std::string("COO -> CSR: ") + cudaGetErrorString(err));
         return err == cudaErrorMemoryAllocation ? PAVA_E_NOMEM : PAVA_E_CUDA;
     };
-    if (e != cudaSuccess) return fail_e(e);  // it allocates and waits
     // entries per row -> row pointer
     e = pool_malloc(&cnt, (size_t)m + 1, s);
     if (e == cudaSuccess) e = pool_malloc(&rp, (size_t)m + 1, s);
