@@ -5,7 +5,9 @@
 #include <thrust/iterator/counting_iterator.h>
 #include <thrust/iterator/transform_iterator.h>
 
+#include <map>
 #include <mutex>
+#include <utility>
 #include <vector>
 
 #include "pava_internal.h"
@@ -23,11 +25,14 @@ namespace {
 constexpr int POOL_DEVICES = 64;
 struct DevicePool {
     cudaMemPool_t pool = nullptr;
-    unsigned long long ctx = 0;  // the context the pool belongs to (a device reset ends it)
     std::vector<void *> waiting;  // freed while the device could not be waited for
 };
 std::mutex g_pool_mutex;
-DevicePool g_pools[POOL_DEVICES];
+// One per device and context: a program may alternate contexts on a device, and a context keeps its
+// pool.  A device reset ends a context and what its pool held; contexts are never numbered alike, so
+// the entry it leaves is not met again.  Never destroyed: handles may be freed at process exit.
+std::map<std::pair<int, unsigned long long>, DevicePool> &g_pools =
+    *new std::map<std::pair<int, unsigned long long>, DevicePool>();
 
 // Identity of the current context; 0 when the driver cannot tell.
 unsigned long long context_id() {
@@ -50,37 +55,37 @@ unsigned long long context_id() {
     return v;
 }
 
-// The current device's pool (made on first use); g_pool_mutex held.
-cudaError_t device_pool(DevicePool **out) {
-    int dev = 0;
-    cudaError_t e = cudaGetDevice(&dev);
+// The current device's and context's entry; g_pool_mutex held.
+cudaError_t device_entry(DevicePool **out, int *dev) {
+    cudaError_t e = cudaGetDevice(dev);
     if (e != cudaSuccess) return e;
-    if (dev < 0 || dev >= POOL_DEVICES) return cudaErrorInvalidDevice;
-    DevicePool &d = g_pools[dev];
+    if (*dev < 0 || *dev >= POOL_DEVICES) return cudaErrorInvalidDevice;
     unsigned long long ctx = context_id();
     if (ctx == 0) {  // a thread's first call: let the runtime make its context current
         e = cudaFree(nullptr);
         if (e != cudaSuccess) return e;
         ctx = context_id();
     }
-    if (d.pool && d.ctx != ctx) d = DevicePool();  // the device was reset: all of it is gone
-    if (!d.pool) {
-        cudaMemPoolProps props = {};
-        props.allocType = cudaMemAllocationTypePinned;
-        props.location.type = cudaMemLocationTypeDevice;
-        props.location.id = dev;
-        e = cudaMemPoolCreate(&d.pool, &props);
-        if (e != cudaSuccess) {
-            d.pool = nullptr;
-            return e;
-        }
-        uint64_t keep = POOL_KEEP;
-        e = cudaMemPoolSetAttribute(d.pool, cudaMemPoolAttrReleaseThreshold, &keep);
-        if (e != cudaSuccess) return e;
-        d.ctx = ctx;
-    }
-    *out = &d;
+    *out = &g_pools[{*dev, ctx}];
     return cudaSuccess;
+}
+
+// The same with its pool, made on first use.
+cudaError_t device_pool(DevicePool **out) {
+    int dev = 0;
+    cudaError_t e = device_entry(out, &dev);
+    if (e != cudaSuccess || (*out)->pool) return e;
+    cudaMemPoolProps props = {};
+    props.allocType = cudaMemAllocationTypePinned;
+    props.location.type = cudaMemLocationTypeDevice;
+    props.location.id = dev;
+    e = cudaMemPoolCreate(&(*out)->pool, &props);
+    if (e != cudaSuccess) {
+        (*out)->pool = nullptr;
+        return e;
+    }
+    uint64_t keep = POOL_KEEP;
+    return cudaMemPoolSetAttribute((*out)->pool, cudaMemPoolAttrReleaseThreshold, &keep);
 }
 
 cudaError_t current_pool(cudaMemPool_t *pool) {
@@ -129,11 +134,14 @@ void pool_free_synced(void *const *ps, int count) {
     const bool waited = cudaDeviceSynchronize() == cudaSuccess;
     {
         std::lock_guard<std::mutex> lock(g_pool_mutex);
-        std::vector<void *> &waiting = g_pools[at.device].waiting;
-        waiting.insert(waiting.end(), ps + i0, ps + count);
-        if (waited) {
-            for (void *p : waiting) cudaFree(p);
-            waiting.clear();
+        DevicePool *d = nullptr;
+        int dev = 0;
+        if (device_entry(&d, &dev) == cudaSuccess) {
+            d->waiting.insert(d->waiting.end(), ps + i0, ps + count);
+            if (waited) {
+                for (void *p : d->waiting) cudaFree(p);
+                d->waiting.clear();
+            }
         }
     }
     if (at.device != cur) cudaSetDevice(cur);

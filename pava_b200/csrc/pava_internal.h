@@ -74,8 +74,8 @@ struct Handle {
     size_t device_bytes = 0;
 };
 
-// Device memory of handles, conversions and their temporaries: a memory pool per device (and
-// context) that keeps at most POOL_KEEP bytes of what was freed, so that converting a new matrix
+// Device memory of handles, conversions and their temporaries: a memory pool per device and
+// context that keeps at most POOL_KEEP bytes of what was freed, so that converting a new matrix
 // does not pay the driver for its buffers each time.  All calls are thread-safe; memory is
 // ordered on the stream it is allocated and freed on.
 constexpr size_t POOL_KEEP = (size_t)1 << 30;
