@@ -25,6 +25,7 @@ namespace {
 constexpr int POOL_DEVICES = 64;
 struct DevicePool {
     cudaMemPool_t pool = nullptr;
+    void *anchor = nullptr;       // keeps the driver's block of small allocations mapped
     std::vector<void *> waiting;  // freed while the device could not be waited for
 };
 std::mutex g_pool_mutex;
@@ -84,8 +85,38 @@ cudaError_t device_pool(DevicePool **out) {
         (*out)->pool = nullptr;
         return e;
     }
+    if (!(*out)->anchor && cudaMalloc(&(*out)->anchor, 1) != cudaSuccess) {
+        (*out)->anchor = nullptr;  // device_wait tries again
+        cudaGetLastError();
+    }
     uint64_t keep = POOL_KEEP;
     return cudaMemPoolSetAttribute((*out)->pool, cudaMemPoolAttrReleaseThreshold, &keep);
+}
+
+// Waits for all work of the device, as cudaFree always does, by an allocation that is freed at once.
+// cudaDeviceSynchronize would end a stream capture that another thread, or this one in relaxed mode, is
+// making; cudaMalloc and cudaFree are allowed beside one.  5 us with the anchor (640 without, as
+// the driver then maps and unmaps a block each time), 3 us for cudaDeviceSynchronize.
+cudaError_t device_wait() {
+    {
+        std::lock_guard<std::mutex> lock(g_pool_mutex);
+        DevicePool *d = nullptr;
+        int dev = 0;
+        cudaError_t e = device_entry(&d, &dev);
+        if (e == cudaSuccess && !d->anchor) {
+            e = cudaMalloc(&d->anchor, 1);
+            if (e != cudaSuccess) d->anchor = nullptr;
+        }
+        if (e != cudaSuccess) {
+            cudaGetLastError();  // not the next launch's error
+            return e;
+        }
+    }
+    void *p = nullptr;
+    cudaError_t e = cudaMalloc(&p, 1);
+    if (e == cudaSuccess) e = cudaFree(p);
+    if (e != cudaSuccess) cudaGetLastError();
+    return e;
 }
 
 cudaError_t current_pool(cudaMemPool_t *pool) {
@@ -107,7 +138,7 @@ cudaError_t pool_malloc(void **p, size_t bytes, cudaStream_t s) {
     e = cudaMallocFromPoolAsync(p, bytes, pool, s);
     if (e == cudaErrorMemoryAllocation) {  // memory freed on other streams may still be on its way
         cudaGetLastError();
-        if (cudaDeviceSynchronize() == cudaSuccess) {
+        if (device_wait() == cudaSuccess || cudaDeviceSynchronize() == cudaSuccess) {
             pool_trim(0);
             e = cudaMallocFromPoolAsync(p, bytes, pool, s);
         }
@@ -131,7 +162,7 @@ void pool_free_synced(void *const *ps, int count) {
         at.device < 0 || at.device >= POOL_DEVICES)
         return;
     if (at.device != cur) cudaSetDevice(at.device);
-    const bool waited = cudaDeviceSynchronize() == cudaSuccess;
+    const bool waited = device_wait() == cudaSuccess;
     {
         std::lock_guard<std::mutex> lock(g_pool_mutex);
         DevicePool *d = nullptr;

@@ -86,8 +86,8 @@ template <typename T> cudaError_t pool_malloc(T **p, size_t count, cudaStream_t 
 // Frees memory whose last use is ordered before this point of s (NULL pointers are skipped).
 void pool_free(void *p, cudaStream_t s);
 // Frees memory that work on any stream may still use: waits for the device first, as cudaFree
-// does.  Where the wait is not possible (a stream is capturing) the memory is kept until a later
-// call can wait.
+// does, and like it leaves a thread-local or relaxed capture elsewhere whole.  Where the wait is not
+// possible (a global capture) the memory is kept until a later call can wait.
 void pool_free_synced(void *const *ps, int count);
 // Bytes the pool holds, and giving back what is unused above `keep`.
 size_t pool_reserved();
