@@ -69,7 +69,7 @@ namespace {
 thread_local std::string g_last_error;
 
 pava_status fail(pava_status st, const std::string &msg) {
-    g_last_error = msg;
+    pava::set_last_error(msg);
     return st;
 }
 
@@ -357,7 +357,12 @@ std::mutex g_wait_mutex;
 }  // namespace
 
 namespace pava {
-void set_last_error(const std::string &msg) { g_last_error = msg; }
+void set_last_error(const std::string &msg) {
+    g_last_error = msg;
+    // The failure is reported: the runtime's record of it is not left for the check after a later
+    // call's launch.
+    cudaGetLastError();
+}
 
 unsigned long long *wait_word() {
     int dev = 0;
