@@ -127,6 +127,7 @@ GPU_SYMBOLS = [
     ("pava_gen_device", c_int, [ctypes.POINTER(PavaGenParams), c_u64, c_void_p,
                                 ctypes.POINTER(PavaCsr)]),
     ("pava_free_device_csr", c_int, [ctypes.POINTER(PavaCsr)]),
+    ("pava_free_device_csr_async", c_int, [ctypes.POINTER(PavaCsr), c_void_p]),
     ("pava_features", c_int, [ctypes.POINTER(PavaCsr), c_void_p, c_void_p]),
     ("pava_variant", c_int, [c_int, ctypes.POINTER(c_int), ctypes.POINTER(PavaOpts)]),
     ("pava_variant_family", c_int, [c_int]),
@@ -145,6 +146,8 @@ GPU_SYMBOLS = [
     ("pava_create_selected", c_int, [ctypes.POINTER(PavaCsr), c_void_p, c_void_p,
                                      ctypes.POINTER(c_void_p), ctypes.POINTER(c_int)]),
     ("pava_coo_to_csr_device", c_int, [c_int, c_int, c_ll, c_void_p, c_void_p, c_void_p, c_int,
+                                       c_int, c_void_p, ctypes.POINTER(PavaCsr)]),
+    ("pava_coo_to_csr_device_pooled", c_int, [c_int, c_int, c_ll, c_void_p, c_void_p, c_void_p, c_int,
                                        c_int, c_void_p, ctypes.POINTER(PavaCsr)]),
     ("pava_conduct", c_int, [c_int, ctypes.POINTER(PavaCsr), c_void_p, c_void_p, c_char_p, c_int,
                              ctypes.POINTER(PavaOpts), ctypes.POINTER(PavaRunRecord)]),

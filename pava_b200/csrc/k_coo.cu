@@ -222,10 +222,13 @@ __global__ void coo_long_unpack_kernel(const int *__restrict__ rp, const int *__
 
 }  // namespace pava
 
-extern "C" pava_status pava_coo_to_csr_device(int m, int n, long long nnz, const int *rows,
-                                              const int *cols, const double *vals,
-                                              int index_base, int symmetric, void *stream,
-                                              pava_csr *out) {
+namespace {
+
+// pooled: the result's arrays come from the library's memory pool, else from cudaMalloc, which CUDA
+// IPC and peer access need.
+pava_status coo_to_csr(int m, int n, long long nnz, const int *rows, const int *cols,
+                       const double *vals, int index_base, int symmetric, void *stream,
+                       pava_csr *out, bool pooled) {
     using namespace pava;
     if (!out) { set_last_error("out is NULL"); return PAVA_E_INVALID_ARG; }
     memset(out, 0, sizeof(*out));
@@ -259,9 +262,13 @@ extern "C" pava_status pava_coo_to_csr_device(int m, int n, long long nnz, const
     };
     auto give_back = [&]() {
         cleanup();
-        pool_free(rp, s); pool_free(ci, s); pool_free(v, s);
+        if (pooled) { pool_free(rp, s); pool_free(ci, s); pool_free(v, s); }
         cudaStreamSynchronize(s);
+        if (!pooled) { cudaFree(rp); cudaFree(ci); cudaFree(v); }
         pool_trim(held);
+    };
+    auto result_malloc = [&](auto **p, size_t count) {
+        return pooled ? pool_malloc(p, count, s) : plain_malloc((void **)p, sizeof(**p) * (count ? count : 1));
     };
     auto fail_e = [&](cudaError_t err) {
         give_back();
@@ -270,7 +277,7 @@ extern "C" pava_status pava_coo_to_csr_device(int m, int n, long long nnz, const
     };
     // entries per row -> row pointer
     e = pool_malloc(&cnt, (size_t)m + 1, s);
-    if (e == cudaSuccess) e = pool_malloc(&rp, (size_t)m + 1, s);
+    if (e == cudaSuccess) e = result_malloc(&rp, (size_t)m + 1);
     if (e == cudaSuccess) e = pool_malloc(&d_st, 1, s);
     if (e == cudaSuccess) e = cudaMemsetAsync(cnt, 0, sizeof(int) * ((size_t)m + 1), s);
     if (e == cudaSuccess) e = cudaMemsetAsync(d_st, 0, sizeof(CooStat), s);
@@ -306,8 +313,8 @@ extern "C" pava_status pava_coo_to_csr_device(int m, int n, long long nnz, const
         return PAVA_E_TOO_LARGE;
     }
     const size_t tz = (size_t)(total ? total : 1);
-    if (e == cudaSuccess) e = pool_malloc(&ci, tz, s);
-    if (e == cudaSuccess) e = pool_malloc(&v, tz, s);
+    if (e == cudaSuccess) e = result_malloc(&ci, tz);
+    if (e == cudaSuccess) e = result_malloc(&v, tz);
     if (total > 0) {
         if (e == cudaSuccess) e = pool_malloc(&rec, tz, s);
         cur = cnt;  // the counts are in rp: their array becomes the rows' cursors
@@ -361,3 +368,32 @@ extern "C" pava_status pava_coo_to_csr_device(int m, int n, long long nnz, const
     out->on_device = 1;
     return PAVA_SUCCESS;
 }
+
+}  // namespace
+
+extern "C" {
+
+pava_status pava_coo_to_csr_device(int m, int n, long long nnz, const int *rows, const int *cols,
+                                   const double *vals, int index_base, int symmetric, void *stream,
+                                   pava_csr *out) {
+    return coo_to_csr(m, n, nnz, rows, cols, vals, index_base, symmetric, stream, out, false);
+}
+
+pava_status pava_coo_to_csr_device_pooled(int m, int n, long long nnz, const int *rows,
+                                          const int *cols, const double *vals, int index_base,
+                                          int symmetric, void *stream, pava_csr *out) {
+    return coo_to_csr(m, n, nnz, rows, cols, vals, index_base, symmetric, stream, out, true);
+}
+
+pava_status pava_free_device_csr_async(pava_csr *A, void *stream) {
+    if (!A) return PAVA_SUCCESS;
+    if (A->on_device) {
+        pava::pool_free((void *)A->row_ptr, (cudaStream_t)stream);
+        pava::pool_free((void *)A->col_idx, (cudaStream_t)stream);
+        pava::pool_free((void *)A->vals, (cudaStream_t)stream);
+    }
+    memset(A, 0, sizeof(*A));
+    return PAVA_SUCCESS;
+}
+
+}  // extern "C"

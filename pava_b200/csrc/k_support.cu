@@ -147,6 +147,19 @@ cudaError_t pool_malloc(void **p, size_t bytes, cudaStream_t s) {
     return e;
 }
 
+cudaError_t plain_malloc(void **p, size_t bytes) {
+    cudaError_t e = cudaMalloc(p, bytes);
+    if (e == cudaErrorMemoryAllocation) {  // the pool may hold it
+        cudaGetLastError();
+        if (device_wait() == cudaSuccess || cudaDeviceSynchronize() == cudaSuccess) {
+            pool_trim(0);
+            e = cudaMalloc(p, bytes);
+        }
+    }
+    if (e != cudaSuccess) *p = nullptr;
+    return e;
+}
+
 void pool_free(void *p, cudaStream_t s) {
     if (p) cudaFreeAsync(p, s);
 }

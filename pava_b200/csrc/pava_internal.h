@@ -83,6 +83,8 @@ cudaError_t pool_malloc(void **p, size_t bytes, cudaStream_t s);
 template <typename T> cudaError_t pool_malloc(T **p, size_t count, cudaStream_t s) {
     return pool_malloc((void **)p, sizeof(T) * (count ? count : 1), s);
 }
+// cudaMalloc, once more after giving back what the pool holds unused.
+cudaError_t plain_malloc(void **p, size_t bytes);
 // Frees memory whose last use is ordered before this point of s (NULL pointers are skipped).
 void pool_free(void *p, cudaStream_t s);
 // Frees memory that work on any stream may still use: waits for the device first, as cudaFree

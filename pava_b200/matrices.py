@@ -175,13 +175,13 @@ def write_mtx(path: str, A: CSR) -> None:
 
 def coo_to_csr_device(m: int, n: int, rows, cols, vals, index_base: int = 0,
                       symmetric: bool = False):
-    """COO on the GPU -> sorted CSR on the GPU (pava_coo_to_csr_device).  rows / cols are
+    """COO on the GPU -> sorted CSR on the GPU (pava_coo_to_csr_device_pooled).  rows / cols are
     int32 CUDA tensors, vals a float64 CUDA tensor.  Returns (rp, ci, v) CUDA tensors."""
     import torch
     A = _abi.PavaCsr()
-    _abi.check(_abi.gpu().pava_coo_to_csr_device(m, n, rows.numel(), rows.data_ptr(),
-                                                 cols.data_ptr(), vals.data_ptr(), index_base,
-                                                 int(symmetric), None, A))
+    _abi.check(_abi.gpu().pava_coo_to_csr_device_pooled(m, n, rows.numel(), rows.data_ptr(),
+                                                        cols.data_ptr(), vals.data_ptr(), index_base,
+                                                        int(symmetric), None, A))
     try:
         out = []
         for ptr, cnt, ts, dt in ((A.row_ptr, m + 1, "<i4", torch.int32),
@@ -192,8 +192,8 @@ def coo_to_csr_device(m: int, n: int, rows, cols, vals, index_base: int = 0,
                 t.copy_(torch.as_tensor(_DevView(ptr, cnt, ts), device="cuda"))
             out.append(t)
         return tuple(out)
-    finally:
-        _abi.gpu().pava_free_device_csr(A)
+    finally:  # after the copies, in their stream
+        _abi.gpu().pava_free_device_csr_async(A, torch.cuda.current_stream().cuda_stream)
 
 
 class _DevView:
