@@ -203,9 +203,14 @@ pava_status pava_spmv_host_wait(pava_handle *h);
 pava_status pava_get_info(const pava_handle *h, pava_info *out);
 
 /* anonymouslibHandle::destroy / asCSR (csr5/anonymouslib_avx512.h:80-104,258-262).  Waits for the
- * handle's device.  The library keeps up to 1 GiB of freed device memory per device for later
- * conversions. */
+ * handle's device.  The library keeps up to 1 GiB of freed device memory per device and context for
+ * later conversions (pava_release_memory gives it back). */
 pava_status pava_destroy(pava_handle *h);
+
+/* Gives back to the driver the device memory that the library keeps unused on the current device
+ * beyond `keep` bytes, for programs whose other allocators need it.  Waits for the device.  No
+ * counterpart in the reference. */
+pava_status pava_release_memory(unsigned long long keep);
 
 /* Message of the last failed call on this thread ("" if none). */
 const char *pava_last_error(void);

@@ -7,11 +7,11 @@ COO->CSR live in include/pava_host.h.  Build with ``python -m pava_b200.build``.
 from . import _abi  # noqa: F401
 from .matrices import CSR  # noqa: F401
 
-__all__ = ["CSR", "SpMatrix", "AnonymousLibHandle", "conduct_cvr", "conduct_csr5"]
+__all__ = ["CSR", "SpMatrix", "AnonymousLibHandle", "conduct_cvr", "conduct_csr5", "release_memory"]
 
 
 def __getattr__(name):
-    if name in ("SpMatrix", "AnonymousLibHandle", "conduct_cvr", "conduct_csr5"):
+    if name in __all__:
         from . import api
         return getattr(api, name)
     raise AttributeError(name)

@@ -89,6 +89,7 @@ class PavaError(RuntimeError):
 GPU_SYMBOLS = [
     ("pava_init", c_int, [c_int]),
     ("pava_set_device_memory_limit", c_int, [ctypes.c_ulonglong]),
+    ("pava_release_memory", c_int, [ctypes.c_ulonglong]),
     ("pava_bounds_checked", c_int, []),
     ("pava_bounds_report", c_int, [c_void_p, c_int]),
     ("pava_wait_report", c_int, [c_void_p, c_int]),

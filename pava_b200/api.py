@@ -5,6 +5,7 @@
 * ``Batch``                -- many independent matrices as one block-diagonal union, one
   launch per SpMV, replayable from a CUDA graph (pava_batch_*)
 * ``autotune``             -- exhaustive search over the candidate forms (pava_autotune)
+* ``release_memory``       -- gives back the device memory kept for later conversions
 * ``AnonymousLibHandle``   -- the CSR5 handle of csr5/anonymouslib_avx512.h:14-276 (inputCSR,
   setX, setSigma, asCSR5, spmv, asCSR, destroy), same names, argument meaning and status codes
 * ``conduct_cvr`` / ``conduct_csr5`` -- the engine entry points of cvr/cvr.h:1953 and
@@ -33,6 +34,12 @@ def _stream_ptr(stream) -> int | None:
         torch = _torch()
         return torch.cuda.current_stream().cuda_stream
     return getattr(stream, "cuda_stream", stream)
+
+
+def release_memory(keep: int = 0) -> None:
+    """Gives the device memory that the library keeps for later conversions back to the driver, but
+    for `keep` bytes (pava_release_memory)."""
+    _abi.check(_abi.gpu().pava_release_memory(keep))
 
 
 class SpMatrix:

@@ -835,6 +835,11 @@ pava_status pava_get_info(const pava_handle *H, pava_info *out) {
     return PAVA_SUCCESS;
 }
 
+pava_status pava_release_memory(unsigned long long keep) {
+    PAVA_CUDA(pava::pool_release((size_t)keep), "releasing memory");
+    return PAVA_SUCCESS;
+}
+
 pava_status pava_destroy(pava_handle *H) {
     if (!H) return PAVA_SUCCESS;
     free_pipe(H->pipe);

@@ -205,6 +205,23 @@ void pool_trim(size_t keep) {
     if (current_pool(&pool) == cudaSuccess) cudaMemPoolTrimTo(pool, keep);
 }
 
+cudaError_t pool_release(size_t keep) {
+    cudaError_t e = device_wait();
+    if (e != cudaSuccess) return e;
+    cudaMemPool_t pool = nullptr;
+    {
+        std::lock_guard<std::mutex> lock(g_pool_mutex);
+        DevicePool *d = nullptr;
+        int dev = 0;
+        e = device_entry(&d, &dev);
+        if (e != cudaSuccess) return e;
+        for (void *p : d->waiting) cudaFree(p);
+        d->waiting.clear();
+        pool = d->pool;
+    }
+    return pool ? cudaMemPoolTrimTo(pool, keep) : cudaSuccess;
+}
+
 namespace {
 
 // Counts violations: row_ptr[0] != 0, row_ptr decreasing, row_ptr[m] != nnz, column outside

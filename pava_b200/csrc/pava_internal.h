@@ -94,6 +94,8 @@ void pool_free_synced(void *const *ps, int count);
 // Bytes the pool holds, and giving back what is unused above `keep`.
 size_t pool_reserved();
 void pool_trim(size_t keep);
+// The same after waiting for the device, with what waits to be freed.
+cudaError_t pool_release(size_t keep);
 
 // Launches a product kernel as a programmatic dependent of the kernel before it in the stream.
 // All product kernels let their dependents launch at once (pdl_trigger) and call pdl_wait before
