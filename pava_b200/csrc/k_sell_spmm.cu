@@ -249,7 +249,7 @@ sell_spmm_kernel(const SellSlice *__restrict__ meta, const VT *__restrict__ vals
         const int done = cs;
         cb += KB;
         if (cb >= nblk) {  // the slice's last piece
-            store_row(cs, acc);
+            if (ok) store_row(cs, acc);  // after a wait that gave up the sums are partial
 #pragma unroll
             for (int p = 0; p < KPL; ++p) acc[p] = 0.0;
             cb = 0;
