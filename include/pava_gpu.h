@@ -281,7 +281,8 @@ pava_status pava_batch_destroy(pava_batch *b);
  * with 32-bit columns and with PAVA_INDEX_AUTO (16-bit offsets where they reach), CSR5 also
  * with the tiles per chunk that fill the last wave of warp chunks best (1..8); for
  * every k, the CSR row-group form over lanes_per_row x col_lanes x cols_per_lane x
- * rows_per_tile, and for k > 1 also with x_window.  entries[0 .. *n_entries) receive every candidate (ms < 0 when it failed,
+ * rows_per_tile, and for k > 1 also with x_window; for k > 32 also in the engine's own shape (every
+ * shape option 0).  entries[0 .. *n_entries) receive every candidate (ms < 0 when it failed,
  * with its status), *best the index of the fastest.  No counterpart in the reference. */
 typedef struct pava_tune_entry {
     int format;

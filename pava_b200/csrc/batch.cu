@@ -174,8 +174,8 @@ pava_status build_union(int count, const pava_csr *mats, cudaStream_t s, pava_ba
 }
 
 // Built-in candidate forms for k right-hand sides: for k = 1 the 32 forms of pava_variant in
-// their order (the selector's space); for k > 1 the row-group shapes (at most 72 for k <= 128)
-// and the SELL SpMM shapes (lanes per row x column form, at most 4).
+// their order (the selector's space); for k > 1 the row-group shapes (at most 72 for k <= 128), the
+// engine's own shape and the SELL SpMM shapes (lanes per row x column form, at most 4).
 std::vector<std::pair<int, pava_opts>> candidates(int k, int precision) {
     std::vector<std::pair<int, pava_opts>> c;
     auto base = [&]() {
@@ -221,6 +221,11 @@ std::vector<std::pair<int, pava_opts>> candidates(int k, int precision) {
                     c.push_back({PAVA_FORMAT_CSR, o});
                 }
     }
+    // The engine's own shape (k_csr_spmm.cu: rows staged per warp).  Up to k = 32 the shapes above include
+    // it; above, its lanes hold 8 columns each, which no option names.  FP64, k = 48 / 64 / 128, us,
+    // the best of the shapes above / this: banded 300,007 rows 339 338 658 / 214 242 428, stencil 70^3 400 402 785 / 313 390 614, dense blocks 120,001
+    // rows 243 257 482 / 193 219 325.
+    if (k > 32) c.push_back({PAVA_FORMAT_CSR, base()});
     // SELL: 4 (k <= 32) or 8 lanes per row, 32-bit columns or 16-bit offsets where they reach
     // (16 lanes per row, an option of pava_create, was never faster on the banded, stencil and
     // batch matrices)
