@@ -376,7 +376,11 @@ csr_window_kernel(const int *__restrict__ rp, const int *__restrict__ ci,
 // off the critical path:
 //
 //  * a row longer than LONG = 4 U GL is summed by the whole warp, WU elements per lane at a time:
-//    in its group it would run len / (U GL) dependent rounds while the other groups wait;
+//    in its group it would run len / (U GL) dependent rounds while the other groups wait.  Narrow
+//    groups (GL <= 4) keep them where so many of a warp's rows are long that one after the other
+//    they would take more rounds (one lane per row, us, each row by the warp / this: banded 500,000
+//    rows of 24 135 / 121 with L2 flushed, in tiles of 512 rows 484 / 128; power law 40,000 rows 45 / 45,
+//    and 73 where half as many rows were enough to stay in the groups);
 //  * a row longer than HUGE_ROW waits until the CTA's tiles are done and is summed by all of its
 //    warps.  Each warp keeps up to LIST such rows (and sums further ones alone), so which rows
 //    take which way depends on the matrix and the launch shape only, and results repeat bit
@@ -453,7 +457,16 @@ csr_spmv_kernel(const int *__restrict__ rp, const int *__restrict__ ci, const VT
                 b = rp[r + 1];
             }
             const int len = b - a;
-            const bool is_long = len > LONG;
+            bool is_long = len > LONG;
+            unsigned todo = __ballot_sync(FULL, is_long && gi == 0);
+            if (GL <= 4 && todo) {  // many of them: the groups are done sooner, all at once
+                const bool mid = is_long && len <= HUGE_ROW;
+                const int most = __reduce_max_sync(FULL, mid ? len : 0);
+                const int count = __popc(__ballot_sync(FULL, mid && gi == 0));
+                if (count * ((most + 32 * WU - 1) / (32 * WU)) >= (most + U * GL - 1) / (U * GL))
+                    is_long = len > HUGE_ROW;
+                todo = __ballot_sync(FULL, is_long && gi == 0);
+            }
             const VT *vr = v + a;
             const int *cr = ci + a;
             Acc<VT> acc;
@@ -475,7 +488,6 @@ csr_spmv_kernel(const int *__restrict__ rp, const int *__restrict__ ci, const VT
             for (int o = 1; o < GL; o <<= 1) s += __shfl_xor_sync(FULL, s, o);
             if (r < (unsigned)m && gi == 0 && !is_long) y[r * ldy] = s;
             // long rows, one after the other, by the whole warp
-            unsigned todo = __ballot_sync(FULL, is_long && gi == 0);
             while (todo) {
                 const int src = __ffs(todo) - 1;
                 todo &= todo - 1;
