@@ -110,10 +110,11 @@ __global__ void __launch_bounds__(GROUP_THREADS, KCT ? COOP_MINB : group_minb<KP
 csr_group_kernel(const int *__restrict__ rp, const int *__restrict__ ci,
                  const VT *__restrict__ v, const VT *X, long long ldx,
                  double *__restrict__ Y, long long ldy, int m, int k, int gl_shift,
-                 int kc_shift, int tile_rows, int n, unsigned long long *err) {
+                 int kc_shift, int tile_rows, unsigned by_cta, unsigned by_warp, int n,
+                 unsigned long long *err) {
     constexpr int U = group_unroll<KPL>();
-    pdl_trigger();
     pdl_wait();
+    pdl_trigger();  // after the wait: one product ahead at most, see deal_tiles
     const int lane = threadIdx.x & 31;
     const int gl = 1 << gl_shift, kc = 1 << kc_shift;
     const int grp = lane >> gl_shift;          // group within the warp
@@ -153,7 +154,7 @@ csr_group_kernel(const int *__restrict__ rp, const int *__restrict__ ci,
         }
     };
 
-    for (long long t = (((long long)blockIdx.x * blockDim.x) + threadIdx.x) >> 5; t < ntiles;
+    for (long long t = (long long)blockIdx.x * by_cta + (threadIdx.x >> 5) * by_warp; t < ntiles;
          t += nwarps) {
         for (int i = 0; i < rounds; ++i) {
             const long long r = t * tile_rows + (long long)i * gpw + grp;
@@ -216,8 +217,8 @@ csr_window_kernel(const int *__restrict__ rp, const int *__restrict__ ci,
     VT *xs = reinterpret_cast<VT *>(smem_raw);
     constexpr int WARPS = GROUP_THREADS / 32;
     __shared__ int s_min[WARPS], s_max[WARPS];
-    pdl_trigger();
     pdl_wait();
+    pdl_trigger();  // after the wait: one product ahead at most, see deal_tiles
     const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
     const int gl = 1 << gl_shift, kc = 1 << kc_shift;
     const int grp = lane >> gl_shift;
@@ -408,8 +409,8 @@ csr_spmv_kernel(const int *__restrict__ rp, const int *__restrict__ ci, const VT
     constexpr int LONG = GL < 32 ? 4 * U * GL : HUGE_ROW;
     __shared__ int s_list[WARPS][LIST], s_cnt[WARPS];
     __shared__ double s_sum[WARPS];
-    pdl_trigger();
     pdl_wait();
+    pdl_trigger();  // after the wait: one product ahead at most, see deal_tiles
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const int grp = lane / GL, gi = lane % GL;
     const uint64_t pf = policy_evict_first(), pl = policy_evict_last();
@@ -524,6 +525,29 @@ csr_spmv_kernel(const int *__restrict__ rp, const int *__restrict__ ci, const VT
     }
 }
 
+// The grid for ntiles tiles of a warp each with `resident` CTAs per SM, and the first tile of warp w of CTA
+// b, b * by_cta + w * by_warp.  Up to a full GPU tile t goes to warp t / grid of CTA t % grid and every
+// SM gets as many CTAs, so that every SM has an even share: FP32C SpMV in a loop, us, before / after:
+// banded 30,000 rows 13.7 / 10.4, dense blocks 30,000 18.6 / 14.1, power law 40,000 21.6 / 17.7.
+// A product's CTAs come in while those of the product before run (of that one only: the kernels let
+// their dependents launch after their own wait).  Where both do not fit at once, the SMs whose CTAs end
+// first would get more of the next, so more than half a GPU takes all of it, and every place is used
+// once.  In a loop, us, before / after: SpMV of banded 500,000 rows, one lane each, 121 / 89, dense blocks
+// 300,000 rows, two lanes, 93 / 67; k = 2 on banded 300,007 rows, one lane, 100 / 54.
+struct TileDeal {
+    unsigned grid, by_cta, by_warp;
+};
+TileDeal deal_tiles(long long ntiles, int sms, int resident) {
+    constexpr int WARPS = GROUP_THREADS / 32;
+    const long long want = (ntiles + WARPS - 1) / WARPS;
+    long long per_sm = (want + sms - 1) / sms;
+    if (per_sm < 1) per_sm = 1;
+    if (2 * per_sm > resident) per_sm = resident;
+    const unsigned grid = (unsigned)(per_sm * sms);
+    const bool one_each = ntiles <= (long long)grid * WARPS;
+    return {grid, one_each ? 1u : (unsigned)WARPS, one_each ? grid : 1u};
+}
+
 int ilog2(int v) {
     int s = 0;
     while ((1 << s) < v) ++s;
@@ -572,21 +596,11 @@ template <typename VT>
 cudaError_t launch_spmv(const Handle &h, const VT *x, long long ldx, double *y, long long ldy,
                         cudaStream_t s) {
     const int tr = h.rows_per_tile;
-    const long long ntiles = ((long long)h.m + tr - 1) / tr;
-    const long long want = (ntiles + (GROUP_THREADS / 32) - 1) / (GROUP_THREADS / 32);
-    const long long cap = (long long)h.sm_count * SPMV_MINB;
-    // Up to a full GPU, as many CTAs on every SM, and tile t to warp t / grid of CTA t % grid, so that
-    // every SM gets an even share, however the CTAs of the product before free their places.  FP32C in a
-    // loop, us, before / after: banded 30,000 rows 13.7 / 10.4, dense blocks 30,000 18.6 / 14.1,
-    // power law 40,000 21.6 / 17.7.
-    const long long even = (want + h.sm_count - 1) / h.sm_count * h.sm_count;
-    const unsigned grid = (unsigned)(even < cap ? (want > 0 ? even : 1) : cap);
-    const bool one_each = ntiles <= (long long)grid * (GROUP_THREADS / 32);
-    const unsigned by_cta = one_each ? 1u : GROUP_THREADS / 32, by_warp = one_each ? grid : 1u;
+    const TileDeal d = deal_tiles(((long long)h.m + tr - 1) / tr, h.sm_count, SPMV_MINB);
     auto go = [&](auto GLC) {
-        return launch_product(csr_spmv_kernel<decltype(GLC)::value, VT>, grid, GROUP_THREADS, 0, s,
-                              h.rp, h.ci, (const VT *)h.v, x, ldx, y, ldy, h.m, tr, by_cta,
-                              by_warp, h.n, guard_word());
+        return launch_product(csr_spmv_kernel<decltype(GLC)::value, VT>, d.grid, GROUP_THREADS, 0, s,
+                              h.rp, h.ci, (const VT *)h.v, x, ldx, y, ldy, h.m, tr, d.by_cta,
+                              d.by_warp, h.n, guard_word());
     };
     switch (h.lanes_per_row) {
         case 1: return go(std::integral_constant<int, 1>());
@@ -604,11 +618,8 @@ cudaError_t launch_rows(const Handle &h, const VT *x, long long ldx, double *y, 
                         int k, cudaStream_t s) {
     const int kc = h.col_lanes;
     const int tr = h.rows_per_tile;
-    const long long ntiles = ((long long)h.m + tr - 1) / tr;
-    const long long want = (ntiles + (GROUP_THREADS / 32) - 1) / (GROUP_THREADS / 32);
-    const int minb = kc > 1 ? COOP_MINB : group_minb<KPL>();
-    const long long cap = (long long)h.sm_count * minb;
-    const unsigned grid = (unsigned)(want < cap ? (want > 0 ? want : 1) : cap);
+    const TileDeal d = deal_tiles(((long long)h.m + tr - 1) / tr, h.sm_count,
+                                  kc > 1 ? COOP_MINB : group_minb<KPL>());
     const int gs = ilog2(h.lanes_per_row), ks = ilog2(kc);
     // pairs of columns per vector read when every pair is whole and 2-element aligned
     const bool vec2 = KPL >= 2 && k % 2 == 0 && ldx % 2 == 0 &&
@@ -620,9 +631,9 @@ cudaError_t launch_rows(const Handle &h, const VT *x, long long ldx, double *y, 
             return cudaErrorInvalidValue;  // one column in one lane: launch_spmv
         } else {
             auto go = [&](auto kernel) {
-                return launch_product(kernel, grid, GROUP_THREADS, 0, s, h.rp, h.ci,
-                                      (const VT *)h.v, x, ldx, y, ldy, h.m, k, gs, ks, tr, h.n,
-                                      guard_word());
+                return launch_product(kernel, d.grid, GROUP_THREADS, 0, s, h.rp, h.ci,
+                                      (const VT *)h.v, x, ldx, y, ldy, h.m, k, gs, ks, tr, d.by_cta,
+                                      d.by_warp, h.n, guard_word());
             };
             return vec2 ? go(csr_group_kernel<KPL, VT, KCT, VW2>)
                         : go(csr_group_kernel<KPL, VT, KCT, 1>);
