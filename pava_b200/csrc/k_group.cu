@@ -40,20 +40,21 @@ struct ColAcc {
 // stream), with the next round's loads in flight while the current round is consumed; each
 // element reaches the lanes that need it by shuffle.  Slice e takes elements e, e + ES, ... in
 // ascending order, as the per-lane loop does, so the sums have the same bits.  The round count
-// is the maximum over the warp's groups so that every shuffle has all 32 lanes.  The X reads of
-// UB elements are in flight together: an element past the row's end has column -1, for which
-// xload gives zeros.
+// is the maximum over the warp's groups so that every shuffle has all 32 lanes.  With eight steps or more
+// a round takes as many as the longest row still needs, rounded up to a half, a quarter or an eighth:
+// rows of five in groups of 32 spent nearly all of it on nothing (Laplacian 700^2, k = 33, 32 lanes of
+// which 16 across k: 816 us with all steps for every row, now 324).  With fewer steps the choice
+// cost more than it saved (power law 200,003 rows, k = 2, two lanes: 555 -> 930 us), as did an end
+// test between the steps, which kept the X reads of the next ones back (banded 300,007 rows, k = 8 on
+// groups of four: 67 -> 96).  The X reads of UB elements are in flight together: an element past the
+// row's end has column -1, for which xload gives zeros.
 template <int KPL, int KCT, typename VT, typename XLOAD>
 __device__ __forceinline__ void coop_row(int a, int b, int gi, int gl, int es, int e, int lane,
                                          const int *__restrict__ ci, const VT *__restrict__ v,
                                          XLOAD xload, ColAcc (&acc)[KPL], uint64_t pf) {
     constexpr int UB = KPL >= 4 ? 1 : (KCT < 4 / KPL ? KCT : 4 / KPL);
-    int rounds = (b - a + gl - 1) / gl;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        const int t = __shfl_xor_sync(FULL, rounds, o);
-        rounds = t > rounds ? t : rounds;
-    }
+    const int most = __reduce_max_sync(FULL, b - a);  // elements of the warp's longest row
+    const int rounds = (int)(((unsigned)most + gl - 1) / gl);
     const int gbase = lane & ~(gl - 1);
     VT pv = VT(0);
     int pc = -1;
@@ -71,19 +72,31 @@ __device__ __forceinline__ void coop_row(int a, int b, int gi, int gl, int es, i
             pv = ld_val(v + base + gl + gi, pf);
             pc = ld_col(ci + base + gl + gi, pf);
         }
+        auto steps = [&](auto count) {
+            constexpr int N = decltype(count)::value, B = UB < N ? UB : N;
 #pragma unroll
-        for (int u0 = 0; u0 < KCT; u0 += UB) {
-            VT val[UB], xv[UB][KPL];
+            for (int u0 = 0; u0 < N; u0 += B) {
+                VT val[B], xv[B][KPL];
 #pragma unroll
-            for (int u = 0; u < UB; ++u) {
-                const int o = gbase + e + (u0 + u) * es;
-                val[u] = __shfl_sync(FULL, cv, o);
-                xload(__shfl_sync(FULL, cc, o), xv[u]);
+                for (int u = 0; u < B; ++u) {
+                    const int o = gbase + e + (u0 + u) * es;
+                    val[u] = __shfl_sync(FULL, cv, o);
+                    xload(__shfl_sync(FULL, cc, o), xv[u]);
+                }
+#pragma unroll
+                for (int u = 0; u < B; ++u)
+#pragma unroll
+                    for (int p = 0; p < KPL; ++p) acc[p].add((double)val[u], (double)xv[u][p]);
             }
-#pragma unroll
-            for (int u = 0; u < UB; ++u)
-#pragma unroll
-                for (int p = 0; p < KPL; ++p) acc[p].add((double)val[u], (double)xv[u][p]);
+        };
+        if constexpr (KCT >= 8) {
+            const int left = most - rd * gl;
+            if (left > es * (KCT / 2)) steps(std::integral_constant<int, KCT>());
+            else if (left > es * (KCT / 4)) steps(std::integral_constant<int, KCT / 2>());
+            else if (left > es * (KCT / 8)) steps(std::integral_constant<int, KCT / 4>());
+            else steps(std::integral_constant<int, KCT / 8>());
+        } else {
+            steps(std::integral_constant<int, KCT>());
         }
     }
 }
