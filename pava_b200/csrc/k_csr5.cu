@@ -205,8 +205,8 @@ __device__ __forceinline__ void tile_combine(double head, double tail, bool seen
     }
 }
 
-// Warps per CTA and CTAs per SM.
-// FP64: 24 warps with 80 registers for 16-bit columns, 20 with 96 for 32-bit ones, which spill at 80 and
+// Warps per CTA and CTAs per SM: one CTA of 24 or 20 warps, or three of 8 (csr5_spmv chooses).
+// FP64: 24 warps with 80 registers for 16-bit columns; 20 with 96 for 32-bit ones, which spill at 80 and
 // keep more of a chunk in flight at 96.  A product in a loop, us, 24 / 20 warps: 32-bit columns, stencil
 // 72^3 37.3 / 30.1, 128^3 158 / 150, dense blocks 17 M nonzeros 56 / 45, power law 66 M 338 / 294;
 // 16-bit columns, stencil 100^3 66.6 / 70.4, 128^3 135 / 143, Laplacian 2000^2 62 / 67 (dense blocks
@@ -214,11 +214,9 @@ __device__ __forceinline__ void tile_combine(double head, double tail, bool seen
 // One CTA puts that many neighbouring chunks on the SM, which share lines of x: 256 stacked small
 // matrices FP32 67 -> 51 us, FP64 105 -> 85, stencil 128^3 FP64 138 -> 135, power law of 102,000 rows
 // FP64 16.0 -> 12.0, against CTAs of 8 or 4 warps; CTAs of 12 or 10 lie between.
-// FP32: one CTA of 24, but three of 8 for 32-bit columns that are not scattered (Handle::scattered):
-// stencil 128^3 115 -> 108, dense blocks 17 M 41.6 -> 38.6; power law 20 M 88 -> 90.
-template <typename VT, typename IT, bool SCAT> struct Csr5Shape {
-    static constexpr bool F64 = sizeof(VT) == 8, ONE = F64 || sizeof(IT) == 2 || SCAT;
-    static constexpr int WARPS = !ONE ? 8 : F64 && sizeof(IT) == 4 ? 20 : 24, CTAS = ONE ? 1 : 3;
+template <int W> struct Csr5Shape {
+    static_assert(W == 24 || W == 20 || W == 8, "launch shape");
+    static constexpr int WARPS = W, CTAS = W == 8 ? 3 : 1;
 };
 
 // CSR5 SpMV (FP64 values; the FP32 form is csr5_spmv_f32_kernel below): one warp per chunk of
@@ -231,19 +229,19 @@ template <typename VT, typename IT, bool SCAT> struct Csr5Shape {
 // so the step has no branch; at the tile end piece 0 (the end of the row the lane started
 // with) joins the cross-lane combine and pieces 1 .. k-1, rows that start and end in the
 // lane, go to y.  Other tiles write each finished row as it ends.
-template <int SIGMA, typename VT, typename IT, bool SCAT>
-__global__ void __launch_bounds__(Csr5Shape<VT, IT, SCAT>::WARPS * 32, Csr5Shape<VT, IT, SCAT>::CTAS)
+template <int SIGMA, typename VT, typename IT, int W>
+__global__ void __launch_bounds__(Csr5Shape<W>::WARPS * 32, Csr5Shape<W>::CTAS)
 csr5_spmv_kernel(const ChunkHdr *__restrict__ hdr, const int *__restrict__ tile_ptr,
                  const unsigned *__restrict__ desc, const VT *__restrict__ vals,
                  const IT *__restrict__ cols, const VT *x,
                  double *__restrict__ y, double *__restrict__ carry_head,
-                 double *__restrict__ carry_tail, ChunkWalk<Csr5Shape<VT, IT, SCAT>::WARPS> walk,
+                 double *__restrict__ carry_tail, ChunkWalk<Csr5Shape<W>::WARPS> walk,
                  int G, int m, int n,
                  unsigned long long *err) {
     constexpr int NBT = SIGMA / 4;  // blocks per tile
-    constexpr int SPMV_WARPS = Csr5Shape<VT, IT, SCAT>::WARPS;
+    constexpr int SPMV_WARPS = Csr5Shape<W>::WARPS;
     pdl_trigger();
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int lane = threadIdx.x & 31;
     const uint64_t pf = policy_evict_first(), pl = policy_evict_last();
     constexpr int KSTK = 4;
     constexpr unsigned SLOT = SPMV_WARPS * 32 * 8;  // bytes between a thread's slots
@@ -392,20 +390,20 @@ template <bool B> struct Flag { static constexpr bool value = B; };
 // choice and the tile-boundary checks are made once per tile instead of once per block.  The
 // compensated add makes this form instruction-issue bound, where the saved instructions are
 // time; the FP64 form is bandwidth bound, and unrolled it spills, so it keeps the block loop.
-template <int SIGMA, typename IT, bool SCAT>
-__global__ void __launch_bounds__(Csr5Shape<float, IT, SCAT>::WARPS * 32, Csr5Shape<float, IT, SCAT>::CTAS)
+template <int SIGMA, typename IT, int W>
+__global__ void __launch_bounds__(Csr5Shape<W>::WARPS * 32, Csr5Shape<W>::CTAS)
 csr5_spmv_f32_kernel(const ChunkHdr *__restrict__ hdr, const int *__restrict__ tile_ptr,
                      const unsigned *__restrict__ desc, const float *__restrict__ vals,
                      const IT *__restrict__ cols, const float *x,
                      double *__restrict__ y, double *__restrict__ carry_head,
                      double *__restrict__ carry_tail,
-                     ChunkWalk<Csr5Shape<float, IT, SCAT>::WARPS> walk, int G, int m, int n,
+                     ChunkWalk<Csr5Shape<W>::WARPS> walk, int G, int m, int n,
                      unsigned long long *err) {
     using VT = float;
     constexpr int NBT = SIGMA / 4;  // blocks per tile
-    constexpr int SPMV_WARPS = Csr5Shape<VT, IT, SCAT>::WARPS;
+    constexpr int SPMV_WARPS = Csr5Shape<W>::WARPS;
     pdl_trigger();
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int lane = threadIdx.x & 31;
     const uint64_t pf = policy_evict_first(), pl = policy_evict_last();
     constexpr int KSTK = 4;
     constexpr unsigned SLOT = SPMV_WARPS * 32 * 8;  // bytes between a thread's slots
@@ -562,9 +560,9 @@ cudaError_t convert_t(Handle &h, const int *rp, const int *ci, const double *v, 
     }
 }
 
-template <int SG, typename VT, typename IT, bool SCAT>
+template <int SG, typename VT, typename IT, int W>
 cudaError_t launch_sg(const Handle &h, const void *x, void *y, cudaStream_t s) {
-    using SH = Csr5Shape<VT, IT, SCAT>;
+    using SH = Csr5Shape<W>;
     const long long cap = (long long)h.sm_count * SH::CTAS;
     const unsigned grid = (unsigned)(h.nchunks < cap ? h.nchunks : cap);
     auto go = [&](auto kernel) {
@@ -574,20 +572,26 @@ cudaError_t launch_sg(const Handle &h, const void *x, void *y, cudaStream_t s) {
                               ChunkWalk<SH::WARPS>::over(h.nchunks, grid), h.G, h.m, h.n,
                               guard_word());
     };
-    if constexpr (sizeof(VT) == 4) return go(csr5_spmv_f32_kernel<SG, IT, SCAT>);
-    else return go(csr5_spmv_kernel<SG, VT, IT, SCAT>);
+    if constexpr (sizeof(VT) == 4) return go(csr5_spmv_f32_kernel<SG, IT, W>);
+    else return go(csr5_spmv_kernel<SG, VT, IT, W>);
 }
 
-template <typename VT, typename IT, bool SCAT>
+template <typename VT, typename IT, int W>
 cudaError_t spmv_t(const Handle &h, const void *x, void *y, cudaStream_t s) {
     switch (h.sigma) {
-        case 8: return launch_sg<8, VT, IT, SCAT>(h, x, y, s);
-        case 12: return launch_sg<12, VT, IT, SCAT>(h, x, y, s);
-        case 16: return launch_sg<16, VT, IT, SCAT>(h, x, y, s);
-        case 24: return launch_sg<24, VT, IT, SCAT>(h, x, y, s);
-        case 32: return launch_sg<32, VT, IT, SCAT>(h, x, y, s);
+        case 8: return launch_sg<8, VT, IT, W>(h, x, y, s);
+        case 12: return launch_sg<12, VT, IT, W>(h, x, y, s);
+        case 16: return launch_sg<16, VT, IT, W>(h, x, y, s);
+        case 24: return launch_sg<24, VT, IT, W>(h, x, y, s);
+        case 32: return launch_sg<32, VT, IT, W>(h, x, y, s);
         default: return cudaErrorInvalidValue;
     }
+}
+
+// Waves of chunks with `warps` resident warps per SM.
+long long waves(const Handle &h, int warps) {
+    const long long w = (long long)warps * h.sm_count;
+    return (h.nchunks + w - 1) / w;
 }
 
 }  // namespace
@@ -606,9 +610,20 @@ cudaError_t csr5_spmv(const Handle &h, const void *x, void *y, cudaStream_t s) {
     if (h.nchunks <= 0) return cudaSuccess;
     const bool f32 = h.precision == PAVA_PREC_FP32C, d16 = h.index_mode == PAVA_INDEX_DELTA16;
     if (d16)  // columns within 65,534 of one another in every chunk
-        return f32 ? spmv_t<float, short, false>(h, x, y, s) : spmv_t<double, short, false>(h, x, y, s);
-    if (!f32) return spmv_t<double, int, false>(h, x, y, s);
-    return h.scattered ? spmv_t<float, int, true>(h, x, y, s) : spmv_t<float, int, false>(h, x, y, s);
+        return f32 ? spmv_t<float, short, 24>(h, x, y, s) : spmv_t<double, short, 24>(h, x, y, s);
+    if (!f32) {
+        // 20 warps per SM, but 24 where they save a second or a third wave of chunks: 24 / 20 warps, us,
+        // banded 500,000 rows, sigma 24, 3,125 chunks 35.5 / 48.4, dense blocks 300,000 rows, sigma 32,
+        // 3,003 chunks 39.4 / 52.0, stencil 110^3, sigma 32, 6,901 chunks 88.6 / 95.7.  Of 38 forms with two
+        // waves of 20 warps and one of 24, one was slower with 24 (by 2 %), of 32 with three against two
+        // three (by 1 to 3 %), of those with more waves most; with as many waves 20 is 15 % faster.
+        const long long w24 = waves(h, 24), w20 = waves(h, 20);
+        return w24 <= 2 && w20 > w24 ? spmv_t<double, int, 24>(h, x, y, s)
+                                     : spmv_t<double, int, 20>(h, x, y, s);
+    }
+    // FP32: one CTA of 24, but three of 8 for 32-bit columns that are not scattered (Handle::scattered):
+    // stencil 128^3 115 -> 108 us, dense blocks 17 M 41.6 -> 38.6; power law 20 M 88 -> 90
+    return h.scattered ? spmv_t<float, int, 24>(h, x, y, s) : spmv_t<float, int, 8>(h, x, y, s);
 }
 
 }  // namespace pava
