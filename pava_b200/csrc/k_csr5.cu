@@ -609,8 +609,16 @@ cudaError_t csr5_convert(Handle &h, const int *rp, const int *ci, const double *
 cudaError_t csr5_spmv(const Handle &h, const void *x, void *y, cudaStream_t s) {
     if (h.nchunks <= 0) return cudaSuccess;
     const bool f32 = h.precision == PAVA_PREC_FP32C, d16 = h.index_mode == PAVA_INDEX_DELTA16;
-    if (d16)  // columns within 65,534 of one another in every chunk
-        return f32 ? spmv_t<float, short, 24>(h, x, y, s) : spmv_t<double, short, 24>(h, x, y, s);
+    if (d16 && !f32) return spmv_t<double, short, 24>(h, x, y, s);
+    if (d16) {
+        // One CTA of 24 warps, but three of 8 where neighbouring nonzeros share lines of x anyway and sigma
+        // is 12, or 32 with more than one wave of chunks.  24 / three of 8, us: sigma 12 stencil 110^3
+        // 88.0 / 77.1, banded 500,000 rows 35.8 / 30.8; sigma 32 stencil 110^3 58.3 / 53.6, banded
+        // 1,048,576 rows 40.0 / 38.8, 60^3 in 1,377 chunks 16.2 / 19.6; sigma 8, 16 and 24 within 3 %,
+        // mostly for 24; 256 stacked matrices (scattered) 48.8 / 67.3.
+        const bool three = !h.scattered && (h.sigma == 12 || (h.sigma == 32 && waves(h, 24) > 1));
+        return three ? spmv_t<float, short, 8>(h, x, y, s) : spmv_t<float, short, 24>(h, x, y, s);
+    }
     if (!f32) {
         // 20 warps per SM, but 24 where they save a second or a third wave of chunks: 24 / 20 warps, us,
         // banded 500,000 rows, sigma 24, 3,125 chunks 35.5 / 48.4, dense blocks 300,000 rows, sigma 32,
