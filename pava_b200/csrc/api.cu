@@ -618,10 +618,12 @@ pava_status pava_create(const pava_csr *A, int format, const pava_opts *opts, vo
         cudaEventDestroy(e0);
         cudaEventDestroy(e1);
     };
-    int *d_chk = nullptr, chk[3] = {0, 0, 0};  // violations, empty rows, sampled lines of x
+    int *d_chk = nullptr, chk[3] = {0, 0, 0};  // violations, empty rows (CSR: the longest row), sampled lines of x
     {
         ce = pava::pool_malloc(&d_chk, 3, s);
-        if (ce == cudaSuccess) ce = pava::launch_validate(rp, ci, h.m, h.n, h.nnz, d_chk, s);
+        if (ce == cudaSuccess)
+            ce = pava::launch_validate(rp, ci, h.m, h.n, h.nnz, d_chk,
+                                       format == PAVA_FORMAT_CSR ? d_chk + 1 : nullptr, s);
         cudaEventRecord(e0, s);
         const bool chunked = format == PAVA_FORMAT_CVR || format == PAVA_FORMAT_CSR5;
         if (ce == cudaSuccess && chunked) ce = dalloc(&h.arp, (size_t)h.m + 2, &h.device_bytes, s);
@@ -629,7 +631,8 @@ pava_status pava_create(const pava_csr *A, int format, const pava_opts *opts, vo
             ce = pava::build_augmented_rowptr(rp, h.m, h.arp, d_chk + 1, s);
         if (ce == cudaSuccess && chunked) ce = pava::sample_lines(ci, h.nnz, d_chk + 2, s);
         if (ce == cudaSuccess)
-            ce = cudaMemcpyAsync(chk, d_chk, sizeof(int) * (chunked ? 3 : 1), cudaMemcpyDeviceToHost, s);
+            ce = cudaMemcpyAsync(chk, d_chk, sizeof(int) * (chunked ? 3 : format == PAVA_FORMAT_CSR ? 2 : 1),
+                                 cudaMemcpyDeviceToHost, s);
         if (ce == cudaSuccess) ce = cudaStreamSynchronize(s);
         pava::pool_free(d_chk, s);
         if (ce != cudaSuccess) {
@@ -654,6 +657,7 @@ pava_status pava_create(const pava_csr *A, int format, const pava_opts *opts, vo
         h.G = pava::csr5_scattered_tiles((long long)h.nnz / (32LL * h.sigma), 20LL * h.sm_count);
         h.L = 32LL * h.sigma * h.G;
     }
+    if (format == PAVA_FORMAT_CSR) h.longest = chk[1];
     st = convert(h, rp, ci, v, chk[1], auto_index, s);
     if (st == PAVA_SUCCESS) {
         cudaEventRecord(e1, s);
@@ -720,18 +724,29 @@ pava_status pava_spmm(pava_handle *H, int k, const void *X, long long ldx, void 
         if (e != cudaSuccess) return fail_cuda(e, "spmm launch");
         return PAVA_SUCCESS;
     }
-    // Handles without a shape of their own: rows staged per warp for k >= 3, two columns per lane
-    // in groups of four lanes for k = 2 (FP64, banded / stencil / blocks: staged 123 / 137 / 98 us,
-    // groups 105 / 123 / 96; k = 3: 127 / 143 / 97 against 154 / 176 / 129).
+    // Handles without a shape of their own: rows staged per warp for k >= 3, two columns per lane in
+    // groups of four lanes for k = 2 (FP64, banded / stencil / blocks: staged 123 / 137 / 98 us, groups
+    // 105 / 123 / 96; k = 3: 127 / 143 / 97 against 154 / 176 / 129).  A staged row is a chain of its
+    // elements for its four to sixteen lanes; where that is longer than the whole product's share, a
+    // warp per row and its lanes side by side along the row: FP64, k = 2 / 8 / 64, us, staged / this:
+    // power law 200,003 rows (longest 3,945 of 3.1 M) 311 468 2,186 / 86 144 880, 1,300,021 rows (7,430
+    // of 20.4 M) 756 1,508 8,008 / 469 781 4,044; banded 300,007 rows with one of 500 (of 7.2 M) 62 89
+    // 519 / 91 120 466, of 1,000 97 137 824 / 93 127 537, of 2,000 174 249 1,415 / 108 148 784; FP32C
+    // alike (of 1,000 81 130 511 / 89 120 467).
     const bool own_shape = h.lanes_per_row || h.col_lanes || h.cols_per_lane || h.rows_per_tile ||
                            h.x_window;
-    if (!own_shape && k > 2) {
+    const bool uneven = (long long)h.longest * 6000 > h.nnz && (long long)h.longest * h.m > 4LL * h.nnz;
+    if (!own_shape && k > 2 && !uneven) {
         const cudaError_t e = pava::csr_spmm_staged(h, X, ldx, Y, ldy, k, 0, 0, (cudaStream_t)stream);
         if (e != cudaSuccess) return fail_cuda(e, "spmm launch");
         return PAVA_SUCCESS;
     }
     pava::Handle g, asked = h;
-    if (!own_shape && k == 2) {
+    if (!own_shape && uneven && k > 1) {
+        asked.lanes_per_row = 32;
+        asked.cols_per_lane = k <= 64 ? 2 : 4;
+        asked.col_lanes = pow2_ceil((k + asked.cols_per_lane - 1) / asked.cols_per_lane);
+    } else if (!own_shape && k == 2) {
         asked.lanes_per_row = 4;
         asked.col_lanes = 1;
         asked.cols_per_lane = 2;

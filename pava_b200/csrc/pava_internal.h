@@ -49,6 +49,7 @@ struct Handle {
     int sigma = 0, G = 0;    // CSR5: elements per lane per tile, tiles per chunk
     long long ntiles = 0;
     int scattered = 0;       // CVR, CSR5: neighbouring nonzeros rarely share lines of x
+    int longest = 0;         // plain CSR: elements of the longest row
     int lanes_per_row = 0;   // plain CSR: lanes per row group (GL)
     int col_lanes = 1;       //   lanes across the right-hand sides (KC)
     int cols_per_lane = 1;   //   right-hand sides per lane (KPL)
@@ -165,8 +166,9 @@ inline int csr5_scattered_tiles(long long tiles, long long warps) {
 }
 
 // Kernel launchers (stream-ordered; return cudaGetLastError()).
+// d_longest (optional): the length of the longest row, where the row pointer is sound.
 cudaError_t launch_validate(const int *rp, const int *ci, int m, int n, int nnz, int *d_err,
-                            cudaStream_t s);
+                            int *d_longest, cudaStream_t s);
 // arp[0..m]; arp[m + 1], the padded total, is the caller's (set_int).
 cudaError_t build_augmented_rowptr(const int *rp, int m, int *arp, int *d_nempty, cudaStream_t s);
 cudaError_t set_int(int *p, int v, cudaStream_t s);
