@@ -149,6 +149,25 @@ int pow2_ceil(int v) {
     return p;
 }
 
+// Whether a product with k right-hand sides takes a warp per row, its lanes side by side along the row
+// (32 lanes, two or four columns each), instead of staged rows.  A staged row is a chain of its elements
+// for its four to sixteen lanes, so the longest row bounds the product, which pays where that is more
+// than its share of the whole.
+// Rows far longer than the others, us, staged / this, k = 2, 8, 64: power law 200,003 rows (longest 3,945
+// of 3.1 M) 311 468 2,186 / 86 110 707, 1,300,021 rows (7,430 of 20.4 M) 756 1,508 8,008 / 465 606 3,281;
+// banded 300,007 rows with one of 500 (of 7.2 M) 62 89 519 / 91 120 466, of 1,000 97 137 824 / 93 127 537,
+// of 2,000 174 249 1,415 / 104 112 660; FP32C alike (of 1,000 81 130 511 / 89 120 467).
+// Small matrices of even rows, k = 3, 16, 64, 128: banded 3,001 rows 10 16 25 22 / 10 10 12 21, 24,001
+// rows 10 21 49 47 / 12 14 34 58; dense blocks 20,000 rows 19 32 83 82 / 14 18 45 79, 40,000 rows 25 44
+// 97 138 / 22 29 82 146; stencil 24^3 12 20 45 51 / 9 13 18 30, 32^3 13 27 54 57 / 14 17 43 74 (FP32C
+// 13 22 49 51 / 13 18 45 80).
+bool warp_per_row(const pava::Handle &h, int k) {
+    const bool even = (long long)h.longest * h.m <= 4LL * h.nnz;
+    if (even && k == 2) return false;
+    const long long rows = !even ? 6000 : k > 32 && k <= 64 && h.precision == PAVA_PREC_FP64 ? 30000 : 14000;
+    return (long long)h.longest * rows > h.nnz;
+}
+
 // The row-group shape of a CSR handle for k right-hand sides: the handle's options where
 // given, otherwise derived from k and the mean row length.  Returns false (with a message)
 // when the given options cannot serve k.
@@ -726,23 +745,17 @@ pava_status pava_spmm(pava_handle *H, int k, const void *X, long long ldx, void 
     }
     // Handles without a shape of their own: rows staged per warp for k >= 3, two columns per lane in
     // groups of four lanes for k = 2 (FP64, banded / stencil / blocks: staged 123 / 137 / 98 us, groups
-    // 105 / 123 / 96; k = 3: 127 / 143 / 97 against 154 / 176 / 129).  A staged row is a chain of its
-    // elements for its four to sixteen lanes; where that is longer than the whole product's share, a
-    // warp per row and its lanes side by side along the row: FP64, k = 2 / 8 / 64, us, staged / this:
-    // power law 200,003 rows (longest 3,945 of 3.1 M) 311 468 2,186 / 86 144 880, 1,300,021 rows (7,430
-    // of 20.4 M) 756 1,508 8,008 / 469 781 4,044; banded 300,007 rows with one of 500 (of 7.2 M) 62 89
-    // 519 / 91 120 466, of 1,000 97 137 824 / 93 127 537, of 2,000 174 249 1,415 / 108 148 784; FP32C
-    // alike (of 1,000 81 130 511 / 89 120 467).
+    // 105 / 123 / 96; k = 3: 127 / 143 / 97 against 154 / 176 / 129), or a warp per row.
     const bool own_shape = h.lanes_per_row || h.col_lanes || h.cols_per_lane || h.rows_per_tile ||
                            h.x_window;
-    const bool uneven = (long long)h.longest * 6000 > h.nnz && (long long)h.longest * h.m > 4LL * h.nnz;
-    if (!own_shape && k > 2 && !uneven) {
+    const bool by_warp = !own_shape && k > 1 && warp_per_row(h, k);
+    if (!own_shape && k > 2 && !by_warp) {
         const cudaError_t e = pava::csr_spmm_staged(h, X, ldx, Y, ldy, k, 0, 0, (cudaStream_t)stream);
         if (e != cudaSuccess) return fail_cuda(e, "spmm launch");
         return PAVA_SUCCESS;
     }
     pava::Handle g, asked = h;
-    if (!own_shape && uneven && k > 1) {
+    if (by_warp) {
         asked.lanes_per_row = 32;
         asked.cols_per_lane = k <= 64 ? 2 : 4;
         asked.col_lanes = pow2_ceil((k + asked.cols_per_lane - 1) / asked.cols_per_lane);

@@ -45,3 +45,21 @@ def test_products(cuda, precision, longest, k):
         for c in sorted({0, k // 2, k - 1}):
             yr, ab = O.csr_ref(A.rp, A.ci, A.v, np.ascontiguousarray(X[:, c]))
             assert O.rel_error(np.ascontiguousarray(out[:, c]), yr, ab, 1e-9 if fp32 else 1e-12)[0] == 0
+
+
+@pytest.mark.parametrize("precision", [_abi.PREC_FP64, _abi.PREC_FP32C])
+@pytest.mark.parametrize("m", [1, 31, 13_999, 14_001, 29_999, 30_001])   # a warp per row up to 14,000 or 30,000
+@pytest.mark.parametrize("k", [2, 3, 32, 33, 64, 65])
+def test_small_matrices_of_even_rows(cuda, precision, m, k):
+    torch = cuda
+    A = M.banded(m, 8, 6, seed=3) if m > 20 else M.from_arrays(m, m, np.arange(m + 1, dtype=np.int32),
+                                                              np.arange(m, dtype=np.int32), np.ones(m))
+    fp32 = precision == _abi.PREC_FP32C
+    A = M.from_arrays(A.m, A.n, A.rp, A.ci, A.v.astype(np.float32).astype(np.float64))
+    mat = SpMatrix(A, "csr", precision=precision)
+    X = M.uniform(A.n * k, seed=5, fp32=True).reshape(A.n, k)
+    Xd = torch.from_numpy(X).cuda()
+    y = mat.spmm(Xd.float() if fp32 else Xd).cpu().numpy()
+    for c in (0, k - 1):
+        yr, ab = O.csr_ref(A.rp, A.ci, A.v, np.ascontiguousarray(X[:, c]))
+        assert O.rel_error(np.ascontiguousarray(y[:, c]), yr, ab, 1e-9 if fp32 else 1e-12)[0] == 0
