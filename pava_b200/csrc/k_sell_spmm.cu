@@ -47,20 +47,33 @@ namespace {
 
 // The shape of G lanes per row: 32 G threads per CTA (32 rows), 32 / G CTAs per SM (32 warps), pieces
 // of KB blocks (100 KB of stages per SM for FP64 values and 32-bit columns with 8 or 16 lanes, which
-// leaves L1 room for the X rows neighbouring slices share).
+// leaves L1 room for the X rows neighbouring slices share).  Four lanes take pieces of 8 blocks, but of 4
+// for FP64 with five columns per lane or more, where 200 KB of stages left X no L1: stencil 90^3, k = 29,
+// 770 -> 430 us.  Eight columns per lane spill 50 to 120 bytes at 64 registers: FP64 pairs read the X of
+// one element at a time for 32-bit columns (k = 64, stencil 60^3 160 -> 150 us) and run 24 warps with 80
+// registers for 16-bit ones (Laplacian 900^2 231 -> 214); so do single FP32 columns beside 32-bit ones
+// (k = 63, Laplacian 900^2 267 -> 240), which beside 16-bit ones is slower (1.3 times).
 constexpr int SPMM_UNROLL = 2;  // blocks of a piece unrolled together
 // Neighbouring slices a CTA takes in a row: they share X rows, but long runs keep distant regions
 // of X alive at once (stencil, k = 16: 249, 251, 254 and 304 us at 1, 2, 4 and 16; FP32C 214, 202,
 // 200, 208).  One at a time where the matrix has few runs per resident CTA: fewer than 4 for FP32
 // (stencil 80^3, k = 32: 202 us one at a time, 196 in runs), 16 for FP64 (169 and 175).
 constexpr int RUN = 2;  // a power of two
-template <int G> struct SpmmShape {
+template <typename VT, typename IT, int G, int KPL, int VW> struct SpmmShape {
     static_assert(G == 4 || G == 8 || G == 16, "lanes per row");
-    static constexpr int THREADS = 32 * G, CTAS_PER_SM = 32 / G, KB = G == 4 ? 8 : G;
+    static constexpr bool F64 = sizeof(VT) == 8, I32 = sizeof(IT) == 4, WIDE = KPL >= 7;
+    static constexpr bool FEWER = WIDE && G <= 8 && (F64 ? VW == 2 && !I32 : VW == 1 && I32);
+    static constexpr int THREADS = 32 * G, CTAS_PER_SM = (FEWER ? 24 : 32) / G;
+    static constexpr int KB = G == 4 ? (F64 && KPL >= 5 ? 4 : 8) : G;
+    // elements of a block whose X reads are in flight together, four where registers allow (pads: in
+    // blocks with padding)
+    static constexpr int together(bool pads) {
+        return VW == 1 && KPL >= 3 ? 1 : F64 && I32 && WIDE ? 1 : KPL > 4 || pads ? 2 : 4;
+    }
 };
-template <typename VT, typename IT, int G> struct SpmmStage {
-    static constexpr int VBYTES = SpmmShape<G>::KB * 128 * (int)sizeof(VT);
-    static constexpr int CBYTES = SpmmShape<G>::KB * 128 * (int)sizeof(IT);
+template <typename VT, typename IT, int G, int KPL, int VW> struct SpmmStage {
+    static constexpr int VBYTES = SpmmShape<VT, IT, G, KPL, VW>::KB * 128 * (int)sizeof(VT);
+    static constexpr int CBYTES = SpmmShape<VT, IT, G, KPL, VW>::KB * 128 * (int)sizeof(IT);
     static constexpr int BYTES = 2 * (VBYTES + CBYTES) + 128;  // two pieces + barriers
 };
 
@@ -88,13 +101,13 @@ __device__ __forceinline__ void row_cols(const short *pc, int i, int r, int (&c)
 
 // LD: the type of X's leading dimension; int makes a row address one multiply-add.
 template <typename VT, typename IT, int G, int KPL, int VW, typename LD>
-__global__ void __launch_bounds__(SpmmShape<G>::THREADS, SpmmShape<G>::CTAS_PER_SM)
+__global__ void __launch_bounds__(SpmmShape<VT, IT, G, KPL, VW>::THREADS, SpmmShape<VT, IT, G, KPL, VW>::CTAS_PER_SM)
 sell_spmm_kernel(const SellSlice *__restrict__ meta, const VT *__restrict__ vals,
                  const IT *__restrict__ cols, const VT *X, LD ldx,
                  double *__restrict__ Y, long long ldy, int ns, int run, int m, int n, int k,
                   unsigned long long *err, unsigned long long *wait_err) {
-    using ST = SpmmStage<VT, IT, G>;
-    constexpr int KB = SpmmShape<G>::KB;
+    using ST = SpmmStage<VT, IT, G, KPL, VW>;
+    constexpr int KB = SpmmShape<VT, IT, G, KPL, VW>::KB;
     extern __shared__ __align__(128) unsigned char smem[];
     pdl_trigger();
     const int tid = threadIdx.x;
@@ -201,8 +214,7 @@ sell_spmm_kernel(const SellSlice *__restrict__ meta, const VT *__restrict__ vals
     const bool last = VW == 2 || spmm_col<G, VW>(lg, KPL - VW) < k;
     auto sum_block = [&](const VT *pv, const IT *pc, int i, auto pads_tag) {
         constexpr bool PADS = decltype(pads_tag)::value;
-        // elements whose X reads are in flight together: a block's four, where registers allow
-        constexpr int QB = VW == 1 && KPL >= 3 ? 1 : KPL > 4 || PADS ? 2 : 4;
+        constexpr int QB = SpmmShape<VT, IT, G, KPL, VW>::together(PADS);
         int c[4];
         row_cols(pc, i, r, c);
         const VBlk<VT> vv = VBlk<VT>::load_smem(pv, i, r);
@@ -278,7 +290,7 @@ sell_spmm_kernel(const SellSlice *__restrict__ meta, const VT *__restrict__ vals
 template <typename VT, typename IT, int G, int KPL, int VW, typename LD = int>
 cudaError_t spmm_launch(const Handle &h, const VT *X, long long ldx, double *Y, long long ldy,
                         int k, cudaStream_t s) {
-    using ST = SpmmStage<VT, IT, G>;
+    using ST = SpmmStage<VT, IT, G, KPL, VW>;
     constexpr auto kernel = sell_spmm_kernel<VT, IT, G, KPL, VW, LD>;
     // more than the default 48 KB of dynamic shared memory: opted into once per device
     static std::atomic<unsigned long long> opted{0};
@@ -290,11 +302,11 @@ cudaError_t spmm_launch(const Handle &h, const VT *X, long long ldx, double *Y, 
         if (e != cudaSuccess) return e;
         opted.fetch_or(bit);
     }
-    const long long cap = (long long)h.sm_count * SpmmShape<G>::CTAS_PER_SM;
+    const long long cap = (long long)h.sm_count * SpmmShape<VT, IT, G, KPL, VW>::CTAS_PER_SM;
     const int run = h.nchunks >= (sizeof(VT) == 8 ? 16 : 4) * RUN * cap ? RUN : 1;
     const long long runs = (h.nchunks + run - 1) / run;
     const unsigned grid = (unsigned)(runs < cap ? runs : cap);
-    return launch_product(kernel, grid, SpmmShape<G>::THREADS, ST::BYTES, s,
+    return launch_product(kernel, grid, SpmmShape<VT, IT, G, KPL, VW>::THREADS, ST::BYTES, s,
                           (const SellSlice *)h.meta, (const VT *)h.vals, (const IT *)h.cols, X,
                           (LD)ldx, Y, ldy, (int)h.nchunks, run, h.m, h.n, k, guard_word(), wait_word());
 }
@@ -340,7 +352,9 @@ cudaError_t spmm_g(const Handle &h, const VT *X, long long ldx, double *Y, long 
 template <typename VT, typename IT>
 cudaError_t spmm_k(const Handle &h, const VT *X, long long ldx, double *Y, long long ldy, int k,
                    cudaStream_t s) {
-    switch (sell_spmm_lanes(h.lanes_per_row, k, sizeof(VT) == 4, (long long)h.nnz >= 16LL * h.m)) {
+    // 16 elements per row and more; very long rows are "short" again for even k
+    const bool long_rows = (long long)h.nnz >= 16LL * h.m && (k % 2 || (long long)h.nnz <= 32LL * h.m);
+    switch (sell_spmm_lanes(h.lanes_per_row, k, sizeof(VT) == 4, long_rows)) {
         case 4: return spmm_g<VT, IT, 4>(h, X, ldx, Y, ldy, k, s);
         case 8: return spmm_g<VT, IT, 8>(h, X, ldx, Y, ldy, k, s);
         case 16: return spmm_g<VT, IT, 16>(h, X, ldx, Y, ldy, k, s);

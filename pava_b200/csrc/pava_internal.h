@@ -216,9 +216,10 @@ cudaError_t sell_spmv(const Handle &h, const void *x, void *y, cudaStream_t s);
 constexpr int SELL_SPMM_MAX_K = 64;
 // The engine's choice (lanes_per_row 0): four lanes, whose warp reads eight rows' X at once, while the
 // sums fit its registers: FP32 up to k = 24, odd k up to 28; FP64 up to k = 12, or 16 where rows are
-// short (under 16 elements).  FP64 in a loop, us, 4 / 8 lanes: stencil 60^3 k = 13 70 / 63, k = 16
-// 58 / 46, banded 500,000 rows k = 15 167 / 119, dense blocks k = 12 75 / 77, Laplacian 900^2 k = 13
-// 75 / 93; FP32 banded k = 20 116 / 160, k = 27 157 / 186, stencil k = 32 101 / 78.
+// short (under 16 elements) or, for even k, long (over 32).  FP64 in a loop, us, 4 / 8 lanes: stencil
+// 60^3 k = 13 70 / 63, k = 16 58 / 46, banded 500,000 rows k = 15 167 / 119, dense blocks k = 12 75 / 77,
+// 300,000 rows on 16-bit columns k = 16 103 / 122 (32-bit 104 / 108), Laplacian 900^2 k = 13 75 / 93; FP32 banded k = 20
+// 116 / 160, k = 27 157 / 186, stencil k = 32 101 / 78.
 inline int sell_spmm_lanes(int lanes_per_row, int k, bool f32 = false, bool long_rows = false) {
     const int four = f32 ? (k % 2 ? 28 : 24) : long_rows ? 12 : 16;
     const int g = lanes_per_row ? lanes_per_row : (k <= four ? 4 : 8);
