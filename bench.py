@@ -85,14 +85,16 @@ def peak_hbm():
         return FALLBACK_HBM_GBS, "fallback"
 
 
-def traffic_from_profiles(kernel_key):
-    """DRAM bytes per launch of the dominant kernel from the committed ncu summary, if any."""
-    path = os.path.join(ROOT, "profiles", "traffic.txt")
+def traffic_from_profiles(matrix, kernel_key, path=None):
+    """DRAM bytes per launch of kernel_key on this matrix (its ``powerlaw_<rows>_<nonzeros>`` key) from
+    the committed ncu summary; None where that pair was not captured."""
+    path = path or os.path.join(ROOT, "profiles", "traffic.txt")
     try:
-        for line in open(path):
-            k, _, v = line.partition("=")
-            if k.strip() == kernel_key:
-                return float(v.split()[0])
+        with open(path) as f:
+            for line in f:
+                k, _, v = line.partition("=")
+                if k.strip() == f"{matrix}.{kernel_key}":
+                    return float(v.split()[0])
     except OSError:
         pass
     return None
@@ -401,7 +403,7 @@ def main():
     peak, peak_kind = peak_hbm()
     achieved = alg / (main_ms * 1e-3) / 1e9
     kernel_key = f"{chosen}_main"
-    traffic = traffic_from_profiles(kernel_key)
+    traffic = traffic_from_profiles(f"powerlaw_{A.m}_{A.nnz}", kernel_key)
     line = None
     if rank == 0:
         cpu = None
