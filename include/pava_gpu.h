@@ -171,7 +171,9 @@ pava_status pava_spmv(pava_handle *h, const void *x, void *y, void *stream);
 
 /* Y = A X for k right-hand sides: X is n x k and Y is m x k, both row-major with leading
  * dimensions ldx >= k and ldy >= k (elements), device memory; FP64, or FP32C with float X and
- * double Y.  CSR handles (the row-group kernel), 1 <= k <= 128, and SELL handles (a CTA per
+ * double Y.  CSR handles (rows staged per warp, or a warp per row on small matrices and those with a
+ * row far longer than the others; the row-group kernel where options name a shape), 1 <= k <= 128,
+ * and SELL handles (a CTA per
  * 32-row slice, the slice's streams in shared memory, opts.lanes_per_row = 4, 8 or 16 lanes
  * per row across k; 0 = chosen by k, precision and row length), 1 <= k <= 64, k <= 32 with 4 lanes
  * (PAVA_E_UNSUPPORTED_PARAMS past it).  The reference has no multi-vector product; k = 1

@@ -1,5 +1,5 @@
 // SpMM on plain CSR for k right-hand sides (Y = A X, X row-major n x k): the kernel of handles whose
-// shape is left to the engine, and of the row-group shapes that give each of a row's lanes its own
+// shape is left to the engine (but for small matrices and very uneven rows, pava_spmm), and of the row-group shapes that give each of a row's lanes its own
 // columns (csr_staged_shape); k_group.cu runs the other shapes that options name.
 //
 // A warp takes 32 / G rows at a time, G lanes per row; lane g of a row's G owns the KPL columns of
@@ -16,7 +16,10 @@
 // the shape the engine chose before / the best row-group shape / this kernel: banded (1,048,576
 // rows, 24 each) k = 8 254 / 188 / 154 and 340 / 217 / 140, k = 16 621 / 295 / 267 and 693 / 383 /
 // 211, k = 32 1,234 / 506 / 366 and 1,420 / 734 / 365; stencil 100^3 k = 8 312 / 209 / 168, k = 32
-// 1,237 / 582 / 410; dense blocks (400,000 rows) k = 8 189 / 148 / 117, k = 32 814 / 371 / 251.
+// 1,237 / 582 / 410; dense blocks (400,000 rows) k = 8 189 / 148 / 117, k = 32 814 / 371 / 251.  In a
+// loop, FP64 / FP32, the shape before / this kernel: banded 300,007 rows k = 33 499 / 248 and 680 / 241,
+// k = 64 396 / 242 and 490 / 193, k = 127 953 / 549 and 1,638 / 463, k = 128 591 / 435 and 993 / 328 (the
+// 8-column forms for odd k spill 150 to 200 bytes; they are still the faster ones).
 // Without the next round's elements in flight k = 8 took 161, 174 and 118 us; with three CTAs per
 // SM 164, 182 and 117.
 //

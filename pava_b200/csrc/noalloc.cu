@@ -10,8 +10,8 @@
 // nnz-balanced chunks of NOALLOC_G tiles of 32 lanes x NOALLOC_SIGMA elements straight from
 // the CSR arrays, finds its rows by binary search in row_ptr, sums per-lane segments, combines
 // the lanes with the same fixed-order suffix scan, and writes rows it does not finish to
-// per-chunk carry slots.  The carry fixup of k_support.cu (unchanged) then adds those in chunk
-// order.  Empty rows are zeroed by a separate pass.
+// per-chunk carry slots.  The carry fixup of k_support.cu, in the form that reads the headers after
+// its wait, then adds those in chunk order.  Empty rows are zeroed by a separate pass.
 //
 // Scratch: one file-scope array of NOALLOC_SCRATCH_BYTES (1 MiB) per device, laid out as
 // [chunk headers | head carries | tail carries] for at most NOALLOC_MAX_CHUNKS chunks.  Every
@@ -181,7 +181,7 @@ extern "C" pava_status pava_spmv_csr_noalloc(int m, int n, int nnz, const int *r
         if (blocks > (long long)sms * 8) blocks = (long long)sms * 8;
         csr_tiles_noalloc_kernel<<<(unsigned)blocks, NA_WARPS * 32, 0, s>>>(
             row_ptr, col_idx, vals, x, y, m, nnz, nchunks, hdr, head, tail, n, guard_word());
-        // the unchanged carry fixup, pointed at the scratch: chunk c's first element is
+        // the carry fixup, pointed at the scratch, whose headers this call's kernel writes: chunk c's first element is
         // c*L and a shared row R starts in chunk row_ptr[R] / L
         Handle h;
         h.m = m;

@@ -99,10 +99,11 @@ void pool_trim(size_t keep);
 cudaError_t pool_release(size_t keep);
 
 // Launches a product kernel as a programmatic dependent of the kernel before it in the stream.
-// All product kernels let their dependents launch at once (pdl_trigger) and call pdl_wait before
-// they read x or write anything, so consecutive products overlap one's launch and first reads of
-// the format, which only conversion writes, with the end of the other; behind any other kernel
-// the launch waits as an ordinary one does.  512 x 512 Laplacian, CVR (SpMV and fixup): 12.3 ->
+// All product kernels let their dependents launch early (pdl_trigger: CVR, CSR5, SELL and the fixup at
+// once, the row groups of plain CSR after their own wait) and call pdl_wait before they read x or
+// write anything, so consecutive products overlap one's launch and first reads of the format, which
+// only conversion writes, with the end of the other; behind any other kernel the launch waits as an
+// ordinary one does.  x is read by ordinary loads: the kernel before may still be writing it.  512 x 512 Laplacian, CVR (SpMV and fixup): 12.3 ->
 // 10.3 us a product in a loop; 128^3 stencil, SELL FP32C: 74.5 -> 71.6 us.
 template <typename... KArgs, typename... Args>
 cudaError_t launch_product(void (*kernel)(KArgs...), unsigned grid, unsigned threads,
@@ -132,8 +133,8 @@ unsigned long long *guard_word();
 unsigned long long *wait_word();
 
 // CSR5 tiles per chunk.  The persistent grid keeps `warps` warps resident (24 per SM; FP64 on 32-bit
-// columns runs 20, and these rules count 24 for it too unless its columns are scattered); each
-// takes chunks in turn, so a chunk count just above a multiple of `warps` leaves a last wave that
+// columns runs 20 where that takes as many waves, and these rules count 24 for it too unless its
+// columns are scattered); each takes chunks in turn, so a chunk count just above a multiple of `warps` leaves a last wave that
 // few warps run.
 // Default: 4 tiles per chunk, fewer when that leaves fewer chunks than warps.
 inline int csr5_default_tiles(long long tiles, long long warps) {
@@ -235,8 +236,8 @@ cudaError_t sell_spmm(const Handle &h, const void *X, long long ldx, void *Y, lo
 cudaError_t csr_spmv(const Handle &h, const void *x, void *y, cudaStream_t s);
 cudaError_t csr_spmm(const Handle &h, const void *X, long long ldx, void *Y, long long ldy,
                      int k, cudaStream_t s);
-// SpMM with the rows staged per warp (k_csr_spmm.cu), k in 1 .. 128, in the engine's own shape for
-// k; csr_spmm runs it too for the shapes csr_staged_shape accepts.
+// SpMM with the rows staged per warp (k_csr_spmm.cu), k in 1 .. 128, in its own shape for k (lanes = 0)
+// or a named one; csr_spmm runs it too for the shapes csr_staged_shape accepts.
 cudaError_t csr_spmm_staged(const Handle &h, const void *X, long long ldx, void *Y, long long ldy,
                             int k, int lanes, int cols, cudaStream_t s);
 bool csr_staged_shape(const Handle &shape, int k);
