@@ -641,8 +641,7 @@ pava_status pava_create(const pava_csr *A, int format, const pava_opts *opts, vo
     {
         ce = pava::pool_malloc(&d_chk, 3, s);
         if (ce == cudaSuccess)
-            ce = pava::launch_validate(rp, ci, h.m, h.n, h.nnz, d_chk,
-                                       format == PAVA_FORMAT_CSR ? d_chk + 1 : nullptr, s);
+            ce = pava::launch_validate(rp, ci, h.m, h.n, h.nnz, d_chk, format == PAVA_FORMAT_CSR, s);
         cudaEventRecord(e0, s);
         const bool chunked = format == PAVA_FORMAT_CVR || format == PAVA_FORMAT_CSR5;
         if (ce == cudaSuccess && chunked) ce = dalloc(&h.arp, (size_t)h.m + 2, &h.device_bytes, s);

@@ -167,9 +167,10 @@ inline int csr5_scattered_tiles(long long tiles, long long warps) {
 }
 
 // Kernel launchers (stream-ordered; return cudaGetLastError()).
-// d_longest (optional): the length of the longest row, where the row pointer is sound.
+// d_err[0]: violations; want_longest: d_err[1] = the length of the longest row, where the row pointer is
+// sound.
 cudaError_t launch_validate(const int *rp, const int *ci, int m, int n, int nnz, int *d_err,
-                            int *d_longest, cudaStream_t s);
+                            bool want_longest, cudaStream_t s);
 // arp[0..m]; arp[m + 1], the padded total, is the caller's (set_int).
 cudaError_t build_augmented_rowptr(const int *rp, int m, int *arp, int *d_nempty, cudaStream_t s);
 cudaError_t set_int(int *p, int v, cudaStream_t s);
