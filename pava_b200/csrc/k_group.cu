@@ -393,8 +393,9 @@ csr_window_kernel(const int *__restrict__ rp, const int *__restrict__ ci,
 //    in its group it would run len / (U GL) dependent rounds while the other groups wait.  Narrow
 //    groups (GL <= 4) keep them where so many of a warp's rows are long that one after the other
 //    they would take more rounds (one lane per row, us, each row by the warp / this: banded 500,000
-//    rows of 24 135 / 121 with L2 flushed, in tiles of 512 rows 484 / 128; power law 40,000 rows 45 / 45,
-//    and 73 where half as many rows were enough to stay in the groups);
+//    rows of 24 140 / 117 with L2 flushed, in tiles of 512 rows 494 / 129; power law 40,000 rows 45 / 43,
+//    and 73 where half as many rows were enough to stay in the groups).  They have a loop of their own:
+//    choosing before the short rows' loop cost Laplacian 1960^2 15 % (77 -> 88 us; this 74);
 //  * a row longer than HUGE_ROW waits until the CTA's tiles are done and is summed by all of its
 //    warps.  Each warp keeps up to LIST such rows (and sums further ones alone), so which rows
 //    take which way depends on the matrix and the launch shape only, and results repeat bit
@@ -471,36 +472,42 @@ csr_spmv_kernel(const int *__restrict__ rp, const int *__restrict__ ci, const VT
                 b = rp[r + 1];
             }
             const int len = b - a;
-            bool is_long = len > LONG;
+            const bool is_long = len > LONG;
+            const VT *vr = v + a;
+            const int *cr = ci + a;
+            auto by_group = [&](int count) -> double {  // the row's first `count` elements, by its group
+                Acc<VT> acc;
+                for (int j = gi; j < count; j += U * GL) {
+                    VT val[U];
+                    int col[U];
+#pragma unroll
+                    for (int u = 0; u < U; ++u) {
+                        const bool in = j + u * GL < len;
+                        val[u] = in ? ld_val(vr + (j + u * GL), pf) : VT(0);
+                        col[u] = in ? ld_col(cr + (j + u * GL), pf) : -1;
+                    }
+#pragma unroll
+                    for (int u = 0; u < U; ++u)
+                        if (col[u] >= 0) acc.add(val[u], gather(col[u]));
+                }
+                double s = acc.value();
+#pragma unroll
+                for (int o = 1; o < GL; o <<= 1) s += __shfl_xor_sync(FULL, s, o);
+                return s;
+            };
+            const double s = by_group(is_long ? 0 : len);
+            if (r < (unsigned)m && gi == 0 && !is_long) y[r * ldy] = s;
             unsigned todo = __ballot_sync(FULL, is_long && gi == 0);
             if (GL <= 4 && todo) {  // many of them: the groups are done sooner, all at once
                 const bool mid = is_long && len <= HUGE_ROW;
                 const int most = __reduce_max_sync(FULL, mid ? len : 0);
                 const int count = __popc(__ballot_sync(FULL, mid && gi == 0));
-                if (count * ((most + 32 * WU - 1) / (32 * WU)) >= (most + U * GL - 1) / (U * GL))
-                    is_long = len > HUGE_ROW;
-                todo = __ballot_sync(FULL, is_long && gi == 0);
-            }
-            const VT *vr = v + a;
-            const int *cr = ci + a;
-            Acc<VT> acc;
-            for (int j = gi; j < (is_long ? 0 : len); j += U * GL) {
-                VT val[U];
-                int col[U];
-#pragma unroll
-                for (int u = 0; u < U; ++u) {
-                    const bool in = j + u * GL < len;
-                    val[u] = in ? ld_val(vr + (j + u * GL), pf) : VT(0);
-                    col[u] = in ? ld_col(cr + (j + u * GL), pf) : -1;
+                if (count * ((most + 32 * WU - 1) / (32 * WU)) >= (most + U * GL - 1) / (U * GL)) {
+                    const double sm = by_group(mid ? len : 0);
+                    if (mid && gi == 0) y[r * ldy] = sm;
+                    todo = __ballot_sync(FULL, is_long && !mid && gi == 0);
                 }
-#pragma unroll
-                for (int u = 0; u < U; ++u)
-                    if (col[u] >= 0) acc.add(val[u], gather(col[u]));
             }
-            double s = acc.value();
-#pragma unroll
-            for (int o = 1; o < GL; o <<= 1) s += __shfl_xor_sync(FULL, s, o);
-            if (r < (unsigned)m && gi == 0 && !is_long) y[r * ldy] = s;
             // long rows, one after the other, by the whole warp
             while (todo) {
                 const int src = __ffs(todo) - 1;
