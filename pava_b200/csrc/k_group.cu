@@ -395,7 +395,10 @@ csr_window_kernel(const int *__restrict__ rp, const int *__restrict__ ci,
 //    they would take more rounds (one lane per row, us, each row by the warp / this: banded 500,000
 //    rows of 24 140 / 117 with L2 flushed, in tiles of 512 rows 494 / 129; power law 40,000 rows 45 / 43,
 //    and 73 where half as many rows were enough to stay in the groups).  They have a loop of their own:
-//    choosing before the short rows' loop cost Laplacian 1960^2 15 % (77 -> 88 us; this 74);
+//    choosing before the short rows' loop cost Laplacian 1960^2 15 % (77 -> 88 us; this 74).  FP64 rows
+//    of one lane stay with the warp where there are more tiles than warps (by_cta > 1), since a lane per
+//    row reads a line per element then: dense blocks 300,000 rows in tiles of 32 219 / 96 us, stencil
+//    110^3 in tiles of 128 528 / 288 by the groups / the warp, L2 flushed;
 //  * a row longer than HUGE_ROW waits until the CTA's tiles are done and is summed by all of its
 //    warps.  Each warp keeps up to LIST such rows (and sums further ones alone), so which rows
 //    take which way depends on the matrix and the launch shape only, and results repeat bit
@@ -498,7 +501,8 @@ csr_spmv_kernel(const int *__restrict__ rp, const int *__restrict__ ci, const VT
             const double s = by_group(is_long ? 0 : len);
             if (r < (unsigned)m && gi == 0 && !is_long) y[r * ldy] = s;
             unsigned todo = __ballot_sync(FULL, is_long && gi == 0);
-            if (GL <= 4 && todo) {  // many of them: the groups are done sooner, all at once
+            // many of them: the groups are done sooner, all at once
+            if (GL <= 4 && todo && !(GL == 1 && sizeof(VT) == 8 && by_cta != 1u)) {
                 const bool mid = is_long && len <= HUGE_ROW;
                 const int most = __reduce_max_sync(FULL, mid ? len : 0);
                 const int count = __popc(__ballot_sync(FULL, mid && gi == 0));

@@ -47,3 +47,26 @@ def test_rounds(cuda, precision, lanes, per_lane, count):
     y = mat.spmv(xd)
     assert O.rel_error(y.cpu().numpy(), yr, ab, 1e-9 if fp32 else 1e-12)[0] == 0  # the stated bounds
     assert torch.equal(y, mat.spmv(xd))
+
+
+@pytest.mark.parametrize("precision", [_abi.PREC_FP64, _abi.PREC_FP32C])
+@pytest.mark.parametrize("rows_per_tile,m", [(32, 32 * 7104), (32, 32 * 7104 + 1), (64, 64 * 7104 + 1)])
+def test_more_tiles_than_warps(cuda, precision, rows_per_tile, m):
+    torch = cuda
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    m = m // 7104 * (48 * sms) + m % 7104                # 48 warps per SM
+    lens = np.full(m, 17)
+    lens[::3] = 5
+    rp = np.concatenate([[0], np.cumsum(lens)]).astype(np.int32)
+    rng = np.random.default_rng(3)
+    n = 4000
+    ci = rng.integers(0, n, int(rp[-1])).astype(np.int32)
+    v = rng.normal(size=len(ci)).astype(np.float32).astype(np.float64)
+    A = M.from_arrays(m, n, rp, ci, v)
+    fp32 = precision == _abi.PREC_FP32C
+    x = M.uniform(n, seed=6, fp32=True)
+    yr, ab = O.csr_ref(A.rp, A.ci, A.v, x)
+    xd = torch.from_numpy(x).cuda()
+    mat = SpMatrix(A, "csr", precision=precision, lanes_per_row=1, rows_per_tile=rows_per_tile)
+    y = mat.spmv(xd.float() if fp32 else xd)
+    assert O.rel_error(y.cpu().numpy(), yr, ab, 1e-9 if fp32 else 1e-12)[0] == 0
