@@ -32,9 +32,9 @@ unsigned grid_of(long long work, long long cap) {
 }
 
 struct CooStat {
-    unsigned long long mirrored;    // entries the symmetric expansion adds
-    unsigned long long long_total;  // nonzeros in rows longer than RANK_MAX
-    int bad, nlong;                 // entries outside the matrix, rows longer than RANK_MAX
+    unsigned long long mirrored;  // entries the symmetric expansion adds
+    unsigned long long longs;     // rows longer than RANK_MAX << 32 | their nonzeros
+    int bad, longest;             // entries outside the matrix, nonzeros of the longest long row
 };
 
 // A record of the scatter: key = column << 32 | mirrored << 31 | input position, and the value.
@@ -101,7 +101,8 @@ coo_count_kernel(const int *__restrict__ rows, const int *__restrict__ cols, lon
 }
 
 // Rows are sorted by counting, for each entry, the smaller keys of its row: up to RANK_MAX
-// entries.  Longer rows (listed here) are sorted by cub's segmented sort.
+// entries.  Longer rows are listed here, with ascending places in the packed array (one atomic
+// hands out both: rows and nonzeros are below 2^31), and sorted by cub.
 constexpr int RANK_MAX = 256;
 __global__ void coo_long_kernel(const int *__restrict__ cnt, int m, CooStat *__restrict__ st,
                                 const int *__restrict__ rp, int *__restrict__ row,
@@ -110,9 +111,11 @@ __global__ void coo_long_kernel(const int *__restrict__ cnt, int m, CooStat *__r
     if (r >= m) return;
     const int len = cnt ? cnt[r] : rp[r + 1] - rp[r];
     if (len <= RANK_MAX) return;
-    const int q = atomicAdd(&st->nlong, 1);
-    const unsigned long long off = atomicAdd(&st->long_total, (unsigned long long)len);
-    if (row) {
+    const unsigned long long at = atomicAdd(&st->longs, (1ull << 32) | (unsigned)len);
+    const unsigned q = (unsigned)(at >> 32), off = (unsigned)at;
+    if (!row) {
+        atomicMax(&st->longest, len);
+    } else {
         row[q] = (int)r;
         begin[q] = (int)off;
         end[q] = (int)off + len;
@@ -218,6 +221,114 @@ __global__ void coo_long_unpack_kernel(const int *__restrict__ rp, const int *__
     }
 }
 
+// cub's segmented sort and the two kernels above give a row to one block, about 13 ns per entry: a
+// row of 20 M entries took 390 ms.  Where the longest row has WIDE_MIN entries and there is less to
+// sort than WIDE_ROWS such rows, all long rows are sorted by the whole device instead: a radix sort
+// of the keys, then, where there are several rows, a stable one of the rows' numbers in the list.
+// Whole conversion, segmented / wide: one row of 8000 225 / 201 us, of 32000 515 / 201, of 3 M
+// 40.6 / 0.59 ms, of 20 M 390 / 2.9 ms; 100 rows of 8000 265 / 318 us, of 16000 411 / 440, of
+// 32000 742 / 663; 300 rows of 16000 780 / 934 us, of 32000 1.52 / 1.61 ms.
+constexpr int WIDE_MIN = 16384, WIDE_ROWS = 148;
+
+// Packed place t -> the listed row that holds it: the last one that begins at or before t.
+__device__ __forceinline__ int listed_row(const int *__restrict__ begin, int nl, int t) {
+    int lo = 0, hi = nl;
+    while (hi - lo > 1) {
+        const int mid = lo + (hi - lo) / 2;
+        if (begin[mid] <= t) lo = mid; else hi = mid;
+    }
+    return lo;
+}
+__global__ void __launch_bounds__(256)
+coo_wide_pack_kernel(const int *__restrict__ rp, const int *__restrict__ row,
+                     const int *__restrict__ begin, int nl, int total,
+                     const CooRec *__restrict__ rec, unsigned long long *__restrict__ keys,
+                     int *__restrict__ which) {
+    const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= total) return;
+    const int q = listed_row(begin, nl, (int)t);
+    keys[t] = rec[rp[row[q]] + ((int)t - begin[q])].key;
+    if (which) which[t] = q;
+}
+__global__ void __launch_bounds__(256)
+coo_wide_unpack_kernel(const int *__restrict__ rp, const int *__restrict__ row,
+                       const int *__restrict__ begin, int total,
+                       const unsigned long long *__restrict__ keys, const int *__restrict__ which,
+                       const double *__restrict__ vals, int *__restrict__ ci,
+                       double *__restrict__ v) {
+    const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= total) return;
+    const int q = which ? which[t] : 0;
+    const int at = rp[row[q]] + ((int)t - begin[q]);
+    const unsigned long long key = keys[t];
+    ci[at] = (int)(key >> 32);
+    v[at] = vals[key & 0x7fffffffull];
+}
+
+int bits_of(unsigned x) {  // of the values below x
+    int b = 1;
+    while (b < 32 && (x - 1) >> b) ++b;
+    return b;
+}
+
+// The long rows' entries from rec, sorted, into ci and v.  `held` takes what is still to be freed.
+// Once packed, rec is where the sorts put their other copy: it is read last by the pack kernels.
+cudaError_t sort_long_rows(int m, int n, const CooStat &h, CooStat *d_st, const int *rp,
+                           CooRec *rec, const double *vals, int *ci, double *v, void **held,
+                           cudaStream_t s) {
+    const int nl = (int)(h.longs >> 32), lt = (int)(unsigned)h.longs;
+    const bool wide = h.longest >= WIDE_MIN && lt / h.longest < WIDE_ROWS;
+    const bool several = wide && nl > 1;
+    const size_t n_l = (size_t)nl, n_t = (size_t)lt;
+    int *seg = nullptr, *which = nullptr;
+    unsigned long long *keys = nullptr;
+    cudaError_t e = pool_malloc(&seg, 3 * n_l, s);
+    held[0] = seg;
+    if (e == cudaSuccess) e = pool_malloc(&keys, n_t, s);
+    held[1] = keys;
+    if (e == cudaSuccess && several) e = pool_malloc(&which, n_t, s);
+    held[2] = which;
+    if (e == cudaSuccess) e = cudaMemsetAsync(d_st, 0, sizeof(CooStat), s);
+    if (e != cudaSuccess) return e;
+    const int *row = seg, *begin = seg + n_l, *end = seg + 2 * n_l;
+    coo_long_kernel<<<(unsigned)(((long long)m + 255) / 256), 256, 0, s>>>(
+        nullptr, m, d_st, rp, seg, seg + n_l, seg + 2 * n_l);
+    const unsigned blocks = (unsigned)((n_t + 255) / 256);
+    if (wide)
+        coo_wide_pack_kernel<<<blocks, 256, 0, s>>>(rp, row, begin, nl, lt, rec, keys, which);
+    else
+        coo_long_pack_kernel<<<(unsigned)nl, 256, 0, s>>>(rp, row, begin, rec, keys);
+    e = cudaGetLastError();
+    if (e != cudaSuccess) return e;
+    // Two buffers each: a sort leaves its result in either
+    cub::DoubleBuffer<unsigned long long> kb(keys, reinterpret_cast<unsigned long long *>(rec));
+    cub::DoubleBuffer<int> wb(which, which ? reinterpret_cast<int *>(rec) + 2 * n_t : nullptr);
+    const int key_bits = 32 + bits_of((unsigned)n), row_bits = bits_of((unsigned)nl);
+    auto sort = [&](int step, void *tmp, size_t &tb) {
+        if (!wide) return cub::DeviceSegmentedSort::SortKeys(tmp, tb, kb, lt, nl, begin, end, s);
+        if (!several) return cub::DeviceRadixSort::SortKeys(tmp, tb, kb, lt, 0, key_bits, s);
+        if (step == 0) return cub::DeviceRadixSort::SortPairs(tmp, tb, kb, wb, lt, 0, key_bits, s);
+        return cub::DeviceRadixSort::SortPairs(tmp, tb, wb, kb, lt, 0, row_bits, s);
+    };
+    size_t tb = 0, tb2 = 0;
+    e = sort(0, nullptr, tb);
+    if (e == cudaSuccess && several) e = sort(1, nullptr, tb2);
+    if (tb < tb2) tb = tb2;
+    char *tmp = nullptr;
+    if (e == cudaSuccess) e = pool_malloc(&tmp, tb, s);
+    held[3] = tmp;
+    if (e == cudaSuccess) e = sort(0, tmp, tb);
+    if (e == cudaSuccess && several) e = sort(1, tmp, tb);
+    if (e != cudaSuccess) return e;
+    if (wide)
+        coo_wide_unpack_kernel<<<blocks, 256, 0, s>>>(rp, row, begin, lt, kb.Current(),
+                                                      wb.Current(), vals, ci, v);
+    else
+        coo_long_unpack_kernel<<<(unsigned)nl, 256, 0, s>>>(rp, row, begin, kb.Current(), vals, ci,
+                                                           v);
+    return cudaGetLastError();
+}
+
 }  // namespace
 
 }  // namespace pava
@@ -239,12 +350,11 @@ pava_status coo_to_csr(int m, int n, long long nnz, const int *rows, const int *
     }
     if (nnz > 2147483000LL) { set_last_error("more than 2^31 entries"); return PAVA_E_TOO_LARGE; }
     cudaStream_t s = (cudaStream_t)stream;
-    int *cnt = nullptr, *cur = nullptr, *rp = nullptr, *ci = nullptr, *seg = nullptr;
+    int *cnt = nullptr, *cur = nullptr, *rp = nullptr, *ci = nullptr;
     CooStat *d_st = nullptr;
     CooRec *rec = nullptr;
-    unsigned long long *keys = nullptr;
     double *v = nullptr;
-    void *tmp = nullptr;
+    void *tmp = nullptr, *held_long[4] = {};
     // it allocates and waits: not on a stream that is being captured.  Nothing is held yet, and a
     // wait or a trim here would end the caller's capture.
     cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
@@ -257,8 +367,9 @@ pava_status coo_to_csr(int m, int n, long long nnz, const int *rows, const int *
     }
     const size_t held = pool_reserved();
     auto cleanup = [&]() {
-        pool_free(cnt, s); pool_free(cur, s); pool_free(seg, s); pool_free(d_st, s);
-        pool_free(rec, s); pool_free(keys, s); pool_free(tmp, s);
+        pool_free(cnt, s); pool_free(cur, s); pool_free(d_st, s); pool_free(rec, s);
+        pool_free(tmp, s);
+        for (void *p : held_long) pool_free(p, s);
     };
     auto give_back = [&]() {
         cleanup();
@@ -330,32 +441,8 @@ pava_status coo_to_csr(int m, int n, long long nnz, const int *rows, const int *
             e = cudaGetLastError();
         }
     }
-    if (e == cudaSuccess && h.nlong > 0) {
-        const size_t nl = (size_t)h.nlong, lt = (size_t)h.long_total;
-        e = pool_malloc(&seg, 3 * nl, s);
-        if (e == cudaSuccess) e = pool_malloc(&keys, 2 * lt, s);
-        if (e == cudaSuccess) e = cudaMemsetAsync(d_st, 0, sizeof(CooStat), s);
-        if (e == cudaSuccess) {
-            coo_long_kernel<<<row_blocks, 256, 0, s>>>(nullptr, m, d_st, rp, seg, seg + nl,
-                                                       seg + 2 * nl);
-            coo_long_pack_kernel<<<(unsigned)nl, 256, 0, s>>>(rp, seg, seg + nl, rec, keys);
-            e = cudaGetLastError();
-        }
-        pool_free(tmp, s);
-        tmp = nullptr;
-        if (e == cudaSuccess)
-            e = cub::DeviceSegmentedSort::SortKeys(nullptr, tb, keys, keys + lt, (int)lt, (int)nl,
-                                                   seg + nl, seg + 2 * nl, s);
-        if (e == cudaSuccess) e = pool_malloc(&tmp, tb, s);
-        if (e == cudaSuccess)
-            e = cub::DeviceSegmentedSort::SortKeys(tmp, tb, keys, keys + lt, (int)lt, (int)nl,
-                                                   seg + nl, seg + 2 * nl, s);
-        if (e == cudaSuccess) {
-            coo_long_unpack_kernel<<<(unsigned)nl, 256, 0, s>>>(rp, seg, seg + nl, keys + lt, vals,
-                                                               ci, v);
-            e = cudaGetLastError();
-        }
-    }
+    if (e == cudaSuccess && h.longs)
+        e = sort_long_rows(m, n, h, d_st, rp, rec, vals, ci, v, held_long, s);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
     if (e != cudaSuccess) return fail_e(e);
     cleanup();
