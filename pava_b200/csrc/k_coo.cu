@@ -43,13 +43,29 @@ struct CooRec {
     double val;
 };
 
-// Adds `on` lanes' counts to their rows' counters, one atomic per run of equal rows in
-// neighbouring lanes (sorted inputs have long ones), and returns the lane's slot.  All 32 lanes.
+// Adds `on` lanes' counts to their rows' counters and returns the lane's slot: one atomic per run of
+// equal rows in neighbouring lanes (sorted inputs have long ones).  Where a lane's row is also that
+// of the lane half a warp away and there are MATCH_MIN runs, one per different row: the atomics of a
+// hot row in shuffled order go to one address, 0.3 ns each.  Whole conversion of 20 M entries, half
+// of them in one row, shuffled: 8.05 -> 2.34 ms; in two rows that alternate 15.4 -> 3.4; random
+// rows, which pay for the test, 1.19 -> 1.22, with every warp matched 1.23 (row order 0.77 -> 0.89
+// then, 0.75 with the test).  All 32 lanes.
+constexpr int MATCH_MIN = 8;
 __device__ __forceinline__ int run_add(int *cnt, int row, bool on, int lane) {
     const int left = __shfl_up_sync(FULL, row, 1);
     const unsigned act = __ballot_sync(FULL, on);
     const bool lead = on && (lane == 0 || !((act >> (lane - 1)) & 1u) || left != row);
     const unsigned leads = __ballot_sync(FULL, lead);
+    const int across = __shfl_xor_sync(FULL, row, 16);
+    const bool far = on && ((act >> (lane ^ 16)) & 1u) && across == row;
+    if (__popc(leads) >= MATCH_MIN && __any_sync(FULL, far)) {
+        const unsigned same = __match_any_sync(FULL, on ? row : -1);
+        const int first = __ffs(same) - 1;
+        int base = 0;
+        if (on && lane == first) base = atomicAdd(&cnt[row], __popc(same));
+        base = __shfl_sync(FULL, base, first);
+        return base + __popc(same & ((1u << lane) - 1u));
+    }
     // a run ends before the next leader or the next inactive lane
     int base = 0, src = lane;
     if (on) src = 31 - __clz(leads & (0xffffffffu >> (31 - lane)));
