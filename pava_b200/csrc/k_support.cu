@@ -7,6 +7,7 @@
 
 #include <map>
 #include <mutex>
+#include <unordered_map>
 #include <utility>
 #include <vector>
 
@@ -27,8 +28,25 @@ struct DevicePool {
     cudaMemPool_t pool = nullptr;
     void *anchor = nullptr;       // keeps the driver's block of small allocations mapped
     std::vector<void *> waiting;  // freed while the device could not be waited for
+    size_t large = 0;             // bytes of the large blocks that are in use out of the pool
 };
 std::mutex g_pool_mutex;
+// The blocks of at least LARGE_MIN bytes that pool_malloc gave and that are in use.
+struct LargeBlock {
+    DevicePool *from;
+    size_t bytes;
+    bool plain;  // by cudaMalloc
+};
+std::unordered_map<void *, LargeBlock> &g_large = *new std::unordered_map<void *, LargeBlock>();
+// Takes p off the list; whether cudaMalloc gave it.  g_pool_mutex held.
+bool forget_large(void *p) {
+    const auto it = g_large.find(p);
+    if (it == g_large.end()) return false;
+    const bool plain = it->second.plain;
+    if (!plain) it->second.from->large -= it->second.bytes;
+    g_large.erase(it);
+    return plain;
+}
 // One per device and context: a program may alternate contexts on a device, and a context keeps its
 // pool.  A device reset ends a context and what its pool held; contexts are never numbered alike, so
 // the entry it leaves is not met again.  Never destroyed: handles may be freed at process exit.
@@ -127,14 +145,51 @@ cudaError_t current_pool(cudaMemPool_t *pool) {
     return e;
 }
 
+// Large blocks that the pool would not keep once they are freed come from cudaMalloc.  What a pool
+// holds above its threshold is mapped and unmapped for each use, at several times cudaMalloc's price:
+// blocks of 1.28, 0.64 and 0.32 GB taken and given back in turn take 14.0 ms from the pool, 3.6 from
+// cudaMalloc; one of 5 GB 50 and 4.8.  Conversion of 200 M nonzeros to CSR5 22.2 -> 4.2 ms,
+// to plain CSR 21.5 -> 2.7; COO -> CSR of 80 M entries 20 -> 7.1; CSR5 of 20 M beside a live matrix of
+// 1.4 GB 2.9 -> 0.22.  The sizes in use are counted here: the pool's own count still holds, for a
+// while, what has been freed.  Below LARGE_MIN cudaMalloc (0.3 ms and more, and cudaFree waits) is no
+// cheaper than mapping.
+constexpr size_t LARGE_MIN = (size_t)64 << 20;
+
+// cudaMalloc and cudaFree beside a capture on another stream, in whichever mode.
+struct RelaxedCapture {
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+    ~RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+};
+
 }  // namespace
 
 cudaError_t pool_malloc(void **p, size_t bytes, cudaStream_t s) {
     *p = nullptr;
     cudaMemPool_t pool = nullptr;
-    cudaError_t e = current_pool(&pool);
-    if (e != cudaSuccess) return e;
+    DevicePool *d = nullptr;
+    bool plain = false;
     if (bytes == 0) bytes = 1;
+    cudaError_t e = cudaSuccess;
+    {
+        std::lock_guard<std::mutex> lock(g_pool_mutex);
+        e = device_pool(&d);
+        if (e != cudaSuccess) return e;
+        pool = d->pool;
+        plain = bytes >= LARGE_MIN && d->large + bytes > POOL_KEEP;
+    }
+    cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
+    if (plain && cudaStreamIsCapturing(s, &capturing) == cudaSuccess &&
+        capturing == cudaStreamCaptureStatusNone) {
+        RelaxedCapture relaxed;
+        if (cudaMalloc(p, bytes) == cudaSuccess) {
+            std::lock_guard<std::mutex> lock(g_pool_mutex);
+            g_large[*p] = {d, bytes, true};
+            return cudaSuccess;
+        }
+        cudaGetLastError();  // the pool may hold it
+        *p = nullptr;
+    }
     e = cudaMallocFromPoolAsync(p, bytes, pool, s);
     if (e == cudaErrorMemoryAllocation) {  // memory freed on other streams may still be on its way
         cudaGetLastError();
@@ -143,8 +198,17 @@ cudaError_t pool_malloc(void **p, size_t bytes, cudaStream_t s) {
             e = cudaMallocFromPoolAsync(p, bytes, pool, s);
         }
     }
-    if (e != cudaSuccess) *p = nullptr;
-    return e;
+    if (e != cudaSuccess) {
+        *p = nullptr;
+        return e;
+    }
+    std::lock_guard<std::mutex> lock(g_pool_mutex);
+    forget_large(*p);  // an address of a context that a reset ended
+    if (bytes >= LARGE_MIN) {
+        d->large += bytes;
+        g_large[*p] = {d, bytes, false};
+    }
+    return cudaSuccess;
 }
 
 cudaError_t plain_malloc(void **p, size_t bytes) {
@@ -161,7 +225,18 @@ cudaError_t plain_malloc(void **p, size_t bytes) {
 }
 
 void pool_free(void *p, cudaStream_t s) {
-    if (p) cudaFreeAsync(p, s);
+    if (!p) return;
+    bool plain;
+    {
+        std::lock_guard<std::mutex> lock(g_pool_mutex);
+        plain = forget_large(p);
+    }
+    if (plain) {
+        RelaxedCapture relaxed;
+        cudaFree(p);  // waits for the device
+    } else {
+        cudaFreeAsync(p, s);
+    }
 }
 
 void pool_free_synced(void *const *ps, int count) {
@@ -182,6 +257,7 @@ void pool_free_synced(void *const *ps, int count) {
         int dev = 0;
         if (device_entry(&d, &dev) == cudaSuccess) {
             d->waiting.insert(d->waiting.end(), ps + i0, ps + count);
+            for (int i = i0; i < count; ++i) forget_large(ps[i]);
             if (waited) {
                 for (void *p : d->waiting) cudaFree(p);
                 d->waiting.clear();

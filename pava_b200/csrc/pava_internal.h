@@ -77,7 +77,8 @@ struct Handle {
 
 // Device memory of handles, conversions and their temporaries: a memory pool per device and
 // context that keeps at most POOL_KEEP bytes of what was freed, so that converting a new matrix
-// does not pay the driver for its buffers each time.  All calls are thread-safe; memory is
+// does not pay the driver for its buffers each time.  Large blocks that it would not keep come from
+// cudaMalloc (k_support.cu); freeing one waits for the device.  All calls are thread-safe; memory is
 // ordered on the stream it is allocated and freed on.
 constexpr size_t POOL_KEEP = (size_t)1 << 30;
 cudaError_t pool_malloc(void **p, size_t bytes, cudaStream_t s);
