@@ -413,7 +413,8 @@ pava_status pava_coo_to_csr_device(int m, int n, long long nnz, const int *rows,
  * device and freed soon: repeated conversions do not pay the driver for them (about 1 ms each at 13.6 M
  * nonzeros).  CUDA IPC handles cannot be made of such arrays, and other devices cannot reach them.
  * pava_free_device_csr_async frees such a result once `stream` has reached the point of the call, without
- * waiting (pava_free_device_csr waits for the device). */
+ * waiting unless an array is too large for the pool to keep (pava_free_device_csr always waits for the
+ * device). */
 pava_status pava_coo_to_csr_device_pooled(int m, int n, long long nnz, const int *rows,
                                    const int *cols, const double *vals, int index_base,
                                    int symmetric, void *stream, pava_csr *out);

@@ -151,8 +151,8 @@ cudaError_t current_pool(cudaMemPool_t *pool) {
 // cudaMalloc; one of 5 GB 50 and 4.8.  Conversion of 200 M nonzeros to CSR5 22.2 -> 4.2 ms,
 // to plain CSR 21.5 -> 2.7; COO -> CSR of 80 M entries 20 -> 7.1; CSR5 of 20 M beside a live matrix of
 // 1.4 GB 2.9 -> 0.22.  The sizes in use are counted here: the pool's own count still holds, for a
-// while, what has been freed.  Below LARGE_MIN cudaMalloc (0.3 ms and more, and cudaFree waits) is no
-// cheaper than mapping.
+// while, what has been freed.  One block, cudaMalloc / the pool's mapping: 4 and 32 MB 0.64 / 0.42 ms, 64 MB
+// 0.65 / 0.80, 256 MB 0.79 / 3.3, 1 GB 1.7 / 12.6.
 constexpr size_t LARGE_MIN = (size_t)64 << 20;
 
 // cudaMalloc and cudaFree beside a capture on another stream, in whichever mode.
